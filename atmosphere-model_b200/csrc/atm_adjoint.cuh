@@ -371,7 +371,7 @@ __device__ __forceinline__ void flush_box(const Sm<double>& a, int w, int h, dou
 }
 
 // ======================================================== mass adjoint ====
-// Adjoint of k_mass2 (C grid: dpc, ptc from dp, pt, ud, vd; D grid: dp, pt
+// Adjoint of the mass sweep (C grid: dpc, ptc from dp, pt, ud, vd; D grid: dp, pt
 // from dp, pt, uc, vc), src/mod_sw_dyn.f90:94-270 and 439-600 (heating off).
 // The update's adjoint needs only the new dp and pt (read from the step's
 // outputs), so the reverse splits by sweep direction into two kernels that
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(NTA, 3) k_mass_adj(const __grid_constant__ CUt
   }
   zero_smem(lam0, p);
 
-  // ---- forward recomputation (as k_mass2)
+  // ---- forward recomputation (the mass sweep)
   if (CGRID) {  // mod_sw_dyn.f90:109-117
     regions(reg<TX + 1, TY + 6>(ox, oy - 3, [&](int x, int y) {
       T ub = T(.5) * (su(x, y) + su(x - 1, y));
@@ -772,7 +772,7 @@ __global__ void __launch_bounds__(NTA, 3) k_mass_adj1(const __grid_constant__ CU
   }
   zero_smem(lam0, p);
 
-  // ---- forward recomputation (as k_mass2)
+  // ---- forward recomputation (the mass sweep)
   if (CGRID) {
     aregion<TX + 1, TY + 6>(ox, oy - 3, [&](int x, int y) {
       T ub = T(.5) * (su(x, y) + su(x - 1, y));
@@ -979,7 +979,7 @@ __global__ void __launch_bounds__(NTA, 3) k_mass_adj1(const __grid_constant__ CU
 }
 
 // =================================================== C-momentum adjoint ====
-// Adjoint of k_c_mom2: uc, vc of layer k from ud, vd of layers k and nlay
+// Adjoint of the C-grid momentum sweep: uc, vc of layer k from ud, vd of layers k and nlay
 // and pkap, gz of levels k, k+1 (src/mod_sw_dyn.f90:294-414).
 template <int TX, int TY>
 struct CMomAdjL {
@@ -1080,7 +1080,7 @@ __global__ void __launch_bounds__(NTA, 3) k_c_mom_adj(const __grid_constant__ CU
   Sm<T> agz1 = carve<T>(p, ox - 1, oy - 1, TX + 1, TY + 1);
   zero_smem(lam0, p);
 
-  // ---- forward recomputation (as k_c_mom2)
+  // ---- forward recomputation (the C-grid momentum sweep)
   aregion<TX + 6, TY + 6>(ox - 3, oy - 3, [&](int x, int y) {
     T ub = T(.5) * (sud(x, y) + sud(x - 1, y));
     uc1(x, y) = T(.5) * (ub + T(.5) * (sud(x, y + 1) + sud(x - 1, y + 1)));
@@ -1280,7 +1280,7 @@ __global__ void __launch_bounds__(NTA, 3) k_c_mom_adj(const __grid_constant__ CU
 }
 
 // =================================================== D-momentum adjoint ====
-// Adjoint of k_d_mom2: ud, vd of layer k from the old ud, vd, uc, vc of
+// Adjoint of the D-grid momentum sweep: ud, vd of layer k from the old ud, vd, uc, vc of
 // layers k and nlay and pkapb, gzb of levels k, k+1 (src/mod_sw_dyn.f90:634-771).
 // The reverse splits into two chains that share only the adjoints of the
 // inputs, which meet in global memory through the flush atomics: the
@@ -1370,7 +1370,7 @@ __global__ void __launch_bounds__(NTA, 4) k_d_mom_adj_ke(const __grid_constant__
   Sm<T> avcL = carve<T>(p, ox - 3, oy, TX + 5, TY + 1);
   zero_smem(lam0, p);
 
-  // ---- forward recomputation (as k_d_mom2): slopes and edges of the KE sweeps
+  // ---- forward recomputation (the D-grid momentum sweep): slopes and edges of the KE sweeps
   regions(reg<TX + 1, TY + 4>(ox, oy - 2, [&](int x, int y) { mvy(x, y) = slope_at(svd.ptr(x, y), Lay::WU); }),
           reg<TX + 4, TY + 1>(ox - 2, oy, [&](int x, int y) { mux(x, y) = slope_at(sud.ptr(x, y), 1); }));
   __syncthreads();
@@ -1527,7 +1527,7 @@ __global__ void __launch_bounds__(NTA, 3) k_d_mom_adj_vf(const __grid_constant__
   Sm<T> agb1 = carve<T>(p, ox, oy, TX + 1, TY + 1);
   zero_smem(lam0, p);
 
-  // ---- forward recomputation (as k_d_mom2): vorticity and its flux sweeps
+  // ---- forward recomputation (the D-grid momentum sweep): vorticity and its flux sweeps
   const T f = c.coriolis;
   aregion<TX + 5, TY + 5>(ox - 3, oy - 3, [&](int x, int y) {
     vor(x, y) = f - (sud(x, y + 1) - sud(x, y)) * rdy + (svd(x + 1, y) - svd(x, y)) * rdx;

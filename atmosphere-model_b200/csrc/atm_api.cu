@@ -305,7 +305,6 @@ int atm_create(atm_ctx** out, int nx, int ny, int nlay, double dx, double dy, co
 
   cudaError_t e;
   if ((e = cudaGetDevice(&ctx->device)) != cudaSuccess) { int r = cuda_fail(ctx, "cudaGetDevice", e); delete ctx; return r; }
-  if ((e = ctx->ops->setup()) != cudaSuccess) { int r = cuda_fail(ctx, "kernel set-up", e); delete ctx; return r; }
   if ((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess) {
     int r = cuda_fail(ctx, "cudaStreamCreate", e); delete ctx; return r;
   }
@@ -544,7 +543,7 @@ int atm_cgrid_step(atm_ctx* ctx, double dt_half) {
   {
     Stage t(ctx, S_CMASS);
     CK(ops.mass(g, k, s[F_DP], s[F_PT], s[F_UD], s[F_VD], heat, ctx->cg[C_DPC], ctx->cg[C_PTC], -2, 2, nullptr,
-                &ctx->status->tma_timeout, true, ctx->stream));
+                true, ctx->stream));
   }
   // plev, pkap, gz (src/mod_sw_dyn.f90:276-292)
   {
@@ -554,8 +553,7 @@ int atm_cgrid_step(atm_ctx* ctx, double dt_half) {
   // uc, vc (src/mod_sw_dyn.f90:294-414)
   {
     Stage t(ctx, S_CMOM);
-    CK(ops.c_mom(g, k, s[F_UD], s[F_VD], ctx->pkap, ctx->gz, ctx->cg[C_UC], ctx->cg[C_VC], &ctx->status->tma_timeout,
-                 ctx->stream));
+    CK(ops.c_mom(g, k, s[F_UD], s[F_VD], ctx->pkap, ctx->gz, ctx->cg[C_UC], ctx->cg[C_VC], ctx->stream));
   }
   return ATM_OK;
 }
@@ -593,7 +591,7 @@ int atm_dgrid_step(atm_ctx* ctx, double dt) {
   {
     Stage t(ctx, S_DMASS);
     CK(ops.mass(g, k, so[F_DP], so[F_PT], ctx->cg[C_UC], ctx->cg[C_VC], heat, sn[F_DP], sn[F_PT], -3, 3,
-                &ctx->status->nonfinite_step, &ctx->status->tma_timeout, false, ctx->stream));
+                &ctx->status->nonfinite_step, false, ctx->stream));
   }
   // plev, pkap, gz, pkapb, gzb (src/mod_sw_dyn.f90:606-632)
   {
@@ -608,7 +606,7 @@ int atm_dgrid_step(atm_ctx* ctx, double dt) {
   {
     Stage t(ctx, S_DMOM);
     CK(ops.d_mom(g, k, so[F_UD], so[F_VD], ctx->cg[C_UC], ctx->cg[C_VC], ctx->pkapb, ctx->gzb, sn[F_UD], sn[F_VD],
-                 &ctx->status->nonfinite_step, &ctx->status->tma_timeout, ctx->stream));
+                 &ctx->status->nonfinite_step, ctx->stream));
   }
   ctx->cur = nxt;
   ctx->flag_valid = true;
@@ -849,10 +847,9 @@ int fwd_c(atm_ctx* ctx, double dt_half, void* const* s) {
   const Geom& g = ctx->geo;
   atm::Consts k = step_consts(ctx, dt_half);
   CK(ops.mass(g, k, s[F_DP], s[F_PT], s[F_UD], s[F_VD], nullptr, ctx->cg[C_DPC], ctx->cg[C_PTC], -2, 2, nullptr,
-              &ctx->status->tma_timeout, true, ctx->stream));
+              true, ctx->stream));
   CK(ops.column(g, k, ctx->cg[C_DPC], ctx->cg[C_PTC], ops.cg_elem, ctx->pkap, ctx->gz, -2, 2, nullptr, ctx->stream));
-  CK(ops.c_mom(g, k, s[F_UD], s[F_VD], ctx->pkap, ctx->gz, ctx->cg[C_UC], ctx->cg[C_VC], &ctx->status->tma_timeout,
-               ctx->stream));
+  CK(ops.c_mom(g, k, s[F_UD], s[F_VD], ctx->pkap, ctx->gz, ctx->cg[C_UC], ctx->cg[C_VC], ctx->stream));
   ctx->launches += 3;
   return ATM_OK;
 }
@@ -864,11 +861,11 @@ int fwd_d(atm_ctx* ctx, double dt, void* const* so, void* const* sn) {
   atm::Consts k = step_consts(ctx, dt);
   CK(ops.ring(g, sn, (const void* const*)so, 4, ctx->L, true, ctx->stream));
   CK(ops.mass(g, k, so[F_DP], so[F_PT], ctx->cg[C_UC], ctx->cg[C_VC], nullptr, sn[F_DP], sn[F_PT], -3, 3,
-              &ctx->status->nonfinite_step, &ctx->status->tma_timeout, false, ctx->stream));
+              &ctx->status->nonfinite_step, false, ctx->stream));
   CK(ops.column(g, k, sn[F_DP], sn[F_PT], ops.elem, ctx->pkap, ctx->gz, -2, 2, nullptr, ctx->stream));
   CK(atm::corners(g, ctx->pkap, ctx->gz, ctx->pkapb, ctx->gzb, 1, 0, ctx->L, ctx->stream));
   CK(ops.d_mom(g, k, so[F_UD], so[F_VD], ctx->cg[C_UC], ctx->cg[C_VC], ctx->pkapb, ctx->gzb, sn[F_UD], sn[F_VD],
-               &ctx->status->nonfinite_step, &ctx->status->tma_timeout, ctx->stream));
+               &ctx->status->nonfinite_step, ctx->stream));
   ctx->launches += 5;
   return ATM_OK;
 }

@@ -112,67 +112,6 @@ __device__ __forceinline__ void slopes(T qm, T q0, T qp, T& dqi, T& mono) {
   mono = cpsign(mn3(fab(dqi), dmin, dmax), dqi);
 }
 
-// Edge anomalies edge_L(i), edge_R(i) of cell i, src/mod_sw_dyn.f90:877-911.
-// q points at cell i; s is the distance between neighbouring cells.
-template <typename T, int V>
-__device__ __forceinline__ void edges(const T* q, int s, T& eL, T& eR) {
-  T qm2 = q[-2 * s], qm1 = q[-s], q0 = q[0], qp1 = q[s], qp2 = q[2 * s];
-  T d_m, mono_m, d_0, mono_0, d_p, mono_p;
-  slopes(qm2, qm1, q0, d_m, mono_m);
-  slopes(qm1, q0, qp1, d_0, mono_0);
-  slopes(q0, qp1, qp2, d_p, mono_p);
-  eL = (qm1 - q0) * T(0.5) + div_const<3>(mono_m - mono_0);
-  eR = (qp1 - q0) * T(0.5) + div_const<3>(mono_0 - mono_p);
-  if (V == PPM_CON || V == PPM_NN) {
-    T lim = T(2) * fab(d_0);
-    eL = -cpsign(mn(lim, fab(eL)), d_0);
-    eR = +cpsign(mn(lim, fab(eR)), d_0);
-    if (V == PPM_NN) {
-      eL = mx(eL, -q0);
-      eR = mx(eR, -q0);
-      T a = eR - eL;
-      T b = T(-3) * (eR + eL);
-      if ((fab(a) < -b) && (q0 + a * a / (T(4) * b) + div_const<12>(b) < T(0))) {
-        if (eL * eR > T(0)) {
-          eL = T(0);
-          eR = T(0);
-        } else if (eL > eR) {
-          eL = T(2) * fab(eR);
-        } else {
-          eR = T(2) * fab(eL);
-        }
-      }
-    }
-  }
-}
-
-// Upwind flux at the interface between cells i-1 and i (src/mod_sw_dyn.f90:
-// 802-838).  q points at cell i, s is the cell spacing in the array, c is the
-// Courant number of the interface.  Reads q[-3s .. 2s].
-template <typename T, int V>
-__device__ __forceinline__ T flux(const T* q, int s, T c) {
-  if (V == PC) return (c > T(0)) ? q[-s] : q[0];
-  T sa = fab(c);
-  T k1 = (T(1) - T(2) * sa) * (T(1) - sa);
-  T k2 = sa * (sa - T(1));
-  if (V == PPM_CON) {
-    T eLm, eRm, eL0, eR0;
-    edges<T, V>(q - s, s, eLm, eRm);
-    edges<T, V>(q, s, eL0, eR0);
-    if ((T(3) * fab(eL0 + eR0) > fab(eL0 - eR0)) && (T(3) * fab(eLm + eRm) > fab(eLm - eRm)))
-      return (c > T(0)) ? q[-s] : q[0];
-    if (c > T(0)) return q[-s] + k1 * eRm + k2 * eLm;
-    return q[0] + k1 * eL0 + k2 * eR0;
-  }
-  T eL, eR;
-  if (c > T(0)) {
-    edges<T, V>(q - s, s, eL, eR);
-    return q[-s] + k1 * eR + k2 * eL;
-  }
-  edges<T, V>(q, s, eL, eR);
-  return q[0] + k1 * eL + k2 * eR;
-}
-
 // A window of a 2-D shared-memory array addressed with absolute interior
 // coordinates (x, y) of the tile's region [x0, x0+w) x [y0, y0+h).
 template <typename T>

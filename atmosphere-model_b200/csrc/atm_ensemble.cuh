@@ -160,10 +160,10 @@ __device__ __forceinline__ int ens_member(const long long* off, int nm, long lon
 }
 
 // one strip item of a marching sweep at the member's strip height
-template <int TYS, typename F>
-__device__ __forceinline__ void ens_strip_item(const Geom& g, int lo, int hi, long long li, F&& body) {
+template <typename F>
+__device__ __forceinline__ void ens_strip_item(const Geom& g, int lo, int hi, int tys, long long li, F&& body) {
   int sxn, syn;
-  ens_strips(g, lo, hi, TYS, sxn, syn);
+  ens_strips(g, lo, hi, tys, sxn, syn);
   const int sx = (int)(li % sxn);
   const int sy = (int)((li / sxn) % syn);
   const int k = (int)(li / ((long long)sxn * syn));
@@ -172,47 +172,47 @@ __device__ __forceinline__ void ens_strip_item(const Geom& g, int lo, int hi, lo
 
 // The stage bodies are not inlined: each keeps the register allocation of
 // its single-domain kernel instead of the union of all of them.
-template <typename T, typename S, typename C, int TYS>
+template <typename T, typename S, typename C>
 __device__ __noinline__ void ens_cmass(const EnsMember& M, int cur, long long li) {
-  ens_strip_item<TYS>(M.g, -2, 2, li, [&](int sx, int sy, int k) {
+  ens_strip_item(M.g, -2, 2, M.tys, li, [&](int sx, int sy, int k) {
     void* const* so = M.st[cur];
-    mass_strip<T, TYS, true, S, C, false>(M.g, M.cc, (const S*)so[0], (const S*)so[1], (const S*)so[2], (const S*)so[3],
-                                   nullptr, (C*)M.cg[0], (C*)M.cg[1], -2, 2, nullptr, sx, sy, k);
+    mass_strip<T, true, S, C, false>(M.g, M.cc, (const S*)so[0], (const S*)so[1], (const S*)so[2], (const S*)so[3],
+                                   nullptr, (C*)M.cg[0], (C*)M.cg[1], -2, 2, nullptr, sx, sy, k, M.tys);
   });
 }
-template <typename T, typename S, typename C, int TYS>
+template <typename T, typename S, typename C>
 __device__ __noinline__ void ens_cmom(const EnsMember& M, int cur, long long li) {
-  ens_strip_item<TYS>(M.g, 0, 0, li, [&](int sx, int sy, int k) {
+  ens_strip_item(M.g, 0, 0, M.tys, li, [&](int sx, int sy, int k) {
     void* const* so = M.st[cur];
-    c_mom_strip<T, TYS, S, C, false>(M.g, M.cc, (const S*)so[2], (const S*)so[3], M.pkap, M.gz, (C*)M.cg[2], (C*)M.cg[3],
-                              sx, sy, k);
+    c_mom_strip<T, S, C, false>(M.g, M.cc, (const S*)so[2], (const S*)so[3], M.pkap, M.gz, (C*)M.cg[2], (C*)M.cg[3],
+                              sx, sy, k, M.tys);
   });
 }
-template <typename T, typename S, typename C, int TYS>
+template <typename T, typename S, typename C>
 __device__ __noinline__ void ens_dmass(const EnsMember& M, int cur, long long li) {
-  ens_strip_item<TYS>(M.g, -3, 3, li, [&](int sx, int sy, int k) {
+  ens_strip_item(M.g, -3, 3, M.tys, li, [&](int sx, int sy, int k) {
     void* const* so = M.st[cur];
     void* const* sn = M.st[cur ^ 1];
-    mass_strip<T, TYS, false, S, C, false>(M.g, M.cd, (const S*)so[0], (const S*)so[1], (const C*)M.cg[2], (const C*)M.cg[3],
-                                    nullptr, (S*)sn[0], (S*)sn[1], -3, 3, &M.status->nonfinite_step, sx, sy, k);
+    mass_strip<T, false, S, C, false>(M.g, M.cd, (const S*)so[0], (const S*)so[1], (const C*)M.cg[2], (const C*)M.cg[3],
+                                    nullptr, (S*)sn[0], (S*)sn[1], -3, 3, &M.status->nonfinite_step, sx, sy, k, M.tys);
   });
 }
-template <typename T, typename S, typename C, int TYS>
+template <typename T, typename S, typename C>
 __device__ __noinline__ void ens_dmom(const EnsMember& M, int cur, long long li) {
-  ens_strip_item<TYS>(M.g, 0, 0, li, [&](int sx, int sy, int k) {
+  ens_strip_item(M.g, 0, 0, M.tys, li, [&](int sx, int sy, int k) {
     void* const* so = M.st[cur];
     void* const* sn = M.st[cur ^ 1];
-    d_mom_strip<T, TYS, S, C, false>(M.g, M.cd, (const S*)so[2], (const S*)so[3], (const C*)M.cg[2], (const C*)M.cg[3],
-                              M.pkapb, M.gzb, (S*)sn[2], (S*)sn[3], &M.status->nonfinite_step, sx, sy, k);
+    d_mom_strip<T, S, C, false>(M.g, M.cd, (const S*)so[2], (const S*)so[3], (const C*)M.cg[2], (const C*)M.cg[3],
+                              M.pkapb, M.gzb, (S*)sn[2], (S*)sn[3], &M.status->nonfinite_step, sx, sy, k, M.tys);
   });
 }
 
-template <typename T, typename S, typename C, int TYS>
+template <typename T, typename S, typename C>
 __device__ __forceinline__ void ens_sweep(int stage, const EnsMember& M, int cur, long long li) {
-  if (stage == E_CMASS) ens_cmass<T, S, C, TYS>(M, cur, li);
-  else if (stage == E_CMOM) ens_cmom<T, S, C, TYS>(M, cur, li);
-  else if (stage == E_DMASS) ens_dmass<T, S, C, TYS>(M, cur, li);
-  else ens_dmom<T, S, C, TYS>(M, cur, li);
+  if (stage == E_CMASS) ens_cmass<T, S, C>(M, cur, li);
+  else if (stage == E_CMOM) ens_cmom<T, S, C>(M, cur, li);
+  else if (stage == E_DMASS) ens_dmass<T, S, C>(M, cur, li);
+  else ens_dmom<T, S, C>(M, cur, li);
 }
 
 template <typename S, int LM>
@@ -248,9 +248,7 @@ __device__ __forceinline__ void ens_item(int stage, const EnsMember& M, int cur,
     case E_CMOM:
     case E_DMASS:
     case E_DMOM:
-      if (M.tys == 16) ens_sweep<T, S, C, 16>(stage, M, cur, li);
-      else if (M.tys == 32) ens_sweep<T, S, C, 32>(stage, M, cur, li);
-      else ens_sweep<T, S, C, 64>(stage, M, cur, li);
+      ens_sweep<T, S, C>(stage, M, cur, li);
       break;
     case E_CCOL:
       column_at<C, FormPow<T>>(g, M.cc, (const C*)M.cg[0], (const C*)M.cg[1], M.pkap, M.gz, -2, 2, nullptr,

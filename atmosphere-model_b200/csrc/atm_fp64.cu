@@ -4,6 +4,7 @@
 #define ATM_FORM_T double
 #define ATM_OPS_NAME ops_fp64
 #include "atm_launch.cuh"
+#include "atm_tma.cuh"
 
 #ifndef ATM_CORNER_CHUNK
 #define ATM_CORNER_CHUNK 8
@@ -42,11 +43,16 @@ static __global__ void k_div_check(unsigned long long n, unsigned long long seed
     unsigned long long b = mix64(seed * 0x100000001b3ULL + i);
     double x = __longlong_as_double((long long)b);
     if (i % 7 == 0) x = (double)(long long)(b % 2000001) - 1000000.0;
+    if (i % 11 == 0) x = __longlong_as_double((long long)(b & 0x800fffffffffffffULL));  // zeros and subnormals
+    if (i % 11 == 1) x = __longlong_as_double((long long)(b & 0x8000000000000003ULL));
+    if (i % 1000003 == 0) x = copysign(__longlong_as_double(0x7ff0000000000000LL), x);
     bool ok = true;
     double q3 = div_const<3>(x), t3 = x / 3.0;
     double q12 = div_const<12>(x), t12 = x / 12.0;
     ok = ok && (__double_as_longlong(q3) == __double_as_longlong(t3) || (q3 != q3 && t3 != t3));
     ok = ok && (__double_as_longlong(q12) == __double_as_longlong(t12) || (q12 != q12 && t12 != t12));
+    const double q = third(x);
+    ok = ok && (__double_as_longlong(q) == __double_as_longlong(t3) || (q != q && t3 != t3));
     if (!ok) ++local;
   }
   if (local) atomicAdd(bad, local);

@@ -2,10 +2,9 @@
 // (double for the FP64 form, float for the mixed form).  Column sums,
 // pkap, gz and the vertical remap always run in double.
 //
-// Every per-layer kernel processes one TX x TY tile of one layer: it stages
-// the tile plus the stencil halo of its inputs in shared memory, runs the
-// stages of the reference's layer loop on that tile, and writes its outputs.
-// Index ranges, staggering shifts and evaluation order follow the
+// Columns, corners, halos, the vertical remap and the reductions; the
+// horizontal sweeps are in atm_march.cuh.  Index ranges, staggering shifts
+// and evaluation order follow the
 // reference line by line (cited per stage).
 #pragma once
 
@@ -16,24 +15,7 @@
 
 namespace atm {
 
-constexpr int NT = 256;  // threads per block of the per-layer kernels
-
-// ---------------------------------------------------------------- loads ----
-// s[(y - y0) * w + (x - x0)] = field(x, y, k) for the box [x0, x0+w) x
-// [y0, y0+h); points outside the stored (halo-padded) array read as zero and
-// only ever feed outputs outside the kernel's output region.
-template <typename T>
-__device__ __forceinline__ void load_box(T* s, const T* __restrict__ f, const Geom& g, int k, int x0, int y0, int w,
-                                         int h) {
-  const T* base = f + (long long)k * g.S;
-  for (int idx = threadIdx.x; idx < w * h; idx += blockDim.x) {
-    int y = idx / w, x = idx - y * w;
-    int gx = x0 + x, gy = y0 + y;
-    T v = T(0);
-    if (gx >= -H && gx < g.nx + H && gy >= -H && gy < g.ny + H) v = base[g.at(gx, gy)];
-    s[idx] = v;
-  }
-}
+constexpr int NT = 256;  // threads per block of the tile kernels
 
 template <typename T>
 __device__ __forceinline__ Sm<T> carve(unsigned char*& p, int x0, int y0, int w, int h) {

@@ -1,25 +1,31 @@
-// Column-marching sweep kernels of the B200 dynamical core.
+// Column-marching sweep kernels of the B200 dynamical core, both forms.
 //
 // A warp owns a strip of one layer: 32 consecutive x columns (lane = column)
 // of which the middle 26 are outputs (3 halo columns on each side feed the
-// PPM stencils), and TYS output rows that it walks through in ascending y.
-// Each lane keeps the y-direction stencil values of its column (the last
-// few rows of every stage) in registers, so that every stage of the
+// PPM stencils), and a number of output rows that it walks through in
+// ascending y.  Each lane keeps the y-direction stencil values of its column
+// (the last few rows of every stage) in registers, so that every stage of the
 // reference's layer loop is evaluated once per cell instead of once per
 // cell of every overlapping tile halo; x-direction neighbours come from the
 // neighbouring lanes by warp shuffles.  No shared memory and no block-wide
-// barrier: the warps of a block are independent.
+// barrier: the warps of a block are independent.  Each iteration loads the
+// inputs of the next row before working on the current one, so that the
+// loads' latency overlaps a row of arithmetic.
 //
-// Each iteration loads the inputs of the next row before working on the
-// current one, so that the loads' latency overlaps a row of arithmetic.
+// The sweeps are bound by instruction issue (HBM traffic is the fields read
+// and written once, 0.5 ms of a kernel at 1024x1024x64), so the formulas are
+// arranged for the fewest instructions that give the reference's bits: a
+// difference of two neighbours is formed once and serves the slopes of both
+// cells and the two edges between them (YLine, xline_flux), each cell's edges
+// are formed and limited once, exact products are fused, and the division by
+// three needs no branch.  Measured on B200 at 1024x1024x64 (ms a launch, C
+// mass / C momentum / D mass / D momentum; before: FP64 sweeps on 32 x 4-8
+// shared-memory tiles, FP32 marching with per-flux edges):
+//   FP64  4.24 / 4.03 / 4.58 / 4.92  ->  1.93 / 2.61 / 2.38 / 2.69
+//   FP32  1.63 / 2.02 / 1.70 / 2.29  ->  1.23 / 1.65 / 1.27 / 1.60
 //
-// The stage formulas, index shifts and evaluation order are those of the
-// tile kernels (atm_sweeps.cuh) and of the reference, so FP64 instances
-// are bit-identical to them (the oracle's parity tests passed with the
-// FP64 form built on these kernels).  The mixed form launches its four
-// sweeps as marching kernels; in FP64 the tiles are faster (the marching
-// FP64 sweeps execute about as many instructions per cell, at 140-174
-// registers a thread and 17 % warps active), so the FP64 form keeps them.
+// Every value is the reference's expression (src/mod_sw_dyn.f90) up to the
+// sign of a zero; FP64 instances are bit-identical to the FP64 restatement.
 // The persistent ensemble kernel runs the same strip functions with plain
 // loads (RO = false), as it reads fields that it wrote earlier in the same
 // launch.
@@ -35,17 +41,25 @@ constexpr int MW = 32;              // lanes (columns) of a strip
 constexpr int MXH = 3;              // halo columns on each side
 constexpr int MOUT = MW - 2 * MXH;  // output columns of a strip
 constexpr int MWARPS = 4;           // independent strips (warps) per block
-// blocks per SM the register budget of the marching kernels is set for: 4
-// (16 warps), which the FP32 sweeps reach without spilling (at most 128
-// registers; the C-momentum sweep would take 131 and fall to 3 blocks)
-#ifndef ATM_MARCH_MINB
-#define ATM_MARCH_MINB 4
-#endif
 
-template <typename T>
-__device__ __forceinline__ T shfl_at(T v, int src) {
-  return __shfl_sync(0xffffffffu, v, src);
-}
+// Register budget (blocks of four warps per SM) and rows per loop body of each
+// marching kernel.  The row windows shift by one register a row; unrolling by
+// n rows does n shifts at once (a window of w doubles costs 2w/n moves a row).
+// Measured on B200 at 1024x1024x64 (ms, C mass / C momentum / D mass / D
+// momentum):
+//   FP64, 3 blocks (168 registers), 1 / 2 / 3 / 4 rows: 2.33 2.68 2.75 2.74 /
+//     2.25 2.63 2.54 3.14 / 1.93 2.61 2.38 2.69 / 2.06 2.58 2.50 2.89;
+//     4 blocks, 1 row (spills): 2.40 3.01 2.58 2.88; 2 blocks: 2.35 3.34 2.80 3.50
+//   FP32, 4 blocks (128 registers), 1 / 2 / 3 / 4 rows: 1.23 1.73 1.58 1.73 /
+//     1.37 1.89 1.35 1.60 / 1.29 1.65 1.27 1.87 / 1.35 1.68 1.27 1.77
+enum { MK_CMASS, MK_DMASS, MK_CMOM, MK_DMOM };
+template <typename T, int K>
+struct MarchL {
+  static constexpr bool F32 = std::is_same_v<T, float>;
+  static constexpr int min_blocks = F32 ? 4 : 3;
+  static constexpr int unroll = !F32 ? 3 : K == MK_CMASS ? 1 : K == MK_DMOM ? 2 : 3;
+};
+
 template <typename T>
 __device__ __forceinline__ T shfl_dn(T v, int d) {
   return __shfl_down_sync(0xffffffffu, v, d);
@@ -63,387 +77,496 @@ __device__ __forceinline__ T shfl_up(T v, int d) {
 __device__ __forceinline__ float fmadd(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fmadd(double a, double b, double c) { return a * b + c; }
 
-// Edge anomalies of a cell from its value and neighbours (qm, q0, qp) and
-// their monotone slopes (mm, m0, mp): the operations of edges_pre.
-template <typename T, int V>
-__device__ __forceinline__ void edges_v(T qm, T q0, T qp, T mm, T m0, T mp, T& eL, T& eR) {
-  eL = fmadd(qm - q0, T(0.5), div_const<3>(mm - m0));
-  eR = fmadd(qp - q0, T(0.5), div_const<3>(m0 - mp));
-  if (V == PPM_CON || V == PPM_NN) {
-    const T d0 = (qp - qm) * T(0.25);
-    const T lim = T(2) * fab(d0);
-    eL = -cpsign(mn(lim, fab(eL)), d0);
-    eR = +cpsign(mn(lim, fab(eR)), d0);
-    if (V == PPM_NN) {
-      eL = mx(eL, -q0);
-      eR = mx(eR, -q0);
-      T a = eR - eL;
-      T b = T(-3) * (eR + eL);
-      if ((fab(a) < -b) && (q0 + a * a / (T(4) * b) + div_const<12>(b) < T(0))) {
-        if (eL * eR > T(0)) {
-          eL = T(0);
-          eR = T(0);
-        } else if (eL > eR) {
-          eL = T(2) * fab(eR);
-        } else {
-          eR = T(2) * fab(eL);
-        }
-      }
+// a * b + c where a * b is exact (a a power of two): one fused operation in
+// either type, with the value of the two separate ones.
+__device__ __forceinline__ float fmx(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fmx(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// v with its sign flipped where s is negative
+__device__ __forceinline__ double xsign(double v, double s) {
+  return __hiloint2double(__double2hiint(v) ^ (__double2hiint(s) & 0x80000000), __double2loint(v));
+}
+__device__ __forceinline__ float xsign(float v, float s) {
+  return __int_as_float(__float_as_int(v) ^ (__float_as_int(s) & 0x80000000));
+}
+// min and max that return NaN where an argument is NaN (one instruction in
+// FP32; in FP64 the compare-and-select of mn and mx, which keeps a NaN first
+// argument)
+__device__ __forceinline__ float mn_nan(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float mx_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ double mn_nan(double a, double b) { return mn(a, b); }
+__device__ __forceinline__ double mx_nan(double a, double b) { return mx(a, b); }
+
+// Monotone slope of a cell (slopes() of atm_common.cuh) from the differences
+// dm = q(0) - q(-1), dp = q(+1) - q(0) and dqi = (q(+1) - q(-1)) / 4.
+// slopes() bounds |dqi| by dmax = max(q(+1), q(0), q(-1)) - q(0) and dmin =
+// q(0) - min(...): where dm and dp agree in sign these two are |dm| and |dp|
+// (the same rounded differences), elsewhere one of them is zero.  So the
+// magnitude is the least of |dqi| and of dm, dp counted positive along dqi,
+// and not below zero: the same value from half the compares and selects, and
+// each difference serves two cells and the edges between them.
+template <typename T>
+__device__ __forceinline__ T slope_d(T dm, T dp, T dqi) {
+  const T m = mn_nan(mn_nan(fab(dqi), xsign(dm, dqi)), xsign(dp, dqi));
+  return cpsign(mx_nan(m, T(0)), dqi);
+}
+
+// x / 3 in FP64, equal to the IEEE quotient for every x, without a branch:
+// the corrected quotient of div_const, whose remainder e is exact (a multiple
+// of the smallest subnormal, and x / 3 is never near half an ulp from two
+// doubles, so the correction rounds rightly among subnormals too); a zero
+// remainder (zeros among them) and a NaN one (infinities) keep q.
+__device__ __forceinline__ double third(double x) {
+  constexpr double r = 1.0 / 3;
+  const double q = x * r;
+  const double e = __fma_rn(-q, 3.0, x);
+  return fabs(e) > 0. ? __fma_rn(e, r, q) : q;
+}
+__device__ __forceinline__ float third(float x) { return div_const<3>(x); }
+
+// The constrained limiter of a cell's raw edge anomalies (edges_pre) with
+// its raw slope dqi.
+__device__ __forceinline__ double lim_min(double lim, double e) { return mn(lim, fabs(e)); }
+__device__ __forceinline__ float lim_min(float lim, float e) { return fminf(lim, fabsf(e)); }
+template <typename T>
+__device__ __forceinline__ void limit_con(T dqi, T& eL, T& eR) {
+  const T lim = T(2) * fab(dqi);
+  eL = -cpsign(lim_min(lim, eL), dqi);
+  eR = cpsign(lim_min(lim, eR), dqi);
+}
+// The same with the positivity filter of PPM_NONNEGATIVE.  Both edges are at
+// most 2 |dqi| in magnitude, so where q0 > 6 |dqi| neither floor at -q0 holds
+// and the parabola's minimum, above q0 - 2 |dqi|, is positive: nothing
+// changes and the filter (and its division) is skipped.
+template <typename T>
+__device__ __forceinline__ void limit_nn(T q0, T dqi, T& eL, T& eR) {
+  limit_con(dqi, eL, eR);
+  if (q0 > T(6) * fab(dqi)) return;
+  eL = mx(eL, -q0);
+  eR = mx(eR, -q0);
+  const T a = eR - eL;
+  const T b = T(-3) * (eR + eL);
+  if ((fab(a) < -b) && (q0 + a * a / (T(4) * b) + div_const<12>(b) < T(0))) {
+    if (eL * eR > T(0)) {
+      eL = T(0);
+      eR = T(0);
+    } else if (eL > eR) {
+      eL = T(2) * fab(eR);
+    } else {
+      eR = T(2) * fab(eL);
     }
   }
 }
 
-// Upwind flux with Courant number c from the values and monotone slopes
-// around the upwind cell (cell i-1 for c > 0, cell i otherwise): the
-// operations of flux_pre.
-template <typename T, int V>
-__device__ __forceinline__ T flux_v(T c, T qm, T q0, T qp, T mm, T m0, T mp) {
-  const T sa = fab(c);
-  const T k1 = fmadd(T(-2), sa, T(1)) * (T(1) - sa);
-  const T k2 = sa * (sa - T(1));
-  T eL, eR;
-  edges_v<T, V>(qm, q0, qp, mm, m0, mp, eL, eR);
-  return (c > T(0)) ? fmadd(k2, eL, fmadd(k1, eR, q0)) : fmadd(k2, eR, fmadd(k1, eL, q0));
-}
-
-// Flux with the edge values of the upwind candidates given (PPM_CONSTRAINED):
-// the operations of flux_con_pre.  qm, q0 are the values of cells i-1 and
-// i, (eLm, eRm) and (eL0, eR0) their edges.
+// Upwind flux with Courant number c at the interface between cells m and 0
+// from their values and edges: the operations of flux_pre.
 template <typename T>
-__device__ __forceinline__ T flux_con_v(T c, T qm, T q0, T eLm, T eRm, T eL0, T eR0) {
-  if ((T(3) * fab(eL0 + eR0) > fab(eL0 - eR0)) && (T(3) * fab(eLm + eRm) > fab(eLm - eRm)))
-    return (c > T(0)) ? qm : q0;
+__device__ __forceinline__ T flux_e(T c, T qm, T eLm, T eRm, T q0, T eL0, T eR0) {
+  const bool pos = c > T(0);
   const T sa = fab(c);
-  const T k1 = fmadd(T(-2), sa, T(1)) * (T(1) - sa);
+  const T k1 = fmx(T(-2), sa, T(1)) * (T(1) - sa);
   const T k2 = sa * (sa - T(1));
-  return (c > T(0)) ? fmadd(k2, eLm, fmadd(k1, eRm, qm)) : fmadd(k2, eR0, fmadd(k1, eL0, q0));
+  return fmadd(k2, pos ? eLm : eR0, fmadd(k1, pos ? eRm : eL0, pos ? qm : q0));
+}
+// PPM_CONSTRAINED: the upwind value itself where both cells' edges are
+// one-sided (flat_e of each), flux_con_pre
+template <typename T>
+__device__ __forceinline__ bool flat_e(T eL, T eR) {
+  return T(3) * fab(eL + eR) > fab(eL - eR);
+}
+template <typename T>
+__device__ __forceinline__ T flux_con_e(T c, T qm, T eLm, T eRm, T q0, T eL0, T eR0, bool flat) {
+  const T f = flux_e(c, qm, eLm, eRm, q0, eL0, eR0);
+  return flat ? ((c > T(0)) ? qm : q0) : f;
 }
 
-__device__ __forceinline__ double slope_v(double qm, double q0, double qp) {
-  double d, m;
-  slopes(qm, q0, qp, d, m);
-  return m;
-}
-__device__ __forceinline__ float slope_v(float qm, float q0, float qp) {
-  float d, m;
-  slopes(qm, q0, qp, d, m);
-  return m;
+// t = .5 (q + den (q - rA (f1 - f0))), the piecewise-constant inner sweep
+template <typename T>
+__device__ __forceinline__ T inner_e(T q, T f0, T f1, T den, T rA) {
+  return T(.5) * fmadd(den, fmadd(-rA, f1 - f0, q), q);
 }
 
-// Row accessor of one level of a stored field: value at (x, y) of the
-// level, zero outside the stored (halo-padded) array.  RO: no thread writes
-// the field during the launch, so it is read through the read-only data
-// path; the persistent ensemble kernel, whose later stages read what earlier
-// stages of the same launch wrote, uses plain (coherent) loads.
-template <typename E, bool RO = true>
-struct Lev {
-  const E* p;  // element (0, 0) of the level
-  int P, nx, ny;
-  __device__ __forceinline__ E operator()(int x, int y) const {
-    if (x < -H || x >= nx + H || y < -H || y >= ny + H) return E(0);
-    const E* a = p + (long long)y * P + x;
-    if constexpr (RO) return __ldg(a);
-    else return *a;
+// A line of one quantity along y, fed a value a row: the windows of its last
+// rows and the edges of its cells, formed once a cell.  After push() of row r:
+// q0 .. q3 are rows r .. r-3, (L2, R2) and (L3, R3) the final edges of cells
+// r-2 and r-3, so that flux() is the flux at the interface between them.
+template <typename T, int V>
+struct YLine {
+  T q0 = 0, q1 = 0, q2 = 0, q3 = 0;
+  T dif = 0, mono = 0, dqi = 0, rawL = 0;  // q0 - q1; slope, dqi and raw lower edge of cell r-1
+  T L2 = 0, R2 = 0, L3 = 0, R3 = 0;
+  bool flat2 = false, flat3 = false;
+  __device__ __forceinline__ void push(T v) {
+    const T dn = v - q0;
+    const T dq = (v - q1) * T(0.25);
+    const T m = slope_d(dif, dn, dq);       // cell r-1
+    const T h = third(mono - m);            // between cells r-2 and r-1
+    L3 = L2;
+    R3 = R2;
+    L2 = rawL;
+    R2 = fmx(T(.5), dif, h);
+    rawL = fmx(T(-.5), dif, h);
+    if (V == PPM_CON) {
+      limit_con(dqi, L2, R2);
+      flat3 = flat2;
+      flat2 = flat_e(L2, R2);
+    }
+    if (V == PPM_NN) limit_nn(q1, dqi, L2, R2);
+    q3 = q2; q2 = q1; q1 = q0; q0 = v;
+    dif = dn;
+    mono = m;
+    dqi = dq;
+  }
+  __device__ __forceinline__ T flux(T c) const {
+    if (V == PPM_CON) return flux_con_e(c, q3, L3, R3, q2, L2, R2, flat2 && flat3);
+    return flux_e(c, q3, L3, R3, q2, L2, R2);
   }
 };
-template <bool RO = true, typename E>
-__device__ __forceinline__ Lev<E, RO> level(const E* f, const Geom& g, int k) {
-  return Lev<E, RO>{f + g.at(0, 0, k), g.P, g.nx, g.ny};
+
+// A line along x, one cell a lane: the flux at the interface between the
+// lane's cell and the cell of the lane below.
+template <typename T, int V>
+__device__ __forceinline__ T xline_flux(T q, T c) {
+  const T qL = shfl_up(q, 1), qR = shfl_dn(q, 1);
+  const T dm = q - qL;
+  const T dqi = (qR - qL) * T(0.25);
+  const T m = slope_d(dm, qR - q, dqi);
+  const T h = third(shfl_up(m, 1) - m);
+  const T rI = fmx(T(.5), dm, h);  // raw upper edge of the cell below
+  T eL = fmx(T(-.5), dm, h);       // raw lower edge of the cell
+  T eR = shfl_dn(rI, 1);
+  if (V == PPM_UNC) return flux_e(c, qL, shfl_up(eL, 1), rI, q, eL, eR);
+  if (V == PPM_NN) {
+    limit_nn(q, dqi, eL, eR);
+    return flux_e(c, qL, shfl_up(eL, 1), shfl_up(eR, 1), q, eL, eR);
+  }
+  limit_con(dqi, eL, eR);
+  const unsigned fl = __ballot_sync(0xffffffffu, flat_e(eL, eR));
+  const int lane = threadIdx.x & (MW - 1);
+  const bool flat = lane > 0 && ((fl >> (lane - 1)) & 3u) == 3u;
+  return flux_con_e(c, qL, shfl_up(eL, 1), shfl_up(eR, 1), q, eL, eR, flat);
+}
+
+// The unconstrained flux at the interface above the lane's cell, with the
+// lane's Courant number.
+template <typename T>
+__device__ __forceinline__ T xline_flux_above(T q, T c) {
+  const T qL = shfl_up(q, 1), qR = shfl_dn(q, 1);
+  const T dp = qR - q;
+  const T m = slope_d(q - qL, dp, (qR - qL) * T(0.25));
+  const T h = third(m - shfl_dn(m, 1));
+  const T rI = fmx(T(.5), dp, h);   // upper edge of the cell
+  const T lI = fmx(T(-.5), dp, h);  // lower edge of the cell above
+  return flux_e(c, q, shfl_up(lI, 1), rI, qR, lI, shfl_dn(rI, 1));
+}
+
+// Column accessor of one level of a stored field: the value at (x, y) with x
+// the lane's column, both brought into the stored (halo-padded) array, so
+// that rows and lanes past it read some stored value (they only feed outputs
+// outside the kernel's range).  RO: no thread writes the field during the
+// launch, so it is read through the read-only data path; the persistent
+// ensemble kernel, whose later stages read what earlier stages of the same
+// launch wrote, uses plain (coherent) loads.  A level holds fewer than 2^32
+// elements (three levels of 17 fields of that size exceed the device memory).
+__device__ __forceinline__ unsigned col_of(const Geom& g, int x) {
+  return (unsigned)(min(max(x, -H), g.nx + H - 1) + H + XOFF);
+}
+__device__ __forceinline__ unsigned row_of(const Geom& g, int y) {
+  return (unsigned)(min(max(y, -H), g.ny + H - 1) + H) * (unsigned)g.P;
+}
+template <bool RO, typename E>
+__device__ __forceinline__ E ld(const E* level, unsigned i) {
+  if constexpr (RO) return __ldg(level + i);
+  else return level[i];
 }
 
 // ---------------------------------------------------------------- mass ----
 // The C-grid (CGRID) or D-grid mass and potential-temperature sweep of one
-// layer (src/mod_sw_dyn.f90:96-268 and 439-598), as k_mass2: S the state
-// type, C the C-grid fields' type, T the sweep arithmetic.  Output region
-// [lo, nx-1+hi] x [lo, ny-1+hi]; strips of TYS rows.
+// layer (src/mod_sw_dyn.f90:96-268 and 439-598): S the state type, C the
+// C-grid fields' type, T the sweep arithmetic.  The FP64 form has S = C = T =
+// double; the mixed form keeps the state in double, the C-grid fields in
+// float and sweeps in float.  Output region [lo, nx-1+hi] x [lo, ny-1+hi];
+// strips of tys rows.
 template <typename T, bool CGRID, typename S, typename C>
 struct MassM {
   using UB = std::conditional_t<CGRID, S, C>;  // u, v inputs
   using O = std::conditional_t<CGRID, C, S>;   // outputs
 };
 
-template <typename T, int TYS, bool CGRID, typename S, typename C, bool RO = true>
-__device__ __forceinline__ void mass_strip(Geom g, Consts c, const S* dp,
-                                                         const S* pt,
-                                                         const typename MassM<T, CGRID, S, C>::UB* u,
-                                                         const typename MassM<T, CGRID, S, C>::UB* v,
-                                                         const double* heat,
-                                                         typename MassM<T, CGRID, S, C>::O* dpo,
-                                                         typename MassM<T, CGRID, S, C>::O* pto, int lo,
-                                                         int hi, int* nonfinite, int sx, int sy, int k) {
+template <typename T, bool CGRID, typename S, typename C, bool RO = true>
+__device__ __forceinline__ void mass_strip(const Geom& g, const Consts& c, const S* dp, const S* pt,
+                                           const typename MassM<T, CGRID, S, C>::UB* u,
+                                           const typename MassM<T, CGRID, S, C>::UB* v, const double* heat,
+                                           typename MassM<T, CGRID, S, C>::O* dpo,
+                                           typename MassM<T, CGRID, S, C>::O* pto, int lo, int hi, int* nonfinite,
+                                           int sx, int sy, int k, int tys) {
   using UB = typename MassM<T, CGRID, S, C>::UB;
   using O = typename MassM<T, CGRID, S, C>::O;
   constexpr int V = CGRID ? PPM_UNC : PPM_NN;
   constexpr bool SAME = std::is_same_v<S, T>;
   const int lane = threadIdx.x & (MW - 1);
   const int ox = lo + sx * MOUT;
-  const int oy = lo + sy * TYS;
+  const int oy = lo + sy * tys;
   const int xhi = g.nx - 1 + hi, yhi = g.ny - 1 + hi;
   if (ox > xhi) return;  // the whole warp is past the region
   const int x = ox - MXH + lane;
   const bool out_lane = lane >= MXH && lane < MXH + MOUT && x <= xhi;
   const T dt = T(c.dt), dtdx = T(c.dtdx), dtdy = T(c.dtdy), rA = T(c.rA);
-  const T rdx2 = T(c.rdx2), rdy2 = T(c.rdy2), rdxy = T(c.rdx2rdy2);
+  const T rdx2 = T(c.rdx2), rdy2 = T(c.rdy2), m2rdxy = T(-2.) * T(c.rdx2rdy2);
   const T dxv = dtdx * T(c.vdx), dyv = dtdy * T(c.vdy), vdx = T(c.vdx), vdy = T(c.vdy);
-  const auto fdp = level<RO>(dp, g, k), fpt = level<RO>(pt, g, k);
-  const auto fu = level<RO>(u, g, k), fv = level<RO>(v, g, k);
+  const long long kS = (long long)k * g.S;
+  dp += kS;
+  pt += kS;
+  u += kS;
+  v += kS;
+  const unsigned xi = col_of(g, x), xr = col_of(g, x + 1);
 
   // register windows of the column, named by their row offset from the
   // newest row j of the current iteration
-  T d4 = 0, d3 = 0, d2 = 0, d1 = 0, d0 = 0;       // dp(j-4 .. j)
-  T p4 = 0, p3 = 0, p2 = 0, p1 = 0, p0 = 0;       // pt(j-4 .. j)
-  T tx4 = 0, tx3 = 0, tx2 = 0, tx1 = 0, tx0 = 0;  // inner x sweep of dp, rows j-4 .. j
-  T tp4 = 0, tp3 = 0, tp2 = 0, tp1 = 0, tp0 = 0;  // ... of pt
-  T my4 = 0, my3 = 0, my2 = 0, my1 = 0;           // its monotone y slopes, rows j-4 .. j-1
-  T mp4 = 0, mp3 = 0, mp2 = 0, mp1 = 0;
-  T fy1 = 0, fy0 = 0, fq1 = 0, fq0 = 0;           // y fluxes of dp and pt at rows j-3, j-2
+  T d3 = 0, d2 = 0, d1 = 0, d0 = 0;               // dp(j-3 .. j)
+  T p3 = 0, p2 = 0, p1 = 0, p0 = 0;               // pt(j-3 .. j)
+  T ds2 = 0, ds1 = 0, ds0 = 0;                    // dp(x+1) + dp(x-1), rows j-2 .. j
+  T ps2 = 0, ps1 = 0, ps0 = 0;                    // ... of pt
+  YLine<T, V> ld_, lp_;                           // the inner x sweeps of dp and pt along y
+  T fd1 = 0, fd0 = 0, fp1 = 0, fp0 = 0;           // piecewise-constant y fluxes of dp, pt at interfaces j-3, j-2
+  T fy1 = 0, fy0 = 0, fq1 = 0, fq0 = 0;           // y fluxes of dp and pt at interfaces j-3, j-2
   T ld2 = 0, ld1 = 0, ld0 = 0, lq2 = 0, lq1 = 0, lq0 = 0;  // Laplacians of dp, pt at rows j-4 .. j-2
   T uc3 = 0, uc2 = 0, uc1 = 0, uc0 = 0;           // C-grid u at rows j-3 .. j
   T vc1 = 0, vc0 = 0;                             // C-grid v at rows j-3, j-2
-  T su_x = 0, su_xm = 0;                          // D-grid u at (x, j), (x-1, j) (C grid)
-  T sv_x = 0, sv_xp = 0;                          // D-grid v at (x, j-3), (x+1, j-3) (C grid)
+  T us = 0;                                       // D-grid u(x, j) + u(x-1, j) (C grid)
+  T va_o = 0, vb_o = 0;                           // D-grid v at (x, j-3), (x+1, j-3) (C grid)
   if constexpr (CGRID) {
-    su_x = T(fu(x, oy - 3));
-    su_xm = T(fu(x - 1, oy - 3));
-    sv_x = T(fv(x, oy - 6));
-    sv_xp = T(fv(x + 1, oy - 6));
+    const T a = T(ld<RO>(u, row_of(g, oy - 3) + xi));
+    us = a + shfl_up(a, 1);
+    const unsigned rv = row_of(g, oy - 6);
+    va_o = T(ld<RO>(v, rv + xi));
+    vb_o = T(ld<RO>(v, rv + xr));
   }
   bool bad = false;
-  const int jend = min(oy + TYS, yhi + 1) + 3;
-  S dn_p = fdp(x, oy - 3), pn_p = fpt(x, oy - 3);
-  UB ua_p = CGRID ? fu(x, oy - 2) : fu(x, oy - 3), ub_p = CGRID ? fu(x - 1, oy - 2) : UB(0);
-  UB va_p = fv(x, oy - 5), vb_p = CGRID ? fv(x + 1, oy - 5) : UB(0);
+  const int jend = min(oy + tys, yhi + 1) + 3;
+  unsigned r = row_of(g, oy - 3);
+  S dn_p = ld<RO>(dp, r + xi), pn_p = ld<RO>(pt, r + xi);
+  UB ua_p = ld<RO>(u, (CGRID ? row_of(g, oy - 2) : r) + xi);
+  r = row_of(g, oy - 5);
+  UB va_p = ld<RO>(v, r + xi), vb_p = CGRID ? ld<RO>(v, r + xr) : UB(0);
+#pragma unroll MarchL<T, CGRID ? MK_CMASS : MK_DMASS>::unroll
   for (int j = oy - 3; j < jend; ++j) {
     // ---- row j: inputs, C-grid u, the inner x sweep (mod_sw_dyn.f90:109-117, 176-185; 503-511)
-    const S d_upd = fdp(x, j - 3), p_upd = fpt(x, j - 3);  // the update's state values of row j-3
-    const T dn = T(dn_p), pn = T(pn_p);
-    const UB ua_c = ua_p, ub_c = ub_p, va_c = va_p, vb_c = vb_p;
-    dn_p = fdp(x, j + 1);
-    pn_p = fpt(x, j + 1);
-    if constexpr (CGRID) {
-      ua_p = fu(x, j + 2);
-      ub_p = fu(x - 1, j + 2);
-      vb_p = fv(x + 1, j - 1);
-    } else {
-      ua_p = fu(x, j + 1);
+    const int y = j - 3;
+    const unsigned oi = row_of(g, y) + xi;
+    S d_upd = 0, p_upd = 0;  // the state values of row y (the update in the state's type)
+    if constexpr (!SAME) {
+      d_upd = ld<RO>(dp, oi);
+      p_upd = ld<RO>(pt, oi);
     }
-    va_p = fv(x, j - 1);
+    const T dn = T(dn_p), pn = T(pn_p);
+    const T ua_c = T(ua_p), va_c = T(va_p), vb_c = T(vb_p);
+    r = row_of(g, j + 1);
+    dn_p = ld<RO>(dp, r + xi);
+    pn_p = ld<RO>(pt, r + xi);
+    ua_p = ld<RO>(u, (CGRID ? row_of(g, j + 2) : r) + xi);
+    r = row_of(g, j - 1);
+    va_p = ld<RO>(v, r + xi);
+    if constexpr (CGRID) vb_p = ld<RO>(v, r + xr);
     T ucn;
-    if constexpr (CGRID) {
-      const T a = T(ua_c), b = T(ub_c);
-      const T ub = T(.5) * (su_x + su_xm);
-      ucn = T(.5) * (ub + T(.5) * (a + b));
-      su_x = a;
-      su_xm = b;
+    if constexpr (CGRID) {  // .5 (.5 (u + u(x-1)) + .5 (the row above)): the halvings are exact
+      const T s = ua_c + shfl_up(ua_c, 1);
+      ucn = T(.25) * (us + s);
+      us = s;
     } else {
-      ucn = T(ua_c);
+      ucn = ua_c;
     }
     const T ucR = shfl_dn(ucn, 1);
     const T dL = shfl_up(dn, 1), dR = shfl_dn(dn, 1);
     const T pL = shfl_up(pn, 1), pR = shfl_dn(pn, 1);
     T txn, tpn;
     {
-      const T cx0 = dtdx * ucn, cx1 = dtdx * ucR;
+      const bool c0 = dtdx * ucn > T(0), c1 = dtdx * ucR > T(0);
       const T den = T(1) / fmadd(-dtdx, ucR - ucn, T(1));
-      T f0 = (cx0 > T(0)) ? dL : dn;
-      T f1 = (cx1 > T(0)) ? dn : dR;
-      txn = T(.5) * fmadd(den, fmadd(-rA, f1 - f0, dn), dn);
-      f0 = (cx0 > T(0)) ? pL : pn;
-      f1 = (cx1 > T(0)) ? pn : pR;
-      tpn = T(.5) * fmadd(den, fmadd(-rA, f1 - f0, pn), pn);
+      txn = inner_e(dn, c0 ? dL : dn, c1 ? dn : dR, den, rA);
+      tpn = inner_e(pn, c0 ? pL : pn, c1 ? pn : pR, den, rA);
     }
     // shift the windows to the new row
-    d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = dn;
-    p4 = p3; p3 = p2; p2 = p1; p1 = p0; p0 = pn;
-    tx4 = tx3; tx3 = tx2; tx2 = tx1; tx1 = tx0; tx0 = txn;
-    tp4 = tp3; tp3 = tp2; tp2 = tp1; tp1 = tp0; tp0 = tpn;
+    d3 = d2; d2 = d1; d1 = d0; d0 = dn;
+    p3 = p2; p2 = p1; p1 = p0; p0 = pn;
+    ds2 = ds1; ds1 = ds0; ds0 = dR + dL;
+    ps2 = ps1; ps1 = ps0; ps0 = pR + pL;
     uc3 = uc2; uc2 = uc1; uc1 = uc0; uc0 = ucn;
-    // monotone y slope of row j-1 (ppm, :870-875)
-    my4 = my3; my3 = my2; my2 = my1; my1 = slope_v(tx2, tx1, tx0);
-    mp4 = mp3; mp3 = mp2; mp2 = mp1; mp1 = slope_v(tp2, tp1, tp0);
+    ld_.push(txn);
+    lp_.push(tpn);
     // C-grid v of row j-2 (:109-117)
-    T vcn;
-    if constexpr (CGRID) {
-      const T a = T(va_c), b = T(vb_c);
-      const T vb = T(.5) * (a + sv_x);
-      vcn = T(.5) * (vb + T(.5) * (b + sv_xp));
-      sv_x = a;
-      sv_xp = b;
-    } else {
-      vcn = T(va_c);
-    }
     vc1 = vc0;
-    vc0 = vcn;
-    {  // outer y sweep (PPM) at the interface below row j-2; the upwind
-       // cell's values selected first: one flux evaluation per lane
+    if constexpr (CGRID) {
+      vc0 = T(.25) * ((va_c + va_o) + (vb_c + vb_o));
+      va_o = va_c;
+      vb_o = vb_c;
+    } else {
+      vc0 = va_c;
+    }
+    {  // inner and outer y sweeps' fluxes at the interface below row j-2
       const T cy = dtdx * vc0;
-      const bool up = cy > T(0);
-      fy1 = fy0;
-      fq1 = fq0;
-      fy0 = flux_v<T, V>(cy, up ? tx4 : tx3, up ? tx3 : tx2, up ? tx2 : tx1, up ? my4 : my3, up ? my3 : my2,
-                         up ? my2 : my1) * cy;
-      fq0 = flux_v<T, V>(cy, up ? tp4 : tp3, up ? tp3 : tp2, up ? tp2 : tp1, up ? mp4 : mp3, up ? mp3 : mp2,
-                         up ? mp2 : mp1);
+      const bool pos = cy > T(0);
+      fd1 = fd0; fp1 = fp0;
+      fd0 = pos ? d3 : d2;
+      fp0 = pos ? p3 : p2;
+      fy1 = fy0; fq1 = fq0;
+      fy0 = ld_.flux(cy) * cy;
+      fq0 = lp_.flux(cy);
     }
     // Laplacians of row j-2 (:158-173)
-    {
-      const T dl = shfl_up(d2, 1), dr = shfl_dn(d2, 1);
-      const T pl = shfl_up(p2, 1), pr = shfl_dn(p2, 1);
-      ld2 = ld1; ld1 = ld0;
-      lq2 = lq1; lq1 = lq0;
-      ld0 = fmadd(d1 + d3, rdy2, fmadd(dr + dl, rdx2, T(-2.) * d2 * rdxy));
-      lq0 = fmadd(p1 + p3, rdy2, fmadd(pr + pl, rdx2, T(-2.) * p2 * rdxy));
-    }
-    const int y = j - 3;
-    if (y < oy) continue;  // warm-up rows of the strip (warp-uniform)
-    // ---- row y: inner y sweep, its x slopes, the outer x sweep, the update
-    T tyd, typ;
-    {
-      const T cy0 = dtdx * vc1, cy1 = dtdx * vc0;
+    ld2 = ld1; ld1 = ld0;
+    lq2 = lq1; lq1 = lq0;
+    ld0 = fmadd(d1 + d3, rdy2, fmadd(ds2, rdx2, d2 * m2rdxy));
+    lq0 = fmadd(p1 + p3, rdy2, fmadd(ps2, rdx2, p2 * m2rdxy));
+    if (y >= oy) {  // (the rows below are the strip's warm-up)
+      // ---- row y: inner y sweep, the outer x sweep, the update
       const T den = T(1) / fmadd(-dtdy, vc0 - vc1, T(1));
-      T f0 = (cy0 > T(0)) ? d4 : d3;
-      T f1 = (cy1 > T(0)) ? d3 : d2;
-      tyd = T(.5) * fmadd(den, fmadd(-rA, f1 - f0, d3), d3);
-      f0 = (cy0 > T(0)) ? p4 : p3;
-      f1 = (cy1 > T(0)) ? p3 : p2;
-      typ = T(.5) * fmadd(den, fmadd(-rA, f1 - f0, p3), p3);
-    }
-    const T mxd = slope_v(shfl_up(tyd, 1), tyd, shfl_dn(tyd, 1));
-    const T mxp = slope_v(shfl_up(typ, 1), typ, shfl_dn(typ, 1));
-    T fxd, fxp;
-    {
+      const T tyd = inner_e(d3, fd1, fd0, den, rA);
+      const T typ = inner_e(p3, fp1, fp0, den, rA);
       const T cx = dtdx * uc3;
-      const int s0 = lane + ((cx > T(0)) ? -1 : 0);  // the upwind cell's lane
-      fxd = flux_v<T, V>(cx, shfl_at(tyd, s0 - 1), shfl_at(tyd, s0), shfl_at(tyd, s0 + 1), shfl_at(mxd, s0 - 1),
-                         shfl_at(mxd, s0), shfl_at(mxd, s0 + 1)) * cx;
-      fxp = flux_v<T, V>(cx, shfl_at(typ, s0 - 1), shfl_at(typ, s0), shfl_at(typ, s0 + 1), shfl_at(mxp, s0 - 1),
-                         shfl_at(mxp, s0), shfl_at(mxp, s0 + 1));
+      const T fxd = xline_flux<T, V>(tyd, cx) * cx;
+      const T fxp = xline_flux<T, V>(typ, cx);
+      const T fxd1 = shfl_dn(fxd, 1), fxp1 = shfl_dn(fxp, 1);
+      const T lxm = shfl_up(ld1, 1), lxp = shfl_dn(ld1, 1);
+      const T qxm = shfl_up(lq1, 1), qxp = shfl_dn(lq1, 1);
+      if (out_lane && y <= yhi) {
+        // updates, mod_sw_dyn.f90:163-172,193-202,230-237,258-267 (C); 490-499,519-528,555-562,582-591 (D)
+        O vo, qo;
+        if constexpr (SAME) {  // the reference's operations, in order
+          const T d = d3;
+          T vv = d - (fxd1 - fxd + dxv * (fmx(T(-2), ld1, lxp) + lxm));
+          vv = vv - (fy0 - fy1 + dyv * (fmx(T(-2), ld1, ld0) + ld2));
+          T q = d * p3 - (fxp1 * fxd1 - fxp * fxd + vdx * ((qxp - lq1) * fxd1 - (lq1 - qxm) * fxd));
+          q = q - (fq0 * fy0 - fq1 * fy1 + vdy * ((lq0 - lq1) * fy0 - (lq1 - lq2) * fy1));
+          if (heat) q = q + dt * d * T(heat[kS + oi]);
+          q = q / vv;
+          vo = O(vv);
+          qo = O(q);
+        } else {
+          // the same update in flux form: interface fluxes (advective plus
+          // vorticity-damping) in the sweep type, their differences applied to
+          // the state's type, so that mass and dp*pt telescope in S
+          const T Fx0 = fmadd(dxv, ld1 - lxm, fxd), Fx1 = fmadd(dxv, lxp - ld1, fxd1);
+          const T Fy0 = fmadd(dyv, ld1 - ld2, fy1), Fy1 = fmadd(dyv, ld0 - ld1, fy0);
+          const T Hx0 = fmadd(vdx, lq1 - qxm, fxp) * fxd, Hx1 = fmadd(vdx, qxp - lq1, fxp1) * fxd1;
+          const T Hy0 = fmadd(vdy, lq1 - lq2, fq1) * fy1, Hy1 = fmadd(vdy, lq0 - lq1, fq0) * fy0;
+          const S d = d_upd;
+          const S vv = d - ((S(Fx1) - S(Fx0)) + (S(Fy1) - S(Fy0)));
+          S q = d * p_upd - ((S(Hx1) - S(Hx0)) + (S(Hy1) - S(Hy0)));
+          if (heat) q = q + S(c.dt) * d * S(heat[kS + oi]);
+          q = q / vv;
+          vo = O(vv);
+          qo = O(q);
+        }
+        dpo[kS + oi] = vo;
+        pto[kS + oi] = qo;
+        const bool inside = x >= 0 && x < g.nx && y >= 0 && y < g.ny;
+        bad = bad || (inside && !(finite_(vo) && finite_(qo)));
+      }
     }
-    const T fxd1 = shfl_dn(fxd, 1), fxp1 = shfl_dn(fxp, 1);
-    const T lxm = shfl_up(ld1, 1), lxp = shfl_dn(ld1, 1);
-    const T qxm = shfl_up(lq1, 1), qxp = shfl_dn(lq1, 1);
-    if (!out_lane || y > yhi) continue;
-    // updates, mod_sw_dyn.f90:163-172,193-202,230-237,258-267 (C); 490-499,519-528,555-562,582-591 (D)
-    O vo, qo;
-    const long long o = g.at(x, y, k);
-    if constexpr (SAME) {  // the reference's operations, in order
-      const T d = d3;
-      T vv = d - (fxd1 - fxd + dxv * (lxp - T(2.) * ld1 + lxm));
-      vv = vv - (fy0 - fy1 + dyv * (ld0 - T(2.) * ld1 + ld2));
-      T q = d * p3 - (fxp1 * fxd1 - fxp * fxd + vdx * ((qxp - lq1) * fxd1 - (lq1 - qxm) * fxd));
-      q = q - (fq0 * fy0 - fq1 * fy1 + vdy * ((lq0 - lq1) * fy0 - (lq1 - lq2) * fy1));
-      if (heat) q = q + dt * d * T(heat[o]);
-      q = q / vv;
-      vo = O(vv);
-      qo = O(q);
-    } else {
-      // the same update in flux form: interface fluxes (advective plus
-      // vorticity-damping) in the sweep type, their differences applied to
-      // the state's type, so that mass and dp*pt telescope in S
-      const T Fx0 = fmadd(dxv, ld1 - lxm, fxd), Fx1 = fmadd(dxv, lxp - ld1, fxd1);
-      const T Fy0 = fmadd(dyv, ld1 - ld2, fy1), Fy1 = fmadd(dyv, ld0 - ld1, fy0);
-      const T Hx0 = fmadd(vdx, lq1 - qxm, fxp) * fxd, Hx1 = fmadd(vdx, qxp - lq1, fxp1) * fxd1;
-      const T Hy0 = fmadd(vdy, lq1 - lq2, fq1) * fy1, Hy1 = fmadd(vdy, lq0 - lq1, fq0) * fy0;
-      const S d = d_upd;
-      const S vv = d - ((S(Fx1) - S(Fx0)) + (S(Fy1) - S(Fy0)));
-      S q = d * p_upd - ((S(Hx1) - S(Hx0)) + (S(Hy1) - S(Hy0)));
-      if (heat) q = q + S(c.dt) * d * S(heat[o]);
-      q = q / vv;
-      vo = O(vv);
-      qo = O(q);
-    }
-    dpo[o] = vo;
-    pto[o] = qo;
-    const bool inside = x >= 0 && x < g.nx && y >= 0 && y < g.ny;
-    bad = bad || (inside && !(finite_(vo) && finite_(qo)));
   }
   if (nonfinite) flag_nonfinite(nonfinite, bad);
 }
 
 // one warp per strip: blockIdx.x * MWARPS + warp across x, blockIdx.y
 // across y, blockIdx.z the layer
-template <typename T, int TYS, bool CGRID, typename S, typename C>
-__global__ void __launch_bounds__(MW * MWARPS, ATM_MARCH_MINB) k_mass_m(Geom g, Consts c, const S* __restrict__ dp,
+template <typename T, bool CGRID, typename S, typename C>
+__global__ void __launch_bounds__(MW * MWARPS, MarchL<T, CGRID ? MK_CMASS : MK_DMASS>::min_blocks) k_mass_m(Geom g, Consts c, const S* __restrict__ dp,
                                                          const S* __restrict__ pt,
                                                          const typename MassM<T, CGRID, S, C>::UB* __restrict__ u,
                                                          const typename MassM<T, CGRID, S, C>::UB* __restrict__ v,
                                                          const double* __restrict__ heat,
                                                          typename MassM<T, CGRID, S, C>::O* __restrict__ dpo,
                                                          typename MassM<T, CGRID, S, C>::O* __restrict__ pto, int lo,
-                                                         int hi, int* nonfinite) {
-  mass_strip<T, TYS, CGRID, S, C>(g, c, dp, pt, u, v, heat, dpo, pto, lo, hi, nonfinite, blockIdx.x * MWARPS + (threadIdx.x >> 5), blockIdx.y, blockIdx.z);
+                                                         int hi, int* nonfinite, int tys) {
+  mass_strip<T, CGRID, S, C>(g, c, dp, pt, u, v, heat, dpo, pto, lo, hi, nonfinite,
+                             blockIdx.x * MWARPS + (threadIdx.x >> 5), blockIdx.y, blockIdx.z, tys);
 }
 
 // ======================================================== C-grid momentum ==
-// The C-grid momentum update of one layer (src/mod_sw_dyn.f90:294-414), as
-// k_c_mom2: kinetic energy from PPM fluxes of the C-grid winds with the
+// The C-grid momentum update of one layer (src/mod_sw_dyn.f90:294-414):
+// kinetic energy from PPM fluxes of the C-grid winds with the
 // layer-nlay A-grid winds (:299-317), absolute vorticity (:319-323), the
 // pressure-gradient force (:325-339) and the vorticity-flux updates of uc
-// and vc (:344-412).  Outputs on the interior; strips of TYS rows.
-template <typename T, int TYS, typename S, typename C, bool RO = true>
-__device__ __forceinline__ void c_mom_strip(Geom g, Consts c, const S* ud,
-                                                          const S* vd, const double* pkap,
-                                                          const double* gz, C* uc,
-                                                          C* vc, int sx, int sy, int k) {
+// and vc (:344-412).  Outputs on the interior; strips of tys rows.
+template <typename T, typename S, typename C, bool RO = true>
+__device__ __forceinline__ void c_mom_strip(const Geom& g, const Consts& c, const S* ud, const S* vd,
+                                            const double* pkap, const double* gz, C* uc, C* vc, int sx, int sy, int k,
+                                            int tys) {
   constexpr int UNC = PPM_UNC;
   const int lane = threadIdx.x & (MW - 1);
   const int ox = sx * MOUT;
-  const int oy = sy * TYS;
-  const int L = g.L;
+  const int oy = sy * tys;
   if (ox >= g.nx) return;  // the whole warp is past the region
   const int x = ox - MXH + lane;
   const bool out_lane = lane >= MXH && lane < MXH + MOUT && x < g.nx;
   const T dt = T(c.dt), dtdx = T(c.dtdx), dtdy = T(c.dtdy), rA = T(c.rA);
   const T rdx = T(c.rdx), rdy = T(c.rdy), f = T(c.coriolis);
-  const T rdx2 = T(c.rdx2), rdy2 = T(c.rdy2), rdxy = T(c.rdx2rdy2);
+  const T rdx2 = T(c.rdx2), rdy2 = T(c.rdy2), m2rdxy = T(-2.) * T(c.rdx2rdy2);
   const T vdx = T(c.vdx), vdy = T(c.vdy);
-  const auto fud = level<RO>(ud, g, k), fvd = level<RO>(vd, g, k);
-  const auto fuL = level<RO>(ud, g, L - 1), fvL = level<RO>(vd, g, L - 1);
-  const auto fpk0 = level<RO>(pkap, g, k), fpk1 = level<RO>(pkap, g, k + 1);
-  const auto fgz0 = level<RO>(gz, g, k), fgz1 = level<RO>(gz, g, k + 1);
+  const long long kS = (long long)k * g.S, LS = (long long)(g.L - 1) * g.S;
+  const S *uk = ud + kS, *vk = vd + kS, *uL = ud + LS, *vL = vd + LS;
+  const double *pka = pkap + kS, *pkb = pka + g.S, *gza = gz + kS, *gzb = gza + g.S;
+  const unsigned xi = col_of(g, x), xl = col_of(g, x - 1), xr = col_of(g, x + 1);
 
   // register windows of the column, named by their row offset from the
   // newest row j of the iteration
-  T u_x = T(fud(x, oy - 3)), u_xm = T(fud(x - 1, oy - 3));  // ud(x, j), ud(x-1, j)
-  T v_x = T(fvd(x, oy - 4)), v_xp = T(fvd(x + 1, oy - 4));  // vd(x, j-1), vd(x+1, j-1)
-  T uw3 = 0, uw2 = 0, uw1 = 0, uw0 = 0;           // ud(x, j-3 .. j)
+  unsigned r = row_of(g, oy - 3);
+  T u_x = T(ld<RO>(uk, r + xi)), u_xm = T(ld<RO>(uk, r + xl));  // ud(x, j), ud(x-1, j)
+  r = row_of(g, oy - 4);
+  T v_x = T(ld<RO>(vk, r + xi)), v_xp = T(ld<RO>(vk, r + xr));  // vd(x, j-1), vd(x+1, j-1)
+  T uw3 = 0, uw2 = 0, uw1 = 0, uw0 = 0;  // ud(x, j-3 .. j)
   T vw4 = 0, vw3 = 0, vw2 = 0, vw1 = 0, vw0 = 0;  // vd(x, j-4 .. j)
-  T a3 = 0, a2 = 0, a1 = 0, a0 = 0;               // C-grid u of this layer, rows j-3 .. j
-  T b4 = 0, b3 = 0, b2 = 0, b1 = 0, b0 = 0;       // C-grid v, rows j-4 .. j
-  T mv4 = 0, mv3 = 0, mv2 = 0, mv1 = 0;           // monotone y slopes of C-grid v, rows j-4 .. j-1
-  T w4 = 0, w3 = 0, w2 = 0, w1 = 0, w0 = 0;       // absolute vorticity, rows j-4 .. j
-  T t4 = 0, t3 = 0, t2 = 0, t1 = 0, t0 = 0;       // inner x sweep of the vorticity, rows j-4 .. j
-  T mt4 = 0, mt3 = 0, mt2 = 0, mt1 = 0;           // its monotone y slopes, rows j-4 .. j-1
-  T lp1 = 0, lp0 = 0;                             // Laplacian of the vorticity, rows j-3, j-2
-  T ke1 = 0, ke0 = 0;                             // kinetic energy, rows j-4, j-3
+  T a3 = 0, a2 = 0, a1 = 0, a0 = 0;      // C-grid u of this layer, rows j-3 .. j
+  YLine<T, UNC> lb;                      // C-grid v of this layer along y
+  YLine<T, UNC> lt;                      // the inner x sweep of the vorticity along y
+  T w3 = 0, w2 = 0, w1 = 0, w0 = 0;      // absolute vorticity, rows j-3 .. j
+  T ws2 = 0, ws1 = 0, ws0 = 0;           // its x(+1) + x(-1), rows j-2 .. j
+  T fw1 = 0, fw0 = 0;                    // its piecewise-constant y flux at interfaces j-3, j-2
+  T lp1 = 0, lp0 = 0;                    // Laplacian of the vorticity, rows j-3, j-2
+  T ke1 = 0, ke0 = 0;                    // kinetic energy, rows j-4, j-3
   double pk0m = 0, pk1m = 0, gz0m = 0, gz1m = 0;  // pkap, gz at k and k+1, row j-4
   // layer-nlay ud at row y and vd at rows y-1, y of the first kinetic-energy row y = oy-1
-  T uL1 = T(fuL(x, oy - 1)), vL2 = T(fvL(x, oy - 2)), vL1 = T(fvL(x, oy - 1));
-  const int jend = min(oy + TYS, g.ny) + 3;
-  S un_p = fud(x, oy - 2), unm_p = fud(x - 1, oy - 2), vn_p = fvd(x, oy - 3), vnp_p = fvd(x + 1, oy - 3);
+  T uL1 = T(ld<RO>(uL, row_of(g, oy - 1) + xi));
+  T vL2 = T(ld<RO>(vL, row_of(g, oy - 2) + xi)), vL1 = T(ld<RO>(vL, row_of(g, oy - 1) + xi));
+  const int jend = min(oy + tys, g.ny) + 3;
+  r = row_of(g, oy - 2);
+  S un_p = ld<RO>(uk, r + xi), unm_p = ld<RO>(uk, r + xl);
+  r = row_of(g, oy - 3);
+  S vn_p = ld<RO>(vk, r + xi), vnp_p = ld<RO>(vk, r + xr);
+#pragma unroll MarchL<T, MK_CMOM>::unroll
   for (int j = oy - 3; j < jend; ++j) {
     // loads of row y = j-3 issued before this row's work
-    const double pk0 = fpk0(x, j - 3), pk1 = fpk1(x, j - 3), gz0 = fgz0(x, j - 3), gz1 = fgz1(x, j - 3);
-    const S uL0_r = fuL(x, j - 2), vL0_r = fvL(x, j - 2);
+    const int y = j - 3;
+    const unsigned oi = row_of(g, y) + xi, ri = row_of(g, j - 2) + xi;
+    const double pk0 = ld<RO>(pka, oi), pk1 = ld<RO>(pkb, oi), gz0 = ld<RO>(gza, oi), gz1 = ld<RO>(gzb, oi);
+    const S uL0_r = ld<RO>(uL, ri), vL0_r = ld<RO>(vL, ri);
     // ---- row j: C-grid winds of the layer (:110-117), vorticity (:319-323),
     // inner x sweep of the vorticity (:353-367)
     const T un = T(un_p), unm = T(unm_p);
     const T vn = T(vn_p), vnp = T(vnp_p);
-    un_p = fud(x, j + 2);
-    unm_p = fud(x - 1, j + 2);
-    vn_p = fvd(x, j + 1);
-    vnp_p = fvd(x + 1, j + 1);
-    const T ucn = T(.5) * (T(.5) * (u_x + u_xm) + T(.5) * (un + unm));
-    const T vcn = T(.5) * (T(.5) * (vn + v_x) + T(.5) * (vnp + v_xp));
+    r = row_of(g, j + 2);
+    un_p = ld<RO>(uk, r + xi);
+    unm_p = ld<RO>(uk, r + xl);
+    r = row_of(g, j + 1);
+    vn_p = ld<RO>(vk, r + xi);
+    vnp_p = ld<RO>(vk, r + xr);
+    const T ucn = T(.25) * ((u_x + u_xm) + (un + unm));  // the reference's halvings are exact
+    const T vcn = T(.25) * ((vn + v_x) + (vnp + v_xp));
     const T vor = fmadd(vcn - shfl_up(vcn, 1), rdx, fmadd(-(ucn - a0), rdy, f));
     const T vl = shfl_up(vor, 1), vr = shfl_dn(vor, 1);
     T tun;
     {
-      const T c0 = dtdx * u_xm, c1 = dtdx * u_x;
       const T den = T(1) / fmadd(-dtdx, u_x - u_xm, T(1));
-      const T f0 = (c0 > T(0)) ? vl : vor;
-      const T f1 = (c1 > T(0)) ? vor : vr;
-      tun = T(.5) * fmadd(den, fmadd(-rA, f1 - f0, vor), vor);
+      tun = inner_e(vor, (dtdx * u_xm > T(0)) ? vl : vor, (dtdx * u_x > T(0)) ? vor : vr, den, rA);
     }
     uw3 = uw2; uw2 = uw1; uw1 = uw0; uw0 = u_x;
     u_x = un;
@@ -452,248 +575,215 @@ __device__ __forceinline__ void c_mom_strip(Geom g, Consts c, const S* ud,
     v_xp = vnp;
     vw4 = vw3; vw3 = vw2; vw2 = vw1; vw1 = vw0; vw0 = vn;
     a3 = a2; a2 = a1; a1 = a0; a0 = ucn;
-    b4 = b3; b3 = b2; b2 = b1; b1 = b0; b0 = vcn;
-    w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = vor;
-    t4 = t3; t3 = t2; t2 = t1; t1 = t0; t0 = tun;
-    mv4 = mv3; mv3 = mv2; mv2 = mv1; mv1 = slope_v(b2, b1, b0);
-    mt4 = mt3; mt3 = mt2; mt2 = mt1; mt1 = slope_v(t2, t1, t0);
-    // Laplacian of the vorticity at row j-2
+    w3 = w2; w2 = w1; w1 = w0; w0 = vor;
+    ws2 = ws1; ws1 = ws0; ws0 = vr + vl;
+    const T b3 = lb.q2;  // C-grid v of row j-3
+    lb.push(vcn);
+    lt.push(tun);
+    // the vorticity's inner y sweep at the interface below row j-2 (vd(x, j-3)), its Laplacian at row j-2
+    fw1 = fw0;
+    fw0 = (dtdx * vw3 > T(0)) ? w3 : w2;
     lp1 = lp0;
-    lp0 = fmadd(w1 + w3, rdy2, fmadd(shfl_dn(w2, 1) + shfl_up(w2, 1), rdx2, T(-2.) * w2 * rdxy));
-    const int y = j - 3;
-    if (y < oy - 1) continue;  // warm-up rows (warp-uniform)
-    // ---- row y: kinetic energy (:299-317) with the layer-nlay A-grid winds
-    // (:110-125 at k = nlay), recomputed where they are read
-    const T uL0 = T(uL0_r), vL0 = T(vL0_r);
-    T ken;
-    {
-      const T ub = T(.5) * (uL1 + shfl_up(uL1, 1));
-      const T ucl = T(.5) * (ub + T(.5) * (uL0 + shfl_up(uL0, 1)));
-      const T ua = T(.5) * (ucl + T(.25) * (shfl_dn(uL1, 1) + uL1 + shfl_dn(uL0, 1) + uL0));
-      const T vb = T(.5) * (vL1 + vL2);
-      const T vL1r = shfl_dn(vL1, 1);
-      const T vcl = T(.5) * (vb + T(.5) * (vL1r + shfl_dn(vL2, 1)));
-      const T va = T(.5) * (vcl + T(.25) * (vL0 + vL1 + shfl_dn(vL0, 1) + vL1r));
-      const T cy = dtdy * va;
-      const bool upy = cy > T(0);
-      const T fy = flux_v<T, UNC>(cy, upy ? b4 : b3, upy ? b3 : b2, upy ? b2 : b1, upy ? mv4 : mv3,
-                                  upy ? mv3 : mv2, upy ? mv2 : mv1);
-      const T kv = va * fy;
-      const T mux = slope_v(shfl_up(a3, 1), a3, shfl_dn(a3, 1));
-      const T cx = dtdx * ua;
-      const int s0 = lane + ((cx > T(0)) ? 0 : 1);  // the upwind cell's lane
-      const T fx = flux_v<T, UNC>(cx, shfl_at(a3, s0 - 1), shfl_at(a3, s0), shfl_at(a3, s0 + 1),
-                                  shfl_at(mux, s0 - 1), shfl_at(mux, s0), shfl_at(mux, s0 + 1));
-      ken = T(.5) * fmadd(ua, fx, kv);
+    lp0 = fmadd(w1 + w3, rdy2, fmadd(ws2, rdx2, w2 * m2rdxy));
+    if (y >= oy - 1) {  // (the rows below are the strip's warm-up)
+      // ---- row y: kinetic energy (:299-317) with the layer-nlay A-grid winds
+      // (:110-125 at k = nlay), recomputed where they are read
+      const T uL0 = T(uL0_r), vL0 = T(vL0_r);
+      T ken;
+      {
+        const T ub = T(.5) * (uL1 + shfl_up(uL1, 1));
+        const T ucl = T(.5) * (ub + T(.5) * (uL0 + shfl_up(uL0, 1)));
+        const T ua = T(.5) * (ucl + T(.25) * (shfl_dn(uL1, 1) + uL1 + shfl_dn(uL0, 1) + uL0));
+        const T vb = T(.5) * (vL1 + vL2);
+        const T vL1r = shfl_dn(vL1, 1);
+        const T vcl = T(.5) * (vb + T(.5) * (vL1r + shfl_dn(vL2, 1)));
+        const T va = T(.5) * (vcl + T(.25) * (vL0 + vL1 + shfl_dn(vL0, 1) + vL1r));
+        const T kv = va * lb.flux(dtdy * va);
+        // the flux at the interface above the lane's cell: that of the next lane's lower interface
+        const T fx = xline_flux_above<T>(a3, dtdx * ua);
+        ken = T(.5) * fmadd(ua, fx, kv);
+      }
+      uL1 = uL0;
+      vL2 = vL1;
+      vL1 = vL0;
+      ke1 = ke0;
+      ke0 = ken;
+      const double pk0l = shfl_up(pk0, 1), pk1l = shfl_up(pk1, 1), gz0l = shfl_up(gz0, 1), gz1l = shfl_up(gz1, 1);
+      const double pk0d = pk0m, pk1d = pk1m, gz0d = gz0m, gz1d = gz1m;  // row y-1
+      pk0m = pk0; pk1m = pk1; gz0m = gz0; gz1m = gz1;
+      if (y >= oy) {
+        // ---- row y: inner y sweep of the vorticity (:388-397), its x sweep, the updates
+        const T den = T(1) / fmadd(-dtdy, vw3 - vw4, T(1));
+        const T tvn = inner_e(w3, fw1, fw0, den, rA);
+        const T ke_l = shfl_up(ke0, 1);
+        const T lp_r = shfl_dn(lp1, 1);
+        const T udx = uw3, vdx_ = vw3;
+        const T fx = xline_flux_above<T>(tvn, dtdx * udx);
+        if (out_lane && y < g.ny) {
+          const double pgx = ((pk0 - pk1l) * (gz0l - gz1) + (pk0l - pk1) * (gz1l - gz0)) / (pk0 - pk1l + pk0l - pk1);
+          const double pgy = ((pk0 - pk1d) * (gz0d - gz1) + (pk0d - pk1) * (gz1d - gz0)) / (pk0 - pk1d + pk0d - pk1);
+          const T fy = lt.flux(dtdx * vdx_);
+          uc[kS + oi] = C(fmadd(-dtdx, ke0 - ke_l - T(pgx), fmadd(dt, fmadd(vdy, lp0 - lp1, vdx_ * fy), a3)));
+          vc[kS + oi] = C(fmadd(-dtdy, ke0 - ke1 - T(pgy), fmadd(-dt, fmadd(vdx, lp_r - lp1, udx * fx), b3)));
+        }
+      }
     }
-    uL1 = uL0;
-    vL2 = vL1;
-    vL1 = vL0;
-    ke1 = ke0;
-    ke0 = ken;
-    const double pk0l = shfl_up(pk0, 1), pk1l = shfl_up(pk1, 1), gz0l = shfl_up(gz0, 1), gz1l = shfl_up(gz1, 1);
-    const double pk0d = pk0m, pk1d = pk1m, gz0d = gz0m, gz1d = gz1m;  // row y-1
-    pk0m = pk0; pk1m = pk1; gz0m = gz0; gz1m = gz1;
-    if (y < oy) continue;
-    // ---- row y: inner y sweep of the vorticity (:388-397), its x slopes, the updates
-    T tvn;
-    {
-      const T c0 = dtdx * vw4, c1 = dtdx * vw3;
-      const T den = T(1) / fmadd(-dtdy, vw3 - vw4, T(1));
-      const T f0 = (c0 > T(0)) ? w4 : w3;
-      const T f1 = (c1 > T(0)) ? w3 : w2;
-      tvn = T(.5) * fmadd(den, fmadd(-rA, f1 - f0, w3), w3);
-    }
-    const T mtv = slope_v(shfl_up(tvn, 1), tvn, shfl_dn(tvn, 1));
-    const T ke_l = shfl_up(ke0, 1);
-    const T lp_r = shfl_dn(lp1, 1);
-    const T udx = uw3, vdx_ = vw3;
-    T fx;
-    {
-      const T cx = dtdx * udx;
-      const int s0 = lane + ((cx > T(0)) ? 0 : 1);
-      fx = flux_v<T, UNC>(cx, shfl_at(tvn, s0 - 1), shfl_at(tvn, s0), shfl_at(tvn, s0 + 1), shfl_at(mtv, s0 - 1),
-                          shfl_at(mtv, s0), shfl_at(mtv, s0 + 1));
-    }
-    if (!out_lane || y >= g.ny) continue;
-    const double pgx = ((pk0 - pk1l) * (gz0l - gz1) + (pk0l - pk1) * (gz1l - gz0)) / (pk0 - pk1l + pk0l - pk1);
-    const double pgy = ((pk0 - pk1d) * (gz0d - gz1) + (pk0d - pk1) * (gz1d - gz0)) / (pk0 - pk1d + pk0d - pk1);
-    T fy;
-    {
-      const T cy = dtdx * vdx_;
-      const bool up = cy > T(0);
-      fy = flux_v<T, UNC>(cy, up ? t4 : t3, up ? t3 : t2, up ? t2 : t1, up ? mt4 : mt3, up ? mt3 : mt2,
-                          up ? mt2 : mt1);
-    }
-    const T u = fmadd(-dtdx, ke0 - ke_l - T(pgx), fmadd(dt, fmadd(vdy, lp0 - lp1, vdx_ * fy), a3));
-    const T v = fmadd(-dtdy, ke0 - ke1 - T(pgy), fmadd(-dt, fmadd(vdx, lp_r - lp1, udx * fx), b3));
-    const long long o = g.at(x, y, k);
-    uc[o] = C(u);
-    vc[o] = C(v);
   }
 }
 
 // one warp per strip: blockIdx.x * MWARPS + warp across x, blockIdx.y
 // across y, blockIdx.z the layer
-template <typename T, int TYS, typename S, typename C>
-__global__ void __launch_bounds__(MW * MWARPS, ATM_MARCH_MINB) k_c_mom_m(Geom g, Consts c, const S* __restrict__ ud,
+template <typename T, typename S, typename C>
+__global__ void __launch_bounds__(MW * MWARPS, MarchL<T, MK_CMOM>::min_blocks) k_c_mom_m(Geom g, Consts c, const S* __restrict__ ud,
                                                           const S* __restrict__ vd, const double* __restrict__ pkap,
                                                           const double* __restrict__ gz, C* __restrict__ uc,
-                                                          C* __restrict__ vc) {
-  c_mom_strip<T, TYS, S, C>(g, c, ud, vd, pkap, gz, uc, vc, blockIdx.x * MWARPS + (threadIdx.x >> 5), blockIdx.y, blockIdx.z);
+                                                          C* __restrict__ vc, int tys) {
+  c_mom_strip<T, S, C>(g, c, ud, vd, pkap, gz, uc, vc, blockIdx.x * MWARPS + (threadIdx.x >> 5), blockIdx.y,
+                       blockIdx.z, tys);
 }
 
 // ======================================================== D-grid momentum ==
-// The D-grid momentum update of one layer (src/mod_sw_dyn.f90:634-771), as
-// k_d_mom2: kinetic energy from constrained-PPM fluxes of ud, vd with the
+// The D-grid momentum update of one layer (src/mod_sw_dyn.f90:634-771):
+// kinetic energy from constrained-PPM fluxes of ud, vd with the
 // layer-nlay B-grid winds (:639-657, 441-444), vorticity (:659-663), the
 // B-grid pressure-gradient force (:665-679), del^4 divergence damping
 // (:682-702) and the vorticity-flux updates (:708-769).  Outputs on the
-// interior; strips of TYS rows.
-template <typename T, int TYS, typename S, typename C, bool RO = true>
-__device__ __forceinline__ void d_mom_strip(Geom g, Consts c, const S* ud,
-                                                          const S* vd, const C* uc,
-                                                          const C* vc, const double* pkapb,
-                                                          const double* gzb, S* udo,
-                                                          S* vdo, int* nonfinite, int sx, int sy, int k) {
+// interior; strips of tys rows.
+template <typename T, typename S, typename C, bool RO = true>
+__device__ __forceinline__ void d_mom_strip(const Geom& g, const Consts& c, const S* ud, const S* vd, const C* uc,
+                                            const C* vc, const double* pkapb, const double* gzb, S* udo, S* vdo,
+                                            int* nonfinite, int sx, int sy, int k, int tys) {
   constexpr int CON = PPM_CON;
+  constexpr bool SAME = std::is_same_v<S, T>;
   const int lane = threadIdx.x & (MW - 1);
   const int ox = sx * MOUT;
-  const int oy = sy * TYS;
-  const int L = g.L;
+  const int oy = sy * tys;
   if (ox >= g.nx) return;  // the whole warp is past the region
   const int x = ox - MXH + lane;
   const bool out_lane = lane >= MXH && lane < MXH + MOUT && x < g.nx;
   const T dt = T(c.dt), dtdx = T(c.dtdx), dtdy = T(c.dtdy), rA = T(c.rA);
   const T rdx = T(c.rdx), rdy = T(c.rdy), f = T(c.coriolis);
-  const T rdx2 = T(c.rdx2), rdy2 = T(c.rdy2), rdxy = T(c.rdx2rdy2);
+  const T rdx2 = T(c.rdx2), rdy2 = T(c.rdy2), m2rdxy = T(-2.) * T(c.rdx2rdy2);
   const T vdx = T(c.vdx), vdy = T(c.vdy), divdamp = T(c.divdamp);
-  const auto fud = level<RO>(ud, g, k), fvd = level<RO>(vd, g, k);
-  const auto fuL = level<RO>(uc, g, L - 1), fvL = level<RO>(vc, g, L - 1);
-  const auto fuc = level<RO>(uc, g, k), fvc = level<RO>(vc, g, k);
-  const auto fpb0 = level<RO>(pkapb, g, k), fpb1 = level<RO>(pkapb, g, k + 1);
-  const auto fgb0 = level<RO>(gzb, g, k), fgb1 = level<RO>(gzb, g, k + 1);
+  const long long kS = (long long)k * g.S, LS = (long long)(g.L - 1) * g.S;
+  const S *uk = ud + kS, *vk = vd + kS;
+  const C *uL = uc + LS, *vL = vc + LS, *ucK = uc + kS, *vcK = vc + kS;
+  const double *pba = pkapb + kS, *pbb = pba + g.S, *gba = gzb + kS, *gbb = gba + g.S;
+  const unsigned xi = col_of(g, x);
 
   // register windows of the column, named by their row offset from the
   // newest row j of the iteration
-  T s2 = 0, s1 = 0, s0 = T(fud(x, oy - 3));                     // ud(x, j-2 .. j)
-  T v3 = 0, v2 = 0, v1 = 0, v0 = T(fvd(x, oy - 3));             // vd(x, j-3 .. j)
-  T mv3 = 0, mv2 = 0, mv1 = 0;                                  // monotone y slopes of vd, rows j-3 .. j-1
-  T lv3 = 0, rv3 = 0, lv2 = 0, rv2 = 0;                         // constrained edges of vd, rows j-3, j-2
-  T q2 = 0, q1 = 0, q0 = 0;                                     // divergence, rows j-2 .. j
-  T e3 = 0, e2 = 0, e1 = 0;                                     // its Laplacian, rows j-3 .. j-1
-  T dd3 = 0, dd2 = 0;                                           // del^4 damping term, rows j-3, j-2
-  T w4 = 0, w3 = 0, w2 = 0, w1 = 0;                             // vorticity, rows j-4 .. j-1
-  T t4 = 0, t3 = 0, t2 = 0, t1 = 0;                             // inner x sweep of the vorticity, rows j-4 .. j-1
-  T mt4 = 0, mt3 = 0, mt2 = 0;                                  // its monotone y slopes, rows j-4 .. j-2
-  T lt4 = 0, rt4 = 0, lt3 = 0, rt3 = 0;                         // its constrained edges, rows j-4, j-3
-  T ke3 = 0, ke2 = 0;                                           // kinetic energy, rows j-3, j-2
-  T lp4 = 0, lp3 = 0, lp2 = 0;                                  // Laplacian of the vorticity, rows j-4 .. j-2
-  T cu3 = 0, cu2 = T(fuL(x, oy - 5)), cu1 = T(fuL(x, oy - 4));  // layer-nlay uc, rows j-3 .. j-1
-  T cv3 = 0, cv2 = T(fvL(x, oy - 5));                           // layer-nlay vc, rows j-3, j-2
-  double pb0y = 0, pb1y = 0, gb0y = 0, gb1y = 0;                // pkapb, gzb at k, k+1, row j-3
+  unsigned r = row_of(g, oy - 3) + xi;
+  T s3 = 0, s2 = 0, s1 = 0, s0 = T(ld<RO>(uk, r));  // ud(x, j-3 .. j)
+  T v0 = T(ld<RO>(vk, r)), v3 = 0;                  // vd(x, j), vd(x, j-3)
+  YLine<T, CON> lv;                                 // vd along y
+  lv.q0 = v0;
+  T q2 = 0, q1 = 0, q0 = 0;                         // divergence, rows j-2 .. j
+  T qs1 = 0, qs0 = 0;                               // its x(+1) + x(-1), rows j-1, j
+  T e3 = 0, e2 = 0, e1 = 0;                         // its Laplacian, rows j-3 .. j-1
+  T es2 = 0, es1 = 0;                               // x(+1) + x(-1) of that, rows j-2, j-1
+  T dd3 = 0, dd2 = 0;                               // del^4 damping term, rows j-3, j-2
+  T w3 = 0, w2 = 0, w1 = 0;                         // vorticity, rows j-3 .. j-1
+  T ws2 = 0, ws1 = 0;                               // its x(+1) + x(-1), rows j-2, j-1
+  YLine<T, CON> lt;                                 // inner x sweep of the vorticity along y (newest row j-1)
+  T fw1 = 0, fw0 = 0;                               // the vorticity's piecewise-constant y flux at interfaces j-3, j-2
+  T ke3 = 0, ke2 = 0;                               // kinetic energy, rows j-3, j-2
+  T lp4 = 0, lp3 = 0, lp2 = 0;                      // Laplacian of the vorticity, rows j-4 .. j-2
+  T cu3 = 0, cu2 = T(ld<RO>(uL, row_of(g, oy - 5) + xi)), cu1 = T(ld<RO>(uL, row_of(g, oy - 4) + xi));  // layer-nlay uc, rows j-3 .. j-1
+  T cv3 = 0, cv2 = T(ld<RO>(vL, row_of(g, oy - 5) + xi));  // layer-nlay vc, rows j-3, j-2
+  double pb0y = 0, pb1y = 0, gb0y = 0, gb1y = 0;    // pkapb, gzb at k, k+1, row j-3
   bool bad = false;
-  const int jend = min(oy + TYS, g.ny) + 3;
-  S sn_p = fud(x, oy - 2), vn_p = fvd(x, oy - 2);
-  C cu_p = fuL(x, oy - 3), cv_p = fvL(x, oy - 4);
+  const int jend = min(oy + tys, g.ny) + 3;
+  r = row_of(g, oy - 2) + xi;
+  S sn_p = ld<RO>(uk, r), vn_p = ld<RO>(vk, r);
+  C cu_p = ld<RO>(uL, row_of(g, oy - 3) + xi), cv_p = ld<RO>(vL, row_of(g, oy - 4) + xi);
+#pragma unroll MarchL<T, MK_DMOM>::unroll
   for (int j = oy - 2; j < jend; ++j) {
     // loads of rows j-2 (pressure terms) and j-3 (the update) issued before this row's work
-    const double pb0n = fpb0(x, j - 2), pb1n = fpb1(x, j - 2), gb0n = fgb0(x, j - 2), gb1n = fgb1(x, j - 2);
-    const C svc_r = fvc(x, j - 3), suc_r = fuc(x, j - 3);
-    const S uo_r = fud(x, j - 3), vo_r = fvd(x, j - 3);
+    const int y = j - 3;
+    r = row_of(g, j - 2) + xi;
+    const double pb0n = ld<RO>(pba, r), pb1n = ld<RO>(pbb, r), gb0n = ld<RO>(gba, r), gb1n = ld<RO>(gbb, r);
+    const unsigned oi = row_of(g, y) + xi;
+    const C svc_r = ld<RO>(vcK, oi), suc_r = ld<RO>(ucK, oi);
+    S uo_r = 0, vo_r = 0;  // the state values of row y (the update in the state's type)
+    if constexpr (!SAME) {
+      uo_r = ld<RO>(uk, oi);
+      vo_r = ld<RO>(vk, oi);
+    }
     // ---- row j inputs; vorticity of row j-1 (:659-663), divergence of row j (:682-685)
     const T sn = T(sn_p), vn = T(vn_p);
     const C cu_c = cu_p, cv_c = cv_p;
-    sn_p = fud(x, j + 1);
-    vn_p = fvd(x, j + 1);
-    cu_p = fuL(x, j);
-    cv_p = fvL(x, j - 1);
+    r = row_of(g, j + 1) + xi;
+    sn_p = ld<RO>(uk, r);
+    vn_p = ld<RO>(vk, r);
+    cu_p = ld<RO>(uL, row_of(g, j) + xi);
+    cv_p = ld<RO>(vL, row_of(g, j - 1) + xi);
     const T vorn = fmadd(shfl_dn(v0, 1) - v0, rdx, fmadd(-(sn - s0), rdy, f));
     const T dvn = fmadd(rdy, vn - v0, rdx * (sn - shfl_up(sn, 1)));
-    s2 = s1; s1 = s0; s0 = sn;
-    v3 = v2; v2 = v1; v1 = v0; v0 = vn;
-    w4 = w3; w3 = w2; w2 = w1; w1 = vorn;
+    s3 = s2; s2 = s1; s1 = s0; s0 = sn;
+    v3 = lv.q2;
+    v0 = vn;
+    w3 = w2; w2 = w1; w1 = vorn;
     q2 = q1; q1 = q0; q0 = dvn;
+    qs1 = qs0; qs0 = shfl_dn(dvn, 1) + shfl_up(dvn, 1);
     cu3 = cu2; cu2 = cu1; cu1 = T(cu_c);
     cv3 = cv2; cv2 = T(cv_c);
-    // monotone slope of vd at row j-1, its edges at row j-2 (:870-911)
-    mv3 = mv2; mv2 = mv1; mv1 = slope_v(v2, v1, v0);
-    lv3 = lv2; rv3 = rv2;
-    edges_v<T, CON>(v3, v2, v1, mv3, mv2, mv1, lv2, rv2);
+    // vd's slope at row j-1, its edges at row j-2 (:870-911)
+    lv.push(vn);
     // del^2 of the divergence at row j-1 (:688-692), del^4 at row j-2 (:695-702)
     e3 = e2; e2 = e1;
-    e1 = fmadd(q0 + q2, rdy2, fmadd(shfl_dn(q1, 1) + shfl_up(q1, 1), rdx2, T(-2.) * q1 * rdxy));
+    e1 = fmadd(q0 + q2, rdy2, fmadd(qs1, rdx2, q1 * m2rdxy));
+    es2 = es1; es1 = shfl_dn(e1, 1) + shfl_up(e1, 1);
     dd3 = dd2;
-    dd2 = divdamp * (fmadd(e1 + e3, rdy2, fmadd(shfl_dn(e2, 1) + shfl_up(e2, 1), rdx2, T(-2.) * e2 * rdxy)));
+    dd2 = divdamp * (fmadd(e1 + e3, rdy2, fmadd(es2, rdx2, e2 * m2rdxy)));
     // inner x sweep of the vorticity at row j-1 with the layer-nlay Courant numbers (:708-722)
     {
       const T cR = shfl_dn(cu1, 1);
-      const T c0 = dtdx * cu1, c1 = dtdx * cR;
       const T den = T(1) / fmadd(-dtdx, cR - cu1, T(1));
       const T wl = shfl_up(w1, 1), wr = shfl_dn(w1, 1);  // every lane takes part in the shuffles
-      const T f0 = (c0 > T(0)) ? wl : w1;
-      const T f1 = (c1 > T(0)) ? w1 : wr;
-      t4 = t3; t3 = t2; t2 = t1;
-      t1 = T(.5) * fmadd(den, fmadd(-rA, f1 - f0, w1), w1);
+      ws2 = ws1; ws1 = wr + wl;
+      lt.push(inner_e(w1, (dtdx * cu1 > T(0)) ? wl : w1, (dtdx * cR > T(0)) ? w1 : wr, den, rA));
     }
-    mt4 = mt3; mt3 = mt2; mt2 = slope_v(t3, t2, t1);
-    lt4 = lt3; rt4 = rt3;
-    edges_v<T, CON>(t4, t3, t2, mt4, mt3, mt2, lt3, rt3);
-    // Laplacian of the vorticity at row j-2
+    // the vorticity's inner y sweep at the interface below row j-2, its Laplacian at row j-2
+    fw1 = fw0;
+    fw0 = (dtdx * cv2 > T(0)) ? w3 : w2;
     lp4 = lp3; lp3 = lp2;
-    lp2 = fmadd(w1 + w3, rdy2, fmadd(shfl_dn(w2, 1) + shfl_up(w2, 1), rdx2, T(-2.) * w2 * rdxy));
+    lp2 = fmadd(w1 + w3, rdy2, fmadd(ws2, rdx2, w2 * m2rdxy));
     // kinetic energy of row j-2 with PPM_CONSTRAINED (:639-657) and the
     // layer-nlay B-grid winds (:441-444)
     {
       const T ubL = T(.5) * (cu2 + cu3);
       const T vbL = T(.5) * (cv2 + shfl_up(cv2, 1));
-      const T fy = flux_con_v(dtdy * vbL, v3, v2, lv3, rv3, lv2, rv2);
-      const T kv = vbL * fy;
-      const T sl = shfl_up(s2, 1), sr = shfl_dn(s2, 1);
-      const T mux = slope_v(sl, s2, sr);
-      T lux, rux;
-      edges_v<T, CON>(sl, s2, sr, shfl_up(mux, 1), mux, shfl_dn(mux, 1), lux, rux);
-      const T fx = flux_con_v(dtdx * ubL, sl, s2, shfl_up(lux, 1), shfl_up(rux, 1), lux, rux);
+      const T kv = vbL * lv.flux(dtdy * vbL);
+      const T fx = xline_flux<T, CON>(s2, dtdx * ubL);
       ke3 = ke2;
       ke2 = T(.5) * fmadd(ubL, fx, kv);
     }
-    const int y = j - 3;
     if (y >= oy) {
-      // ---- row y: inner y sweep of the vorticity (:744-753), its x slopes and
-      // edges, the updates of ud, vd (:724-738, 755-769) with the B-grid PGF
-      T tv;
-      {
-        const T c0 = dtdx * cv3, c1 = dtdx * cv2;
-        const T den = T(1) / fmadd(-dtdy, cv2 - cv3, T(1));
-        const T f0 = (c0 > T(0)) ? w4 : w3;
-        const T f1 = (c1 > T(0)) ? w3 : w2;
-        tv = T(.5) * fmadd(den, fmadd(-rA, f1 - f0, w3), w3);
-      }
-      const T tl = shfl_up(tv, 1), tr = shfl_dn(tv, 1);
-      const T mtv = slope_v(tl, tv, tr);
-      T ltv, rtv;
-      edges_v<T, CON>(tl, tv, tr, shfl_up(mtv, 1), mtv, shfl_dn(mtv, 1), ltv, rtv);
-      const T fx = flux_con_v(dtdx * cu3, tl, tv, shfl_up(ltv, 1), shfl_up(rtv, 1), ltv, rtv);
-      const T fy = flux_con_v(dtdx * cv3, t4, t3, lt4, rt4, lt3, rt3);
+      // ---- row y: inner y sweep of the vorticity (:744-753), its x sweep, the
+      // updates of ud, vd (:724-738, 755-769) with the B-grid PGF
+      const T den = T(1) / fmadd(-dtdy, cv2 - cv3, T(1));
+      const T tv = inner_e(w3, fw1, fw0, den, rA);
+      const T fx = xline_flux<T, CON>(tv, dtdx * cu3);
+      const T fy = lt.flux(dtdx * cv3);
       const T ke_r = shfl_dn(ke3, 1), dd_r = shfl_dn(dd3, 1), lp_l = shfl_up(lp3, 1);
       const double pb0r = shfl_dn(pb0y, 1), pb1r = shfl_dn(pb1y, 1), gb0r = shfl_dn(gb0y, 1), gb1r = shfl_dn(gb1y, 1);
       if (out_lane && y < g.ny) {
         const double pgx = ((pb0r - pb1y) * (gb0y - gb1r) + (pb0y - pb1r) * (gb1y - gb0r)) / (pb0r - pb1y + pb0y - pb1r);
         const double pgy = ((pb0n - pb1y) * (gb0y - gb1n) + (pb0y - pb1n) * (gb1y - gb0n)) / (pb0n - pb1y + pb0y - pb1n);
-        const long long o = g.at(x, y, k);
         const T svc = T(svc_r), suc = T(suc_r);
         S u, v;
-        if constexpr (std::is_same_v<S, T>) {  // the reference's operations, in order
-          u = uo_r + dt * (svc * fy + vdy * (lp3 - lp4)) - dtdx * (ke_r - ke3 - dd_r + dd3 - T(pgx));
-          v = vo_r - dt * (suc * fx + vdx * (lp3 - lp_l)) - dtdy * (ke2 - ke3 - dd2 + dd3 - T(pgy));
+        if constexpr (SAME) {  // the reference's operations, in order
+          u = s3 + dt * (svc * fy + vdy * (lp3 - lp4)) - dtdx * (ke_r - ke3 - dd_r + dd3 - T(pgx));
+          v = v3 - dt * (suc * fx + vdx * (lp3 - lp_l)) - dtdy * (ke2 - ke3 - dd2 + dd3 - T(pgy));
         } else {  // the tendency in the sweep type added to the state's type
           const T du = fmadd(-dtdx, ke_r - ke3 - dd_r + dd3 - T(pgx), dt * fmadd(vdy, lp3 - lp4, svc * fy));
           const T dv = fmadd(-dtdy, ke2 - ke3 - dd2 + dd3 - T(pgy), -dt * fmadd(vdx, lp3 - lp_l, suc * fx));
           u = uo_r + S(du);
           v = vo_r + S(dv);
         }
-        udo[o] = u;
-        vdo[o] = v;
+        udo[kS + oi] = u;
+        vdo[kS + oi] = v;
         bad = bad || !(finite_(u) && finite_(v));
       }
     }
@@ -704,13 +794,14 @@ __device__ __forceinline__ void d_mom_strip(Geom g, Consts c, const S* ud,
 
 // one warp per strip: blockIdx.x * MWARPS + warp across x, blockIdx.y
 // across y, blockIdx.z the layer
-template <typename T, int TYS, typename S, typename C>
-__global__ void __launch_bounds__(MW * MWARPS, ATM_MARCH_MINB) k_d_mom_m(Geom g, Consts c, const S* __restrict__ ud,
+template <typename T, typename S, typename C>
+__global__ void __launch_bounds__(MW * MWARPS, MarchL<T, MK_DMOM>::min_blocks) k_d_mom_m(Geom g, Consts c, const S* __restrict__ ud,
                                                           const S* __restrict__ vd, const C* __restrict__ uc,
                                                           const C* __restrict__ vc, const double* __restrict__ pkapb,
                                                           const double* __restrict__ gzb, S* __restrict__ udo,
-                                                          S* __restrict__ vdo, int* nonfinite) {
-  d_mom_strip<T, TYS, S, C>(g, c, ud, vd, uc, vc, pkapb, gzb, udo, vdo, nonfinite, blockIdx.x * MWARPS + (threadIdx.x >> 5), blockIdx.y, blockIdx.z);
+                                                          S* __restrict__ vdo, int* nonfinite, int tys) {
+  d_mom_strip<T, S, C>(g, c, ud, vd, uc, vc, pkapb, gzb, udo, vdo, nonfinite,
+                       blockIdx.x * MWARPS + (threadIdx.x >> 5), blockIdx.y, blockIdx.z, tys);
 }
 
 }  // namespace atm

@@ -4,7 +4,6 @@
 // vertical remap and the global mass sum stay in FP64.
 #define ATM_FORM_T float
 #define ATM_OPS_NAME ops_mixed
-#define ATM_MARCH_SWEEPS 1  // the four sweeps as column-marching kernels
 #include "atm_launch.cuh"
 
 // ---- the persistent ensemble kernel of the mixed form (atm_ensemble.cuh)

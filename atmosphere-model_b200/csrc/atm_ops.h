@@ -13,20 +13,19 @@ namespace atm {
 struct Ops {
   int elem;     // bytes of an element of the prognostic state (dp, pt, ud, vd)
   int cg_elem;  // bytes of an element of the C-grid fields (dpc, ptc, uc, vc)
-  cudaError_t (*setup)();
   // C- or D-grid mass/potential-temperature sweep of every layer
   cudaError_t (*mass)(const Geom&, const Consts&, const void* dp, const void* pt, const void* u, const void* v,
-                      const double* heat, void* dpo, void* pto, int lo, int hi, int* nonfinite, int* timeout,
-                      bool cgrid, cudaStream_t);
+                      const double* heat, void* dpo, void* pto, int lo, int hi, int* nonfinite, bool cgrid,
+                      cudaStream_t);
   // plev/pkap/gz columns over [lo, n-1+hi]^2 from dp, pt of element size es
   cudaError_t (*column)(const Geom&, const Consts&, const void* dpl, const void* ptl, int es, double* pkap,
                         double* gz, int lo, int hi, double* plev, cudaStream_t);
   cudaError_t (*heating)(const Geom&, const Consts&, const void* dpl, int es, const double* net_flux, double* heat,
                          cudaStream_t);
   cudaError_t (*c_mom)(const Geom&, const Consts&, const void* ud, const void* vd, const double* pkap,
-                       const double* gz, void* uc, void* vc, int* timeout, cudaStream_t);
+                       const double* gz, void* uc, void* vc, cudaStream_t);
   cudaError_t (*d_mom)(const Geom&, const Consts&, const void* ud, const void* vd, const void* uc, const void* vc,
-                       const double* pkapb, const double* gzb, void* udo, void* vdo, int* nonfinite, int* timeout,
+                       const double* pkapb, const double* gzb, void* udo, void* vdo, int* nonfinite,
                        cudaStream_t);
   // periodic halo fill (copy = false) or ring copy src -> f (copy = true) of
   // nf state fields (ring) or C-grid fields (ring_cg)

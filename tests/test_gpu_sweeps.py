@@ -1,0 +1,49 @@
+"""The marching sweeps at the edges of their strips (26 output columns a warp,
+four warps a block, 4 to 128 output rows), bit for bit against the oracle: one
+step on smooth and on rough fields, whose slopes switch every limiter and the
+positivity filter."""
+import numpy as np
+import pytest
+
+from atmdyn import ic, Dycore
+import pyoracle
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = (('dp', pyoracle.DP), ('pt', pyoracle.PT), ('ud', pyoracle.UD), ('vd', pyoracle.VD))
+
+
+def rough(nx, ny, nlay, seed):
+    """Log-normal thickness and potential temperature (ratios of neighbours up
+    to about a hundred), winds of both signs and some exact ties."""
+    st = ic.bubble_case(nx, ny, nlay, 50e3, 50e3, seed=seed)
+    rng = np.random.default_rng(seed)
+    st.dp = st.dp * np.exp(rng.normal(0, 1.2, st.dp.shape))
+    st.pt = st.pt * np.exp(rng.normal(0, 1.2, st.pt.shape))
+    st.u = np.round(rng.normal(0, 15.0, st.u.shape), 0)
+    st.v = rng.normal(0, 15.0, st.v.shape)
+    return st
+
+
+# nx, ny around the strip widths (104 columns a block, halo rows and columns
+# 2-3 wide), the smallest domain, and one tall enough for 128-row strips
+SIZES = [(7, 7, 3), (26, 33, 5), (27, 8, 4), (100, 9, 3), (105, 131, 3), (416, 270, 24)]
+
+
+@pytest.mark.parametrize('nx,ny,nlay', SIZES)
+@pytest.mark.parametrize('fields', ['smooth', 'rough'])
+def test_step_bit_exact(nx, ny, nlay, fields):
+    st = rough(nx, ny, nlay, nx) if fields == 'rough' else ic.jet_case(nx, ny, nlay, 400e3, 400e3, width=900e3, seed=ny)
+    dt = 20.0 if fields == 'rough' else 60.0
+    g, o = Dycore(st), pyoracle.OracleModel(st, threads=8)
+    for a in (g, o):
+        a.cgrid_step(dt / 2)
+        a.cgrid_halo()
+    for name, f in (('dpc', pyoracle.DPC), ('ptc', pyoracle.PTC), ('uc', pyoracle.UC), ('vc', pyoracle.VC)):
+        np.testing.assert_array_equal(g.get(name, halo=True), o.get(f, halo=True), err_msg=name)
+    for a in (g, o):
+        a.dgrid_step(dt)
+        a.dgrid_halo()
+    for name, f in FIELDS:
+        np.testing.assert_array_equal(g.get(name, halo=True), o.get(f, halo=True), err_msg=name)
+    g.close()
