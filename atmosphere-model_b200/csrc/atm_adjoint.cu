@@ -1,122 +1,114 @@
-// Launchers of the FP64 adjoint kernels (atm_adjoint.cuh).  Compiled with
-// --fmad=false like the FP64 form: the adjoint kernels recompute the
-// forward's intermediates with the forward's exact operations, so every
+// Launchers of the FP64 adjoint kernels (atm_adj_march.cuh, atm_adjoint.cuh).
+// Compiled with --fmad=false like the FP64 form: the adjoint kernels recompute
+// the forward's intermediates with the forward's exact operations, so every
 // limiter and upwind branch is taken as in the forward step.
+#include "atm_adj_march.cuh"
 #include "atm_adjoint.cuh"
 #include "atm_ops.h"
-#include "atm_tmap.h"
 
 namespace atm {
 namespace {
 
-// tiles of the adjoints, measured: C-grid mass TXA x TYC (3 CTAs per SM),
-// D-grid mass TXA x TYA (2 CTAs per SM; 32 x 4 is no faster there), the
-// momentum adjoints TXA x TYM
-constexpr int TXA = 32, TYC = 4, TYA = 8, TYM = 4;
-
-inline dim3 tiles_a(int lo, int hi, const Geom& g, int ty) {
-  int w = g.nx - lo + hi, h = g.ny - lo + hi;
-  return dim3((w + TXA - 1) / TXA, (h + ty - 1) / ty, g.L);
+// grid of a marching reverse over w columns (out a warp) and h rows in strips of tys
+inline dim3 adj_strips(int w, int h, int layers, int out, int tys) {
+  return dim3((w + out * MWARPS - 1) / (out * MWARPS), (h + tys - 1) / tys, layers);
 }
 
-template <typename K>
-cudaError_t smem_attr(K kernel, size_t bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+// strip height of a marching reverse with `warm` rows beside the strip's own,
+// as strip_rows of atm_launch.cuh
+inline int adj_rows(int w, int h, int layers, int out, int warm) {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    sms = 148;
+  const long long slots = (long long)sms * 3;
+  int best = 8;
+  long long cost = -1;
+  for (int r = 128; r >= 4; r >>= 1) {
+    const dim3 b = adj_strips(w, h, layers, out, r);
+    const long long t = (((long long)b.x * b.y * b.z + slots - 1) / slots) * (min(r, h) + warm);
+    if (cost < 0 || t < cost) {
+      cost = t;
+      best = r;
+    }
+  }
+  return best;
 }
 
 }  // namespace
 
-cudaError_t adj_setup() {
-  cudaError_t e;
-  if ((e = smem_attr(k_mass_adj1<TXA, TYC, true>, MassAdj1L<TXA, TYC, true>::bytes))) return e;
-  if ((e = smem_attr(k_mass_adj<TXA, TYA, false, true>, MassAdjBL<TXA, TYA, false>::bytes))) return e;
-  if ((e = smem_attr(k_mass_adj<TXA, TYA, false, false>, MassAdjBL<TXA, TYA, false>::bytes))) return e;
-  if ((e = smem_attr(k_c_mom_adj<TXA, TYM>, CMomAdjL<TXA, TYM>::bytes))) return e;
-  if ((e = smem_attr(k_d_mom_adj_ke<TXA, TYM>, DMomKeAdjL<TXA, TYM>::bytes))) return e;
-  if ((e = smem_attr(k_d_mom_adj_vf<TXA, TYM>, DMomVfAdjL<TXA, TYM>::bytes))) return e;
-  return cudaSuccess;
-}
-
 cudaError_t adj_mass(const Geom& g, const Consts& c, const double* dp, const double* pt, const double* u,
                      const double* v, const double* dpo, const double* pto, const double* lam_dpo,
                      const double* lam_pto, double* lam_dp, double* lam_pt, double* lam_u, double* lam_v, int lo,
-                     int hi, int* timeout, bool cgrid, cudaStream_t s, int parts) {
-  CUtensorMap md, mp, mu, mv;
-  cudaError_t e;
-  if (cgrid) {  // one kernel (the update recomputed from the fluxes)
-    using Lay = MassL<double, TXA, TYC, true>;
-    if ((e = tmap(dp, 8, g, g.L, Lay::WD, Lay::HD, &md)) || (e = tmap(pt, 8, g, g.L, Lay::WD, Lay::HD, &mp)) ||
-        (e = tmap(u, 8, g, g.L, Lay::WU, Lay::HU, &mu)) || (e = tmap(v, 8, g, g.L, Lay::WV, Lay::HV, &mv)))
-      return e;
-    (void)dpo;
-    (void)pto;
-    k_mass_adj1<TXA, TYC, true><<<tiles_a(lo, hi, g, TYC), NTA, MassAdj1L<TXA, TYC, true>::bytes, s>>>(
-        md, mp, mu, mv, g, c, lam_dpo, lam_pto, lam_dp, lam_pt, lam_u, lam_v, lo, hi, timeout);
-  } else {  // the x branch (with the direct terms) and the y branch, both adding into the same global adjoints
-    using Lay = MassL<double, TXA, TYA, false>;
-    constexpr size_t bytes = MassAdjBL<TXA, TYA, false>::bytes;
-    if ((e = tmap(dp, 8, g, g.L, Lay::WD, Lay::HD, &md)) || (e = tmap(pt, 8, g, g.L, Lay::WD, Lay::HD, &mp)) ||
-        (e = tmap(u, 8, g, g.L, Lay::WU, Lay::HU, &mu)) || (e = tmap(v, 8, g, g.L, Lay::WV, Lay::HV, &mv)))
-      return e;
-    const dim3 grid = tiles_a(lo, hi, g, TYA);
-    if (parts & 1)
-      k_mass_adj<TXA, TYA, false, true><<<grid, NTA, bytes, s>>>(md, mp, mu, mv, g, c, dpo, pto, lam_dpo, lam_pto,
-                                                                  lam_dp, lam_pt, lam_u, lam_v, lo, hi, timeout);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if (parts & 2)
-      k_mass_adj<TXA, TYA, false, false><<<grid, NTA, bytes, s>>>(md, mp, mu, mv, g, c, dpo, pto, lam_dpo, lam_pto,
-                                                                   lam_dp, lam_pt, lam_u, lam_v, lo, hi, timeout);
+                     int hi, bool cgrid, cudaStream_t s, int part) {
+  const MassAdjArgs a{dp, pt, u, v, dpo, pto, lam_dpo, lam_pto, lam_dp, lam_pt, lam_u, lam_v};
+  const int w = g.nx - lo + hi, h = g.ny - lo + hi;
+  if (part == 1) {
+    const int rows = adj_rows(w, h, g.L, MOUT, 4);
+    const dim3 grid = adj_strips(w, h, g.L, MOUT, rows);
+    if (cgrid) k_mass_adj_x<true><<<grid, MW * MWARPS, 0, s>>>(g, c, a, lo, hi, rows);
+    else k_mass_adj_x<false><<<grid, MW * MWARPS, 0, s>>>(g, c, a, lo, hi, rows);
+  } else {
+    const int rows = adj_rows(w, h, g.L, YOUT_MASS, 11);
+    const dim3 grid = adj_strips(w, h, g.L, YOUT_MASS, rows);
+    if (cgrid) k_mass_adj_y<true><<<grid, MW * MWARPS, 0, s>>>(g, c, a, lo, hi, rows);
+    else k_mass_adj_y<false><<<grid, MW * MWARPS, 0, s>>>(g, c, a, lo, hi, rows);
   }
   return cudaGetLastError();
 }
 
-cudaError_t adj_c_mom(const Geom& g, const Consts& c, const double* ud, const double* vd, const double* pkap,
-                      const double* gz, const double* lam_uc, const double* lam_vc, double* lam_ud, double* lam_vd,
-                      double* lam_pk, double* lam_gz, int* timeout, cudaStream_t s) {
-  using Lay = CMomL<double, TXA, TYM>;
-  CUtensorMap mu, mv, muL, mvL, mpk, mgz;
+cudaError_t adj_c_mom(const Geom& g, const Consts& c, const double* ud, const double* vd, const double* lam_uc,
+                      const double* lam_vc, double* lam_ud, double* lam_vd, double* lam_w, double* lam_uc1,
+                      double* lam_vc1, double* lam_nlay, cudaStream_t s) {
+  const CMomAdjArgs a{ud, vd, lam_uc, lam_vc, lam_ud, lam_vd, lam_w, lam_uc1, lam_vc1, lam_nlay, lam_nlay + g.S};
   cudaError_t e;
-  if ((e = tmap(ud, 8, g, g.L, Lay::WU, Lay::HU, &mu)) || (e = tmap(vd, 8, g, g.L, Lay::WV, Lay::HV, &mv)) ||
-      (e = tmap(ud, 8, g, g.L, Lay::WL, Lay::HL, &muL)) || (e = tmap(vd, 8, g, g.L, Lay::WL, Lay::HL, &mvL)) ||
-      (e = tmap(pkap, 8, g, g.L + 1, Lay::WP, Lay::HP, &mpk)) || (e = tmap(gz, 8, g, g.L + 1, Lay::WP, Lay::HP, &mgz)))
+  const size_t lay = (size_t)g.S * g.L * 8;
+  if ((e = cudaMemsetAsync(lam_w, 0, lay, s)) || (e = cudaMemsetAsync(lam_uc1, 0, lay, s)) ||
+      (e = cudaMemsetAsync(lam_vc1, 0, lay, s)) || (e = cudaMemsetAsync(lam_nlay, 0, (size_t)g.S * 2 * 8, s)))
     return e;
-  k_c_mom_adj<TXA, TYM><<<tiles_a(0, 0, g, TYM), NTA, CMomAdjL<TXA, TYM>::bytes, s>>>(
-      mu, mv, muL, mvL, mpk, mgz, g, c, lam_uc, lam_vc, lam_ud, lam_vd, lam_pk, lam_gz, timeout);
+  int rows = adj_rows(g.nx, g.ny, g.L, MOUT, 3);
+  k_c_mom_adj_x<<<adj_strips(g.nx, g.ny, g.L, MOUT, rows), MW * MWARPS, 0, s>>>(g, c, a, rows);
+  rows = adj_rows(g.nx + 1, g.ny + 1, g.L, YOUT_CMOM, 10);
+  k_c_mom_adj_y<<<adj_strips(g.nx + 1, g.ny + 1, g.L, YOUT_CMOM, rows), MW * MWARPS, 0, s>>>(g, c, a, rows);
+  k_c_mom_adj_fin<<<dim3((g.nx + 8 + 127) / 128, g.ny + 8, g.L), 128, 0, s>>>(g, c, a);
   return cudaGetLastError();
 }
 
 cudaError_t adj_d_mom(const Geom& g, const Consts& c, const double* ud, const double* vd, const double* uc,
-                      const double* vc, const double* pkapb, const double* gzb, const double* lam_udo,
-                      const double* lam_vdo, double* lam_ud, double* lam_vd, double* lam_uc, double* lam_vc,
-                      double* lam_pkb, double* lam_gzb, int* timeout, cudaStream_t s, int parts) {
-  using Lay = DMomL<double, TXA, TYM>;
-  CUtensorMap mu, mv, muL, mvL, muc, mvc, mpb, mgb;
-  cudaError_t e;
-  if ((e = tmap(ud, 8, g, g.L, Lay::WU, Lay::HU, &mu)) || (e = tmap(vd, 8, g, g.L, Lay::WU, Lay::HU, &mv)) ||
-      (e = tmap(uc, 8, g, g.L, Lay::WUL, Lay::HUL, &muL)) || (e = tmap(vc, 8, g, g.L, Lay::WVL, Lay::HVL, &mvL)) ||
-      (e = tmap(uc, 8, g, g.L, Lay::WC, Lay::HC, &muc)) || (e = tmap(vc, 8, g, g.L, Lay::WC, Lay::HC, &mvc)) ||
-      (e = tmap(pkapb, 8, g, g.L + 1, Lay::WP, Lay::HP, &mpb)) || (e = tmap(gzb, 8, g, g.L + 1, Lay::WP, Lay::HP, &mgb)))
-    return e;
-  // the kinetic-energy chain and the rest, both adding into the same
-  // global adjoints
-  if (parts & 1)
-    k_d_mom_adj_ke<TXA, TYM><<<tiles_a(0, 0, g, TYM), NTA, DMomKeAdjL<TXA, TYM>::bytes, s>>>(
-        mu, mv, muL, mvL, g, c, lam_udo, lam_vdo, lam_ud, lam_vd, lam_uc, lam_vc, timeout);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if (parts & 2)
-    k_d_mom_adj_vf<TXA, TYM><<<tiles_a(0, 0, g, TYM), NTA, DMomVfAdjL<TXA, TYM>::bytes, s>>>(
-        mu, mv, muL, mvL, muc, mvc, mpb, mgb, g, c, lam_udo, lam_vdo, lam_ud, lam_vd, lam_uc, lam_vc, lam_pkb,
-        lam_gzb, timeout);
+                      const double* vc, const double* lam_udo, const double* lam_vdo, double* lam_ud, double* lam_vd,
+                      double* lam_uc, double* lam_vc, cudaStream_t s, int part) {
+  const DMomAdjArgs a{ud, vd, uc, vc, lam_udo, lam_vdo, lam_ud, lam_vd, lam_uc, lam_vc};
+  if (part == 1) {
+    const int rows = adj_rows(g.nx, g.ny, g.L, MOUT, 6);
+    k_d_mom_adj_x<<<adj_strips(g.nx, g.ny, g.L, MOUT, rows), MW * MWARPS, 0, s>>>(g, c, a, rows);
+  } else {
+    const int rows = adj_rows(g.nx + 1, g.ny + 1, g.L, YOUT_DMOM, 11);
+    k_d_mom_adj_y<<<adj_strips(g.nx + 1, g.ny + 1, g.L, YOUT_DMOM, rows), MW * MWARPS, 0, s>>>(g, c, a, rows);
+  }
   return cudaGetLastError();
 }
 
-cudaError_t adj_column(const Geom& g, const Consts& c, const double* dp, const double* pt, const double* lam_pk,
-                       const double* lam_gz, double* lam_dp, double* lam_pt, int lo, int hi, cudaStream_t s) {
-  const int n = (g.nx - lo + hi) * (g.ny - lo + hi);
-  const int nb = (n + 127) / 128;
-  if (g.L <= 32) k_column_adj<32><<<nb, 128, 0, s>>>(g, c, dp, pt, lam_pk, lam_gz, lam_dp, lam_pt, lo, hi);
-  else if (g.L <= 64) k_column_adj<64><<<nb, 128, 0, s>>>(g, c, dp, pt, lam_pk, lam_gz, lam_dp, lam_pt, lo, hi);
-  else k_column_adj<MAX_LAYERS><<<nb, 128, 0, s>>>(g, c, dp, pt, lam_pk, lam_gz, lam_dp, lam_pt, lo, hi);
+cudaError_t adj_c_column(const Geom& g, const Consts& c, const double* dp, const double* pt, const double* pkap,
+                         const double* gz, const double* lam_uc, const double* lam_vc, double* tmp, double* lam_dp,
+                         double* lam_pt, cudaStream_t s) {
+  const int n = (g.nx + 4) * (g.ny + 4);
+  k_column_adj<true><<<(n + 127) / 128, 128, 0, s>>>(g, c, dp, pt, pkap, gz, lam_uc, lam_vc, tmp, lam_dp, lam_pt);
+  return cudaGetLastError();
+}
+
+cudaError_t adj_d_column(const Geom& g, const Consts& c, const double* dp, const double* pt, const double* lam_pk,
+                         const double* lam_gz, double* tmp, double* lam_dp, double* lam_pt, cudaStream_t s) {
+  const int n = (g.nx + 4) * (g.ny + 4);
+  k_column_adj<false><<<(n + 127) / 128, 128, 0, s>>>(g, c, dp, pt, nullptr, nullptr, lam_pk, lam_gz, tmp, lam_dp,
+                                                      lam_pt);
+  return cudaGetLastError();
+}
+
+cudaError_t adj_pgf_corners(const Geom& g, const Consts& c, const double* pkapb, const double* gzb,
+                            const double* lam_udo, const double* lam_vdo, double* lam_pkb, double* lam_gzb,
+                            cudaStream_t s) {
+  const int n = (g.nx + 1) * (g.ny + 1);
+  k_pgf_adj_corners<<<dim3((n + 127) / 128, (g.L + PGF_CHUNK - 1) / PGF_CHUNK), 128, 0, s>>>(
+      g, c, pkapb, gzb, lam_udo, lam_vdo, lam_pkb, lam_gzb);
   return cudaGetLastError();
 }
 

@@ -219,14 +219,14 @@ cudaError_t d2h_pitched(atm_ctx* c, double* host, const double* dev, int K) {
 const char* const STAGE_NAMES[] = {"c_mass",  "c_column", "c_mom",        "c_halo",      "d_ring",
                                    "d_mass",  "d_column", "d_corners",    "d_mom",       "remap_ring",
                                    "remap_winds", "remap_energy", "d_halo", "heating", "check",
-                                   "adj_forward", "adj_remap", "adj_d_mom_ke", "adj_d_column", "adj_d_mass_x",
-                                   "adj_c_column", "adj_c_mom", "adj_c_mass", "adj_halo",
-                                   "phys_tend", "phys_apply", "phys_halo", "adj_d_mom_vf", "adj_d_mass_y",
-                                   "radiation", "radiation_halo"};
-constexpr int NSTAGE = 31;
+                                   "adj_forward", "adj_remap", "adj_d_mom_x", "adj_d_column", "adj_d_mass_x",
+                                   "adj_c_column", "adj_c_mom", "adj_c_mass_x", "adj_halo",
+                                   "phys_tend", "phys_apply", "phys_halo", "adj_d_mom_y", "adj_d_mass_y",
+                                   "radiation", "radiation_halo", "adj_c_mass_y"};
+constexpr int NSTAGE = 32;
 enum { S_CMASS, S_CCOL, S_CMOM, S_CHALO, S_DRING, S_DMASS, S_DCOL, S_DCORN, S_DMOM, S_RRING, S_RWIND, S_RENER,
        S_DHALO, S_HEAT, S_CHECK, S_AFWD, S_ARMP, S_ADMOM, S_ADCOL, S_ADMASS, S_ACCOL, S_ACMOM, S_ACMASS, S_AHALO,
-       S_PHYS_TEND, S_PHYS_APPLY, S_PHYS_HALO, S_ADMOM_VF, S_ADMASS_Y, S_RAD, S_RAD_HALO };
+       S_PHYS_TEND, S_PHYS_APPLY, S_PHYS_HALO, S_ADMOM_Y, S_ADMASS_Y, S_RAD, S_RAD_HALO, S_ACMASS_Y };
 
 // Brackets one stage (one kernel launch unless noted) with CUDA events on
 // the context's stream when profiling is on, and counts the launch.
@@ -682,7 +682,6 @@ int atm_check_stability(atm_ctx* ctx, int* stable) {
   }
   CK(cudaMemcpyAsync(ctx->h_status, ctx->status, sizeof(atm::Status), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  if (ctx->h_status->tma_timeout) return fail(ctx, ATM_ERR_CUDA, "a TMA tile load did not complete (wait limit)");
   int bad = !ctx->flag_valid ? ctx->h_status->nonfinite_check
                              : (ctx->remapped ? ctx->h_status->nonfinite_remap : ctx->h_status->nonfinite_step);
   *stable = bad ? 0 : 1;
@@ -877,27 +876,24 @@ int adj_c(atm_ctx* ctx, double dt_half, void* const* s, double* const* lin, cons
   const double* const* sd = (const double* const*)s;
   const double* const* cg = (const double* const*)cgf;
   {
-    Stage t(ctx, S_ACCOL, 2);
+    Stage t(ctx, S_ACCOL);
     CK(ctx->ops->column(g, k, cg[C_DPC], cg[C_PTC], ctx->ops->cg_elem, ctx->pkap, ctx->gz, -2, 2, nullptr,
                         ctx->stream));
-    CK(cudaMemsetAsync(ctx->lam_pk, 0, (size_t)g.S * (ctx->L + 1) * 8, ctx->stream));
-    CK(cudaMemsetAsync(ctx->lam_gz, 0, (size_t)g.S * (ctx->L + 1) * 8, ctx->stream));
   }
   {
-    Stage t(ctx, S_ACMOM);
-    CK(atm::adj_c_mom(g, k, sd[F_UD], sd[F_VD], ctx->pkap, ctx->gz, ctx->lam_cg[C_UC], ctx->lam_cg[C_VC], lin[F_UD],
-                      lin[F_VD], ctx->lam_pk, ctx->lam_gz, &ctx->status->tma_timeout, ctx->stream));
+    Stage t(ctx, S_ACMOM, 3);  // the fields of the D step's corners and of the remap serve as scratch
+    CK(atm::adj_c_mom(g, k, sd[F_UD], sd[F_VD], ctx->lam_cg[C_UC], ctx->lam_cg[C_VC], lin[F_UD], lin[F_VD],
+                      ctx->lam_gzb, ctx->lam_ur, ctx->lam_vr, ctx->lam_pkb, ctx->stream));
   }
   {
     Stage t(ctx, S_ACCOL);
-    CK(atm::adj_column(g, k, cg[C_DPC], cg[C_PTC], ctx->lam_pk, ctx->lam_gz, ctx->lam_cg[C_DPC], ctx->lam_cg[C_PTC], -2,
-                       2, ctx->stream));
+    CK(atm::adj_c_column(g, k, cg[C_DPC], cg[C_PTC], ctx->pkap, ctx->gz, ctx->lam_cg[C_UC], ctx->lam_cg[C_VC],
+                         ctx->stage, ctx->lam_cg[C_DPC], ctx->lam_cg[C_PTC], ctx->stream));
   }
-  {
-    Stage t(ctx, S_ACMASS);
+  for (int part = 1; part <= 2; ++part) {
+    Stage t(ctx, part == 1 ? S_ACMASS : S_ACMASS_Y);
     CK(atm::adj_mass(g, k, sd[F_DP], sd[F_PT], sd[F_UD], sd[F_VD], cg[C_DPC], cg[C_PTC], ctx->lam_cg[C_DPC],
-                     ctx->lam_cg[C_PTC], lin[F_DP],
-                     lin[F_PT], lin[F_UD], lin[F_VD], -2, 2, &ctx->status->tma_timeout, true, ctx->stream));
+                     ctx->lam_cg[C_PTC], lin[F_DP], lin[F_PT], lin[F_UD], lin[F_VD], -2, 2, true, ctx->stream, part));
   }
   return ATM_OK;
 }
@@ -911,30 +907,24 @@ int adj_d(atm_ctx* ctx, double dt, const void* const* so, const void* const* sn,
   const double* const* o = (const double* const*)so;
   const double* const* n = (const double* const*)sn;
   const double* const* cg = (const double* const*)cgf;
-  const size_t lev = (size_t)g.S * (ctx->L + 1) * 8;
-  CK(cudaMemsetAsync(ctx->lam_pk, 0, lev, ctx->stream));
-  CK(cudaMemsetAsync(ctx->lam_gz, 0, lev, ctx->stream));
-  CK(cudaMemsetAsync(ctx->lam_pkb, 0, lev, ctx->stream));
-  CK(cudaMemsetAsync(ctx->lam_gzb, 0, lev, ctx->stream));
-  // the kinetic-energy chain and the rest of the D-momentum reverse, each
-  // its own kernel and profiled stage
+  // each sweep's x and y branch is its own kernel and profiled stage
   for (int part = 1; part <= 2; ++part) {
-    Stage t(ctx, part == 1 ? S_ADMOM : S_ADMOM_VF);
-    CK(atm::adj_d_mom(g, k, o[F_UD], o[F_VD], cg[C_UC], cg[C_VC], ctx->pkapb, ctx->gzb, lout[F_UD], lout[F_VD],
-                      lin[F_UD], lin[F_VD], ctx->lam_cg[C_UC], ctx->lam_cg[C_VC], ctx->lam_pkb, ctx->lam_gzb,
-                      &ctx->status->tma_timeout, ctx->stream, part));
+    Stage t(ctx, part == 1 ? S_ADMOM : S_ADMOM_Y);
+    CK(atm::adj_d_mom(g, k, o[F_UD], o[F_VD], cg[C_UC], cg[C_VC], lout[F_UD], lout[F_VD], lin[F_UD], lin[F_VD],
+                      ctx->lam_cg[C_UC], ctx->lam_cg[C_VC], ctx->stream, part));
   }
   {
-    Stage t(ctx, S_ADCOL, 2);
+    Stage t(ctx, S_ADCOL, 3);
+    CK(atm::adj_pgf_corners(g, k, ctx->pkapb, ctx->gzb, lout[F_UD], lout[F_VD], ctx->lam_pkb, ctx->lam_gzb,
+                            ctx->stream));
     CK(atm::adj_corners(g, ctx->lam_pkb, ctx->lam_gzb, ctx->lam_pk, ctx->lam_gz, ctx->stream));
-    CK(atm::adj_column(g, k, n[F_DP], n[F_PT], ctx->lam_pk, ctx->lam_gz, lout[F_DP], lout[F_PT], -2, 2, ctx->stream));
+    CK(atm::adj_d_column(g, k, n[F_DP], n[F_PT], ctx->lam_pk, ctx->lam_gz, ctx->stage, lout[F_DP], lout[F_PT],
+                         ctx->stream));
   }
-  // the x and the y branch of the D-grid mass reverse
   for (int part = 1; part <= 2; ++part) {
     Stage t(ctx, part == 1 ? S_ADMASS : S_ADMASS_Y);
     CK(atm::adj_mass(g, k, o[F_DP], o[F_PT], cg[C_UC], cg[C_VC], n[F_DP], n[F_PT], lout[F_DP], lout[F_PT], lin[F_DP],
-                     lin[F_PT], ctx->lam_cg[C_UC], ctx->lam_cg[C_VC], -3, 3, &ctx->status->tma_timeout, false,
-                     ctx->stream, part));
+                     lin[F_PT], ctx->lam_cg[C_UC], ctx->lam_cg[C_VC], -3, 3, false, ctx->stream, part));
   }
   {
     Stage t(ctx, S_AHALO);
@@ -980,8 +970,6 @@ int atm_adj_enable(atm_ctx* ctx) {
   if (!ctx) return ATM_ERR_ARG;
   if (ctx->precision != ATM_FP64) return fail(ctx, ATM_ERR_UNSUPPORTED, "the adjoint is defined for the FP64 form");
   if (ctx->adj) return atm_adj_zero(ctx);
-  cudaError_t e = atm::adj_setup();
-  if (e != cudaSuccess) return cuda_fail(ctx, "adjoint kernel set-up", e);
   const size_t lay = (size_t)ctx->geo.S * ctx->L * 8, lev = (size_t)ctx->geo.S * (ctx->L + 1) * 8;
   bool ok = true;
   auto alloc = [&](double** p, size_t bytes) {

@@ -60,7 +60,6 @@ struct Status {
   int nonfinite_remap;  // ... or the vertical remap
   int nonfinite_check;  // standalone stability check
   int fallback_pairs;   // columns whose remap used the all-pairs search
-  int tma_timeout;      // a TMA tile load did not complete within its wait limit
   int radiation_range;  // a radiation table lookup left its table
 };
 
@@ -111,15 +110,5 @@ __device__ __forceinline__ void slopes(T qm, T q0, T qp, T& dqi, T& mono) {
   T dmin = q0 - mn3(qp, q0, qm);
   mono = cpsign(mn3(fab(dqi), dmin, dmax), dqi);
 }
-
-// A window of a 2-D shared-memory array addressed with absolute interior
-// coordinates (x, y) of the tile's region [x0, x0+w) x [y0, y0+h).
-template <typename T>
-struct Sm {
-  T* p;
-  int x0, y0, w;
-  __device__ __forceinline__ T& operator()(int x, int y) const { return p[(y - y0) * w + (x - x0)]; }
-  __device__ __forceinline__ T* ptr(int x, int y) const { return p + (y - y0) * w + (x - x0); }
-};
 
 }  // namespace atm

@@ -4,7 +4,6 @@
 #define ATM_FORM_T double
 #define ATM_OPS_NAME ops_fp64
 #include "atm_launch.cuh"
-#include "atm_tma.cuh"
 
 #ifndef ATM_CORNER_CHUNK
 #define ATM_CORNER_CHUNK 8
@@ -63,10 +62,44 @@ cudaError_t device_div_check(unsigned long long n, unsigned long long seed, unsi
   return cudaGetLastError();
 }
 
-// The bounded wait of the TMA loads, made to run out: one thread arms an
-// mbarrier for 16 bytes of transactions that no copy ever brings (no copy
-// is issued) and waits on it with mbar_wait's poll limit, as tma_fetch
-// does; it must come back with the failure recorded in *flag.
+// A bounded mbarrier wait, made to run out: one thread arms an mbarrier for 16
+// bytes of transactions that no copy ever brings (no copy is issued) and waits
+// on it with a poll limit; it must come back with the failure recorded in
+// *flag.
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ void fence_mbar_init() {
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
+               : "memory");
+}
+
+// wait for a phase of the barrier, at most max_iter polls of at most ~1 us
+// each; true on success
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, int max_iter) {
+  uint32_t done = 0;
+  for (int it = 0; it < max_iter; ++it) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(smem_u32(bar)), "r"(phase)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+
 static __global__ void k_wait_timeout(int max_polls, int* flag) {
   __shared__ __align__(8) uint64_t bar;
   if (threadIdx.x == 0) {

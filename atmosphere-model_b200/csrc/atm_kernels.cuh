@@ -15,19 +15,6 @@
 
 namespace atm {
 
-constexpr int NT = 256;  // threads per block of the tile kernels
-
-template <typename T>
-__device__ __forceinline__ Sm<T> carve(unsigned char*& p, int x0, int y0, int w, int h) {
-  Sm<T> s{reinterpret_cast<T*>(p), x0, y0, w};
-  p += ((size_t)w * h * sizeof(T) + 15) & ~(size_t)15;
-  return s;
-}
-template <typename T>
-__host__ __device__ constexpr size_t box_bytes(int w, int h) {
-  return ((size_t)w * h * sizeof(T) + 15) & ~(size_t)15;
-}
-
 // Raise a context's non-finite flag (bad values are rare: one atomic each).
 __device__ __forceinline__ void flag_nonfinite(int* flag, bool bad) {
   if (bad) atomicOr(flag, 1);

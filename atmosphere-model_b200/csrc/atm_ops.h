@@ -58,28 +58,35 @@ cudaError_t device_kappa_pow(const double* x, double* out, int n, cudaStream_t);
 
 // count of arguments where div_const<3>/<12> differs from IEEE division (tests)
 cudaError_t device_div_check(unsigned long long n, unsigned long long seed, unsigned long long* bad, cudaStream_t);
-// the TMA loads' bounded mbarrier wait on a barrier nothing completes: *flag = 1 when it gave up
+// a bounded mbarrier wait on a barrier nothing completes: *flag = 1 when it gave up
 cudaError_t device_wait_timeout(int max_polls, int* flag, cudaStream_t);
 
 // ---- FP64 adjoint (atm_adjoint.cu); lam_* are adjoint fields laid out like
 // the fields they belong to, accumulated with +=
-cudaError_t adj_setup();
-// dpo, pto: the new dp and pt the forward sweep wrote; parts (D grid): 1
-// the x branch, 2 the y branch, 3 both (the C grid is one kernel)
+// dpo, pto: the new dp and pt the forward sweep wrote; part: 1 the x branch,
+// 2 the y branch
 cudaError_t adj_mass(const Geom&, const Consts&, const double* dp, const double* pt, const double* u, const double* v,
                      const double* dpo, const double* pto, const double* lam_dpo, const double* lam_pto, double* lam_dp,
-                     double* lam_pt, double* lam_u, double* lam_v, int lo, int hi, int* timeout, bool cgrid,
-                     cudaStream_t, int parts = 3);
-cudaError_t adj_c_mom(const Geom&, const Consts&, const double* ud, const double* vd, const double* pkap,
-                      const double* gz, const double* lam_uc, const double* lam_vc, double* lam_ud, double* lam_vd,
-                      double* lam_pk, double* lam_gz, int* timeout, cudaStream_t);
-// parts: 1 the kinetic-energy chain, 2 the rest, 3 both
+                     double* lam_pt, double* lam_u, double* lam_v, int lo, int hi, bool cgrid, cudaStream_t, int part);
+// lam_w, lam_uc1, lam_vc1 (nlay levels), lam_nlay (2 levels): scratch
+cudaError_t adj_c_mom(const Geom&, const Consts&, const double* ud, const double* vd, const double* lam_uc,
+                      const double* lam_vc, double* lam_ud, double* lam_vd, double* lam_w, double* lam_uc1,
+                      double* lam_vc1, double* lam_nlay, cudaStream_t);
+// without the pressure-gradient force; part: 1 the x branch, 2 the y branch
 cudaError_t adj_d_mom(const Geom&, const Consts&, const double* ud, const double* vd, const double* uc,
-                      const double* vc, const double* pkapb, const double* gzb, const double* lam_udo,
-                      const double* lam_vdo, double* lam_ud, double* lam_vd, double* lam_uc, double* lam_vc,
-                      double* lam_pkb, double* lam_gzb, int* timeout, cudaStream_t, int parts = 3);
-cudaError_t adj_column(const Geom&, const Consts&, const double* dp, const double* pt, const double* lam_pk,
-                       const double* lam_gz, double* lam_dp, double* lam_pt, int lo, int hi, cudaStream_t);
+                      const double* vc, const double* lam_udo, const double* lam_vdo, double* lam_ud, double* lam_vd,
+                      double* lam_uc, double* lam_vc, cudaStream_t, int part);
+// lam_pkb (levels 1..nlay), lam_gzb = the D grid's pressure-gradient force reversed
+cudaError_t adj_pgf_corners(const Geom&, const Consts&, const double* pkapb, const double* gzb, const double* lam_udo,
+                            const double* lam_vdo, double* lam_pkb, double* lam_gzb, cudaStream_t);
+// columns over [-2, n+1]^2, on the C grid with the pressure-gradient force;
+// tmp: scratch of nlay + 1 levels
+cudaError_t adj_c_column(const Geom&, const Consts&, const double* dp, const double* pt, const double* pkap,
+                         const double* gz, const double* lam_uc, const double* lam_vc, double* tmp, double* lam_dp,
+                         double* lam_pt, cudaStream_t);
+cudaError_t adj_d_column(const Geom&, const Consts&, const double* dp, const double* pt, const double* lam_pk,
+                         const double* lam_gz, double* tmp, double* lam_dp, double* lam_pt, cudaStream_t);
+// lam_pk (levels 1..nlay), lam_gz (2..nlay+1) = the corner interpolation reversed
 cudaError_t adj_corners(const Geom&, const double* lam_pkb, const double* lam_gzb, double* lam_pk, double* lam_gz,
                         cudaStream_t);
 cudaError_t adj_ring_fold(const Geom&, double* const* f, int nf, int K, cudaStream_t);

@@ -571,18 +571,17 @@ def probe_radiation(args):
 # adjoints it reads, and a read and a write of every adjoint it adds into
 # (layer-nlay slabs excluded, as for the forward).
 ADJ_WORDS = {
-    'adj_c_mass': 14,    # dp, pt, ud, vd; lam dpc, ptc; += lam dp, pt, ud, vd
-    'adj_c_mom': 14,     # ud, vd, pkap, gz; lam uc, vc; += lam ud, vd, pkap, gz
-    'adj_d_mom_ke': 8,   # ud, vd; lam ud, vd (out); += lam ud, vd (in)
-    'adj_d_mom_vf': 20,  # ud, vd, uc, vc, pkapb, gzb; lam ud, vd (out); += lam ud, vd, uc, vc, pkapb, gzb
+    'adj_c_mass_x': 16,  # dp, pt, ud, vd, dpc, ptc; lam dpc, ptc; += lam dp, pt, ud, vd
+    'adj_c_mass_y': 16,
+    'adj_d_mom_x': 11,   # ud, vd, uc; lam ud, vd (out); += lam ud, vd, uc
+    'adj_d_mom_y': 11,   # ud, vd, vc; lam ud, vd (out); += lam ud, vd, vc
     'adj_d_mass_x': 16,  # dp, pt, uc, vc, new dp, pt; lam dp, pt (out); += lam dp, pt, uc, vc
     'adj_d_mass_y': 16,
 }
 # DRAM bytes per interior cell and launch of the adjoint kernels measured by
 # ncu (dram__bytes_read.sum + dram__bytes_write.sum, dense adjoint of the
 # jet at 512x512x32, scaled by cells)
-TRAFFIC_PER_CELL_ADJ = {'adj_c_mass': 113.3, 'adj_c_mom': 114.2, 'adj_d_mass_x': 130.9, 'adj_d_mass_y': 131.1,
-                        'adj_d_mom_ke': 64.7, 'adj_d_mom_vf': 165.2}
+TRAFFIC_PER_CELL_ADJ = {}
 
 
 def grad_leg(args, torch, barrier, max_over_ranks, world, peak, peak_kind):

@@ -102,6 +102,37 @@ def test_dgrid_step_dot_product():
     assert rel(lhs, rhs) <= TOL, (lhs, rhs)
 
 
+@pytest.mark.parametrize('nx,ny,nlay', [(7, 7, 3), (27, 9, 3), (31, 40, 4), (113, 13, 3), (121, 131, 3)])
+def test_strip_edges_dot_product(nx, ny, nlay):
+    """The C and D step together at the edges of the reverse kernels' strips
+    (26 to 30 columns a warp, four warps a block, 4 to 128 rows), on log-normal
+    thickness and potential temperature, whose slopes reach the positivity
+    filter and both sides of every limiter."""
+    st = generic_state(nx, ny, nlay, seed=nx)
+    rng = np.random.default_rng(ny)
+    st.dp = st.dp * np.exp(rng.normal(0, 1.0, st.dp.shape))
+    st.pt = st.pt * np.exp(rng.normal(0, 1.0, st.pt.shape))
+    st.u = st.u + rng.normal(0, 15.0, st.u.shape)
+    st.v = st.v + rng.normal(0, 15.0, st.v.shape)
+    dt = 30.0
+    g = Dycore(st)
+    g.adj_enable()
+    vs = {n: rand(rng, st, n) for n in NAMES}
+    t = tlm_from_gpu(g, st, vs)
+    t.cgrid_step(dt / 2)
+    t.cgrid_halo()
+    t.dgrid_step(dt)
+    w = {n: rand(rng, st, n) for n in NAMES}
+    lhs = sum(np.sum(w[n] * t.get(STATE[n], halo=True)[1]) for n in NAMES)
+    for n in NAMES:
+        g.adj_set('out', n, w[n])
+    g.adj_dgrid_step(dt)
+    g.adj_cgrid_halo()
+    g.adj_cgrid_step(dt / 2)
+    rhs = sum(np.sum(vs[n] * g.adj_get('in', n)) for n in NAMES)
+    assert rel(lhs, rhs) <= TOL, (lhs, rhs)
+
+
 def test_remap_dot_product():
     st = generic_state(seed=4)
     rng = np.random.default_rng(5)
