@@ -126,6 +126,91 @@ __global__ void __launch_bounds__(128) k_column(Geom g, Consts c, const T* __res
   column_at<T, PW>(g, c, dpl, ptl, pkap, gz, lo, hi, plev_out, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
+// The same with a block's four warps sharing the levels of 32 columns (lane =
+// column): the first warp runs the two sums, whose order fixes their bits, and
+// all warps share the powers between them, the long part of a column and
+// independent once the pressures stand (in shared memory, one array of
+// nlay x 32).  For domains of few columns, where one thread a column leaves the
+// GPU waiting for nlay powers in a row (64x64x20: 21.5 -> 12.8 us; 128x128x20:
+// 22.5 -> 13.1; 8 warps 11.1 and 18.5, 2 warps 14.8 and 16.0); with the GPU
+// full, the idle warps of the sums cost more than they save (1024x1024x64:
+// 0.83 ms against 0.63).
+constexpr int COL_WARPS = 4;
+template <typename T, typename PW = PortablePow>
+__global__ void __launch_bounds__(32 * COL_WARPS) k_column_split(Geom g, Consts c, const T* __restrict__ dpl,
+                                                                 const T* __restrict__ ptl, double* __restrict__ pkap,
+                                                                 double* __restrict__ gz, int lo, int hi,
+                                                                 double* __restrict__ plev_out) {
+  extern __shared__ double col_sm[];
+  constexpr int B = 8;  // levels whose loads are in flight together
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int w = g.nx - lo + hi, hgt = g.ny - lo + hi;
+  const int col = blockIdx.x * 32 + lane;
+  const bool in = col < w * hgt;
+  const int cc = in ? col : 0;
+  const long long o = g.at(lo + cc % w, lo + cc / w);
+  const long long S = g.S;
+  const int L = g.L;
+  double* sp = col_sm + lane;
+  if (warp == 0) {
+    double plev = c.ptop;
+    if (plev_out && in) plev_out[o + (long long)L * S] = plev;
+    T dn[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) dn[u] = L - 1 - u >= 0 ? dpl[o + (long long)(L - 1 - u) * S] : T(0);
+    for (int k0 = L - 1; k0 >= 0; k0 -= B) {
+      T dv[B];
+#pragma unroll
+      for (int u = 0; u < B; ++u) {
+        dv[u] = dn[u];
+        const int k = k0 - B - u;
+        if (k >= 0) dn[u] = dpl[o + (long long)k * S];
+      }
+#pragma unroll
+      for (int u = 0; u < B; ++u) {
+        const int k = k0 - u;
+        if (k < 0) break;
+        plev = plev + (double)dv[u];
+        if (plev_out && in) plev_out[o + (long long)k * S] = plev;
+        sp[k * 32] = plev;
+      }
+    }
+  }
+  __syncthreads();
+  for (int k = warp; k < L; k += COL_WARPS) {
+    const double pk = PW::kappa(sp[k * 32]);
+    sp[k * 32] = pk;
+    if (in) pkap[o + (long long)k * S] = pk;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    double z = gz[o];
+    double pk0 = sp[0];
+    T pn[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) pn[u] = u < L ? ptl[o + (long long)u * S] : T(0);
+    for (int k0 = 0; k0 < L; k0 += B) {
+      T pv[B];
+      double pk[B];
+#pragma unroll
+      for (int u = 0; u < B; ++u) {
+        pv[u] = pn[u];
+        const int k = k0 + u;
+        if (k + B < L) pn[u] = ptl[o + (long long)(k + B) * S];
+        pk[u] = k + 1 < L ? sp[(k + 1) * 32] : c.pk_top;
+      }
+#pragma unroll
+      for (int u = 0; u < B; ++u) {
+        const int k = k0 + u;
+        if (k >= L) break;
+        z = z + CP_DRY * (double)pv[u] * (pk0 - pk[u]);
+        if (in) gz[o + (long long)(k + 1) * S] = z;
+        pk0 = pk[u];
+      }
+    }
+  }
+}
+
 // Heating rate of the layer from the radiative net flux,
 // src/mod_sw_dyn.f90:89-106 (C) and 433-464 (D): pkap from dp (C step) or
 // dpc (D step) over the whole padded domain, playkap, then
@@ -195,9 +280,10 @@ __device__ __forceinline__ void corner_at(const Geom& g, const double* pkap, con
   }
 }
 
-// blockIdx.y selects a chunk of `chunk` levels (8: 0.67 ms at 1024x1024x64,
-// against 0.72 / 0.67 / 0.68 / 0.73 at 1 / 4 / 16 / 64), so that more threads share
-// the levels' independent loads
+// blockIdx.y selects a chunk of `chunk` levels, so that more threads share the
+// levels' independent loads: 8 (0.67 ms at 1024x1024x64, against 0.72 / 0.67 /
+// 0.68 / 0.73 at 1 / 4 / 16 / 64), or 1 on domains of few columns (64x64x20:
+// 8.7 us against 12.0 and 16.9 at 4 and 8)
 static __global__ void k_corners(Geom g, const double* __restrict__ pkap, const double* __restrict__ gz,
                           double* __restrict__ pkapb, double* __restrict__ gzb, int with_pkap, int lev0, int nlev,
                           int chunk) {

@@ -60,13 +60,24 @@ cudaError_t mass(const Geom& g, const Consts& c, const void* dp, const void* pt,
 
 cudaError_t column(const Geom& g, const Consts& c, const void* dpl, const void* ptl, int es, double* pkap, double* gz,
                    int lo, int hi, double* plev, cudaStream_t s) {
-  int n = (g.nx - lo + hi) * (g.ny - lo + hi);
+  const int n = (g.nx - lo + hi) * (g.ny - lo + hi);
+  if (few_columns(n)) {
+    const int nb = (n + 31) / 32, nt = 32 * COL_WARPS;
+    const size_t sm = (size_t)g.L * 32 * sizeof(double);  // at most 32 KB (128 layers)
+    if (es == 8)
+      k_column_split<double, FormPow<T>><<<nb, nt, sm, s>>>(g, c, (const double*)dpl, (const double*)ptl, pkap, gz, lo,
+                                                            hi, plev);
+    else
+      k_column_split<float, FormPow<T>><<<nb, nt, sm, s>>>(g, c, (const float*)dpl, (const float*)ptl, pkap, gz, lo, hi,
+                                                           plev);
+    return cudaGetLastError();
+  }
   if (es == 8)
-    k_column<double, FormPow<T>><<<(n + 127) / 128, 128, 0, s>>>(g, c, (const double*)dpl, (const double*)ptl, pkap, gz, lo, hi,
-                                                     plev);
+    k_column<double, FormPow<T>><<<(n + 127) / 128, 128, 0, s>>>(g, c, (const double*)dpl, (const double*)ptl, pkap, gz,
+                                                                 lo, hi, plev);
   else
-    k_column<float, FormPow<T>><<<(n + 127) / 128, 128, 0, s>>>(g, c, (const float*)dpl, (const float*)ptl, pkap, gz, lo, hi,
-                                                    plev);
+    k_column<float, FormPow<T>><<<(n + 127) / 128, 128, 0, s>>>(g, c, (const float*)dpl, (const float*)ptl, pkap, gz, lo,
+                                                                hi, plev);
   return cudaGetLastError();
 }
 

@@ -107,6 +107,12 @@ struct EnsPlan;
 int ensemble_max_blocks();
 cudaError_t ensemble_launch(const EnsPlan& plan, int blocks, cudaStream_t);
 
+// whether n columns leave a kernel of one thread a column with no more than four
+// blocks of 128 a multiprocessor, where levels are better shared (measured on B200,
+// FP64 column pass: 251x187x27 34 -> 29 us, 301x203x40 50 -> 44, 256x256x32 43 ->
+// 41; 350x350x64 111 -> 119, 512x512x64 191 -> 231)
+inline bool few_columns(long long n) { return n <= 148LL * 512; }
+
 // largest number of layers the vertical remap supports
 constexpr int MAX_LAYERS = 128;
 
