@@ -461,6 +461,35 @@ __device__ __forceinline__ int pair_add(double& acc, double btm, double top, dou
   return which;
 }
 
+// The same for layers of monotone coordinates that overlap (sk1 < d0, d1 < sk):
+// the four cases are the four combinations of d1 <= sk1 and sk <= d0, exactly
+// one of them holds, and only its quotients are formed.
+__device__ __forceinline__ int pair_add_case(double& acc, double btm, double top, double cv, double vk, double sk,
+                                             double sk1, double d0, double d1) {
+  const double dsrc = sk1 - sk;
+  const double f = dsrc / (d1 - d0);
+  const bool over = d1 <= sk1, under = sk <= d0;
+  if (over && under) {
+    acc = acc + vk * f;
+    return 5;
+  }
+  if (over) {
+    const double s1 = (d0 - sk) / dsrc;
+    const double tmp3 = 2. * s1 * s1, tmp1 = s1 - 1., tmp2 = s1 + 1.;
+    acc = acc + div_const<6>(tmp1) * (3. * (btm * tmp1 - top * tmp2) + cv * (tmp3 - tmp2)) * f;
+    return 3;
+  }
+  const double s2 = (d1 - sk) / dsrc;
+  if (under) {
+    acc = acc + (s2 / 2.) * (btm * (2. - s2) + s2 * (top + cv * (1. - C2_3 * s2))) * f;
+    return 4;
+  }
+  const double s1 = (d0 - sk) / dsrc;
+  const double tmp3 = 2. * s1 * s1, tmp1 = s1 + s2;
+  acc = acc + div_const<6>(s1 - s2) * (3. * (btm * (tmp1 - 2.) - top * tmp1) + cv * (tmp3 + tmp1 * (2. * s2 - 3.))) * f;
+  return 6;
+}
+
 template <int LM>
 __device__ __forceinline__ int remap_pair(const PPMWork<LM>& w, const double* src_var, double* dst_var,
                                           const double* sc, const double* dc, int k, int m) {
@@ -677,7 +706,7 @@ __device__ __forceinline__ void remap_merge(int L, ColArr sc, LA lv, LA gam, con
       const double sk = sc[k];
       if (!(sk > d1)) break;
       while (ly.k < k) ly.next();
-      const int which = pair_add(acc, ly.btm, ly.top, ly.curv, ly.vk, sk, sc[k + 1], d0, d1);
+      const int which = pair_add_case(acc, ly.btm, ly.top, ly.curv, ly.vk, sk, sc[k + 1], d0, d1);
       if (first < 0) {
         first = k;
         w0 = which;
@@ -827,19 +856,6 @@ __device__ __forceinline__ void remap_winds_at(const Geom& g, const RemapArgs& r
   }
   auto var = [&](int k) { return (double)f[oa + (long long)(k - 1) * S]; };
   remap_merge(L, sc, lv, gam, var, dc, [&](int m, double v) { r[oa + (long long)(m - 1) * S] = T(v); }, tr, 1);
-}
-
-// 16 blocks of 64 threads per SM (a 64-register budget, the column arrays in
-// local memory either way): more columns in flight hide more of the local
-// memory latency (measured at 1024x1024x64: 4.67 ms against 5.88 at the
-// compiler's own budget, 5.34 at 24 blocks, 7.05 at 32).
-template <typename T, int LM, typename E = double>
-__global__ void __launch_bounds__(64, 16) k_remap_winds(Geom g, RemapArgs ra, const T* __restrict__ dp,
-                                                    const T* __restrict__ ud, const T* __restrict__ vd,
-                                                    T* __restrict__ urem, T* __restrict__ vrem, int* trace,
-                                                    Status* st) {
-  remap_winds_at<T, LM, E>(g, ra, dp, ud, vd, urem, vrem, trace, st, blockIdx.x * blockDim.x + threadIdx.x,
-                           blockIdx.y);
 }
 
 // Energy remap and potential-temperature recovery on the interior,
@@ -1008,18 +1024,6 @@ __device__ __forceinline__ void remap_energy_at(const Geom& g, const RemapArgs& 
   };
   remap_merge(L, plev, lv, gam, [&](int k) { return en[k]; }, tpl, put, tr, 1);
   flag_nonfinite(&st->nonfinite_remap, bad);
-}
-
-// 16 blocks per SM, as k_remap_winds (4.91 ms against 5.45)
-template <typename T, int LM, typename PW = PortablePow>
-__global__ void __launch_bounds__(64, 16) k_remap_energy(Geom g, RemapArgs ra, const T* __restrict__ dp,
-                                                     const T* __restrict__ pt, const T* __restrict__ ud,
-                                                     const T* __restrict__ vd, const T* __restrict__ urem,
-                                                     const T* __restrict__ vrem, const double* __restrict__ gzs,
-                                                     T* __restrict__ dpo, T* __restrict__ pto, T* __restrict__ udo,
-                                                     T* __restrict__ vdo, int* trace, Status* st) {
-  remap_energy_at<T, LM, PW>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, dpo, pto, udo, vdo, trace, st,
-                             blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // ============================================================ reductions ===

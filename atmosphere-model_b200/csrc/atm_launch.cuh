@@ -6,6 +6,7 @@
 #include "atm_kernels.cuh"
 #include "atm_march.cuh"
 #include "atm_ops.h"
+#include "atm_remap.cuh"
 
 namespace atm {
 namespace {
@@ -130,38 +131,28 @@ cudaError_t ring_cg(const Geom& g, void* const* f, const void* const* src, int n
   return ring_t<C>(g, f, src, nf, K, copy, s);
 }
 
-template <int LM>
-cudaError_t remap_winds_lm(const Geom& g, const RemapArgs& ra, const void* dp, const void* ud, const void* vd,
-                           void* urem, void* vrem, int* trace, Status* st, cudaStream_t s) {
-  int n = (g.nx + 2) * (g.ny + 2);
-  k_remap_winds<S, LM, T><<<dim3((n + 63) / 64, 2), 64, 0, s>>>(g, ra, (const S*)dp, (const S*)ud, (const S*)vd, (S*)urem,
-                                                    (S*)vrem, trace, st);
-  return cudaGetLastError();
-}
-template <int LM>
-cudaError_t remap_energy_lm(const Geom& g, const RemapArgs& ra, const void* dp, const void* pt, const void* ud,
-                            const void* vd, const void* urem, const void* vrem, const double* gzs, void* dpo,
-                            void* pto, void* udo, void* vdo, int* trace, Status* st, cudaStream_t s) {
-  int n = g.nx * g.ny;
-  k_remap_energy<S, LM, FormPow<T>><<<(n + 63) / 64, 64, 0, s>>>(g, ra, (const S*)dp, (const S*)pt, (const S*)ud, (const S*)vd,
-                                                     (const S*)urem, (const S*)vrem, gzs, (S*)dpo, (S*)pto, (S*)udo,
-                                                     (S*)vdo, trace, st);
-  return cudaGetLastError();
-}
-
 cudaError_t remap_winds(const Geom& g, const RemapArgs& ra, const void* dp, const void* ud, const void* vd, void* urem,
                         void* vrem, int* trace, Status* st, cudaStream_t s) {
-  if (g.L <= 32) return remap_winds_lm<32>(g, ra, dp, ud, vd, urem, vrem, trace, st, s);
-  if (g.L <= 64) return remap_winds_lm<64>(g, ra, dp, ud, vd, urem, vrem, trace, st, s);
-  return remap_winds_lm<MAX_LAYERS>(g, ra, dp, ud, vd, urem, vrem, trace, st, s);
+  auto run = [&](auto lm) {
+    return launch_remap_winds<S, decltype(lm)::value, T>(g, ra, (const S*)dp, (const S*)ud, (const S*)vd, (S*)urem,
+                                                         (S*)vrem, trace, st, s);
+  };
+  if (g.L <= 32) return run(std::integral_constant<int, 32>{});
+  if (g.L <= 64) return run(std::integral_constant<int, 64>{});
+  return run(std::integral_constant<int, MAX_LAYERS>{});
 }
 
 cudaError_t remap_energy(const Geom& g, const RemapArgs& ra, const void* dp, const void* pt, const void* ud,
                          const void* vd, const void* urem, const void* vrem, const double* gzs, void* dpo, void* pto,
                          void* udo, void* vdo, int* trace, Status* st, cudaStream_t s) {
-  if (g.L <= 32) return remap_energy_lm<32>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, dpo, pto, udo, vdo, trace, st, s);
-  if (g.L <= 64) return remap_energy_lm<64>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, dpo, pto, udo, vdo, trace, st, s);
-  return remap_energy_lm<MAX_LAYERS>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, dpo, pto, udo, vdo, trace, st, s);
+  auto run = [&](auto lm) {
+    return launch_remap_energy<S, decltype(lm)::value, FormPow<T>>(
+        g, ra, (const S*)dp, (const S*)pt, (const S*)ud, (const S*)vd, (const S*)urem, (const S*)vrem, gzs, (S*)dpo,
+        (S*)pto, (S*)udo, (S*)vdo, trace, st, s);
+  };
+  if (g.L <= 32) return run(std::integral_constant<int, 32>{});
+  if (g.L <= 64) return run(std::integral_constant<int, 64>{});
+  return run(std::integral_constant<int, MAX_LAYERS>{});
 }
 
 cudaError_t check_finite(const Geom& g, const void* const* f, int* flag, cudaStream_t s) {

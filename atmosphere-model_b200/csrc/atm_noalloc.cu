@@ -14,7 +14,7 @@
 #include <mutex>
 
 #include "atmdyn.h"
-#include "atm_kernels.cuh"
+#include "atm_remap.cuh"
 #include "atm_ops.h"
 
 namespace {
@@ -51,12 +51,9 @@ template <int LM>
 cudaError_t launch(const atm::Geom& g, const atm::RemapArgs& ra, const double* dp, const double* pt,
                    const double* ud, const double* vd, const double* gzs, double* urem, double* vrem, double* dpo,
                    double* pto, double* udo, double* vdo, atm::Status* st, cudaStream_t s) {
-  int nw = (g.nx + 2) * (g.ny + 2);
-  atm::k_remap_winds<double, LM><<<dim3((nw + 63) / 64, 2), 64, 0, s>>>(g, ra, dp, ud, vd, urem, vrem, nullptr, st);
-  int ne = g.nx * g.ny;
-  atm::k_remap_energy<double, LM><<<(ne + 63) / 64, 64, 0, s>>>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, dpo, pto,
-                                                                udo, vdo, nullptr, st);
-  return cudaGetLastError();
+  const cudaError_t e = atm::launch_remap_winds<double, LM>(g, ra, dp, ud, vd, urem, vrem, nullptr, st, s);
+  if (e != cudaSuccess) return e;
+  return atm::launch_remap_energy<double, LM>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, dpo, pto, udo, vdo, nullptr, st, s);
 }
 
 }  // namespace

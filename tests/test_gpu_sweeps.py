@@ -1,7 +1,7 @@
 """The marching sweeps at the edges of their strips (26 output columns a warp,
-four warps a block, 4 to 128 output rows), bit for bit against the oracle: one
-step on smooth and on rough fields, whose slopes switch every limiter and the
-positivity filter."""
+four warps a block, 4 to 128 output rows) and the two forms of the remap, bit
+for bit against the oracle: one step on smooth and on rough fields, whose
+slopes switch every limiter and the positivity filter."""
 import numpy as np
 import pytest
 
@@ -46,4 +46,37 @@ def test_step_bit_exact(nx, ny, nlay, fields):
         a.dgrid_halo()
     for name, f in FIELDS:
         np.testing.assert_array_equal(g.get(name, halo=True), o.get(f, halo=True), err_msg=name)
+    g.close()
+
+
+@pytest.mark.parametrize('nx,ny,nlay', [(9, 8, 3), (23, 17, 32), (40, 33, 33), (20, 18, 65), (12, 11, 128),
+                                        (300, 270, 8)])
+@pytest.mark.parametrize('fields', ['smooth', 'rough', 'crossed'])
+def test_remap_bit_exact(nx, ny, nlay, fields):
+    """The remap alone, in its shared-level form (few columns; the three layer
+    ranges) and with one thread a column (the last size), with its layer-pair
+    trace; crossed: some columns whose interfaces are not monotone, which take
+    the all-pairs search."""
+    st = ic.jet_case(nx, ny, nlay, 400e3, 400e3, width=900e3, seed=ny)
+    rng = np.random.default_rng(nlay)
+    if fields != 'smooth':
+        st.dp = st.dp * np.exp(rng.normal(0, 0.7, st.dp.shape))
+        st.pt = st.pt * np.exp(rng.normal(0, 0.1, st.pt.shape))
+        st.u = st.u + rng.normal(0, 15.0, st.u.shape)
+        st.v = st.v + rng.normal(0, 15.0, st.v.shape)
+    if fields == 'crossed':
+        st.dp[1] = np.where(rng.random((ny, nx)) < 0.03, -0.2 * st.dp[1], st.dp[1])
+    g, o = Dycore(st), pyoracle.OracleModel(st, threads=8)
+    small = nx < 100
+    if small:
+        trace_o = o.enable_trace()
+        trace_g, fallback = g.remap_trace()
+    g.remap()
+    o.remap()
+    for name, f in FIELDS:
+        np.testing.assert_array_equal(g.get(name, halo=True), o.get(f, halo=True), err_msg=name)
+    if small:
+        np.testing.assert_array_equal(trace_g, trace_o)
+        # (the face interpolation crosses some coordinates of the rough fields too)
+        assert fallback.value > 0 if fields == 'crossed' else fields == 'rough' or fallback.value == 0
     g.close()
