@@ -1386,7 +1386,13 @@ int atm_set_gas_optics(atm_ctx* ctx, const atm_gas_optics* t) {
   size_t off[8];
   for (int q = 0, at = 0; q < 8; at += (int)len[q], ++q) {
     off[q] = (size_t)at;
-    std::memcpy(h.data() + at, src[q], len[q] * 8);
+    if (q == 2 || q == 4 || q == 6) {  // absorption and Planck tables: the g-point last on the device
+      const size_t m = len[q] / ng;
+      for (size_t gp = 0; gp < ng; ++gp)
+        for (size_t e = 0; e < m; ++e) h[(size_t)at + e * ng + gp] = src[q][gp * m + e];
+    } else {
+      std::memcpy(h.data() + at, src[q], len[q] * 8);
+    }
   }
   if (ctx->rad_block) {
     CK(cudaStreamSynchronize(ctx->stream));

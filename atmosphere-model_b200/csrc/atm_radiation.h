@@ -7,19 +7,19 @@
 
 namespace atm {
 
-// The gas-optics tables on the device, in the reference's index order
-// (flattened from the last Fortran index): temps[p][t] is temperatures(t, p),
-// sw_abs[g][p][t] is shortwave_absorption_lut(t, p, g), planck[g][t] is
-// planckian_lut(t, g).
+// The gas-optics tables on the device: temps[p][t] is temperatures(t, p); the
+// tables that depend on the g-point have it last, as neighbouring lanes read
+// neighbouring g-points of one entry: sw_abs[p][t][g] is
+// shortwave_absorption_lut(t, p, g), plk[t][g] is planckian_lut(t, g).
 struct RadTables {
   int ng, np, nt, npl;
   const double* pressures;  // [np]
   const double* temps;      // [np][nt]
-  const double* sw_abs;     // [ng][np][nt]
+  const double* sw_abs;     // [np][nt][ng]
   const double* sw_sca;     // [ng]
-  const double* lw_abs;     // [ng][np][nt]
+  const double* lw_abs;     // [np][nt][ng]
   const double* plk_t;      // [npl]
-  const double* plk;        // [ng][npl]
+  const double* plk;        // [npl][ng]
   const double* frac;       // [ng], irradiance_fraction
 };
 

@@ -59,6 +59,22 @@ def test_net_flux_bit_exact(nlay, which):
     dy.close()
 
 
+@pytest.mark.parametrize('n_g,nx,ny,nlay', [(1, 9, 7, 3), (5, 8, 8, 17), (16, 13, 11, 64), (19, 10, 9, 33),
+                                            (40, 7, 7, 8)])
+def test_g_point_counts_bit_exact(n_g, nx, ny, nlay):
+    """Fewer and more g-points than the 16 lanes a column has (whole and partial
+    rounds), column counts that leave a block part empty, and layer counts
+    around the batches of levels."""
+    go = gas_optics.synthetic(4, n_g=n_g)
+    st = radiative_state(nx, ny, nlay, seed=n_g)
+    xc, yc = ic.cell_axes(st)
+    dy = Dycore(st)
+    dy.set_radiation(go, xc, yc)
+    dy.radiative_heating(0.0)
+    np.testing.assert_array_equal(dy.get('net_flux'), oracle_flux(st, go, dy, xc, yc))
+    dy.close()
+
+
 def test_mixed_form_and_parameters():
     """The radiation is FP64 in the mixed form too (its state is FP64);
     non-default zenith angle, albedo and emissivity."""
