@@ -24,12 +24,16 @@
 // return.  A strip whose output adjoints are all zero returns at once (a loss
 // over a sub-domain reaches only its domain of dependence).
 //
-// Bound by instruction issue, like the forward.  Measured on B200 at
-// 512x512x32 (ms a launch; before: one or two kernels on 32 x 4-8 tiles that
+// Bound by the latency of the FP64 chains at the three blocks an SM that the
+// registers leave, once the loads run ahead (RowRing).  Measured on B200 at
+// 512x512x32 (ms a launch; first: one or two kernels on 32 x 4-8 tiles that
 // kept every intermediate and its adjoint in shared memory, with shared-memory
 // atomics and block barriers between about ten stages, ~6000 instructions a
-// cell): C mass 3.37 -> 0.58 + 0.87, C momentum 3.27 -> 1.05, D mass 1.76 +
-// 1.77 -> 0.63 + 1.02, D momentum 1.42 + 2.74 -> 0.59 + 0.57.
+// cell; then this march with its loads at their use, then with the rings):
+// C mass 3.37, 0.58 + 0.87, 0.37 + 0.56; C momentum 3.27, 1.05, 0.89; D mass
+// 3.53, 0.63 + 1.02, 0.47 + 0.79; D momentum 4.16, 0.59 + 0.57, 0.40 + 0.50.
+// With the rings, rows unrolled 2 or 3 times gain up to 4% in the momentum x
+// kernels and lose 10-25% in the y kernels; four blocks an SM lose 50% there.
 #pragma once
 
 #include "atm_march.cuh"
@@ -258,6 +262,30 @@ struct YLineAdj {
   }
 };
 
+// The rows a strip is about to need, brought into shared memory by asynchronous
+// copies two iterations ahead: NF values a lane and iteration, each lane its own
+// (no barrier), DEPTH iterations kept.  Loaded at their use, or a row ahead into
+// registers, these left the reverse mass kernels waiting for 3 of 6 cycles an
+// issued instruction; the gradient at 512x512x32 went from 52.0 to 45.4 ms.
+template <int NF, int DEPTH>
+struct RowRing {
+  static constexpr int bytes = NF * DEPTH * MW * 8;  // of a warp
+  double* p;
+  unsigned s;
+  __device__ __forceinline__ explicit RowRing(double* sm) {
+    p = sm + (threadIdx.x >> 5) * (bytes / 8) + (threadIdx.x & (MW - 1));
+    s = (unsigned)__cvta_generic_to_shared(p);
+  }
+  __device__ __forceinline__ static int slot(int r, int f) { return ((r & (DEPTH - 1)) * NF + f) * MW; }
+  __device__ __forceinline__ void copy(int r, int f, const double* g) const {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s + slot(r, f) * 8), "l"(g) : "memory");
+  }
+  __device__ __forceinline__ static void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+  // every group but the newest two has arrived
+  __device__ __forceinline__ static void wait() { asm volatile("cp.async.wait_group 2;" ::: "memory"); }
+  __device__ __forceinline__ double get(int r, int f) const { return p[slot(r, f)]; }
+};
+
 // add v to a global adjoint (ok: the point is stored)
 __device__ __forceinline__ void radd(double* f, unsigned i, double v, bool ok) {
   if (ok && v != 0.) atomicAdd(f + i, v);
@@ -295,16 +323,17 @@ struct MassAdjArgs {
   double *lam_dp, *lam_pt, *lam_u, *lam_v;
 };
 
-// lv, lq of one output point
-__device__ __forceinline__ void mass_out_adj(const MassAdjArgs& a, long long i, double& lv, double& lq) {
-  lq = a.lam_pto[i] / a.dpo[i];
-  lv = a.lam_dpo[i] - a.pto[i] * lq;
+// lv, lq of an output point with new fields d, t and their adjoints ld, lt
+__device__ __forceinline__ void mass_out_adj(double ld, double lt, double d, double t, double& lv, double& lq) {
+  lq = lt / d;
+  lv = ld - t * lq;
 }
 
 // The x branch: the outer x fluxes, the inner y sweeps, the direct dependence
 // of the new fields on the old, and the whole damping of dp.
 template <bool CGRID>
 __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_x(Geom g, Consts c, MassAdjArgs a, int lo, int hi, int tys) {
+  extern __shared__ double adj_sm[];
   constexpr int V = CGRID ? PPM_UNC : PPM_NN;
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
   const int xhi = g.nx - 1 + hi, yhi = g.ny - 1 + hi;
@@ -321,51 +350,60 @@ __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_x(Geom g, Consts c,
   const double *dp = a.dp + kS, *pt = a.pt + kS, *u = a.u + kS, *v = a.v + kS;
   double *lam_dp = a.lam_dp + kS, *lam_pt = a.lam_pt + kS, *lam_u = a.lam_u + kS, *lam_v = a.lam_v + kS;
 
-  unsigned rm = row_of(g, oy - 1), r0 = row_of(g, oy), r1 = row_of(g, oy + 1);
-  double dm = dp[rm + xi], d0 = dp[r0 + xi], d1n = dp[r1 + xi];
-  double pm = pt[rm + xi], p0 = pt[r0 + xi], p1n = pt[r1 + xi];
-  // C grid: sums of the D-grid winds that the C-grid winds average; D grid: the winds themselves
-  double us = 0., un = 0., vc0 = v[r0 + xi], vn = v[r1 + xi], vnr = 0., vo = 0., vor_ = 0.;
+  // iteration r brings rows r+1 of dp, pt, v and u (D grid: row r of u), and
+  // row r of the outputs and their adjoints
+  enum { F_DP, F_PT, F_U, F_V, F_LD, F_LP, F_DO, F_PO, F_VR };
+  const RowRing<CGRID ? 9 : 8, 4> ring(adj_sm);
+  auto issue = [&](int r) {
+    if (r < yend + 4) {
+      const unsigned i1 = row_of(g, r + 1), i0 = row_of(g, r) + xi;
+      ring.copy(r, F_DP, dp + (i1 + xi));
+      ring.copy(r, F_PT, pt + (i1 + xi));
+      ring.copy(r, F_U, u + (CGRID ? i1 + xi : i0));
+      ring.copy(r, F_V, v + (i1 + xi));
+      if (CGRID) ring.copy(r, F_VR, v + (i1 + xr));
+      if (r < yend) {
+        ring.copy(r, F_LD, a.lam_dpo + (kS + i0));
+        ring.copy(r, F_LP, a.lam_pto + (kS + i0));
+        ring.copy(r, F_DO, a.dpo + (kS + i0));
+        ring.copy(r, F_PO, a.pto + (kS + i0));
+      }
+    }
+    ring.commit();
+  };
+  issue(oy);
+  issue(oy + 1);
+  const unsigned rm = row_of(g, oy - 1), r0 = row_of(g, oy);
+  double dm = dp[rm + xi], d0 = dp[r0 + xi], pm = pt[rm + xi], p0 = pt[r0 + xi];
+  // C grid: sums of the D-grid winds that the C-grid winds average
+  double us = 0., vc0 = v[r0 + xi], vo = 0., vor_ = 0.;
   if constexpr (CGRID) {
     const double ur = u[r0 + xi];
     us = ur + shfl_up(ur, 1);
-    un = u[r1 + xi];
     vo = vc0;
     vor_ = v[r0 + xr];
     vc0 = .25 * ((vo + v[rm + xi]) + (vor_ + v[rm + xr]));
-    vnr = v[r1 + xr];
-  } else {
-    un = u[r0 + xi];
   }
   double aD2 = 0, aD1 = 0, aD0 = 0, aP2 = 0, aP1 = 0, aP0 = 0;  // adjoints of dp, pt of rows r-2, r-1, r
   double lv1 = 0, lv2 = 0, x1 = 0, alp1 = 0;                    // lv of rows r-1, r-2; x damping term, pt Laplacian's adjoint of r-1
   double lwp = 0, Up = 0, Wp = 0;
 #pragma unroll 1
   for (int r = oy; r < yend + 4; ++r) {
+    issue(r + 2);
+    ring.wait();
     const unsigned ri = row_of(g, r) + xi;
-    const double d1 = d1n, p1 = p1n;
+    const double d1 = ring.get(r, F_DP), p1 = ring.get(r, F_PT), ur = ring.get(r, F_U), vn = ring.get(r, F_V);
     double lv = 0., lq = 0.;
     const bool live = r < yend;
-    if (live && own) mass_out_adj(a, kS + ri, lv, lq);
-    const unsigned r2 = row_of(g, r + 2);
-    d1n = dp[r2 + xi];
-    p1n = pt[r2 + xi];
-    double uc, vc1;
+    if (live && own) mass_out_adj(ring.get(r, F_LD), ring.get(r, F_LP), ring.get(r, F_DO), ring.get(r, F_PO), lv, lq);
+    double uc = ur, vc1 = vn;
     if constexpr (CGRID) {
-      const double s = un + shfl_up(un, 1);
-      uc = .25 * (us + s);
-      us = s;
-      un = u[r2 + xi];
+      const double vnr = ring.get(r, F_VR), su = ur + shfl_up(ur, 1);
+      uc = .25 * (us + su);
+      us = su;
       vc1 = .25 * ((vn + vo) + (vnr + vor_));
       vo = vn;
       vor_ = vnr;
-      vn = v[r2 + xi];
-      vnr = v[r2 + xr];
-    } else {
-      uc = un;
-      un = u[row_of(g, r + 1) + xi];
-      vc1 = vn;
-      vn = v[r2 + xi];
     }
     double luc = 0., lw = 0., alp = 0., aD = 0., aP = 0., X = 0.;
     const double lvL = up0(lv), lvR = dn0(lv);
@@ -441,8 +479,12 @@ __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_x(Geom g, Consts c,
 // The y branch: the outer y fluxes, the inner x sweeps, the y part of the
 // damping of pt.  Own columns: lanes 1 to 30.
 constexpr int YOUT_MASS = 30;
+constexpr size_t mass_adj_smem(bool cgrid, bool xb) {
+  return MWARPS * (size_t)(!xb ? RowRing<8, 8>::bytes : cgrid ? RowRing<9, 4>::bytes : RowRing<8, 4>::bytes);
+}
 template <bool CGRID>
 __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_y(Geom g, Consts c, MassAdjArgs a, int lo, int hi, int tys) {
+  extern __shared__ double adj_sm[];
   constexpr int V = CGRID ? PPM_UNC : PPM_NN;
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
   const int xhi = g.nx - 1 + hi, yhi = g.ny - 1 + hi;
@@ -458,6 +500,30 @@ __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_y(Geom g, Consts c,
   const double *dp = a.dp + kS, *pt = a.pt + kS, *u = a.u + kS, *v = a.v + kS;
   double *lam_dp = a.lam_dp + kS, *lam_pt = a.lam_pt + kS, *lam_u = a.lam_u + kS, *lam_v = a.lam_v + kS;
 
+  // iteration r brings row r of dp, pt and u (C grid: row r+1 of u), kept until
+  // the reverse of the inner sweep at row s = r-5 reads them again, and row i =
+  // r-2 of v, the outputs and their adjoints
+  enum { F_DP, F_PT, F_U, F_V, F_LD, F_LP, F_DO, F_PO };
+  const RowRing<8, 8> ring(adj_sm);
+  const int rend = yend + 8 + (CGRID ? 1 : 0);
+  auto issue = [&](int r) {
+    if (r < rend) {
+      const unsigned i0 = row_of(g, r) + xi, ii = row_of(g, r - 2) + xi;
+      ring.copy(r, F_DP, dp + i0);
+      ring.copy(r, F_PT, pt + i0);
+      ring.copy(r, F_U, u + (CGRID ? row_of(g, r + 1) + xi : i0));
+      ring.copy(r, F_V, v + ii);
+      if (r - 2 >= oy && r - 2 < yend) {
+        ring.copy(r, F_LD, a.lam_dpo + (kS + ii));
+        ring.copy(r, F_LP, a.lam_pto + (kS + ii));
+        ring.copy(r, F_DO, a.dpo + (kS + ii));
+        ring.copy(r, F_PO, a.pto + (kS + ii));
+      }
+    }
+    ring.commit();
+  };
+  issue(oy - 3);
+  issue(oy - 2);
   YLineAdj<V> yd, yp;
   double p1 = 0, p2 = 0, ps1 = 0;                   // pt of rows r-1, r-2; pt(x+1) + pt(x-1) of row r-1
   double lp1 = 0, lp2 = 0, lp3 = 0;                 // Laplacian of pt of rows r-1 .. r-3
@@ -467,29 +533,20 @@ __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_y(Geom g, Consts c,
   if constexpr (CGRID) {
     const double ur = u[row_of(g, oy - 3) + xi];
     us = ur + shfl_up(ur, 1);
+    uss = us;
     vo = v[row_of(g, oy - 6) + xi];
-    const double uq = u[row_of(g, oy - 8) + xi];
-    uss = uq + shfl_up(uq, 1);
   }
-  const int rend = yend + 8 + (CGRID ? 1 : 0);
-  unsigned r0 = row_of(g, oy - 3);
-  double dn = dp[r0 + xi], pn = pt[r0 + xi], un = u[(CGRID ? row_of(g, oy - 2) : r0) + xi];
-  double vn = v[row_of(g, oy - 5) + xi];
 #pragma unroll 1
   for (int r = oy - 3; r < rend; ++r) {
+    issue(r + 2);
+    ring.wait();
     const int i = r - 2, s = r - 5;
     const unsigned si = row_of(g, s) + xi, ii = row_of(g, i) + xi;
     double lv = 0., lq = 0.;
-    if (i >= oy && i < yend && own) mass_out_adj(a, kS + ii, lv, lq);
-    // row s, which the reverse of the inner sweep reads again
-    const double ds = dp[si], ps = pt[si], usr = u[(CGRID ? row_of(g, s + 1) + xi : si)];
+    if (i >= oy && i < yend && own)
+      mass_out_adj(ring.get(r, F_LD), ring.get(r, F_LP), ring.get(r, F_DO), ring.get(r, F_PO), lv, lq);
     // ---- forward: row r
-    const double d = dn, p = pn, ur = un, vr = vn;
-    const unsigned r1 = row_of(g, r + 1);
-    dn = dp[r1 + xi];
-    pn = pt[r1 + xi];
-    un = u[(CGRID ? row_of(g, r + 2) : r1) + xi];
-    vn = v[row_of(g, r - 1) + xi];
+    const double d = ring.get(r, F_DP), p = ring.get(r, F_PT), ur = ring.get(r, F_U), vr = ring.get(r, F_V);
     double uc = ur, vc = vr;
     if constexpr (CGRID) {
       const double su = ur + shfl_up(ur, 1), sv = vr + vo;
@@ -525,24 +582,29 @@ __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_y(Geom g, Consts c,
     const double al3 = vdy * (Gp - G);
     Gp = G;
     // ---- row s: the inner x sweep
-    double ucs = usr;
-    if constexpr (CGRID) {
-      const double su = usr + shfl_up(usr, 1);
-      ucs = .25 * (uss + su);
-      uss = su;
+    double lu = 0.;
+    if (s >= oy - 3) {
+      const double ds = ring.get(s, F_DP), ps = ring.get(s, F_PT), usr = ring.get(s, F_U);
+      double ucs = usr;
+      if constexpr (CGRID) {
+        const double su = usr + shfl_up(usr, 1);
+        ucs = .25 * (uss + su);
+        uss = su;
+      }
+      const double ucR = shfl_dn(ucs, 1);
+      const double dL = shfl_up(ds, 1), dR = shfl_dn(ds, 1), qL = shfl_up(ps, 1), qR = shfl_dn(ps, 1);
+      const bool c0 = dtdx * ucs > 0., c1 = dtdx * ucR > 0.;
+      const double den = 1. / (1. - dtdx * (ucR - ucs));
+      double am, a0, ap, lden = 0.;
+      inner_e_adj(ds, c0 ? dL : ds, c1 ? ds : dR, c0, c1, den, rA, lamd, am, a0, ap, lden);
+      radd(lam_dp, si, a0 + dn0(am) + up0(ap), in);
+      inner_e_adj(ps, c0 ? qL : ps, c1 ? ps : qR, c0, c1, den, rA, lamp, am, a0, ap, lden);
+      radd(lam_pt, si, a0 + dn0(am) + up0(ap) + rdy2 * (al6 + al4) + (m2rdxy * al5 + rdx2 * (up0(al5) + dn0(al5))),
+           in);
+      const double lw = dtdx * den * den * lden;
+      lu = up0(lw) - lw;
     }
-    const double ucR = shfl_dn(ucs, 1);
-    const double dL = shfl_up(ds, 1), dR = shfl_dn(ds, 1), qL = shfl_up(ps, 1), qR = shfl_dn(ps, 1);
-    const bool c0 = dtdx * ucs > 0., c1 = dtdx * ucR > 0.;
-    const double den = 1. / (1. - dtdx * (ucR - ucs));
-    double am, a0, ap, lden = 0.;
-    inner_e_adj(ds, c0 ? dL : ds, c1 ? ds : dR, c0, c1, den, rA, lamd, am, a0, ap, lden);
-    radd(lam_dp, si, a0 + dn0(am) + up0(ap), in);
-    inner_e_adj(ps, c0 ? qL : ps, c1 ? ps : qR, c0, c1, den, rA, lamp, am, a0, ap, lden);
-    radd(lam_pt, si, a0 + dn0(am) + up0(ap) + rdy2 * (al6 + al4) + (m2rdxy * al5 + rdx2 * (up0(al5) + dn0(al5))), in);
     al6 = al5; al5 = al4; al4 = al3;
-    const double lw = dtdx * den * den * lden;
-    const double lu = up0(lw) - lw;
     if constexpr (CGRID) {
       const double U = lu + dn0(lu);
       radd(lam_u, si, .25 * (U + Up), in);
@@ -573,6 +635,7 @@ struct CMomAdjArgs {
 // The x branch: the x fluxes of the vorticity and of the kinetic energy, the
 // damping.
 static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_x(Geom g, Consts c, CMomAdjArgs a, int tys) {
+  extern __shared__ double adj_sm[];
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
   const int ox = (int)(blockIdx.x * MWARPS + (threadIdx.x >> 5)) * MOUT, oy = (int)blockIdx.y * tys;
   if (ox >= g.nx) return;
@@ -587,6 +650,26 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_x(Geom g, C
   const double *ud = a.ud + kS, *vd = a.vd + kS, *uL = a.ud + LS;
   double *lam_ud = a.lam_ud + kS, *lam_vd = a.lam_vd + kS, *lam_w = a.lam_w + kS, *lam_uc1 = a.lam_uc1 + kS;
 
+  // iteration r brings rows r+2 of ud, r+1 of vd and of layer-nlay ud, r of lam_uc, lam_vc
+  enum { F_U, F_UL, F_V, F_VR, F_UN, F_LU, F_LV };
+  const RowRing<7, 4> ring(adj_sm);
+  auto issue = [&](int r) {
+    if (r < yend + 3) {
+      const unsigned r0 = row_of(g, r) + xi, r1 = row_of(g, r + 1), r2 = row_of(g, r + 2);
+      ring.copy(r, F_U, ud + (r2 + xi));
+      ring.copy(r, F_UL, ud + (r2 + xl));
+      ring.copy(r, F_V, vd + (r1 + xi));
+      ring.copy(r, F_VR, vd + (r1 + xr));
+      ring.copy(r, F_UN, uL + (r1 + xi));
+      if (r < yend) {
+        ring.copy(r, F_LU, lam_uc + r0);
+        ring.copy(r, F_LV, lam_vc + r0);
+      }
+    }
+    ring.commit();
+  };
+  issue(oy);
+  issue(oy + 1);
   // rows of the layer's C-grid winds and vorticity: a0 = uc1(r), aN = uc1(r+1), w = vor(r-1, r, r+1)
   auto uavg = [&](unsigned ra, unsigned rb) { return .25 * ((ud[ra + xi] + ud[ra + xl]) + (ud[rb + xi] + ud[rb + xl])); };
   auto vavg = [&](unsigned ra, unsigned rb) { return .25 * ((vd[rb + xi] + vd[ra + xi]) + (vd[rb + xr] + vd[ra + xr])); };
@@ -597,21 +680,27 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_x(Geom g, C
   double w0 = f - (uc_1 - uc_0) * rdy + (vc_1 - shfl_up(vc_1, 1)) * rdx;
   double ucr = uc_1, ucm = uc_0;                 // uc1 of rows r, r-1
   double v_m = vd[q1 + xi], v_0 = vd[q0 + xi];   // vd(x) of rows r-1, r
+  double vR0 = vd[q0 + xr];                      // vd(x+1) of row r
+  double u0 = ud[q0 + xi], u1 = ud[p1 + xi];     // ud(x) of rows r, r+1
+  double su1 = u1 + ud[p1 + xl];                 // ud(x) + ud(x-1) of row r+1
   double uLm = uL[q1 + xi], uL0 = uL[q0 + xi];   // layer-nlay ud of rows r-1, r
   double lu1 = 0, lv1 = 0, lwd1 = 0;             // lam_uc, lam_vc, den's adjoint of row r-1
   double aW1 = 0, aW0 = 0;                       // adjoints of the vorticity of rows r-1, r
 #pragma unroll 1
   for (int r = oy; r < yend + 3; ++r) {
-    const unsigned rr = row_of(g, r), ra = row_of(g, r + 1), rb = row_of(g, r + 2);
+    issue(r + 2);
+    ring.wait();
+    const unsigned rr = row_of(g, r);
     const bool live = r < yend;
     double lu = 0., lv = 0.;
     if (live && own) {
-      lu = lam_uc[rr + xi];
-      lv = lam_vc[rr + xi];
+      lu = ring.get(r, F_LU);
+      lv = ring.get(r, F_LV);
     }
-    const double uc_n = uavg(ra, rb), vc_n = vavg(rr, ra);
+    const double u2 = ring.get(r, F_U), su2 = u2 + ring.get(r, F_UL);
+    const double v_n = ring.get(r, F_V), vR_n = ring.get(r, F_VR), uL1 = ring.get(r, F_UN);
+    const double uc_n = .25 * (su1 + su2), vc_n = .25 * ((v_n + v_0) + (vR_n + vR0));
     const double wp = f - (uc_n - ucr) * rdy + (vc_n - shfl_up(vc_n, 1)) * rdx;
-    const double u0 = ud[rr + xi], uL1 = uL[ra + xi];
     double lwd = 0., aW = 0.;
     if (live && __any_sync(0xffffffffu, lv != 0.)) {
       // v = vc1 - dt (ud fx + ...): the flux above the cell, reversed as the one below the next lane's
@@ -664,7 +753,11 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_x(Geom g, C
     wm = w0;
     w0 = wp;
     v_m = v_0;
-    v_0 = vd[ra + xi];
+    v_0 = v_n;
+    vR0 = vR_n;
+    u0 = u1;
+    u1 = u2;
+    su1 = su2;
     uLm = uL0;
     uL0 = uL1;
   }
@@ -674,6 +767,7 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_x(Geom g, C
 // columns: lanes 2 to 29, over [-1, n-1] (the kinetic energy's range).
 constexpr int YOUT_CMOM = 28;
 static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_y(Geom g, Consts c, CMomAdjArgs a, int tys) {
+  extern __shared__ double adj_sm[];
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
   const int ox = -1 + (int)(blockIdx.x * MWARPS + (threadIdx.x >> 5)) * YOUT_CMOM, oy = -1 + (int)blockIdx.y * tys;
   if (ox >= g.nx) return;
@@ -688,31 +782,51 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_y(Geom g, C
   const double *ud = a.ud + kS, *vd = a.vd + kS, *vL = a.vd + LS;
   double *lam_ud = a.lam_ud + kS, *lam_vd = a.lam_vd + kS, *lam_w = a.lam_w + kS, *lam_vc1 = a.lam_vc1 + kS;
 
+  // iteration r brings rows r+1 of ud and r of vd and, with y = r-3, rows y of
+  // lam_uc, y+1 of lam_vc, y of vd, r-5 of ud and y+1 of layer-nlay vd
+  enum { F_U, F_V, F_LU, F_LV, F_VY, F_US, F_VN };
+  const RowRing<7, 4> ring(adj_sm);
+  auto issue = [&](int r) {
+    if (r < yend + 8) {
+      const int y = r - 3;
+      const unsigned y0 = row_of(g, y) + xi, y1 = row_of(g, y + 1) + xi;
+      ring.copy(r, F_U, ud + (row_of(g, r + 1) + xi));
+      ring.copy(r, F_V, vd + (row_of(g, r) + xi));
+      if (y >= 0 && y < g.ny) ring.copy(r, F_LU, lam_uc + y0);
+      if (y >= -1 && y < g.ny - 1) ring.copy(r, F_LV, lam_vc + y1);
+      ring.copy(r, F_VY, vd + y0);
+      ring.copy(r, F_US, ud + (row_of(g, r - 5) + xi));
+      ring.copy(r, F_VN, vL + y1);
+    }
+    ring.commit();
+  };
+  issue(oy - 2);
+  issue(oy - 1);
   YLineAdj<PPM_UNC> lt, lb;  // the inner x sweep of the vorticity, the layer's C-grid v, along y
   double w0 = 0, w1 = 0, w2 = 0, w3 = 0, w4 = 0, w5 = 0;  // vorticity of rows r .. r-5
   int r = oy - 2;
   unsigned rm = row_of(g, r - 1), r0 = row_of(g, r);
-  double u0 = ud[r0 + xi], un = ud[row_of(g, r + 1) + xi];  // ud of rows r, r+1
+  double u0 = ud[r0 + xi];                                  // ud of row r
   double us = u0 + shfl_up(u0, 1);                          // u(x) + u(x-1) of row r
   double ucp = ud[rm + xi];                                 // uc1 of row r-1
   ucp = .25 * ((ucp + shfl_up(ucp, 1)) + us);
-  double vo = vd[rm + xi], vn = vd[r0 + xi];                // vd of rows r-1, r
+  double vo = vd[rm + xi];                                  // vd of row r-1
   // layer-nlay vd of rows y-1, y with y = r-3
   double vL2 = vL[row_of(g, r - 4) + xi], vL1 = vL[row_of(g, r - 3) + xi];
   double lv3 = 0;                                           // lam_vc of row y
 #pragma unroll 1
   for (; r < yend + 8; ++r) {
+    issue(r + 2);
+    ring.wait();
     const int y = r - 3, s = r - 5;
     const unsigned yi = row_of(g, y) + xi, si = row_of(g, s) + xi;
     const bool ownr = own && y >= oy && y < yend;
     double lu = 0., lvn = 0.;  // lam_uc of row y, lam_vc of row y+1, over the domain
-    if (dom && y >= 0 && y < g.ny) lu = lam_uc[yi];
-    if (dom && y >= -1 && y < g.ny - 1) lvn = lam_vc[row_of(g, y + 1) + xi];
-    const double vy = vd[yi], uxs = ud[si], vL0 = vL[row_of(g, y + 1) + xi];
+    if (dom && y >= 0 && y < g.ny) lu = ring.get(r, F_LU);
+    if (dom && y >= -1 && y < g.ny - 1) lvn = ring.get(r, F_LV);
+    const double vy = ring.get(r, F_VY), uxs = ring.get(r, F_US), vL0 = ring.get(r, F_VN);
     // ---- forward: row r
-    const double u1 = un, v = vn;
-    un = ud[row_of(g, r + 2) + xi];
-    vn = vd[row_of(g, r + 1) + xi];
+    const double u1 = ring.get(r, F_U), v = ring.get(r, F_V);
     const double su = u1 + shfl_up(u1, 1), sv = v + vo;
     const double uc = .25 * (us + su), vc = .25 * (sv + shfl_dn(sv, 1));
     const double w = f - (uc - ucp) * rdy + (vc - shfl_up(vc, 1)) * rdx;
@@ -964,6 +1078,7 @@ struct DMomAdjArgs {
 // The x branch: the x fluxes of the vorticity and of the kinetic energy, the
 // direct terms and both dampings.
 static __global__ void __launch_bounds__(MW * MWARPS, 3) k_d_mom_adj_x(Geom g, Consts c, DMomAdjArgs a, int tys) {
+  extern __shared__ double adj_sm[];
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
   const int ox = (int)(blockIdx.x * MWARPS + (threadIdx.x >> 5)) * MOUT, oy = (int)blockIdx.y * tys;
   if (ox >= g.nx) return;
@@ -979,12 +1094,32 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_d_mom_adj_x(Geom g, C
   double *lam_ud = a.lam_ud + kS, *lam_vd = a.lam_vd + kS, *lam_uc = a.lam_uc + kS;
   double *lam_uL = a.lam_uc + LS, *lam_vL = a.lam_vc + LS;
 
+  // iteration r brings rows r+2 of ud, r+1 of vd, r of uc and of layer-nlay uc,
+  // r+1 of layer-nlay vc, r of lam_udo, lam_vdo
+  enum { F_U, F_V, F_UC, F_UN, F_VN, F_LU, F_LV };
+  const RowRing<7, 4> ring(adj_sm);
+  auto issue = [&](int r) {
+    if (r < yend + 6) {
+      const unsigned r0 = row_of(g, r) + xi, r1 = row_of(g, r + 1) + xi;
+      ring.copy(r, F_U, ud + (row_of(g, r + 2) + xi));
+      ring.copy(r, F_V, vd + r1);
+      ring.copy(r, F_UN, uL + r0);
+      ring.copy(r, F_VN, vL + r1);
+      if (r < yend) {
+        ring.copy(r, F_UC, uck + r0);
+        ring.copy(r, F_LU, lam_udo + r0);
+        ring.copy(r, F_LV, lam_vdo + r0);
+      }
+    }
+    ring.commit();
+  };
+  issue(oy);
+  issue(oy + 1);
   auto row = [&](const double* q, int y) { return q[row_of(g, y) + xi]; };
-  double um = row(ud, oy - 1), u0 = row(ud, oy), u1 = row(ud, oy + 1), un = row(ud, oy + 2);  // rows r-1 .. r+2
-  double v1 = row(vd, oy + 1);
+  double um = row(ud, oy - 1), u0 = row(ud, oy), u1 = row(ud, oy + 1);  // rows r-1, r, r+1
   auto vort = [&](double ub, double ut, double v) { return f - (ut - ub) * rdy + (shfl_dn(v, 1) - v) * rdx; };
   double wm = vort(um, u0, row(vd, oy - 1)), w0 = vort(u0, u1, row(vd, oy));  // vorticity of rows r-1, r
-  double cum = row(uL, oy - 1), cu0 = row(uL, oy), cv0 = row(vL, oy), cv1 = row(vL, oy + 1);
+  double cum = row(uL, oy - 1), cv0 = row(vL, oy);
   double lu1 = 0, lv1 = 0, lwp = 0, lubp = 0, e1 = 0;       // of row r-1: lam_udo, lam_vdo, den's, half ubL's, ud line's
   double e2 = 0, dir2 = 0, dirv2 = 0, dirv3 = 0;            // ud line's adjoint of row r-2, lam_udo of r-2, lam_vdo of r-2, r-3
   double aW2 = 0, aW1 = 0, aW0 = 0, W3 = 0;                 // adjoints of the vorticity of rows r-2 .. r, and (complete) r-3
@@ -994,18 +1129,21 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_d_mom_adj_x(Geom g, C
   double g3 = 0;                                            // adjoint of the divergence, row r-3
 #pragma unroll 1
   for (int r = oy; r < yend + 6; ++r) {
+    issue(r + 2);
+    ring.wait();
     const unsigned rr = row_of(g, r) + xi;
     const bool live = r < yend;
     double lu = 0., lv = 0.;
     if (live && own) {
-      lu = lam_udo[rr];
-      lv = lam_vdo[rr];
+      lu = ring.get(r, F_LU);
+      lv = ring.get(r, F_LV);
     }
-    const double w1 = vort(u1, un, v1);
+    const double un = ring.get(r, F_U), cu0 = ring.get(r, F_UN), cv1 = ring.get(r, F_VN);
+    const double w1 = vort(u1, un, ring.get(r, F_V));
     double lwv = 0., lcu = 0., aW = 0.;
     if (live && __any_sync(0xffffffffu, lv != 0.)) {
       // v = vd - dt (uc fx + ...), the flux below the cell with the layer-nlay Courant number
-      const double uc = uck[rr];
+      const double uc = ring.get(r, F_UC);
       const bool c0 = dtdx * cv0 > 0., c1 = dtdx * cv1 > 0.;
       const double den = 1. / (1. - dtdy * (cv1 - cv0));
       const double f0 = c0 ? wm : w0, f1 = c1 ? w0 : w1;
@@ -1067,14 +1205,10 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_d_mom_adj_x(Geom g, C
     lv1 = lv;
     u0 = u1;
     u1 = un;
-    un = row(ud, r + 3);
-    v1 = row(vd, r + 2);
     wm = w0;
     w0 = w1;
     cum = cu0;
-    cu0 = row(uL, r + 1);
     cv0 = cv1;
-    cv1 = row(vL, r + 2);
   }
 }
 
@@ -1082,6 +1216,7 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_d_mom_adj_x(Geom g, C
 // columns: lanes 1 to 29, over [0, n]^2 (the kinetic energy's range).
 constexpr int YOUT_DMOM = 29;
 static __global__ void __launch_bounds__(MW * MWARPS, 3) k_d_mom_adj_y(Geom g, Consts c, DMomAdjArgs a, int tys) {
+  extern __shared__ double adj_sm[];
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
   const int ox = (int)(blockIdx.x * MWARPS + (threadIdx.x >> 5)) * YOUT_DMOM, oy = (int)blockIdx.y * tys;
   if (ox > g.nx) return;
@@ -1097,27 +1232,48 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_d_mom_adj_y(Geom g, C
   double *lam_ud = a.lam_ud + kS, *lam_vd = a.lam_vd + kS, *lam_vc = a.lam_vc + kS;
   double *lam_uL = a.lam_uc + LS, *lam_vL = a.lam_vc + LS;
 
-  auto row = [&](const double* q, int y) { return q[row_of(g, y) + xi]; };
+  // iteration r brings rows r+1 of ud, r of vd and of layer-nlay uc and, with
+  // i = r-2, rows i of lam_udo, lam_vdo, vc and layer-nlay vc, r-5 of layer-nlay uc
+  enum { F_U, F_V, F_C, F_LU, F_LV, F_VC, F_CV, F_CS };
+  const RowRing<8, 4> ring(adj_sm);
+  auto issue = [&](int r) {
+    if (r < yend + 8) {
+      const int i = r - 2;
+      const unsigned r0 = row_of(g, r) + xi, i0 = row_of(g, i) + xi;
+      ring.copy(r, F_U, ud + (row_of(g, r + 1) + xi));
+      ring.copy(r, F_V, vd + r0);
+      ring.copy(r, F_C, uL + r0);
+      if (i >= 0 && i < g.ny) {
+        ring.copy(r, F_LU, lam_udo + i0);
+        ring.copy(r, F_LV, lam_vdo + i0);
+      }
+      ring.copy(r, F_VC, vck + i0);
+      ring.copy(r, F_CV, vL + i0);
+      ring.copy(r, F_CS, uL + (row_of(g, r - 5) + xi));
+    }
+    ring.commit();
+  };
+  issue(oy - 3);
+  issue(oy - 2);
   YLineAdj<PPM_CON> lt, lv_;  // the inner x sweep of the vorticity, vd, along y
   double w1 = 0, w2 = 0, w3 = 0, w4 = 0, w5 = 0;  // vorticity of rows r-1 .. r-5
-  double u0 = row(ud, oy - 3), un = row(ud, oy - 2), vn = row(vd, oy - 3), cn = row(uL, oy - 3);
+  double u0 = ud[row_of(g, oy - 3) + xi];
   double lvp = 0, Wp = 0;                         // lam_vdo of row i-1; adjoint of the vorticity of row s-1
 #pragma unroll 1
   for (int r = oy - 3; r < yend + 8; ++r) {
+    issue(r + 2);
+    ring.wait();
     const int i = r - 2, s = r - 5;
     const unsigned ii = row_of(g, i) + xi, si = row_of(g, s) + xi;
     const bool ownr = own && i >= oy && i < yend;
     double lu = 0., lv = 0.;  // lam_udo, lam_vdo of row i over the domain
     if (dom && i >= 0 && i < g.ny) {
-      lu = lam_udo[ii];
-      lv = lam_vdo[ii];
+      lu = ring.get(r, F_LU);
+      lv = ring.get(r, F_LV);
     }
-    const double vc = vck[ii], cv = vL[ii], cus = uL[si];
+    const double vc = ring.get(r, F_VC), cv = ring.get(r, F_CV), cus = ring.get(r, F_CS);
     // ---- forward: row r
-    const double u1 = un, v = vn, cu = cn;
-    un = row(ud, r + 2);
-    vn = row(vd, r + 1);
-    cn = row(uL, r + 1);
+    const double u1 = ring.get(r, F_U), v = ring.get(r, F_V), cu = ring.get(r, F_C);
     const double w = f - (u1 - u0) * rdy + (shfl_dn(v, 1) - v) * rdx;
     u0 = u1;
     {

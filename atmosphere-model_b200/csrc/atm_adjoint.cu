@@ -42,19 +42,21 @@ cudaError_t adj_mass(const Geom& g, const Consts& c, const double* dp, const dou
                      int hi, bool cgrid, cudaStream_t s, int part) {
   const MassAdjArgs a{dp, pt, u, v, dpo, pto, lam_dpo, lam_pto, lam_dp, lam_pt, lam_u, lam_v};
   const int w = g.nx - lo + hi, h = g.ny - lo + hi;
-  if (part == 1) {
-    const int rows = adj_rows(w, h, g.L, MOUT, 4);
-    const dim3 grid = adj_strips(w, h, g.L, MOUT, rows);
-    if (cgrid) k_mass_adj_x<true><<<grid, MW * MWARPS, 0, s>>>(g, c, a, lo, hi, rows);
-    else k_mass_adj_x<false><<<grid, MW * MWARPS, 0, s>>>(g, c, a, lo, hi, rows);
-  } else {
-    const int rows = adj_rows(w, h, g.L, YOUT_MASS, 11);
-    const dim3 grid = adj_strips(w, h, g.L, YOUT_MASS, rows);
-    if (cgrid) k_mass_adj_y<true><<<grid, MW * MWARPS, 0, s>>>(g, c, a, lo, hi, rows);
-    else k_mass_adj_y<false><<<grid, MW * MWARPS, 0, s>>>(g, c, a, lo, hi, rows);
-  }
-  return cudaGetLastError();
+  const bool xb = part == 1;
+  const int out = xb ? MOUT : YOUT_MASS, rows = adj_rows(w, h, g.L, out, xb ? 4 : 11);
+  const size_t sm = mass_adj_smem(cgrid, xb);
+  auto run = [&](auto kernel) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    kernel<<<adj_strips(w, h, g.L, out, rows), MW * MWARPS, sm, s>>>(g, c, a, lo, hi, rows);
+    return cudaGetLastError();
+  };
+  if (xb) return cgrid ? run(k_mass_adj_x<true>) : run(k_mass_adj_x<false>);
+  return cgrid ? run(k_mass_adj_y<true>) : run(k_mass_adj_y<false>);
 }
+
+// shared memory of a block's row rings (at most 32 KB)
+constexpr size_t ADJ_RING7 = MWARPS * RowRing<7, 4>::bytes, ADJ_RING8 = MWARPS * RowRing<8, 4>::bytes;
 
 cudaError_t adj_c_mom(const Geom& g, const Consts& c, const double* ud, const double* vd, const double* lam_uc,
                       const double* lam_vc, double* lam_ud, double* lam_vd, double* lam_w, double* lam_uc1,
@@ -66,9 +68,9 @@ cudaError_t adj_c_mom(const Geom& g, const Consts& c, const double* ud, const do
       (e = cudaMemsetAsync(lam_vc1, 0, lay, s)) || (e = cudaMemsetAsync(lam_nlay, 0, (size_t)g.S * 2 * 8, s)))
     return e;
   int rows = adj_rows(g.nx, g.ny, g.L, MOUT, 3);
-  k_c_mom_adj_x<<<adj_strips(g.nx, g.ny, g.L, MOUT, rows), MW * MWARPS, 0, s>>>(g, c, a, rows);
+  k_c_mom_adj_x<<<adj_strips(g.nx, g.ny, g.L, MOUT, rows), MW * MWARPS, ADJ_RING7, s>>>(g, c, a, rows);
   rows = adj_rows(g.nx + 1, g.ny + 1, g.L, YOUT_CMOM, 10);
-  k_c_mom_adj_y<<<adj_strips(g.nx + 1, g.ny + 1, g.L, YOUT_CMOM, rows), MW * MWARPS, 0, s>>>(g, c, a, rows);
+  k_c_mom_adj_y<<<adj_strips(g.nx + 1, g.ny + 1, g.L, YOUT_CMOM, rows), MW * MWARPS, ADJ_RING7, s>>>(g, c, a, rows);
   k_c_mom_adj_fin<<<dim3((g.nx + 8 + 127) / 128, g.ny + 8, g.L), 128, 0, s>>>(g, c, a);
   return cudaGetLastError();
 }
@@ -79,10 +81,10 @@ cudaError_t adj_d_mom(const Geom& g, const Consts& c, const double* ud, const do
   const DMomAdjArgs a{ud, vd, uc, vc, lam_udo, lam_vdo, lam_ud, lam_vd, lam_uc, lam_vc};
   if (part == 1) {
     const int rows = adj_rows(g.nx, g.ny, g.L, MOUT, 6);
-    k_d_mom_adj_x<<<adj_strips(g.nx, g.ny, g.L, MOUT, rows), MW * MWARPS, 0, s>>>(g, c, a, rows);
+    k_d_mom_adj_x<<<adj_strips(g.nx, g.ny, g.L, MOUT, rows), MW * MWARPS, ADJ_RING7, s>>>(g, c, a, rows);
   } else {
     const int rows = adj_rows(g.nx + 1, g.ny + 1, g.L, YOUT_DMOM, 11);
-    k_d_mom_adj_y<<<adj_strips(g.nx + 1, g.ny + 1, g.L, YOUT_DMOM, rows), MW * MWARPS, 0, s>>>(g, c, a, rows);
+    k_d_mom_adj_y<<<adj_strips(g.nx + 1, g.ny + 1, g.L, YOUT_DMOM, rows), MW * MWARPS, ADJ_RING8, s>>>(g, c, a, rows);
   }
   return cudaGetLastError();
 }
