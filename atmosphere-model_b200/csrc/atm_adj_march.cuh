@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_x(Geom g, Consts c,
   constexpr int V = CGRID ? PPM_UNC : PPM_NN;
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
   const int xhi = g.nx - 1 + hi, yhi = g.ny - 1 + hi;
-  const int ox = lo + (int)(blockIdx.x * MWARPS + (threadIdx.x >> 5)) * MOUT, oy = lo + (int)blockIdx.y * tys;
+  const int ox = lo + strip_x() * MOUT, oy = lo + (int)blockIdx.y * tys;
   if (ox > xhi) return;
   const int x = ox - MXH + lane, yend = min(oy + tys, yhi + 1);
   const bool own = lane >= MXH && lane < MXH + MOUT && x <= xhi, in = x < g.nx + H;
@@ -479,8 +479,8 @@ __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_x(Geom g, Consts c,
 // The y branch: the outer y fluxes, the inner x sweeps, the y part of the
 // damping of pt.  Own columns: lanes 1 to 30.
 constexpr int YOUT_MASS = 30;
-constexpr size_t mass_adj_smem(bool cgrid, bool xb) {
-  return MWARPS * (size_t)(!xb ? RowRing<8, 8>::bytes : cgrid ? RowRing<9, 4>::bytes : RowRing<8, 4>::bytes);
+constexpr int mass_adj_smem(bool cgrid, bool xb) {  // of a warp
+  return (!xb ? RowRing<8, 8>::bytes : cgrid ? RowRing<9, 4>::bytes : RowRing<8, 4>::bytes);
 }
 template <bool CGRID>
 __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_y(Geom g, Consts c, MassAdjArgs a, int lo, int hi, int tys) {
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_y(Geom g, Consts c,
   constexpr int V = CGRID ? PPM_UNC : PPM_NN;
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
   const int xhi = g.nx - 1 + hi, yhi = g.ny - 1 + hi;
-  const int ox = lo + (int)(blockIdx.x * MWARPS + (threadIdx.x >> 5)) * YOUT_MASS, oy = lo + (int)blockIdx.y * tys;
+  const int ox = lo + strip_x() * YOUT_MASS, oy = lo + (int)blockIdx.y * tys;
   if (ox > xhi) return;
   const int x = ox - 1 + lane, yend = min(oy + tys, yhi + 1);
   const bool own = lane >= 1 && lane <= YOUT_MASS && x <= xhi, in = x < g.nx + H;
@@ -637,7 +637,7 @@ struct CMomAdjArgs {
 static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_x(Geom g, Consts c, CMomAdjArgs a, int tys) {
   extern __shared__ double adj_sm[];
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
-  const int ox = (int)(blockIdx.x * MWARPS + (threadIdx.x >> 5)) * MOUT, oy = (int)blockIdx.y * tys;
+  const int ox = strip_x() * MOUT, oy = (int)blockIdx.y * tys;
   if (ox >= g.nx) return;
   const int x = ox - MXH + lane, yend = min(oy + tys, g.ny);
   const bool own = lane >= MXH && lane < MXH + MOUT && x < g.nx, in = x < g.nx + H;
@@ -769,7 +769,7 @@ constexpr int YOUT_CMOM = 28;
 static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_y(Geom g, Consts c, CMomAdjArgs a, int tys) {
   extern __shared__ double adj_sm[];
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
-  const int ox = -1 + (int)(blockIdx.x * MWARPS + (threadIdx.x >> 5)) * YOUT_CMOM, oy = -1 + (int)blockIdx.y * tys;
+  const int ox = -1 + strip_x() * YOUT_CMOM, oy = -1 + (int)blockIdx.y * tys;
   if (ox >= g.nx) return;
   const int x = ox - 2 + lane, yend = min(oy + tys, g.ny);
   const bool own = lane >= 2 && lane < 2 + YOUT_CMOM && x < g.nx, in = x < g.nx + H;
@@ -1080,7 +1080,7 @@ struct DMomAdjArgs {
 static __global__ void __launch_bounds__(MW * MWARPS, 3) k_d_mom_adj_x(Geom g, Consts c, DMomAdjArgs a, int tys) {
   extern __shared__ double adj_sm[];
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
-  const int ox = (int)(blockIdx.x * MWARPS + (threadIdx.x >> 5)) * MOUT, oy = (int)blockIdx.y * tys;
+  const int ox = strip_x() * MOUT, oy = (int)blockIdx.y * tys;
   if (ox >= g.nx) return;
   const int x = ox - MXH + lane, yend = min(oy + tys, g.ny);
   const bool own = lane >= MXH && lane < MXH + MOUT && x < g.nx, in = x < g.nx + H;
@@ -1218,7 +1218,7 @@ constexpr int YOUT_DMOM = 29;
 static __global__ void __launch_bounds__(MW * MWARPS, 3) k_d_mom_adj_y(Geom g, Consts c, DMomAdjArgs a, int tys) {
   extern __shared__ double adj_sm[];
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
-  const int ox = (int)(blockIdx.x * MWARPS + (threadIdx.x >> 5)) * YOUT_DMOM, oy = (int)blockIdx.y * tys;
+  const int ox = strip_x() * YOUT_DMOM, oy = (int)blockIdx.y * tys;
   if (ox > g.nx) return;
   const int x = ox - 1 + lane, yend = min(oy + tys, g.ny + 1);
   const bool own = lane >= 1 && lane <= YOUT_DMOM && x <= g.nx, in = x < g.nx + H;

@@ -5,33 +5,14 @@
 #include "atm_adj_march.cuh"
 #include "atm_adjoint.cuh"
 #include "atm_ops.h"
+#include "atm_strips.h"
 
 namespace atm {
 namespace {
 
-// grid of a marching reverse over w columns (out a warp) and h rows in strips of tys
-inline dim3 adj_strips(int w, int h, int layers, int out, int tys) {
-  return dim3((w + out * MWARPS - 1) / (out * MWARPS), (h + tys - 1) / tys, layers);
-}
-
-// strip height of a marching reverse with `warm` rows beside the strip's own,
-// as strip_rows of atm_launch.cuh
-inline int adj_rows(int w, int h, int layers, int out, int warm) {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    sms = 148;
-  const long long slots = (long long)sms * 3;
-  int best = 8;
-  long long cost = -1;
-  for (int r = 128; r >= 4; r >>= 1) {
-    const dim3 b = adj_strips(w, h, layers, out, r);
-    const long long t = (((long long)b.x * b.y * b.z + slots - 1) / slots) * (min(r, h) + warm);
-    if (cost < 0 || t < cost) {
-      cost = t;
-      best = r;
-    }
-  }
-  return best;
+// strips of a marching reverse over w x h points, `warm` rows beside the strip's own
+inline StripPlan adj_strips(int w, int h, int layers, int out, int warm) {
+  return plan_strips(w, h, layers, out, warm, 3 * MWARPS);
 }
 
 }  // namespace
@@ -43,20 +24,21 @@ cudaError_t adj_mass(const Geom& g, const Consts& c, const double* dp, const dou
   const MassAdjArgs a{dp, pt, u, v, dpo, pto, lam_dpo, lam_pto, lam_dp, lam_pt, lam_u, lam_v};
   const int w = g.nx - lo + hi, h = g.ny - lo + hi;
   const bool xb = part == 1;
-  const int out = xb ? MOUT : YOUT_MASS, rows = adj_rows(w, h, g.L, out, xb ? 4 : 11);
-  const size_t sm = mass_adj_smem(cgrid, xb);
+  const StripPlan p = adj_strips(w, h, g.L, xb ? MOUT : YOUT_MASS, xb ? 4 : 11);
+  const int sm = p.threads / MW * mass_adj_smem(cgrid, xb);
   auto run = [&](auto kernel) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               MWARPS * mass_adj_smem(cgrid, xb));
     if (e != cudaSuccess) return e;
-    kernel<<<adj_strips(w, h, g.L, out, rows), MW * MWARPS, sm, s>>>(g, c, a, lo, hi, rows);
+    kernel<<<p.grid, p.threads, sm, s>>>(g, c, a, lo, hi, p.rows);
     return cudaGetLastError();
   };
   if (xb) return cgrid ? run(k_mass_adj_x<true>) : run(k_mass_adj_x<false>);
   return cgrid ? run(k_mass_adj_y<true>) : run(k_mass_adj_y<false>);
 }
 
-// shared memory of a block's row rings (at most 32 KB)
-constexpr size_t ADJ_RING7 = MWARPS * RowRing<7, 4>::bytes, ADJ_RING8 = MWARPS * RowRing<8, 4>::bytes;
+// shared memory of a warp's row ring (at most 32 KB a block)
+constexpr int ADJ_RING7 = RowRing<7, 4>::bytes, ADJ_RING8 = RowRing<8, 4>::bytes;
 
 cudaError_t adj_c_mom(const Geom& g, const Consts& c, const double* ud, const double* vd, const double* lam_uc,
                       const double* lam_vc, double* lam_ud, double* lam_vd, double* lam_w, double* lam_uc1,
@@ -67,10 +49,10 @@ cudaError_t adj_c_mom(const Geom& g, const Consts& c, const double* ud, const do
   if ((e = cudaMemsetAsync(lam_w, 0, lay, s)) || (e = cudaMemsetAsync(lam_uc1, 0, lay, s)) ||
       (e = cudaMemsetAsync(lam_vc1, 0, lay, s)) || (e = cudaMemsetAsync(lam_nlay, 0, (size_t)g.S * 2 * 8, s)))
     return e;
-  int rows = adj_rows(g.nx, g.ny, g.L, MOUT, 3);
-  k_c_mom_adj_x<<<adj_strips(g.nx, g.ny, g.L, MOUT, rows), MW * MWARPS, ADJ_RING7, s>>>(g, c, a, rows);
-  rows = adj_rows(g.nx + 1, g.ny + 1, g.L, YOUT_CMOM, 10);
-  k_c_mom_adj_y<<<adj_strips(g.nx + 1, g.ny + 1, g.L, YOUT_CMOM, rows), MW * MWARPS, ADJ_RING7, s>>>(g, c, a, rows);
+  StripPlan p = adj_strips(g.nx, g.ny, g.L, MOUT, 3);
+  k_c_mom_adj_x<<<p.grid, p.threads, p.threads / MW * ADJ_RING7, s>>>(g, c, a, p.rows);
+  p = adj_strips(g.nx + 1, g.ny + 1, g.L, YOUT_CMOM, 10);
+  k_c_mom_adj_y<<<p.grid, p.threads, p.threads / MW * ADJ_RING7, s>>>(g, c, a, p.rows);
   k_c_mom_adj_fin<<<dim3((g.nx + 8 + 127) / 128, g.ny + 8, g.L), 128, 0, s>>>(g, c, a);
   return cudaGetLastError();
 }
@@ -80,11 +62,11 @@ cudaError_t adj_d_mom(const Geom& g, const Consts& c, const double* ud, const do
                       double* lam_uc, double* lam_vc, cudaStream_t s, int part) {
   const DMomAdjArgs a{ud, vd, uc, vc, lam_udo, lam_vdo, lam_ud, lam_vd, lam_uc, lam_vc};
   if (part == 1) {
-    const int rows = adj_rows(g.nx, g.ny, g.L, MOUT, 6);
-    k_d_mom_adj_x<<<adj_strips(g.nx, g.ny, g.L, MOUT, rows), MW * MWARPS, ADJ_RING7, s>>>(g, c, a, rows);
+    const StripPlan p = adj_strips(g.nx, g.ny, g.L, MOUT, 6);
+    k_d_mom_adj_x<<<p.grid, p.threads, p.threads / MW * ADJ_RING7, s>>>(g, c, a, p.rows);
   } else {
-    const int rows = adj_rows(g.nx + 1, g.ny + 1, g.L, YOUT_DMOM, 11);
-    k_d_mom_adj_y<<<adj_strips(g.nx + 1, g.ny + 1, g.L, YOUT_DMOM, rows), MW * MWARPS, ADJ_RING8, s>>>(g, c, a, rows);
+    const StripPlan p = adj_strips(g.nx + 1, g.ny + 1, g.L, YOUT_DMOM, 11);
+    k_d_mom_adj_y<<<p.grid, p.threads, p.threads / MW * ADJ_RING8, s>>>(g, c, a, p.rows);
   }
   return cudaGetLastError();
 }

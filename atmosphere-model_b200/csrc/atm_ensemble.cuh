@@ -177,7 +177,7 @@ __device__ __noinline__ void ens_cmass(const EnsMember& M, int cur, long long li
   ens_strip_item(M.g, -2, 2, M.tys, li, [&](int sx, int sy, int k) {
     void* const* so = M.st[cur];
     mass_strip<T, true, S, C, false>(M.g, M.cc, (const S*)so[0], (const S*)so[1], (const S*)so[2], (const S*)so[3],
-                                   nullptr, (C*)M.cg[0], (C*)M.cg[1], -2, 2, nullptr, sx, sy, k, M.tys);
+                                   nullptr, (C*)M.cg[0], (C*)M.cg[1], -2, 2, nullptr, sx, sy, k, M.tys, nullptr);
   });
 }
 template <typename T, typename S, typename C>
@@ -185,7 +185,7 @@ __device__ __noinline__ void ens_cmom(const EnsMember& M, int cur, long long li)
   ens_strip_item(M.g, 0, 0, M.tys, li, [&](int sx, int sy, int k) {
     void* const* so = M.st[cur];
     c_mom_strip<T, S, C, false>(M.g, M.cc, (const S*)so[2], (const S*)so[3], M.pkap, M.gz, (C*)M.cg[2], (C*)M.cg[3],
-                              sx, sy, k, M.tys);
+                              sx, sy, k, M.tys, nullptr);
   });
 }
 template <typename T, typename S, typename C>
@@ -194,7 +194,7 @@ __device__ __noinline__ void ens_dmass(const EnsMember& M, int cur, long long li
     void* const* so = M.st[cur];
     void* const* sn = M.st[cur ^ 1];
     mass_strip<T, false, S, C, false>(M.g, M.cd, (const S*)so[0], (const S*)so[1], (const C*)M.cg[2], (const C*)M.cg[3],
-                                    nullptr, (S*)sn[0], (S*)sn[1], -3, 3, &M.status->nonfinite_step, sx, sy, k, M.tys);
+                                    nullptr, (S*)sn[0], (S*)sn[1], -3, 3, &M.status->nonfinite_step, sx, sy, k, M.tys, nullptr);
   });
 }
 template <typename T, typename S, typename C>
@@ -203,7 +203,7 @@ __device__ __noinline__ void ens_dmom(const EnsMember& M, int cur, long long li)
     void* const* so = M.st[cur];
     void* const* sn = M.st[cur ^ 1];
     d_mom_strip<T, S, C, false>(M.g, M.cd, (const S*)so[2], (const S*)so[3], (const C*)M.cg[2], (const C*)M.cg[3],
-                              M.pkapb, M.gzb, (S*)sn[2], (S*)sn[3], &M.status->nonfinite_step, sx, sy, k, M.tys);
+                              M.pkapb, M.gzb, (S*)sn[2], (S*)sn[3], &M.status->nonfinite_step, sx, sy, k, M.tys, nullptr);
   });
 }
 

@@ -7,6 +7,7 @@
 #include "atm_march.cuh"
 #include "atm_ops.h"
 #include "atm_remap.cuh"
+#include "atm_strips.h"
 
 namespace atm {
 namespace {
@@ -14,47 +15,22 @@ namespace {
 using T = ATM_FORM_T;  // sweep arithmetic
 using S = double;      // prognostic state (dp, pt, ud, vd), both forms
 using C = T;           // C-grid fields (dpc, ptc, uc, vc)
-// strips of tys output rows of the marching sweeps over [lo, n-1+hi]^2
-inline dim3 strips(int lo, int hi, const Geom& g, int tys) {
-  int w = g.nx - lo + hi, h = g.ny - lo + hi;
-  return dim3((w + MOUT * MWARPS - 1) / (MOUT * MWARPS), (h + tys - 1) / tys, g.L);
-}
-
-// Strip height (output rows a warp walks through), chosen per launch: a strip
-// costs its rows and six warm-up rows, and the launch as many strips as the
-// resident blocks take in turn.
-// Measured on B200, mixed form: 150x130x48 C mass 0.061 ms at 32 rows, 0.047
-// at the 16 this picks; 1024x1024x64 takes 128.
+// strips of kernel K over [lo, n-1+hi]^2 (six rows fill the windows)
 template <int K>
-inline int strip_rows(int lo, int hi, const Geom& g) {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    sms = 148;
-  const long long slots = (long long)sms * MarchL<T, K>::min_blocks;
-  int best = 8;
-  long long cost = -1;
-  for (int r = 128; r >= 4; r >>= 1) {
-    const dim3 b = strips(lo, hi, g, r);
-    const long long waves = ((long long)b.x * b.y * b.z + slots - 1) / slots;
-    const long long t = waves * (min(r, g.ny - lo + hi) + 6);
-    if (cost < 0 || t < cost) {
-      cost = t;
-      best = r;
-    }
-  }
-  return best;
+inline StripPlan strips(int lo, int hi, const Geom& g) {
+  return plan_strips(g.nx - lo + hi, g.ny - lo + hi, g.L, MOUT, 6, MarchL<T, K>::min_blocks * MWARPS);
 }
 
 cudaError_t mass(const Geom& g, const Consts& c, const void* dp, const void* pt, const void* u, const void* v,
                  const double* heat, void* dpo, void* pto, int lo, int hi, int* nonfinite, bool cgrid, cudaStream_t s) {
   if (cgrid) {  // state in, C-grid fields out
-    const int rows = strip_rows<MK_CMASS>(lo, hi, g);
-    k_mass_m<T, true, S, C><<<strips(lo, hi, g, rows), MW * MWARPS, 0, s>>>(
-        g, c, (const S*)dp, (const S*)pt, (const S*)u, (const S*)v, heat, (C*)dpo, (C*)pto, lo, hi, nonfinite, rows);
+    const StripPlan p = strips<MK_CMASS>(lo, hi, g);
+    k_mass_m<T, true, S, C><<<p.grid, p.threads, p.threads / MW * MASS_SMEM<T, true, S> + FEED_PAD, s>>>(
+        g, c, (const S*)dp, (const S*)pt, (const S*)u, (const S*)v, heat, (C*)dpo, (C*)pto, lo, hi, nonfinite, p.rows);
   } else {  // state and C-grid winds in, state out
-    const int rows = strip_rows<MK_DMASS>(lo, hi, g);
-    k_mass_m<T, false, S, C><<<strips(lo, hi, g, rows), MW * MWARPS, 0, s>>>(
-        g, c, (const S*)dp, (const S*)pt, (const C*)u, (const C*)v, heat, (S*)dpo, (S*)pto, lo, hi, nonfinite, rows);
+    const StripPlan p = strips<MK_DMASS>(lo, hi, g);
+    k_mass_m<T, false, S, C><<<p.grid, p.threads, p.threads / MW * MASS_SMEM<T, false, S> + FEED_PAD, s>>>(
+        g, c, (const S*)dp, (const S*)pt, (const C*)u, (const C*)v, heat, (S*)dpo, (S*)pto, lo, hi, nonfinite, p.rows);
   }
   return cudaGetLastError();
 }
@@ -92,17 +68,17 @@ cudaError_t heating(const Geom& g, const Consts& c, const void* dpl, int es, con
 
 cudaError_t c_mom(const Geom& g, const Consts& c, const void* ud, const void* vd, const double* pkap, const double* gz,
                   void* uc, void* vc, cudaStream_t s) {
-  const int rows = strip_rows<MK_CMOM>(0, 0, g);
-  k_c_mom_m<T, S, C><<<strips(0, 0, g, rows), MW * MWARPS, 0, s>>>(g, c, (const S*)ud, (const S*)vd, pkap, gz, (C*)uc,
-                                                                    (C*)vc, rows);
+  const StripPlan p = strips<MK_CMOM>(0, 0, g);
+  k_c_mom_m<T, S, C><<<p.grid, p.threads, p.threads / MW * FEED_BYTES<CMOM_NF, 0>, s>>>(
+      g, c, (const S*)ud, (const S*)vd, pkap, gz, (C*)uc, (C*)vc, p.rows);
   return cudaGetLastError();
 }
 
 cudaError_t d_mom(const Geom& g, const Consts& c, const void* ud, const void* vd, const void* uc, const void* vc,
                   const double* pkapb, const double* gzb, void* udo, void* vdo, int* nonfinite, cudaStream_t s) {
-  const int rows = strip_rows<MK_DMOM>(0, 0, g);
-  k_d_mom_m<T, S, C><<<strips(0, 0, g, rows), MW * MWARPS, 0, s>>>(
-      g, c, (const S*)ud, (const S*)vd, (const C*)uc, (const C*)vc, pkapb, gzb, (S*)udo, (S*)vdo, nonfinite, rows);
+  const StripPlan p = strips<MK_DMOM>(0, 0, g);
+  k_d_mom_m<T, S, C><<<p.grid, p.threads, p.threads / MW * FEED_BYTES<DMOM_NF<std::is_same_v<S, T>>, 0>, s>>>(
+      g, c, (const S*)ud, (const S*)vd, (const C*)uc, (const C*)vc, pkapb, gzb, (S*)udo, (S*)vdo, nonfinite, p.rows);
   return cudaGetLastError();
 }
 

@@ -7,22 +7,23 @@
 // (the last few rows of every stage) in registers, so that every stage of the
 // reference's layer loop is evaluated once per cell instead of once per
 // cell of every overlapping tile halo; x-direction neighbours come from the
-// neighbouring lanes by warp shuffles.  No shared memory and no block-wide
-// barrier: the warps of a block are independent.  Each iteration loads the
-// inputs of the next row before working on the current one, so that the
-// loads' latency overlaps a row of arithmetic.
+// neighbouring lanes by warp shuffles.  The warps of a block are independent
+// (no block-wide barrier); each row's inputs are copied into the warp's part of
+// shared memory two rows ahead (FeedRing).
 //
-// The sweeps are bound by instruction issue (HBM traffic is the fields read
-// and written once, 0.5 ms of a kernel at 1024x1024x64), so the formulas are
-// arranged for the fewest instructions that give the reference's bits: a
-// difference of two neighbours is formed once and serves the slopes of both
-// cells and the two edges between them (YLine, xline_flux), each cell's edges
-// are formed and limited once, exact products are fused, and the division by
-// three needs no branch.  Measured on B200 at 1024x1024x64 (ms a launch, C
-// mass / C momentum / D mass / D momentum; before: FP64 sweeps on 32 x 4-8
-// shared-memory tiles, FP32 marching with per-flux edges):
-//   FP64  4.24 / 4.03 / 4.58 / 4.92  ->  1.93 / 2.61 / 2.38 / 2.69
-//   FP32  1.63 / 2.02 / 1.70 / 2.29  ->  1.23 / 1.65 / 1.27 / 1.60
+// The sweeps are bound by the latency of their FP64 (FP32) chains at the warps
+// that the registers leave, then by instruction issue (HBM traffic is the
+// fields read and written once, 0.5 ms of a kernel at 1024x1024x64), so the
+// formulas are arranged for the fewest instructions that give the reference's
+// bits: a difference of two neighbours is formed once and serves the slopes of
+// both cells and the two edges between them (YLine, xline_flux), each cell's
+// edges are formed and limited once, exact products are fused, and the
+// division by three needs no branch.  Measured on B200 at 1024x1024x64 (ms a
+// launch, C mass / C momentum / D mass / D momentum; first: FP64 sweeps on 32 x
+// 4-8 shared-memory tiles, FP32 marching with per-flux edges; then marching
+// with each row loaded a row ahead into registers; now):
+//   FP64  4.24 / 4.03 / 4.58 / 4.92  ->  1.93 / 2.61 / 2.38 / 2.69  ->  1.73 / 2.17 / 2.05 / 2.39
+//   FP32  1.63 / 2.02 / 1.70 / 2.29  ->  1.23 / 1.65 / 1.27 / 1.60  ->  1.16 / 1.37 / 1.24 / 1.56
 //
 // Every value is the reference's expression (src/mod_sw_dyn.f90) up to the
 // sign of a zero; FP64 instances are bit-identical to the FP64 restatement.
@@ -40,24 +41,26 @@ namespace atm {
 constexpr int MW = 32;              // lanes (columns) of a strip
 constexpr int MXH = 3;              // halo columns on each side
 constexpr int MOUT = MW - 2 * MXH;  // output columns of a strip
-constexpr int MWARPS = 4;           // independent strips (warps) per block
+constexpr int MWARPS = 4;           // independent strips (warps) per block at most (atm_strips.h)
 
 // Register budget (blocks of four warps per SM) and rows per loop body of each
 // marching kernel.  The row windows shift by one register a row; unrolling by
 // n rows does n shifts at once (a window of w doubles costs 2w/n moves a row).
 // Measured on B200 at 1024x1024x64 (ms, C mass / C momentum / D mass / D
-// momentum):
-//   FP64, 3 blocks (168 registers), 1 / 2 / 3 / 4 rows: 2.33 2.68 2.75 2.74 /
-//     2.25 2.63 2.54 3.14 / 1.93 2.61 2.38 2.69 / 2.06 2.58 2.50 2.89;
-//     4 blocks, 1 row (spills): 2.40 3.01 2.58 2.88; 2 blocks: 2.35 3.34 2.80 3.50
-//   FP32, 4 blocks (128 registers), 1 / 2 / 3 / 4 rows: 1.23 1.73 1.58 1.73 /
-//     1.37 1.89 1.35 1.60 / 1.29 1.65 1.27 1.87 / 1.35 1.68 1.27 1.77
+// momentum), rows fed through shared memory:
+//   FP64, 3 blocks (168 registers), 1 / 2 / 3 / 4 rows: 1.93 2.18 2.26 2.42 /
+//     1.78 2.33 2.32 2.44 / 1.77 2.31 2.25 2.43 / 1.75 2.43 2.20 2.52;
+//     4 blocks (128 registers) with the windows of the inputs read back from
+//     shared memory instead of kept in registers, 1 / 2 rows: 1.91 2.35 2.13
+//     2.66 / 1.84 2.65 2.17 3.18: taken for D mass
+//   FP32, 4 blocks (128 registers), 1 / 2 / 3 / 4 rows: 1.22 1.47 1.34 1.62 /
+//     1.18 1.41 1.30 1.57 / 1.22 1.45 1.30 1.59 / 1.15 1.39 1.33 1.63
 enum { MK_CMASS, MK_DMASS, MK_CMOM, MK_DMOM };
 template <typename T, int K>
 struct MarchL {
   static constexpr bool F32 = std::is_same_v<T, float>;
-  static constexpr int min_blocks = F32 ? 4 : 3;
-  static constexpr int unroll = !F32 ? 3 : K == MK_CMASS ? 1 : K == MK_DMOM ? 2 : 3;
+  static constexpr int min_blocks = F32 || K == MK_DMASS ? 4 : 3;
+  static constexpr int unroll = F32 ? (K == MK_DMOM ? 2 : K == MK_DMASS ? 3 : 4) : K == MK_CMASS ? 4 : 1;
 };
 
 template <typename T>
@@ -288,6 +291,100 @@ __device__ __forceinline__ E ld(const E* level, unsigned i) {
   else return level[i];
 }
 
+// The inputs of a strip's rows, brought ahead of the row that works on them.
+// Ring: into shared memory by asynchronous copies two rows ahead, NF values a
+// lane and row; the first N8 fields keep eight rows, the others four.  Each
+// lane copies its own column and may read its neighbours' (d = -1, 1; past
+// the warp's ends some other value, which only feeds halo lanes).  early()
+// and late() issue the copies of one row.  Loads a row ahead into registers left
+// the FP64 sweeps waiting on them for 0.6 to 1.5 cycles an issued instruction:
+// 9.6 -> 8.6 ms a step of 1024x1024x64.
+template <int NF, int N8> constexpr int FEED_BYTES = (N8 * 8 + (NF - N8) * 4) * MW * 8;  // of a warp
+template <int NF, int N8>
+struct FeedRing {
+  char* p;
+  unsigned s;
+  __device__ __forceinline__ explicit FeedRing(char* sm) {
+    p = sm + (threadIdx.x >> 5) * FEED_BYTES<NF, N8>;
+    s = (unsigned)__cvta_generic_to_shared(p);
+  }
+  __device__ __forceinline__ static int slot(int r, int f) {
+    return (f < N8 ? (r & 7) * N8 + f : N8 * 8 + (r & 3) * (NF - N8) + (f - N8)) * (MW * 8);
+  }
+  template <typename E>
+  __device__ __forceinline__ void early(int r, int f, const E* q) const {
+    const unsigned to = s + slot(r, f) + (threadIdx.x & (MW - 1)) * sizeof(E);
+    if constexpr (sizeof(E) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to), "l"(q) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(q) : "memory");
+  }
+  template <typename E>
+  __device__ __forceinline__ void late(int r, int f, const E* q) const {
+    early(r, f, q);
+  }
+  __device__ __forceinline__ static void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+  template <typename A, typename B>
+  __device__ __forceinline__ void start(const A& e, const B& l, int j) const {
+    e(j);
+    l(j);
+    commit();
+    e(j + 1);
+    l(j + 1);
+    commit();
+  }
+  // the values of row j are there (all but the newest two groups have landed, in every lane)
+  template <typename A, typename B>
+  __device__ __forceinline__ void next(const A& e, const B& l, int j, int jend) const {
+    if (j + 2 < jend) {
+      e(j + 2);
+      l(j + 2);
+    }
+    commit();
+    asm volatile("cp.async.wait_group 2;" ::: "memory");
+    __syncwarp();
+  }
+  template <typename E>
+  __device__ __forceinline__ E get(int r, int f, int d = 0) const {
+    return *reinterpret_cast<const E*>(p + slot(r, f) + ((int)(threadIdx.x & (MW - 1)) + d) * (int)sizeof(E));
+  }
+};
+// Registers, for fields that the launch itself writes: early() a row ahead,
+// late() at the row's start; neighbours by shuffles.
+template <int NF, int N8>
+struct FeedRegs {
+  double cur[NF], nxt[NF];
+  __device__ __forceinline__ explicit FeedRegs(char*) {}
+  __device__ __forceinline__ static double bits(double v) { return v; }
+  __device__ __forceinline__ static double bits(float v) { return __hiloint2double(0, __float_as_int(v)); }
+  template <typename E>
+  __device__ __forceinline__ void early(int, int f, const E* q) {
+    nxt[f] = bits(*q);
+  }
+  template <typename E>
+  __device__ __forceinline__ void late(int, int f, const E* q) {
+    cur[f] = bits(*q);
+  }
+  template <typename A, typename B>
+  __device__ __forceinline__ void start(const A& e, const B&, int j) {
+    e(j);
+  }
+  template <typename A, typename B>
+  __device__ __forceinline__ void next(const A& e, const B& l, int j, int) {
+#pragma unroll
+    for (int f = 0; f < NF; ++f) cur[f] = nxt[f];
+    e(j + 1);
+    l(j);
+  }
+  template <typename E>
+  __device__ __forceinline__ E get(int, int f, int d = 0) const {
+    E v;
+    if constexpr (sizeof(E) == 8) v = cur[f];
+    else v = __int_as_float(__double2loint(cur[f]));
+    return d < 0 ? shfl_up(v, 1) : d > 0 ? shfl_dn(v, 1) : v;
+  }
+};
+template <bool RO, int NF, int N8>
+using Feed = std::conditional_t<RO, FeedRing<NF, N8>, FeedRegs<NF, N8>>;
+
 // ---------------------------------------------------------------- mass ----
 // The C-grid (CGRID) or D-grid mass and potential-temperature sweep of one
 // layer (src/mod_sw_dyn.f90:96-268 and 439-598): S the state type, C the
@@ -301,17 +398,20 @@ struct MassM {
   using O = std::conditional_t<CGRID, C, S>;   // outputs
 };
 
+template <bool RO, bool CGRID, bool SAME> constexpr int MASS_NF = SAME || RO ? (CGRID ? 5 : 4) : 7;
+template <bool CGRID, bool SAME> constexpr int MASS_N8 = !CGRID ? 3 : SAME ? 0 : 2;
 template <typename T, bool CGRID, typename S, typename C, bool RO = true>
 __device__ __forceinline__ void mass_strip(const Geom& g, const Consts& c, const S* dp, const S* pt,
                                            const typename MassM<T, CGRID, S, C>::UB* u,
                                            const typename MassM<T, CGRID, S, C>::UB* v, const double* heat,
                                            typename MassM<T, CGRID, S, C>::O* dpo,
                                            typename MassM<T, CGRID, S, C>::O* pto, int lo, int hi, int* nonfinite,
-                                           int sx, int sy, int k, int tys) {
+                                           int sx, int sy, int k, int tys, char* sm) {
   using UB = typename MassM<T, CGRID, S, C>::UB;
   using O = typename MassM<T, CGRID, S, C>::O;
   constexpr int V = CGRID ? PPM_UNC : PPM_NN;
   constexpr bool SAME = std::is_same_v<S, T>;
+  constexpr bool KEPT = SAME && RO && !CGRID;  // windows of dp, pt read back from the ring
   const int lane = threadIdx.x & (MW - 1);
   const int ox = lo + sx * MOUT;
   const int oy = lo + sy * tys;
@@ -352,30 +452,38 @@ __device__ __forceinline__ void mass_strip(const Geom& g, const Consts& c, const
   }
   bool bad = false;
   const int jend = min(oy + tys, yhi + 1) + 3;
-  unsigned r = row_of(g, oy - 3);
-  S dn_p = ld<RO>(dp, r + xi), pn_p = ld<RO>(pt, r + xi);
-  UB ua_p = ld<RO>(u, (CGRID ? row_of(g, oy - 2) : r) + xi);
-  r = row_of(g, oy - 5);
-  UB va_p = ld<RO>(v, r + xi), vb_p = CGRID ? ld<RO>(v, r + xr) : UB(0);
+  enum { F_DP, F_PT, F_U, F_V, F_VB, F_DU, F_PU };
+  Feed<RO, MASS_NF<RO, CGRID, SAME>, MASS_N8<CGRID, SAME>> feed(sm);
+  auto early = [&](int j) {
+    const unsigned r = row_of(g, j) + xi, rv = row_of(g, j - 2);
+    feed.early(j, F_DP, dp + r);
+    feed.early(j, F_PT, pt + r);
+    feed.early(j, F_U, u + (CGRID ? row_of(g, j + 1) + xi : r));
+    feed.early(j, F_V, v + (rv + xi));
+    if constexpr (CGRID) feed.early(j, F_VB, v + (rv + xr));
+  };
+  auto late = [&](int j) {  // the state values of row y (the update in the state's type)
+    if constexpr (!SAME && !RO) {
+      const unsigned r = row_of(g, j - 3) + xi;
+      feed.late(j, F_DU, dp + r);
+      feed.late(j, F_PU, pt + r);
+    }
+  };
+  feed.start(early, late, oy - 3);
 #pragma unroll MarchL<T, CGRID ? MK_CMASS : MK_DMASS>::unroll
   for (int j = oy - 3; j < jend; ++j) {
     // ---- row j: inputs, C-grid u, the inner x sweep (mod_sw_dyn.f90:109-117, 176-185; 503-511)
     const int y = j - 3;
     const unsigned oi = row_of(g, y) + xi;
-    S d_upd = 0, p_upd = 0;  // the state values of row y (the update in the state's type)
+    feed.next(early, late, j, jend);
+    S d_upd = 0, p_upd = 0;  // the state values of row y
     if constexpr (!SAME) {
-      d_upd = ld<RO>(dp, oi);
-      p_upd = ld<RO>(pt, oi);
+      d_upd = RO ? feed.template get<S>(y, F_DP) : feed.template get<S>(j, F_DU);
+      p_upd = RO ? feed.template get<S>(y, F_PT) : feed.template get<S>(j, F_PU);
     }
-    const T dn = T(dn_p), pn = T(pn_p);
-    const T ua_c = T(ua_p), va_c = T(va_p), vb_c = T(vb_p);
-    r = row_of(g, j + 1);
-    dn_p = ld<RO>(dp, r + xi);
-    pn_p = ld<RO>(pt, r + xi);
-    ua_p = ld<RO>(u, (CGRID ? row_of(g, j + 2) : r) + xi);
-    r = row_of(g, j - 1);
-    va_p = ld<RO>(v, r + xi);
-    if constexpr (CGRID) vb_p = ld<RO>(v, r + xr);
+    const T dn = T(feed.template get<S>(j, F_DP)), pn = T(feed.template get<S>(j, F_PT));
+    const T ua_c = T(feed.template get<UB>(j, F_U)), va_c = T(feed.template get<UB>(j, F_V));
+    const T vb_c = CGRID ? T(feed.template get<UB>(j, F_VB)) : T(0);
     T ucn;
     if constexpr (CGRID) {  // .5 (.5 (u + u(x-1)) + .5 (the row above)): the halvings are exact
       const T s = ua_c + shfl_up(ua_c, 1);
@@ -385,8 +493,18 @@ __device__ __forceinline__ void mass_strip(const Geom& g, const Consts& c, const
       ucn = ua_c;
     }
     const T ucR = shfl_dn(ucn, 1);
-    const T dL = shfl_up(dn, 1), dR = shfl_dn(dn, 1);
-    const T pL = shfl_up(pn, 1), pR = shfl_dn(pn, 1);
+    T dL, dR, pL, pR;
+    if constexpr (KEPT) {
+      dL = feed.template get<S>(j, F_DP, -1);
+      dR = feed.template get<S>(j, F_DP, 1);
+      pL = feed.template get<S>(j, F_PT, -1);
+      pR = feed.template get<S>(j, F_PT, 1);
+    } else {
+      dL = shfl_up(dn, 1);
+      dR = shfl_dn(dn, 1);
+      pL = shfl_up(pn, 1);
+      pR = shfl_dn(pn, 1);
+    }
     T txn, tpn;
     {
       const bool c0 = dtdx * ucn > T(0), c1 = dtdx * ucR > T(0);
@@ -395,11 +513,26 @@ __device__ __forceinline__ void mass_strip(const Geom& g, const Consts& c, const
       tpn = inner_e(pn, c0 ? pL : pn, c1 ? pn : pR, den, rA);
     }
     // shift the windows to the new row
-    d3 = d2; d2 = d1; d1 = d0; d0 = dn;
-    p3 = p2; p2 = p1; p1 = p0; p0 = pn;
-    ds2 = ds1; ds1 = ds0; ds0 = dR + dL;
-    ps2 = ps1; ps1 = ps0; ps0 = pR + pL;
-    uc3 = uc2; uc2 = uc1; uc1 = uc0; uc0 = ucn;
+    if constexpr (KEPT) {
+      d1 = feed.template get<S>(j - 1, F_DP);
+      d2 = feed.template get<S>(j - 2, F_DP);
+      d3 = feed.template get<S>(y, F_DP);
+      p1 = feed.template get<S>(j - 1, F_PT);
+      p2 = feed.template get<S>(j - 2, F_PT);
+      p3 = feed.template get<S>(y, F_PT);
+      ds2 = feed.template get<S>(j - 2, F_DP, 1) + feed.template get<S>(j - 2, F_DP, -1);
+      ps2 = feed.template get<S>(j - 2, F_PT, 1) + feed.template get<S>(j - 2, F_PT, -1);
+    } else {
+      d3 = d2; d2 = d1; d1 = d0; d0 = dn;
+      p3 = p2; p2 = p1; p1 = p0; p0 = pn;
+      ds2 = ds1; ds1 = ds0; ds0 = dR + dL;
+      ps2 = ps1; ps1 = ps0; ps0 = pR + pL;
+    }
+    if constexpr (RO && !CGRID) {
+      uc3 = T(feed.template get<UB>(y, F_U));
+    } else {
+      uc3 = uc2; uc2 = uc1; uc1 = uc0; uc0 = ucn;
+    }
     ld_.push(txn);
     lp_.push(tpn);
     // C-grid v of row j-2 (:109-117)
@@ -476,8 +609,15 @@ __device__ __forceinline__ void mass_strip(const Geom& g, const Consts& c, const
   if (nonfinite) flag_nonfinite(nonfinite, bad);
 }
 
-// one warp per strip: blockIdx.x * MWARPS + warp across x, blockIdx.y
+// shared memory of a warp, and of a block beside its warps' (the values past
+// the ends of the first and last warps' rows)
+constexpr int FEED_PAD = 16;
+template <typename T, bool CGRID, typename S>
+constexpr int MASS_SMEM = FEED_BYTES<MASS_NF<true, CGRID, std::is_same_v<S, T>>, MASS_N8<CGRID, std::is_same_v<S, T>>>;
+
+// one warp per strip: across x within the block and blockIdx.x, blockIdx.y
 // across y, blockIdx.z the layer
+__device__ __forceinline__ int strip_x() { return (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); }
 template <typename T, bool CGRID, typename S, typename C>
 __global__ void __launch_bounds__(MW * MWARPS, MarchL<T, CGRID ? MK_CMASS : MK_DMASS>::min_blocks) k_mass_m(Geom g, Consts c, const S* __restrict__ dp,
                                                          const S* __restrict__ pt,
@@ -487,8 +627,9 @@ __global__ void __launch_bounds__(MW * MWARPS, MarchL<T, CGRID ? MK_CMASS : MK_D
                                                          typename MassM<T, CGRID, S, C>::O* __restrict__ dpo,
                                                          typename MassM<T, CGRID, S, C>::O* __restrict__ pto, int lo,
                                                          int hi, int* nonfinite, int tys) {
-  mass_strip<T, CGRID, S, C>(g, c, dp, pt, u, v, heat, dpo, pto, lo, hi, nonfinite,
-                             blockIdx.x * MWARPS + (threadIdx.x >> 5), blockIdx.y, blockIdx.z, tys);
+  extern __shared__ __align__(16) char feed_sm[];
+  mass_strip<T, CGRID, S, C>(g, c, dp, pt, u, v, heat, dpo, pto, lo, hi, nonfinite, strip_x(), blockIdx.y, blockIdx.z,
+                             tys, feed_sm + 8);
 }
 
 // ======================================================== C-grid momentum ==
@@ -497,10 +638,11 @@ __global__ void __launch_bounds__(MW * MWARPS, MarchL<T, CGRID ? MK_CMASS : MK_D
 // layer-nlay A-grid winds (:299-317), absolute vorticity (:319-323), the
 // pressure-gradient force (:325-339) and the vorticity-flux updates of uc
 // and vc (:344-412).  Outputs on the interior; strips of tys rows.
+constexpr int CMOM_NF = 10;
 template <typename T, typename S, typename C, bool RO = true>
 __device__ __forceinline__ void c_mom_strip(const Geom& g, const Consts& c, const S* ud, const S* vd,
                                             const double* pkap, const double* gz, C* uc, C* vc, int sx, int sy, int k,
-                                            int tys) {
+                                            int tys, char* sm) {
   constexpr int UNC = PPM_UNC;
   const int lane = threadIdx.x & (MW - 1);
   const int ox = sx * MOUT;
@@ -538,27 +680,34 @@ __device__ __forceinline__ void c_mom_strip(const Geom& g, const Consts& c, cons
   T uL1 = T(ld<RO>(uL, row_of(g, oy - 1) + xi));
   T vL2 = T(ld<RO>(vL, row_of(g, oy - 2) + xi)), vL1 = T(ld<RO>(vL, row_of(g, oy - 1) + xi));
   const int jend = min(oy + tys, g.ny) + 3;
-  r = row_of(g, oy - 2);
-  S un_p = ld<RO>(uk, r + xi), unm_p = ld<RO>(uk, r + xl);
-  r = row_of(g, oy - 3);
-  S vn_p = ld<RO>(vk, r + xi), vnp_p = ld<RO>(vk, r + xr);
+  enum { F_U, F_UM, F_V, F_VP, F_P0, F_P1, F_G0, F_G1, F_UN, F_VN };
+  Feed<RO, CMOM_NF, 0> feed(sm);
+  auto early = [&](int j) {
+    const unsigned ru = row_of(g, j + 1), rv = row_of(g, j);
+    feed.early(j, F_U, uk + (ru + xi));
+    feed.early(j, F_UM, uk + (ru + xl));
+    feed.early(j, F_V, vk + (rv + xi));
+    feed.early(j, F_VP, vk + (rv + xr));
+  };
+  auto late = [&](int j) {  // the pressure terms of row y = j-3, layer-nlay winds of row y+1
+    const unsigned oi = row_of(g, j - 3) + xi, ri = row_of(g, j - 2) + xi;
+    feed.late(j, F_P0, pka + oi);
+    feed.late(j, F_P1, pkb + oi);
+    feed.late(j, F_G0, gza + oi);
+    feed.late(j, F_G1, gzb + oi);
+    feed.late(j, F_UN, uL + ri);
+    feed.late(j, F_VN, vL + ri);
+  };
+  feed.start(early, late, oy - 3);
 #pragma unroll MarchL<T, MK_CMOM>::unroll
   for (int j = oy - 3; j < jend; ++j) {
-    // loads of row y = j-3 issued before this row's work
     const int y = j - 3;
-    const unsigned oi = row_of(g, y) + xi, ri = row_of(g, j - 2) + xi;
-    const double pk0 = ld<RO>(pka, oi), pk1 = ld<RO>(pkb, oi), gz0 = ld<RO>(gza, oi), gz1 = ld<RO>(gzb, oi);
-    const S uL0_r = ld<RO>(uL, ri), vL0_r = ld<RO>(vL, ri);
+    const unsigned oi = row_of(g, y) + xi;
+    feed.next(early, late, j, jend);
     // ---- row j: C-grid winds of the layer (:110-117), vorticity (:319-323),
     // inner x sweep of the vorticity (:353-367)
-    const T un = T(un_p), unm = T(unm_p);
-    const T vn = T(vn_p), vnp = T(vnp_p);
-    r = row_of(g, j + 2);
-    un_p = ld<RO>(uk, r + xi);
-    unm_p = ld<RO>(uk, r + xl);
-    r = row_of(g, j + 1);
-    vn_p = ld<RO>(vk, r + xi);
-    vnp_p = ld<RO>(vk, r + xr);
+    const T un = T(feed.template get<S>(j, F_U)), unm = T(feed.template get<S>(j, F_UM));
+    const T vn = T(feed.template get<S>(j, F_V)), vnp = T(feed.template get<S>(j, F_VP));
     const T ucn = T(.25) * ((u_x + u_xm) + (un + unm));  // the reference's halvings are exact
     const T vcn = T(.25) * ((vn + v_x) + (vnp + v_xp));
     const T vor = fmadd(vcn - shfl_up(vcn, 1), rdx, fmadd(-(ucn - a0), rdy, f));
@@ -588,7 +737,7 @@ __device__ __forceinline__ void c_mom_strip(const Geom& g, const Consts& c, cons
     if (y >= oy - 1) {  // (the rows below are the strip's warm-up)
       // ---- row y: kinetic energy (:299-317) with the layer-nlay A-grid winds
       // (:110-125 at k = nlay), recomputed where they are read
-      const T uL0 = T(uL0_r), vL0 = T(vL0_r);
+      const T uL0 = T(feed.template get<S>(j, F_UN)), vL0 = T(feed.template get<S>(j, F_VN));
       T ken;
       {
         const T ub = T(.5) * (uL1 + shfl_up(uL1, 1));
@@ -608,6 +757,8 @@ __device__ __forceinline__ void c_mom_strip(const Geom& g, const Consts& c, cons
       vL1 = vL0;
       ke1 = ke0;
       ke0 = ken;
+      const double pk0 = feed.template get<double>(j, F_P0), pk1 = feed.template get<double>(j, F_P1);
+      const double gz0 = feed.template get<double>(j, F_G0), gz1 = feed.template get<double>(j, F_G1);
       const double pk0l = shfl_up(pk0, 1), pk1l = shfl_up(pk1, 1), gz0l = shfl_up(gz0, 1), gz1l = shfl_up(gz1, 1);
       const double pk0d = pk0m, pk1d = pk1m, gz0d = gz0m, gz1d = gz1m;  // row y-1
       pk0m = pk0; pk1m = pk1; gz0m = gz0; gz1m = gz1;
@@ -631,15 +782,13 @@ __device__ __forceinline__ void c_mom_strip(const Geom& g, const Consts& c, cons
   }
 }
 
-// one warp per strip: blockIdx.x * MWARPS + warp across x, blockIdx.y
-// across y, blockIdx.z the layer
 template <typename T, typename S, typename C>
 __global__ void __launch_bounds__(MW * MWARPS, MarchL<T, MK_CMOM>::min_blocks) k_c_mom_m(Geom g, Consts c, const S* __restrict__ ud,
                                                           const S* __restrict__ vd, const double* __restrict__ pkap,
                                                           const double* __restrict__ gz, C* __restrict__ uc,
                                                           C* __restrict__ vc, int tys) {
-  c_mom_strip<T, S, C>(g, c, ud, vd, pkap, gz, uc, vc, blockIdx.x * MWARPS + (threadIdx.x >> 5), blockIdx.y,
-                       blockIdx.z, tys);
+  extern __shared__ __align__(16) char feed_sm[];
+  c_mom_strip<T, S, C>(g, c, ud, vd, pkap, gz, uc, vc, strip_x(), blockIdx.y, blockIdx.z, tys, feed_sm);
 }
 
 // ======================================================== D-grid momentum ==
@@ -649,10 +798,11 @@ __global__ void __launch_bounds__(MW * MWARPS, MarchL<T, MK_CMOM>::min_blocks) k
 // B-grid pressure-gradient force (:665-679), del^4 divergence damping
 // (:682-702) and the vorticity-flux updates (:708-769).  Outputs on the
 // interior; strips of tys rows.
+template <bool SAME> constexpr int DMOM_NF = SAME ? 10 : 12;
 template <typename T, typename S, typename C, bool RO = true>
 __device__ __forceinline__ void d_mom_strip(const Geom& g, const Consts& c, const S* ud, const S* vd, const C* uc,
                                             const C* vc, const double* pkapb, const double* gzb, S* udo, S* vdo,
-                                            int* nonfinite, int sx, int sy, int k, int tys) {
+                                            int* nonfinite, int sx, int sy, int k, int tys, char* sm) {
   constexpr int CON = PPM_CON;
   constexpr bool SAME = std::is_same_v<S, T>;
   const int lane = threadIdx.x & (MW - 1);
@@ -694,30 +844,37 @@ __device__ __forceinline__ void d_mom_strip(const Geom& g, const Consts& c, cons
   double pb0y = 0, pb1y = 0, gb0y = 0, gb1y = 0;    // pkapb, gzb at k, k+1, row j-3
   bool bad = false;
   const int jend = min(oy + tys, g.ny) + 3;
-  r = row_of(g, oy - 2) + xi;
-  S sn_p = ld<RO>(uk, r), vn_p = ld<RO>(vk, r);
-  C cu_p = ld<RO>(uL, row_of(g, oy - 3) + xi), cv_p = ld<RO>(vL, row_of(g, oy - 4) + xi);
+  enum { F_U, F_V, F_CU, F_CV, F_P0, F_P1, F_G0, F_G1, F_UC, F_VC, F_UO, F_VO };
+  Feed<RO, DMOM_NF<SAME>, 0> feed(sm);
+  auto early = [&](int j) {
+    const unsigned r = row_of(g, j) + xi;
+    feed.early(j, F_U, uk + r);
+    feed.early(j, F_V, vk + r);
+    feed.early(j, F_CU, uL + (row_of(g, j - 1) + xi));
+    feed.early(j, F_CV, vL + (row_of(g, j - 2) + xi));
+  };
+  auto late = [&](int j) {  // the pressure terms of row j-2, the winds of row y = j-3
+    const unsigned r = row_of(g, j - 2) + xi, oi = row_of(g, j - 3) + xi;
+    feed.late(j, F_P0, pba + r);
+    feed.late(j, F_P1, pbb + r);
+    feed.late(j, F_G0, gba + r);
+    feed.late(j, F_G1, gbb + r);
+    feed.late(j, F_UC, ucK + oi);
+    feed.late(j, F_VC, vcK + oi);
+    if constexpr (!SAME) {
+      feed.late(j, F_UO, uk + oi);
+      feed.late(j, F_VO, vk + oi);
+    }
+  };
+  feed.start(early, late, oy - 2);
 #pragma unroll MarchL<T, MK_DMOM>::unroll
   for (int j = oy - 2; j < jend; ++j) {
-    // loads of rows j-2 (pressure terms) and j-3 (the update) issued before this row's work
     const int y = j - 3;
-    r = row_of(g, j - 2) + xi;
-    const double pb0n = ld<RO>(pba, r), pb1n = ld<RO>(pbb, r), gb0n = ld<RO>(gba, r), gb1n = ld<RO>(gbb, r);
     const unsigned oi = row_of(g, y) + xi;
-    const C svc_r = ld<RO>(vcK, oi), suc_r = ld<RO>(ucK, oi);
-    S uo_r = 0, vo_r = 0;  // the state values of row y (the update in the state's type)
-    if constexpr (!SAME) {
-      uo_r = ld<RO>(uk, oi);
-      vo_r = ld<RO>(vk, oi);
-    }
+    feed.next(early, late, j, jend);
     // ---- row j inputs; vorticity of row j-1 (:659-663), divergence of row j (:682-685)
-    const T sn = T(sn_p), vn = T(vn_p);
-    const C cu_c = cu_p, cv_c = cv_p;
-    r = row_of(g, j + 1) + xi;
-    sn_p = ld<RO>(uk, r);
-    vn_p = ld<RO>(vk, r);
-    cu_p = ld<RO>(uL, row_of(g, j) + xi);
-    cv_p = ld<RO>(vL, row_of(g, j - 1) + xi);
+    const T sn = T(feed.template get<S>(j, F_U)), vn = T(feed.template get<S>(j, F_V));
+    const C cu_c = feed.template get<C>(j, F_CU), cv_c = feed.template get<C>(j, F_CV);
     const T vorn = fmadd(shfl_dn(v0, 1) - v0, rdx, fmadd(-(sn - s0), rdy, f));
     const T dvn = fmadd(rdy, vn - v0, rdx * (sn - shfl_up(sn, 1)));
     s3 = s2; s2 = s1; s1 = s0; s0 = sn;
@@ -767,11 +924,13 @@ __device__ __forceinline__ void d_mom_strip(const Geom& g, const Consts& c, cons
       const T fx = xline_flux<T, CON>(tv, dtdx * cu3);
       const T fy = lt.flux(dtdx * cv3);
       const T ke_r = shfl_dn(ke3, 1), dd_r = shfl_dn(dd3, 1), lp_l = shfl_up(lp3, 1);
+      const double pb0n = feed.template get<double>(j, F_P0), pb1n = feed.template get<double>(j, F_P1);
+      const double gb0n = feed.template get<double>(j, F_G0), gb1n = feed.template get<double>(j, F_G1);
       const double pb0r = shfl_dn(pb0y, 1), pb1r = shfl_dn(pb1y, 1), gb0r = shfl_dn(gb0y, 1), gb1r = shfl_dn(gb1y, 1);
       if (out_lane && y < g.ny) {
         const double pgx = ((pb0r - pb1y) * (gb0y - gb1r) + (pb0y - pb1r) * (gb1y - gb0r)) / (pb0r - pb1y + pb0y - pb1r);
         const double pgy = ((pb0n - pb1y) * (gb0y - gb1n) + (pb0y - pb1n) * (gb1y - gb0n)) / (pb0n - pb1y + pb0y - pb1n);
-        const T svc = T(svc_r), suc = T(suc_r);
+        const T svc = T(feed.template get<C>(j, F_VC)), suc = T(feed.template get<C>(j, F_UC));
         S u, v;
         if constexpr (SAME) {  // the reference's operations, in order
           u = s3 + dt * (svc * fy + vdy * (lp3 - lp4)) - dtdx * (ke_r - ke3 - dd_r + dd3 - T(pgx));
@@ -779,29 +938,33 @@ __device__ __forceinline__ void d_mom_strip(const Geom& g, const Consts& c, cons
         } else {  // the tendency in the sweep type added to the state's type
           const T du = fmadd(-dtdx, ke_r - ke3 - dd_r + dd3 - T(pgx), dt * fmadd(vdy, lp3 - lp4, svc * fy));
           const T dv = fmadd(-dtdy, ke2 - ke3 - dd2 + dd3 - T(pgy), -dt * fmadd(vdx, lp3 - lp_l, suc * fx));
-          u = uo_r + S(du);
-          v = vo_r + S(dv);
+          u = feed.template get<S>(j, F_UO) + S(du);
+          v = feed.template get<S>(j, F_VO) + S(dv);
         }
         udo[kS + oi] = u;
         vdo[kS + oi] = v;
         bad = bad || !(finite_(u) && finite_(v));
       }
     }
-    pb0y = pb0n; pb1y = pb1n; gb0y = gb0n; gb1y = gb1n;
+    if (y >= oy - 1) {
+      pb0y = feed.template get<double>(j, F_P0);
+      pb1y = feed.template get<double>(j, F_P1);
+      gb0y = feed.template get<double>(j, F_G0);
+      gb1y = feed.template get<double>(j, F_G1);
+    }
   }
   flag_nonfinite(nonfinite, bad);
 }
 
-// one warp per strip: blockIdx.x * MWARPS + warp across x, blockIdx.y
-// across y, blockIdx.z the layer
 template <typename T, typename S, typename C>
 __global__ void __launch_bounds__(MW * MWARPS, MarchL<T, MK_DMOM>::min_blocks) k_d_mom_m(Geom g, Consts c, const S* __restrict__ ud,
                                                           const S* __restrict__ vd, const C* __restrict__ uc,
                                                           const C* __restrict__ vc, const double* __restrict__ pkapb,
                                                           const double* __restrict__ gzb, S* __restrict__ udo,
                                                           S* __restrict__ vdo, int* nonfinite, int tys) {
-  d_mom_strip<T, S, C>(g, c, ud, vd, uc, vc, pkapb, gzb, udo, vdo, nonfinite,
-                       blockIdx.x * MWARPS + (threadIdx.x >> 5), blockIdx.y, blockIdx.z, tys);
+  extern __shared__ __align__(16) char feed_sm[];
+  d_mom_strip<T, S, C>(g, c, ud, vd, uc, vc, pkapb, gzb, udo, vdo, nonfinite, strip_x(), blockIdx.y, blockIdx.z, tys,
+                       feed_sm);
 }
 
 }  // namespace atm

@@ -49,6 +49,12 @@ def test_step_bit_exact(nx, ny, nlay, fields):
     g.close()
 
 
+@pytest.mark.parametrize('nx,ny,nlay', [(60, 9, 3), (140, 41, 3), (235, 18, 3)])
+def test_narrow_blocks_bit_exact(nx, ny, nlay):
+    """Widths of 3, 6 and 10 strips, whose blocks hold three, three and two."""
+    test_step_bit_exact(nx, ny, nlay, 'rough')
+
+
 @pytest.mark.parametrize('nx,ny,nlay', [(9, 8, 3), (23, 17, 32), (40, 33, 33), (20, 18, 65), (12, 11, 128),
                                         (300, 270, 8)])
 @pytest.mark.parametrize('fields', ['smooth', 'rough', 'crossed'])
