@@ -4,6 +4,7 @@
 // limiter and upwind branch is taken as in the forward step.
 #include "atm_adj_march.cuh"
 #include "atm_adjoint.cuh"
+#include "atm_remap_adj.cuh"
 #include "atm_ops.h"
 #include "atm_strips.h"
 
@@ -71,20 +72,27 @@ cudaError_t adj_d_mom(const Geom& g, const Consts& c, const double* ud, const do
   return cudaGetLastError();
 }
 
-cudaError_t adj_c_column(const Geom& g, const Consts& c, const double* dp, const double* pt, const double* pkap,
-                         const double* gz, const double* lam_uc, const double* lam_vc, double* tmp, double* lam_dp,
-                         double* lam_pt, cudaStream_t s) {
+template <bool CGRID>
+static cudaError_t column_adj(const Geom& g, const Consts& c, const double* dp, const double* pt, const double* pkap,
+                              const double* gz, const double* lam_u, const double* lam_v, double* lam_dp,
+                              double* lam_pt, cudaStream_t s) {
   const int n = (g.nx + 4) * (g.ny + 4);
-  k_column_adj<true><<<(n + 127) / 128, 128, 0, s>>>(g, c, dp, pt, pkap, gz, lam_uc, lam_vc, tmp, lam_dp, lam_pt);
+  const size_t sm = column_adj_smem(g.L);
+  const cudaError_t e = remap_smem_attr(k_column_adj<CGRID>, sm);
+  if (e != cudaSuccess) return e;
+  k_column_adj<CGRID><<<(n + 31) / 32, 32 * CADJ_WARPS, sm, s>>>(g, c, dp, pt, pkap, gz, lam_u, lam_v, lam_dp, lam_pt);
   return cudaGetLastError();
 }
 
+cudaError_t adj_c_column(const Geom& g, const Consts& c, const double* dp, const double* pt, const double* pkap,
+                         const double* gz, const double* lam_uc, const double* lam_vc, double* lam_dp, double* lam_pt,
+                         cudaStream_t s) {
+  return column_adj<true>(g, c, dp, pt, pkap, gz, lam_uc, lam_vc, lam_dp, lam_pt, s);
+}
+
 cudaError_t adj_d_column(const Geom& g, const Consts& c, const double* dp, const double* pt, const double* lam_pk,
-                         const double* lam_gz, double* tmp, double* lam_dp, double* lam_pt, cudaStream_t s) {
-  const int n = (g.nx + 4) * (g.ny + 4);
-  k_column_adj<false><<<(n + 127) / 128, 128, 0, s>>>(g, c, dp, pt, nullptr, nullptr, lam_pk, lam_gz, tmp, lam_dp,
-                                                      lam_pt);
-  return cudaGetLastError();
+                         const double* lam_gz, double* lam_dp, double* lam_pt, cudaStream_t s) {
+  return column_adj<false>(g, c, dp, pt, nullptr, nullptr, lam_pk, lam_gz, lam_dp, lam_pt, s);
 }
 
 cudaError_t adj_pgf_corners(const Geom& g, const Consts& c, const double* pkapb, const double* gzb,
@@ -126,8 +134,35 @@ static cudaError_t remap_energy_adj_lm(const Geom& g, const RemapArgs& ra, const
                                        const double* lam_udo, const double* lam_vdo, double* lam_dp, double* lam_pt,
                                        double* lam_ud, double* lam_vd, double* lam_ur, double* lam_vr, cudaStream_t s) {
   const int n = g.nx * g.ny;
-  k_remap_energy_adj<LM><<<(n + 63) / 64, 64, 0, s>>>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, lam_dpo, lam_pto,
-                                                      lam_udo, lam_vdo, lam_dp, lam_pt, lam_ud, lam_vd, lam_ur, lam_vr);
+  if constexpr (LM > 64) {
+    k_remap_energy_adj<LM><<<(n + 63) / 64, 64, 0, s>>>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, lam_dpo, lam_pto,
+                                                        lam_udo, lam_vdo, lam_dp, lam_pt, lam_ud, lam_vd, lam_ur, lam_vr);
+  } else {
+    const size_t sm = remap_smem(g.L, 8);
+    const cudaError_t e = remap_smem_attr(k_remap_energy_adj_split<LM>, sm);
+    if (e != cudaSuccess) return e;
+    k_remap_energy_adj_split<LM><<<(n + RM_LANES - 1) / RM_LANES, RM_LANES * RMA_WARPS, sm, s>>>(
+        g, ra, dp, pt, ud, vd, urem, vrem, gzs, lam_dpo, lam_pto, lam_udo, lam_vdo, lam_dp, lam_pt, lam_ud, lam_vd, lam_ur,
+        lam_vr);
+  }
+  return cudaGetLastError();
+}
+
+template <int LM>
+static cudaError_t remap_winds_adj_lm(const Geom& g, const RemapArgs& ra, const double* dp, const double* ud,
+                                      const double* vd, const double* lam_ur, const double* lam_vr, double* lam_dp,
+                                      double* lam_ud, double* lam_vd, cudaStream_t s) {
+  const int n = (g.nx + 2) * (g.ny + 2);
+  if constexpr (LM > 64) {
+    k_remap_winds_adj<LM><<<dim3((n + 63) / 64, 2), 64, 0, s>>>(g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud,
+                                                                lam_vd);
+  } else {
+    const size_t sm = remap_smem(g.L, 6);
+    const cudaError_t e = remap_smem_attr(k_remap_winds_adj_split<LM>, sm);
+    if (e != cudaSuccess) return e;
+    k_remap_winds_adj_split<LM><<<dim3((n + RM_LANES - 1) / RM_LANES, 2), RM_LANES * RMA_WARPS, sm, s>>>(
+        g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud, lam_vd);
+  }
   return cudaGetLastError();
 }
 
@@ -149,12 +184,9 @@ cudaError_t adj_remap_energy(const Geom& g, const RemapArgs& ra, const double* d
 cudaError_t adj_remap_winds(const Geom& g, const RemapArgs& ra, const double* dp, const double* ud, const double* vd,
                             const double* lam_ur, const double* lam_vr, double* lam_dp, double* lam_ud, double* lam_vd,
                             cudaStream_t s) {
-  const int n = (g.nx + 2) * (g.ny + 2);
-  const int nb = (n + 63) / 64;
-  if (g.L <= 32) k_remap_winds_adj<32><<<nb, 64, 0, s>>>(g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud, lam_vd);
-  else if (g.L <= 64) k_remap_winds_adj<64><<<nb, 64, 0, s>>>(g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud, lam_vd);
-  else k_remap_winds_adj<MAX_LAYERS><<<nb, 64, 0, s>>>(g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud, lam_vd);
-  return cudaGetLastError();
+  if (g.L <= 32) return remap_winds_adj_lm<32>(g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud, lam_vd, s);
+  if (g.L <= 64) return remap_winds_adj_lm<64>(g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud, lam_vd, s);
+  return remap_winds_adj_lm<MAX_LAYERS>(g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud, lam_vd, s);
 }
 
 }  // namespace atm

@@ -504,24 +504,14 @@ __device__ __noinline__ void remap_energy_pairs(int L, const double* en, double*
 // interior: adjoints of the remapped dp, pt, ud, vd in; adjoints of the
 // pre-remap dp, pt (this column), ud, vd (its A-grid neighbours) and of the
 // remapped face winds urem, vrem out.
-// 16 blocks of 64 threads per SM (64 registers; more columns in flight to
-// hide the local-memory latency of the column arrays): both remap adjoints
-// 51.1 ms per remap at 1024x1024x64 against 73.9 at the compiler's own
-// budget, 60.4 at 12 blocks, 58.0 at 24
+// One thread per column, its arrays in local memory: more than 64 layers, and
+// columns whose coordinates are not monotone (atm_remap_adj.cuh has the others).
 template <int LM>
-__global__ void __launch_bounds__(64, 16) k_remap_energy_adj(Geom g, RemapArgs ra, const double* __restrict__ dp,
-                                                         const double* __restrict__ pt, const double* __restrict__ ud,
-                                                         const double* __restrict__ vd, const double* __restrict__ urem,
-                                                         const double* __restrict__ vrem, const double* __restrict__ gzs,
-                                                         const double* __restrict__ lam_dpo,
-                                                         const double* __restrict__ lam_pto,
-                                                         const double* __restrict__ lam_udo,
-                                                         const double* __restrict__ lam_vdo, double* lam_dp,
-                                                         double* lam_pt, double* lam_ud, double* lam_vd, double* lam_ur,
-                                                         double* lam_vr) {
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= g.nx * g.ny) return;
-  const int i = col % g.nx, j = col / g.nx;
+__device__ __noinline__ void remap_energy_adj_at(const Geom& g, const RemapArgs& ra, const double* dp, const double* pt,
+                                                 const double* ud, const double* vd, const double* urem,
+                                                 const double* vrem, const double* gzs, const double* lam_dpo,
+                                                 const double* lam_pto, double* lam_dp, double* lam_pt, double* lam_ud,
+                                                 double* lam_vd, double* lam_ur, double* lam_vr, int i, int j) {
   const int L = g.L;
   const long long S = g.S;
   const long long o = g.at(i, j);
@@ -530,16 +520,6 @@ __global__ void __launch_bounds__(64, 16) k_remap_energy_adj(Geom g, RemapArgs r
   double en[LM + 2], ptr[LM + 2];
   double Lplev[LM + 2], Ltpl[LM + 2], Lpk[LM + 2], Ltpk[LM + 2], Ler[LM + 2];
   RemapAdjWork<LM> wk;
-  // ud = urem and vd = vrem (:156-161); the column's energy and pressure
-  // adjoints are zero unless its new dp or pt carry an adjoint
-  bool any = false;
-  for (int k = 1; k <= L; ++k) {
-    long long ok = o + (long long)(k - 1) * S;
-    if (lam_udo[ok] != 0.) atomicAdd(lam_ur + ok, lam_udo[ok]);
-    if (lam_vdo[ok] != 0.) atomicAdd(lam_vr + ok, lam_vdo[ok]);
-    any = any || lam_dpo[ok] != 0. || lam_pto[ok] != 0.;
-  }
-  if (!any) return;
   // forward recomputation, as k_remap_energy
   plev[L + 1] = ra.ptop;
   pk[L + 1] = ra.pk_top;
@@ -708,9 +688,101 @@ __global__ void __launch_bounds__(64, 16) k_remap_energy_adj(Geom g, RemapArgs r
   }
 }
 
-// Adjoint of k_remap_winds (src/mod_remap.f90:80-105) on [-1, nx] x [-1, ny]:
-// the adjoints of urem, vrem in; ud, vd of the column and dp of the seven
-// columns that form its source and target interface pressures out.
+// 16 blocks of 64 threads per SM (64 registers; more columns in flight to
+// hide the local-memory latency of the column arrays)
+template <int LM>
+__global__ void __launch_bounds__(64, 16) k_remap_energy_adj(Geom g, RemapArgs ra, const double* __restrict__ dp,
+                                                         const double* __restrict__ pt, const double* __restrict__ ud,
+                                                         const double* __restrict__ vd, const double* __restrict__ urem,
+                                                         const double* __restrict__ vrem, const double* __restrict__ gzs,
+                                                         const double* __restrict__ lam_dpo,
+                                                         const double* __restrict__ lam_pto,
+                                                         const double* __restrict__ lam_udo,
+                                                         const double* __restrict__ lam_vdo, double* lam_dp,
+                                                         double* lam_pt, double* lam_ud, double* lam_vd, double* lam_ur,
+                                                         double* lam_vr) {
+  const int col = blockIdx.x * blockDim.x + threadIdx.x;
+  if (col >= g.nx * g.ny) return;
+  const int i = col % g.nx, j = col / g.nx;
+  const long long o = g.at(i, j);
+  // ud = urem and vd = vrem (:156-161); the column's energy and pressure
+  // adjoints are zero unless its new dp or pt carry an adjoint
+  bool any = false;
+  for (int k = 0; k < g.L; ++k) {
+    const long long ok = o + (long long)k * g.S;
+    if (lam_udo[ok] != 0.) atomicAdd(lam_ur + ok, lam_udo[ok]);
+    if (lam_vdo[ok] != 0.) atomicAdd(lam_vr + ok, lam_vdo[ok]);
+    any = any || lam_dpo[ok] != 0. || lam_pto[ok] != 0.;
+  }
+  if (any)
+    remap_energy_adj_at<LM>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, lam_dpo, lam_pto, lam_dp, lam_pt, lam_ud, lam_vd,
+                            lam_ur, lam_vr, i, j);
+}
+
+// Adjoint of k_remap_winds (src/mod_remap.f90:80-105) of direction dir at a
+// point of [-1, nx] x [-1, ny]: the adjoint lr of the remapped wind in; that of
+// the wind f of the column (lf) and of dp of the four columns that form its
+// source and target interface pressures out.
+template <int LM>
+__device__ __noinline__ void remap_winds_adj_at(const Geom& g, const RemapArgs& ra, const double* dp, const double* f,
+                                                const double* lr, double* lam_dp, double* lf, int i, int j, int dir) {
+  const int L = g.L;
+  double sc[LM + 2], dc[LM + 2], var[LM + 2], Ld[LM + 2], Lv[LM + 2], Ls[LM + 2], Lt[LM + 2];
+  RemapAdjWork<LM> wk;
+  const long long o = g.at(i, j), oa = o;
+  const long long ob = dir == 0 ? g.at(i, j - 1) : g.at(i - 1, j);
+  const long long oc = dir == 0 ? g.at(i, j + 1) : g.at(i + 1, j);
+  const long long od = dir == 0 ? g.at(i, j - 2) : g.at(i - 2, j);
+  double pa = ra.ptop, pb = ra.ptop, pc = ra.ptop, pd = ra.ptop;
+  bool any = false;
+  for (int k = L + 1; k >= 1; --k) {
+    if (k <= L) {
+      const long long kk = (long long)(k - 1) * g.S;
+      pa = pa + dp[oa + kk];
+      pb = pb + dp[ob + kk];
+      pc = pc + dp[oc + kk];
+      pd = pd + dp[od + kk];
+      var[k] = f[o + kk];
+      Ld[k] = lr[o + kk];
+      any = any || Ld[k] != 0.;
+    }
+    sc[k] = C7_12 * (pa + pb) - C1_12 * (pc + pd);
+  }
+  if (!any) return;
+  for (int k = 1; k <= L + 1; ++k) {
+    double ta, tb, tc, td;
+    if (k <= L) {
+      const double a = ra.ak[k - 1], b = ra.bk[k - 1];
+      ta = a + b * (pa - ra.ptop);
+      tb = a + b * (pb - ra.ptop);
+      tc = a + b * (pc - ra.ptop);
+      td = a + b * (pd - ra.ptop);
+    } else {
+      ta = tb = tc = td = ra.ptop;
+    }
+    dc[k] = C7_12 * (ta + tb) - C1_12 * (tc + td);
+  }
+  for (int k = 0; k <= L + 1; ++k) { Lv[k] = 0.; Ls[k] = 0.; Lt[k] = 0.; }
+  remap_column_adj<LM>(wk, L, var, Ld, sc, dc, Lv, Ls, Lt);
+  for (int k = 1; k <= L; ++k) lf[o + (long long)(k - 1) * g.S] += Lv[k];
+  // sc(k) = 7/12 (pa + pb) - 1/12 (pc + pd), p(k) = ptop + sum of dp(m >= k);
+  // dc(k) = 7/12 (ta + tb) - 1/12 (tc + td), t = ak + bk (ps - ptop)
+  double Z = 0.;
+  for (int k = 1; k <= L; ++k) Z += ra.bk[k - 1] * Lt[k];
+  double P = 0.;
+  for (int m = 1; m <= L; ++m) {
+    P += Ls[m];
+    const double v = P + Z;
+    if (v == 0.) continue;
+    const long long kk = (long long)(m - 1) * g.S;
+    atomicAdd(lam_dp + oa + kk, C7_12 * v);
+    atomicAdd(lam_dp + ob + kk, C7_12 * v);
+    atomicAdd(lam_dp + oc + kk, -C1_12 * v);
+    atomicAdd(lam_dp + od + kk, -C1_12 * v);
+  }
+}
+
+// (blockIdx.y: the direction)
 template <int LM>
 __global__ void __launch_bounds__(64, 16) k_remap_winds_adj(Geom g, RemapArgs ra, const double* __restrict__ dp,
                                                         const double* __restrict__ ud, const double* __restrict__ vd,
@@ -720,74 +792,9 @@ __global__ void __launch_bounds__(64, 16) k_remap_winds_adj(Geom g, RemapArgs ra
   const int w = g.nx + 2, h = g.ny + 2;
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= w * h) return;
-  const int i = -1 + col % w, j = -1 + col / w;
-  const int L = g.L;
-  double sc[LM + 2], dc[LM + 2], var[LM + 2], Ld[LM + 2], Lv[LM + 2], Ls[LM + 2], Lt[LM + 2];
-  RemapAdjWork<LM> wk;
-  const int cx[7] = {i, i, i, i, i - 2, i - 1, i + 1};
-  const int cy[7] = {j - 2, j - 1, j, j + 1, j, j, j};
-  double ps[7];
-  for (int q = 0; q < 7; ++q) {
-    long long oq = g.at(cx[q], cy[q]);
-    double pl = ra.ptop;
-    for (int k = L - 1; k >= 0; --k) pl = pl + dp[oq + (long long)k * g.S];
-    ps[q] = pl;
-  }
-  for (int dir = 0; dir < 2; ++dir) {
-    const int qa = 2, qb = dir == 0 ? 1 : 5, qc = dir == 0 ? 3 : 6, qd = dir == 0 ? 0 : 4;
-    long long oa = g.at(cx[qa], cy[qa]), ob = g.at(cx[qb], cy[qb]), oc = g.at(cx[qc], cy[qc]), od = g.at(cx[qd], cy[qd]);
-    double pa = ra.ptop, pb = ra.ptop, pc = ra.ptop, pd = ra.ptop;
-    for (int k = L + 1; k >= 1; --k) {
-      if (k <= L) {
-        long long kk = (long long)(k - 1) * g.S;
-        pa = pa + dp[oa + kk];
-        pb = pb + dp[ob + kk];
-        pc = pc + dp[oc + kk];
-        pd = pd + dp[od + kk];
-      }
-      sc[k] = C7_12 * (pa + pb) - C1_12 * (pc + pd);
-      double ta, tb, tc, td;
-      if (k <= L) {
-        double a = ra.ak[k - 1], b = ra.bk[k - 1];
-        ta = a + b * (ps[qa] - ra.ptop);
-        tb = a + b * (ps[qb] - ra.ptop);
-        tc = a + b * (ps[qc] - ra.ptop);
-        td = a + b * (ps[qd] - ra.ptop);
-      } else {
-        ta = tb = tc = td = ra.ptop;
-      }
-      dc[k] = C7_12 * (ta + tb) - C1_12 * (tc + td);
-    }
-    const double* f = dir == 0 ? ud : vd;
-    const double* lr = dir == 0 ? lam_ur : lam_vr;
-    long long o = g.at(i, j);
-    bool any = false;
-    for (int k = 1; k <= L; ++k) {
-      var[k] = f[o + (long long)(k - 1) * g.S];
-      Ld[k] = lr[o + (long long)(k - 1) * g.S];
-      any = any || Ld[k] != 0.;
-    }
-    if (!any) continue;
-    for (int k = 0; k <= L + 1; ++k) { Lv[k] = 0.; Ls[k] = 0.; Lt[k] = 0.; }
-    remap_column_adj<LM>(wk, L, var, Ld, sc, dc, Lv, Ls, Lt);
-    double* lf = dir == 0 ? lam_ud : lam_vd;
-    for (int k = 1; k <= L; ++k) lf[o + (long long)(k - 1) * g.S] += Lv[k];
-    // sc(k) = 7/12 (pa + pb) - 1/12 (pc + pd), p(k) = ptop + sum of dp(m >= k);
-    // dc(k) = 7/12 (ta + tb) - 1/12 (tc + td), t = ak + bk (ps - ptop)
-    double Z = 0.;
-    for (int k = 1; k <= L; ++k) Z += ra.bk[k - 1] * Lt[k];
-    double P = 0.;
-    for (int m = 1; m <= L; ++m) {
-      P += Ls[m];
-      const double v = P + Z;
-      if (v == 0.) continue;
-      long long kk = (long long)(m - 1) * g.S;
-      atomicAdd(lam_dp + oa + kk, C7_12 * v);
-      atomicAdd(lam_dp + ob + kk, C7_12 * v);
-      atomicAdd(lam_dp + oc + kk, -C1_12 * v);
-      atomicAdd(lam_dp + od + kk, -C1_12 * v);
-    }
-  }
+  const int i = -1 + col % w, j = -1 + col / w, dir = blockIdx.y;
+  remap_winds_adj_at<LM>(g, ra, dp, dir == 0 ? ud : vd, dir == 0 ? lam_ur : lam_vr, lam_dp, dir == 0 ? lam_ud : lam_vd,
+                         i, j, dir);
 }
 
 }  // namespace atm

@@ -888,7 +888,7 @@ int adj_c(atm_ctx* ctx, double dt_half, void* const* s, double* const* lin, cons
   {
     Stage t(ctx, S_ACCOL);
     CK(atm::adj_c_column(g, k, cg[C_DPC], cg[C_PTC], ctx->pkap, ctx->gz, ctx->lam_cg[C_UC], ctx->lam_cg[C_VC],
-                         ctx->stage, ctx->lam_cg[C_DPC], ctx->lam_cg[C_PTC], ctx->stream));
+                         ctx->lam_cg[C_DPC], ctx->lam_cg[C_PTC], ctx->stream));
   }
   for (int part = 1; part <= 2; ++part) {
     Stage t(ctx, part == 1 ? S_ACMASS : S_ACMASS_Y);
@@ -918,7 +918,7 @@ int adj_d(atm_ctx* ctx, double dt, const void* const* so, const void* const* sn,
     CK(atm::adj_pgf_corners(g, k, ctx->pkapb, ctx->gzb, lout[F_UD], lout[F_VD], ctx->lam_pkb, ctx->lam_gzb,
                             ctx->stream));
     CK(atm::adj_corners(g, ctx->lam_pkb, ctx->lam_gzb, ctx->lam_pk, ctx->lam_gz, ctx->stream));
-    CK(atm::adj_d_column(g, k, n[F_DP], n[F_PT], ctx->lam_pk, ctx->lam_gz, ctx->stage, lout[F_DP], lout[F_PT],
+    CK(atm::adj_d_column(g, k, n[F_DP], n[F_PT], ctx->lam_pk, ctx->lam_gz, lout[F_DP], lout[F_PT],
                          ctx->stream));
   }
   for (int part = 1; part <= 2; ++part) {

@@ -79,13 +79,12 @@ cudaError_t adj_d_mom(const Geom&, const Consts&, const double* ud, const double
 // lam_pkb (levels 1..nlay), lam_gzb = the D grid's pressure-gradient force reversed
 cudaError_t adj_pgf_corners(const Geom&, const Consts&, const double* pkapb, const double* gzb, const double* lam_udo,
                             const double* lam_vdo, double* lam_pkb, double* lam_gzb, cudaStream_t);
-// columns over [-2, n+1]^2, on the C grid with the pressure-gradient force;
-// tmp: scratch of nlay + 1 levels
+// columns over [-2, n+1]^2, on the C grid with the pressure-gradient force
 cudaError_t adj_c_column(const Geom&, const Consts&, const double* dp, const double* pt, const double* pkap,
-                         const double* gz, const double* lam_uc, const double* lam_vc, double* tmp, double* lam_dp,
+                         const double* gz, const double* lam_uc, const double* lam_vc, double* lam_dp,
                          double* lam_pt, cudaStream_t);
 cudaError_t adj_d_column(const Geom&, const Consts&, const double* dp, const double* pt, const double* lam_pk,
-                         const double* lam_gz, double* tmp, double* lam_dp, double* lam_pt, cudaStream_t);
+                         const double* lam_gz, double* lam_dp, double* lam_pt, cudaStream_t);
 // lam_pk (levels 1..nlay), lam_gz (2..nlay+1) = the corner interpolation reversed
 cudaError_t adj_corners(const Geom&, const double* lam_pkb, const double* lam_gzb, double* lam_pk, double* lam_gz,
                         cudaStream_t);

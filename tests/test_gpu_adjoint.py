@@ -237,3 +237,51 @@ def test_three_steps_dot_product(remap_every):
         g.close()
     rhs = sum(np.sum(v[n] * lam[n]) for n in NAMES)
     assert rel(lhs, rhs) <= TOL, (lhs, rhs)
+
+
+@pytest.mark.parametrize('nx,ny,nlay', [(9, 8, 3), (13, 9, 20), (20, 17, 32), (9, 8, 33), (11, 8, 64), (8, 7, 65),
+                                        (7, 8, 128)])
+def test_layer_counts_dot_product(nx, ny, nlay):
+    """The columns' and the remap's reverse over the ranges of their column
+    arrays (up to 32, 64 and 128 layers), on columns that differ enough for
+    layers to overlap several targets and for all pair cases.  The bound is on
+    the sum of the products' magnitudes: the reverse rounds each term a few
+    hundred times at most."""
+    st = generic_state(nx, ny, nlay, seed=nlay)
+    rng = np.random.default_rng(nx)
+    st.dp = st.dp * np.exp(rng.normal(0, 0.3, st.dp.shape))
+    g = Dycore(st)
+    g.adj_enable()
+    v = {n: rand(rng, st, n) for n in NAMES}
+    t = tlm_from_gpu(g, st, v)
+    dt = 10.0
+    for a in (t, g):
+        a.cgrid_step(dt / 2)
+        a.cgrid_halo()
+        a.dgrid_step(dt)
+        a.remap()
+    w = {n: rand(rng, st, n) for n in NAMES}
+    terms = [w[n] * t.get(STATE[n], halo=True)[1] for n in NAMES]
+    g.close()
+    g = Dycore(st)
+    g.adj_enable()
+    g.cgrid_step(dt / 2)
+    g.cgrid_halo()
+    g.dgrid_step(dt)
+    for n in NAMES:
+        g.adj_set('out', n, w[n])
+    g.adj_remap()
+    back = {n: g.adj_get('in', n) for n in NAMES}
+    g.close()
+    # the step before the remap, from its initial state
+    g = Dycore(st)
+    g.adj_enable()
+    for n in NAMES:
+        g.adj_set('out', n, back[n])
+    g.adj_dgrid_step(dt)
+    g.adj_cgrid_halo()
+    g.adj_cgrid_step(dt / 2)
+    rhs = sum(np.sum(v[n] * g.adj_get('in', n)) for n in NAMES)
+    lhs, scale = sum(np.sum(x) for x in terms), sum(np.sum(np.abs(x)) for x in terms)
+    assert abs(lhs - rhs) <= TOL * scale, (lhs, rhs, scale)
+    g.close()
