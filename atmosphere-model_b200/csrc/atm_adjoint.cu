@@ -78,7 +78,7 @@ static cudaError_t column_adj(const Geom& g, const Consts& c, const double* dp, 
                               double* lam_pt, cudaStream_t s) {
   const int n = (g.nx + 4) * (g.ny + 4);
   const size_t sm = column_adj_smem(g.L);
-  const cudaError_t e = remap_smem_attr(k_column_adj<CGRID>, sm);
+  const cudaError_t e = remap_smem_attr(k_column_adj<CGRID>, column_adj_smem(MAX_LAYERS));
   if (e != cudaSuccess) return e;
   k_column_adj<CGRID><<<(n + 31) / 32, 32 * CADJ_WARPS, sm, s>>>(g, c, dp, pt, pkap, gz, lam_u, lam_v, lam_dp, lam_pt);
   return cudaGetLastError();
@@ -139,7 +139,7 @@ static cudaError_t remap_energy_adj_lm(const Geom& g, const RemapArgs& ra, const
                                                         lam_udo, lam_vdo, lam_dp, lam_pt, lam_ud, lam_vd, lam_ur, lam_vr);
   } else {
     const size_t sm = remap_smem(g.L, 8);
-    const cudaError_t e = remap_smem_attr(k_remap_energy_adj_split<LM>, sm);
+    const cudaError_t e = remap_smem_attr(k_remap_energy_adj_split<LM>, remap_smem(LM, 8));
     if (e != cudaSuccess) return e;
     k_remap_energy_adj_split<LM><<<(n + RM_LANES - 1) / RM_LANES, RM_LANES * RMA_WARPS, sm, s>>>(
         g, ra, dp, pt, ud, vd, urem, vrem, gzs, lam_dpo, lam_pto, lam_udo, lam_vdo, lam_dp, lam_pt, lam_ud, lam_vd, lam_ur,
@@ -158,7 +158,7 @@ static cudaError_t remap_winds_adj_lm(const Geom& g, const RemapArgs& ra, const 
                                                                 lam_vd);
   } else {
     const size_t sm = remap_smem(g.L, 6);
-    const cudaError_t e = remap_smem_attr(k_remap_winds_adj_split<LM>, sm);
+    const cudaError_t e = remap_smem_attr(k_remap_winds_adj_split<LM>, remap_smem(LM, 6));
     if (e != cudaSuccess) return e;
     k_remap_winds_adj_split<LM><<<dim3((n + RM_LANES - 1) / RM_LANES, 2), RM_LANES * RMA_WARPS, sm, s>>>(
         g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud, lam_vd);

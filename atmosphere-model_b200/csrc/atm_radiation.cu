@@ -428,8 +428,9 @@ template <int LM>
 cudaError_t launch(const Geom& g, const RadTables& t, const RadArgs& a, cudaStream_t s) {
   const int n = g.nx * g.ny;
   const size_t sm = (size_t)RC * rad_doubles(g.L) * sizeof(double);
-  const cudaError_t e =
-      cudaFuncSetAttribute(k_radiation<LM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  // what LM layers take whatever L is: launches on several threads set the same value
+  const cudaError_t e = cudaFuncSetAttribute(k_radiation<LM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(RC * rad_doubles(LM) * sizeof(double)));
   if (e != cudaSuccess) return e;
   k_radiation<LM><<<(n + RC - 1) / RC, RG * RC, sm, s>>>(g, t, a);
   return cudaGetLastError();

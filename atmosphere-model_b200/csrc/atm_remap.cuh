@@ -474,10 +474,12 @@ __global__ void __launch_bounds__(64, 16) k_remap_energy(Geom g, RemapArgs ra, c
 // 256x256x32 232 / 293, 301x203x40 291 / 357, 350x350x64 893 / 709.
 constexpr long long RM_WINDS_FEW = 148LL * 256, RM_ENERGY_FEW = 148LL * 512;
 
+// Shared memory above the default limit, which the kernel's own variables count
+// against too: always what the kernel's largest layer count takes, so that
+// launches of different layer counts on several threads set the same value.
 template <typename K>
-inline cudaError_t remap_smem_attr(K kernel, size_t bytes) {  // shared memory above the default limit
-  return bytes <= 48 * 1024 ? cudaSuccess
-                            : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+inline cudaError_t remap_smem_attr(K kernel, size_t bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 template <typename T, int LM, typename E = double>
 cudaError_t launch_remap_winds(const Geom& g, const RemapArgs& ra, const T* dp, const T* ud, const T* vd, T* urem,
@@ -488,7 +490,7 @@ cudaError_t launch_remap_winds(const Geom& g, const RemapArgs& ra, const T* dp, 
     return cudaGetLastError();
   }
   const size_t sm = remap_smem(g.L, 3);
-  const cudaError_t e = remap_smem_attr(k_remap_winds_split<T, LM, E>, sm);
+  const cudaError_t e = remap_smem_attr(k_remap_winds_split<T, LM, E>, remap_smem(LM, 3));
   if (e != cudaSuccess) return e;
   k_remap_winds_split<T, LM, E><<<dim3((n + RM_LANES - 1) / RM_LANES, 2), RM_LANES * RM_WARPS, sm, s>>>(
       g, ra, dp, ud, vd, urem, vrem, trace, st);
@@ -505,7 +507,7 @@ cudaError_t launch_remap_energy(const Geom& g, const RemapArgs& ra, const T* dp,
     return cudaGetLastError();
   }
   const size_t sm = remap_smem(g.L, 4);
-  const cudaError_t e = remap_smem_attr(k_remap_energy_split<T, LM, PW>, sm);
+  const cudaError_t e = remap_smem_attr(k_remap_energy_split<T, LM, PW>, remap_smem(LM, 4));
   if (e != cudaSuccess) return e;
   k_remap_energy_split<T, LM, PW><<<(n + RM_LANES - 1) / RM_LANES, RM_LANES * RM_WARPS, sm, s>>>(
       g, ra, dp, pt, ud, vd, urem, vrem, gzs, dpo, pto, udo, vdo, trace, st);

@@ -86,3 +86,19 @@ def test_remap_bit_exact(nx, ny, nlay, fields):
         # (the face interpolation crosses some coordinates of the rough fields too)
         assert fallback.value > 0 if fields == 'crossed' else fields == 'rough' or fallback.value == 0
     g.close()
+
+
+@pytest.mark.parametrize('nlay', [21, 30, 45, 46, 47, 61, 62, 63])
+def test_layer_counts_near_shared_limit(nlay):
+    """Layer counts whose column arrays fill the 48 KB that a block may take
+    without opting in, with and without room for the kernels' own variables:
+    the remap and its reverse launch, first thing in the process for some."""
+    st = ic.jet_case(9, 8, nlay, 400e3, 400e3, width=900e3, seed=nlay)
+    g, o = Dycore(st), pyoracle.OracleModel(st, threads=8)
+    g.adj_enable()
+    g.adj_remap()
+    g.remap()
+    o.remap()
+    for name, f in FIELDS:
+        np.testing.assert_array_equal(g.get(name, halo=True), o.get(f, halo=True), err_msg=name)
+    g.close()
