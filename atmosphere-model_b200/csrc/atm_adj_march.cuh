@@ -333,6 +333,7 @@ __device__ __forceinline__ void mass_out_adj(double ld, double lt, double d, dou
 // of the new fields on the old, and the whole damping of dp.
 template <bool CGRID>
 __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_x(Geom g, Consts c, MassAdjArgs a, int lo, int hi, int tys) {
+  stream_order();
   extern __shared__ double adj_sm[];
   constexpr int V = CGRID ? PPM_UNC : PPM_NN;
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
@@ -484,6 +485,7 @@ constexpr int mass_adj_smem(bool cgrid, bool xb) {  // of a warp
 }
 template <bool CGRID>
 __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_y(Geom g, Consts c, MassAdjArgs a, int lo, int hi, int tys) {
+  stream_order();
   extern __shared__ double adj_sm[];
   constexpr int V = CGRID ? PPM_UNC : PPM_NN;
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
@@ -635,6 +637,7 @@ struct CMomAdjArgs {
 // The x branch: the x fluxes of the vorticity and of the kinetic energy, the
 // damping.
 static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_x(Geom g, Consts c, CMomAdjArgs a, int tys) {
+  stream_order();
   extern __shared__ double adj_sm[];
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
   const int ox = strip_x() * MOUT, oy = (int)blockIdx.y * tys;
@@ -767,6 +770,7 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_x(Geom g, C
 // columns: lanes 2 to 29, over [-1, n-1] (the kinetic energy's range).
 constexpr int YOUT_CMOM = 28;
 static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_y(Geom g, Consts c, CMomAdjArgs a, int tys) {
+  stream_order();
   extern __shared__ double adj_sm[];
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
   const int ox = -1 + strip_x() * YOUT_CMOM, oy = -1 + (int)blockIdx.y * tys;
@@ -884,6 +888,7 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_y(Geom g, C
 // nlay, of the A-grid winds of the kinetic energy.  A thread a point of
 // [-4, n+3]^2 (blockIdx.y: row, blockIdx.z: layer).
 static __global__ void __launch_bounds__(128) k_c_mom_adj_fin(Geom g, Consts c, CMomAdjArgs a) {
+  stream_order();
   const int x = -4 + (int)(blockIdx.x * blockDim.x + threadIdx.x), y = -4 + (int)blockIdx.y, k = blockIdx.z;
   if (x >= g.nx + 4) return;
   const long long o = g.at(x, y, k);
@@ -1002,6 +1007,7 @@ __global__ void __launch_bounds__(32 * CADJ_WARPS) k_column_adj(Geom g, Consts c
                                                                 const double* __restrict__ lam_u,
                                                                 const double* __restrict__ lam_v, double* lam_dp,
                                                                 double* lam_pt) {
+  stream_order();
   extern __shared__ double adj_sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int w = g.nx + 4, L = g.L;
@@ -1084,6 +1090,7 @@ static __global__ void __launch_bounds__(128) k_pgf_adj_corners(Geom g, Consts c
                                                                 const double* __restrict__ lam_v,
                                                                 double* __restrict__ lam_pkb,
                                                                 double* __restrict__ lam_gzb) {
+  stream_order();
   const int w = g.nx + 1;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= w * (g.ny + 1)) return;
@@ -1113,6 +1120,7 @@ struct DMomAdjArgs {
 // The x branch: the x fluxes of the vorticity and of the kinetic energy, the
 // direct terms and both dampings.
 static __global__ void __launch_bounds__(MW * MWARPS, 3) k_d_mom_adj_x(Geom g, Consts c, DMomAdjArgs a, int tys) {
+  stream_order();
   extern __shared__ double adj_sm[];
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
   const int ox = strip_x() * MOUT, oy = (int)blockIdx.y * tys;
@@ -1251,6 +1259,7 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_d_mom_adj_x(Geom g, C
 // columns: lanes 1 to 29, over [0, n]^2 (the kinetic energy's range).
 constexpr int YOUT_DMOM = 29;
 static __global__ void __launch_bounds__(MW * MWARPS, 3) k_d_mom_adj_y(Geom g, Consts c, DMomAdjArgs a, int tys) {
+  stream_order();
   extern __shared__ double adj_sm[];
   const int lane = threadIdx.x & (MW - 1), k = blockIdx.z;
   const int ox = strip_x() * YOUT_DMOM, oy = (int)blockIdx.y * tys;

@@ -31,8 +31,7 @@ cudaError_t adj_mass(const Geom& g, const Consts& c, const double* dp, const dou
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                MWARPS * mass_adj_smem(cgrid, xb));
     if (e != cudaSuccess) return e;
-    kernel<<<p.grid, p.threads, sm, s>>>(g, c, a, lo, hi, p.rows);
-    return cudaGetLastError();
+    return launch(kernel, p.grid, p.threads, sm, s, g, c, a, lo, hi, p.rows);
   };
   if (xb) return cgrid ? run(k_mass_adj_x<true>) : run(k_mass_adj_x<false>);
   return cgrid ? run(k_mass_adj_y<true>) : run(k_mass_adj_y<false>);
@@ -51,10 +50,10 @@ cudaError_t adj_c_mom(const Geom& g, const Consts& c, const double* ud, const do
       (e = cudaMemsetAsync(lam_vc1, 0, lay, s)) || (e = cudaMemsetAsync(lam_nlay, 0, (size_t)g.S * 2 * 8, s)))
     return e;
   StripPlan p = adj_strips(g.nx, g.ny, g.L, MOUT, 3);
-  k_c_mom_adj_x<<<p.grid, p.threads, p.threads / MW * ADJ_RING7, s>>>(g, c, a, p.rows);
+  launch(k_c_mom_adj_x, p.grid, p.threads, p.threads / MW * ADJ_RING7, s, g, c, a, p.rows);
   p = adj_strips(g.nx + 1, g.ny + 1, g.L, YOUT_CMOM, 10);
-  k_c_mom_adj_y<<<p.grid, p.threads, p.threads / MW * ADJ_RING7, s>>>(g, c, a, p.rows);
-  k_c_mom_adj_fin<<<dim3((g.nx + 8 + 127) / 128, g.ny + 8, g.L), 128, 0, s>>>(g, c, a);
+  launch(k_c_mom_adj_y, p.grid, p.threads, p.threads / MW * ADJ_RING7, s, g, c, a, p.rows);
+  launch(k_c_mom_adj_fin, dim3((g.nx + 8 + 127) / 128, g.ny + 8, g.L), 128, 0, s, g, c, a);
   return cudaGetLastError();
 }
 
@@ -64,10 +63,10 @@ cudaError_t adj_d_mom(const Geom& g, const Consts& c, const double* ud, const do
   const DMomAdjArgs a{ud, vd, uc, vc, lam_udo, lam_vdo, lam_ud, lam_vd, lam_uc, lam_vc};
   if (part == 1) {
     const StripPlan p = adj_strips(g.nx, g.ny, g.L, MOUT, 6);
-    k_d_mom_adj_x<<<p.grid, p.threads, p.threads / MW * ADJ_RING7, s>>>(g, c, a, p.rows);
+    launch(k_d_mom_adj_x, p.grid, p.threads, p.threads / MW * ADJ_RING7, s, g, c, a, p.rows);
   } else {
     const StripPlan p = adj_strips(g.nx + 1, g.ny + 1, g.L, YOUT_DMOM, 11);
-    k_d_mom_adj_y<<<p.grid, p.threads, p.threads / MW * ADJ_RING8, s>>>(g, c, a, p.rows);
+    launch(k_d_mom_adj_y, p.grid, p.threads, p.threads / MW * ADJ_RING8, s, g, c, a, p.rows);
   }
   return cudaGetLastError();
 }
@@ -80,7 +79,7 @@ static cudaError_t column_adj(const Geom& g, const Consts& c, const double* dp, 
   const size_t sm = column_adj_smem(g.L);
   const cudaError_t e = remap_smem_attr(k_column_adj<CGRID>, column_adj_smem(MAX_LAYERS));
   if (e != cudaSuccess) return e;
-  k_column_adj<CGRID><<<(n + 31) / 32, 32 * CADJ_WARPS, sm, s>>>(g, c, dp, pt, pkap, gz, lam_u, lam_v, lam_dp, lam_pt);
+  launch(k_column_adj<CGRID>, (n + 31) / 32, 32 * CADJ_WARPS, sm, s, g, c, dp, pt, pkap, gz, lam_u, lam_v, lam_dp, lam_pt);
   return cudaGetLastError();
 }
 
@@ -99,7 +98,7 @@ cudaError_t adj_pgf_corners(const Geom& g, const Consts& c, const double* pkapb,
                             const double* lam_udo, const double* lam_vdo, double* lam_pkb, double* lam_gzb,
                             cudaStream_t s) {
   const int n = (g.nx + 1) * (g.ny + 1);
-  k_pgf_adj_corners<<<dim3((n + 127) / 128, (g.L + PGF_CHUNK - 1) / PGF_CHUNK), 128, 0, s>>>(
+  launch(k_pgf_adj_corners, dim3((n + 127) / 128, (g.L + PGF_CHUNK - 1) / PGF_CHUNK), 128, 0, s, 
       g, c, pkapb, gzb, lam_udo, lam_vdo, lam_pkb, lam_gzb);
   return cudaGetLastError();
 }
@@ -107,7 +106,7 @@ cudaError_t adj_pgf_corners(const Geom& g, const Consts& c, const double* pkapb,
 cudaError_t adj_corners(const Geom& g, const double* lam_pkb, const double* lam_gzb, double* lam_pk, double* lam_gz,
                         cudaStream_t s) {
   const int n = (g.nx + 4) * (g.ny + 4);
-  k_corners_adj<<<dim3((n + 255) / 256, g.L), 256, 0, s>>>(g, lam_pkb, lam_gzb, lam_pk, lam_gz);
+  launch(k_corners_adj, dim3((n + 255) / 256, g.L), 256, 0, s, g, lam_pkb, lam_gzb, lam_pk, lam_gz);
   return cudaGetLastError();
 }
 
@@ -115,14 +114,14 @@ cudaError_t adj_ring_fold(const Geom& g, double* const* f, int nf, int K, cudaSt
   const int nring = 2 * H * (g.nx + 2 * H) + 2 * H * g.ny;
   double* d[4] = {nullptr, nullptr, nullptr, nullptr};
   for (int i = 0; i < nf; ++i) d[i] = f[i];
-  k_ring_fold<<<dim3((nring + 255) / 256, K, nf), 256, 0, s>>>(g, d[0], d[1], d[2], d[3], K);
+  launch(k_ring_fold, dim3((nring + 255) / 256, K, nf), 256, 0, s, g, d[0], d[1], d[2], d[3], K);
   return cudaGetLastError();
 }
 
 cudaError_t adj_ring_copy(const Geom& g, double* const* dst, double* const* src, int K, int band01, int band23,
                           cudaStream_t s) {
   const int nring = 2 * H * (g.nx + 2 * H) + 2 * H * g.ny;
-  k_ring_copy_adj<<<dim3((nring + 255) / 256, K, 4), 256, 0, s>>>(g, dst[0], dst[1], dst[2], dst[3], src[0], src[1],
+  launch(k_ring_copy_adj, dim3((nring + 255) / 256, K, 4), 256, 0, s, g, dst[0], dst[1], dst[2], dst[3], src[0], src[1],
                                                                    src[2], src[3], K, band01, band23);
   return cudaGetLastError();
 }
@@ -135,13 +134,13 @@ static cudaError_t remap_energy_adj_lm(const Geom& g, const RemapArgs& ra, const
                                        double* lam_ud, double* lam_vd, double* lam_ur, double* lam_vr, cudaStream_t s) {
   const int n = g.nx * g.ny;
   if constexpr (LM > 64) {
-    k_remap_energy_adj<LM><<<(n + 63) / 64, 64, 0, s>>>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, lam_dpo, lam_pto,
+    launch(k_remap_energy_adj<LM>, (n + 63) / 64, 64, 0, s, g, ra, dp, pt, ud, vd, urem, vrem, gzs, lam_dpo, lam_pto,
                                                         lam_udo, lam_vdo, lam_dp, lam_pt, lam_ud, lam_vd, lam_ur, lam_vr);
   } else {
     const size_t sm = remap_smem(g.L, 8);
     const cudaError_t e = remap_smem_attr(k_remap_energy_adj_split<LM>, remap_smem(LM, 8));
     if (e != cudaSuccess) return e;
-    k_remap_energy_adj_split<LM><<<(n + RM_LANES - 1) / RM_LANES, RM_LANES * RMA_WARPS, sm, s>>>(
+    launch(k_remap_energy_adj_split<LM>, (n + RM_LANES - 1) / RM_LANES, RM_LANES * RMA_WARPS, sm, s, 
         g, ra, dp, pt, ud, vd, urem, vrem, gzs, lam_dpo, lam_pto, lam_udo, lam_vdo, lam_dp, lam_pt, lam_ud, lam_vd, lam_ur,
         lam_vr);
   }
@@ -154,13 +153,13 @@ static cudaError_t remap_winds_adj_lm(const Geom& g, const RemapArgs& ra, const 
                                       double* lam_ud, double* lam_vd, cudaStream_t s) {
   const int n = (g.nx + 2) * (g.ny + 2);
   if constexpr (LM > 64) {
-    k_remap_winds_adj<LM><<<dim3((n + 63) / 64, 2), 64, 0, s>>>(g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud,
+    launch(k_remap_winds_adj<LM>, dim3((n + 63) / 64, 2), 64, 0, s, g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud,
                                                                 lam_vd);
   } else {
     const size_t sm = remap_smem(g.L, 6);
     const cudaError_t e = remap_smem_attr(k_remap_winds_adj_split<LM>, remap_smem(LM, 6));
     if (e != cudaSuccess) return e;
-    k_remap_winds_adj_split<LM><<<dim3((n + RM_LANES - 1) / RM_LANES, 2), RM_LANES * RMA_WARPS, sm, s>>>(
+    launch(k_remap_winds_adj_split<LM>, dim3((n + RM_LANES - 1) / RM_LANES, 2), RM_LANES * RMA_WARPS, sm, s, 
         g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud, lam_vd);
   }
   return cudaGetLastError();

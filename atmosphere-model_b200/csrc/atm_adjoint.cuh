@@ -30,6 +30,7 @@ __device__ __forceinline__ int sel_mx3(double a, double b, double c) {
 // the results are stored, not added.
 __global__ void k_corners_adj(Geom g, const double* __restrict__ lam_pkb, const double* __restrict__ lam_gzb,
                               double* lam_pk, double* lam_gz) {
+  stream_order();
   // one thread per point and level (blockIdx.y): the 16-point gathers of a
   // block's row of points hit L1, and every level runs in parallel
   const int w = g.nx + 4, h = g.ny + 4;
@@ -63,6 +64,7 @@ __global__ void k_corners_adj(Geom g, const double* __restrict__ lam_pkb, const 
 // point's adjoint is added to its periodic image in the interior and
 // cleared.
 __global__ void k_ring_fold(Geom g, double* f0, double* f1, double* f2, double* f3, int K) {
+  stream_order();
   const int wide = g.nx + 2 * H;
   const int nband = 2 * H * wide;
   const int nring = nband + 2 * H * g.ny;
@@ -98,6 +100,7 @@ __global__ void k_ring_fold(Geom g, double* f0, double* f1, double* f2, double* 
 // [-band23, n+band23)^2 were recomputed and keep their adjoint.
 __global__ void k_ring_copy_adj(Geom g, double* d0, double* d1, double* d2, double* d3, double* s0, double* s1,
                                 double* s2, double* s3, int K, int band01, int band23) {
+  stream_order();
   const int wide = g.nx + 2 * H;
   const int nband = 2 * H * wide;
   const int nring = nband + 2 * H * g.ny;
@@ -701,6 +704,7 @@ __global__ void __launch_bounds__(64, 16) k_remap_energy_adj(Geom g, RemapArgs r
                                                          const double* __restrict__ lam_vdo, double* lam_dp,
                                                          double* lam_pt, double* lam_ud, double* lam_vd, double* lam_ur,
                                                          double* lam_vr) {
+  stream_order();
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= g.nx * g.ny) return;
   const int i = col % g.nx, j = col / g.nx;
@@ -789,6 +793,7 @@ __global__ void __launch_bounds__(64, 16) k_remap_winds_adj(Geom g, RemapArgs ra
                                                         const double* __restrict__ lam_ur,
                                                         const double* __restrict__ lam_vr, double* lam_dp,
                                                         double* lam_ud, double* lam_vd) {
+  stream_order();
   const int w = g.nx + 2, h = g.ny + 2;
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= w * h) return;

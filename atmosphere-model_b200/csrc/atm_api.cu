@@ -562,13 +562,13 @@ int atm_cgrid_halo(atm_ctx* ctx) {
   int r = require_init(ctx);
   if (r) return r;
   Stage t(ctx, S_CHALO);
-  CK(ctx->ops->ring_cg(ctx->geo, ctx->cg, nullptr, 4, ctx->L, false, ctx->stream));
+  CK(ctx->ops->ring_cg(ctx->geo, ctx->cg, 4, ctx->L, nullptr, false, ctx->stream));
   return ATM_OK;
 }
 
-int atm_dgrid_step(atm_ctx* ctx, double dt) {
-  int r = require_init(ctx);
-  if (r) return r;
+// The D-grid step.  ring: give the new time level the old halo; reset: clear the
+// step's status word.
+static int dgrid_step(atm_ctx* ctx, double dt, bool ring, bool reset) {
   const atm::Ops& ops = *ctx->ops;
   const Geom& g = ctx->geo;
   atm::Consts k = step_consts(ctx, dt);
@@ -582,11 +582,11 @@ int atm_dgrid_step(atm_ctx* ctx, double dt) {
     heat = ctx->heat;
   }
   // the new time level keeps the old halo until the D-grid halo exchange
-  {
+  if (ring) {
     Stage t(ctx, S_DRING);
     CK(ops.ring(g, ctx->st[nxt], (const void* const*)ctx->st[old], 4, ctx->L, true, ctx->stream));
   }
-  CK(cudaMemsetAsync(&ctx->status->nonfinite_step, 0, sizeof(int), ctx->stream));
+  if (reset) CK(cudaMemsetAsync(&ctx->status->nonfinite_step, 0, sizeof(int), ctx->stream));
   // dp, pt on is+4:ie-4 (src/mod_sw_dyn.f90:439-600)
   {
     Stage t(ctx, S_DMASS);
@@ -614,21 +614,28 @@ int atm_dgrid_step(atm_ctx* ctx, double dt) {
   return ATM_OK;
 }
 
-int atm_remap(atm_ctx* ctx) {
+int atm_dgrid_step(atm_ctx* ctx, double dt) {
   int r = require_init(ctx);
   if (r) return r;
+  return dgrid_step(ctx, dt, true, true);
+}
+
+// The remap; ring and reset as for dgrid_step.
+static int remap(atm_ctx* ctx, bool ring, bool reset) {
   const atm::Ops& ops = *ctx->ops;
   const Geom& g = ctx->geo;
   const int src = ctx->cur, dst = 1 - ctx->cur;
   void* const* s = ctx->st[src];
   void* const* d = ctx->st[dst];
   // outside the interior the remapped fields keep the arrays' current values
-  {
+  if (ring) {
     Stage t(ctx, S_RRING);
     CK(ops.ring(g, ctx->st[dst], (const void* const*)ctx->st[src], 4, ctx->L, true, ctx->stream));
   }
-  CK(cudaMemsetAsync(&ctx->status->nonfinite_remap, 0, sizeof(int), ctx->stream));
-  CK(cudaMemsetAsync(&ctx->status->fallback_pairs, 0, sizeof(int), ctx->stream));
+  if (reset) {
+    CK(cudaMemsetAsync(&ctx->status->nonfinite_remap, 0, sizeof(int), ctx->stream));
+    CK(cudaMemsetAsync(&ctx->status->fallback_pairs, 0, sizeof(int), ctx->stream));
+  }
   int* trace = nullptr;
   if (ctx->trace_host) {
     size_t n = (size_t)3 * (ctx->ny + 2) * (ctx->nx + 2) * ctx->L * 5;
@@ -662,6 +669,12 @@ int atm_remap(atm_ctx* ctx) {
     ctx->trace_fallback = nullptr;
   }
   return ATM_OK;
+}
+
+int atm_remap(atm_ctx* ctx) {
+  int r = require_init(ctx);
+  if (r) return r;
+  return remap(ctx, true, true);
 }
 
 int atm_dgrid_halo(atm_ctx* ctx) {
@@ -700,9 +713,14 @@ int atm_mass(atm_ctx* ctx, double* total) {
 int atm_step(atm_ctx* ctx, double dt, int do_remap, int* stable) {
   int r;
   if ((r = atm_cgrid_step(ctx, dt / 2.))) return r;  // src/mod_model.f90:147
-  if ((r = atm_cgrid_halo(ctx))) return r;
-  if ((r = atm_dgrid_step(ctx, dt))) return r;
-  if (do_remap && (r = atm_remap(ctx))) return r;
+  {
+    Stage t(ctx, S_CHALO);  // and the step's status words
+    CK(ctx->ops->ring_cg(ctx->geo, ctx->cg, 4, ctx->L, ctx->status, do_remap != 0, ctx->stream));
+  }
+  // the last halo fill writes every ring point, so the old ring is only worth
+  // copying where the remap reads it (the winds' first ring points)
+  if ((r = dgrid_step(ctx, dt, do_remap != 0, false))) return r;
+  if (do_remap && (r = remap(ctx, false, false))) return r;
   if ((r = atm_dgrid_halo(ctx))) return r;
   if (stable) return atm_check_stability(ctx, stable);
   return ATM_OK;
@@ -1077,7 +1095,7 @@ int atm_adj_dgrid_step(atm_ctx* ctx, double dt) {
   {
     Stage t(ctx, S_AFWD, 1);
     if ((r = fwd_c(ctx, dt / 2., ctx->st[cur]))) return r;
-    CK(ctx->ops->ring_cg(ctx->geo, ctx->cg, nullptr, 4, ctx->L, false, ctx->stream));
+    CK(ctx->ops->ring_cg(ctx->geo, ctx->cg, 4, ctx->L, nullptr, false, ctx->stream));
     if ((r = fwd_d(ctx, dt, ctx->st[cur], ctx->st[1 - cur]))) return r;
   }
   return adj_d(ctx, dt, (const void* const*)ctx->st[cur], (const void* const*)ctx->st[1 - cur],
@@ -1142,7 +1160,7 @@ int atm_adj_step(atm_ctx* ctx, double dt, int do_remap) {
   {
     Stage t(ctx, S_AFWD, 1);
     if ((r = fwd_c(ctx, dt / 2., ctx->st[cur]))) return r;
-    CK(ctx->ops->ring_cg(g, ctx->cg, nullptr, 4, ctx->L, false, ctx->stream));
+    CK(ctx->ops->ring_cg(g, ctx->cg, 4, ctx->L, nullptr, false, ctx->stream));
     if ((r = fwd_d(ctx, dt, ctx->st[cur], ctx->st[nxt]))) return r;
   }
   return adj_step_given(ctx, dt, do_remap, (const void* const*)ctx->st[cur], (const void* const*)ctx->cg,

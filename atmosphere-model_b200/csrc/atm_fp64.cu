@@ -11,7 +11,7 @@ cudaError_t corners(const Geom& g, const double* pkap, const double* gz, double*
                     int lev0, int nlev, cudaStream_t s) {
   int n = (g.nx + 1) * (g.ny + 1);
   const int chunk = few_columns(n) ? 1 : 8;
-  k_corners<<<dim3((n + 255) / 256, (nlev + chunk - 1) / chunk), 256, 0, s>>>(g, pkap, gz, pkapb, gzb, with_pkap,
+  launch(k_corners, dim3((n + 255) / 256, (nlev + chunk - 1) / chunk), 256, 0, s, g, pkap, gz, pkapb, gzb, with_pkap,
                                                                              lev0, nlev, chunk);
   return cudaGetLastError();
 }

@@ -11,6 +11,7 @@
 #include <type_traits>
 
 #include "atm_common.cuh"
+#include "atm_stream.h"
 #include "atm_kappa_tables.h"
 
 namespace atm {
@@ -123,6 +124,7 @@ template <typename T, typename PW = PortablePow>
 __global__ void __launch_bounds__(128) k_column(Geom g, Consts c, const T* __restrict__ dpl, const T* __restrict__ ptl,
                                                 double* __restrict__ pkap, double* __restrict__ gz, int lo, int hi,
                                                 double* __restrict__ plev_out) {
+  stream_order();
   column_at<T, PW>(g, c, dpl, ptl, pkap, gz, lo, hi, plev_out, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -141,6 +143,7 @@ __global__ void __launch_bounds__(32 * COL_WARPS) k_column_split(Geom g, Consts 
                                                                  const T* __restrict__ ptl, double* __restrict__ pkap,
                                                                  double* __restrict__ gz, int lo, int hi,
                                                                  double* __restrict__ plev_out) {
+  stream_order();
   extern __shared__ double col_sm[];
   constexpr int B = 8;  // levels whose loads are in flight together
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -218,6 +221,7 @@ __global__ void __launch_bounds__(32 * COL_WARPS) k_column_split(Geom g, Consts 
 template <typename T>
 __global__ void __launch_bounds__(64) k_heating(Geom g, Consts c, const T* __restrict__ dpl,
                                                 const double* __restrict__ nf, double* __restrict__ heat) {
+  stream_order();
   const int w = g.nx + 2 * H;
   const int col = blockIdx.x * 64 + threadIdx.x;
   if (col >= w * g.NYP) return;
@@ -287,6 +291,7 @@ __device__ __forceinline__ void corner_at(const Geom& g, const double* pkap, con
 static __global__ void k_corners(Geom g, const double* __restrict__ pkap, const double* __restrict__ gz,
                           double* __restrict__ pkapb, double* __restrict__ gzb, int with_pkap, int lev0, int nlev,
                           int chunk) {
+  stream_order();
   const int l0 = lev0 + blockIdx.y * chunk;
   const int n = min(chunk, lev0 + nlev - l0);
   if (n > 0) corner_at(g, pkap, gz, pkapb, gzb, with_pkap, l0, n, blockIdx.x * blockDim.x + threadIdx.x);
@@ -360,7 +365,13 @@ __device__ __forceinline__ void ring_batch(const Geom& g, T* f, const T* s, int 
 }
 
 template <typename T, bool COPY>
-__global__ void k_ring(Geom g, T* f0, T* f1, T* f2, T* f3, const T* s0, const T* s1, const T* s2, const T* s3, int K) {
+__global__ void k_ring(Geom g, T* f0, T* f1, T* f2, T* f3, const T* s0, const T* s1, const T* s2, const T* s3, int K,
+                       Status* reset, bool remap) {
+  stream_order();
+  if (reset && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) {
+    reset->nonfinite_step = 0;
+    if (remap) reset->nonfinite_remap = reset->fallback_pairs = 0;
+  }
   const int k = blockIdx.y;
   if (k >= K) return;
   const int fld = blockIdx.z;

@@ -25,11 +25,11 @@ cudaError_t mass(const Geom& g, const Consts& c, const void* dp, const void* pt,
                  const double* heat, void* dpo, void* pto, int lo, int hi, int* nonfinite, bool cgrid, cudaStream_t s) {
   if (cgrid) {  // state in, C-grid fields out
     const StripPlan p = strips<MK_CMASS>(lo, hi, g);
-    k_mass_m<T, true, S, C><<<p.grid, p.threads, p.threads / MW * MASS_SMEM<T, true, S> + FEED_PAD, s>>>(
+    launch(k_mass_m<T, true, S, C>, p.grid, p.threads, p.threads / MW * MASS_SMEM<T, true, S> + FEED_PAD, s, 
         g, c, (const S*)dp, (const S*)pt, (const S*)u, (const S*)v, heat, (C*)dpo, (C*)pto, lo, hi, nonfinite, p.rows);
   } else {  // state and C-grid winds in, state out
     const StripPlan p = strips<MK_DMASS>(lo, hi, g);
-    k_mass_m<T, false, S, C><<<p.grid, p.threads, p.threads / MW * MASS_SMEM<T, false, S> + FEED_PAD, s>>>(
+    launch(k_mass_m<T, false, S, C>, p.grid, p.threads, p.threads / MW * MASS_SMEM<T, false, S> + FEED_PAD, s, 
         g, c, (const S*)dp, (const S*)pt, (const C*)u, (const C*)v, heat, (S*)dpo, (S*)pto, lo, hi, nonfinite, p.rows);
   }
   return cudaGetLastError();
@@ -42,18 +42,18 @@ cudaError_t column(const Geom& g, const Consts& c, const void* dpl, const void* 
     const int nb = (n + 31) / 32, nt = 32 * COL_WARPS;
     const size_t sm = (size_t)g.L * 32 * sizeof(double);  // at most 32 KB (128 layers)
     if (es == 8)
-      k_column_split<double, FormPow<T>><<<nb, nt, sm, s>>>(g, c, (const double*)dpl, (const double*)ptl, pkap, gz, lo,
+      launch(k_column_split<double, FormPow<T>>, nb, nt, sm, s, g, c, (const double*)dpl, (const double*)ptl, pkap, gz, lo,
                                                             hi, plev);
     else
-      k_column_split<float, FormPow<T>><<<nb, nt, sm, s>>>(g, c, (const float*)dpl, (const float*)ptl, pkap, gz, lo, hi,
+      launch(k_column_split<float, FormPow<T>>, nb, nt, sm, s, g, c, (const float*)dpl, (const float*)ptl, pkap, gz, lo, hi,
                                                            plev);
     return cudaGetLastError();
   }
   if (es == 8)
-    k_column<double, FormPow<T>><<<(n + 127) / 128, 128, 0, s>>>(g, c, (const double*)dpl, (const double*)ptl, pkap, gz,
+    launch(k_column<double, FormPow<T>>, (n + 127) / 128, 128, 0, s, g, c, (const double*)dpl, (const double*)ptl, pkap, gz,
                                                                  lo, hi, plev);
   else
-    k_column<float, FormPow<T>><<<(n + 127) / 128, 128, 0, s>>>(g, c, (const float*)dpl, (const float*)ptl, pkap, gz, lo,
+    launch(k_column<float, FormPow<T>>, (n + 127) / 128, 128, 0, s, g, c, (const float*)dpl, (const float*)ptl, pkap, gz, lo,
                                                                 hi, plev);
   return cudaGetLastError();
 }
@@ -61,15 +61,15 @@ cudaError_t column(const Geom& g, const Consts& c, const void* dpl, const void* 
 cudaError_t heating(const Geom& g, const Consts& c, const void* dpl, int es, const double* nf, double* heat,
                     cudaStream_t s) {
   int n = (g.nx + 2 * H) * g.NYP;
-  if (es == 8) k_heating<double><<<(n + 63) / 64, 64, 0, s>>>(g, c, (const double*)dpl, nf, heat);
-  else k_heating<float><<<(n + 63) / 64, 64, 0, s>>>(g, c, (const float*)dpl, nf, heat);
+  if (es == 8) launch(k_heating<double>, (n + 63) / 64, 64, 0, s, g, c, (const double*)dpl, nf, heat);
+  else launch(k_heating<float>, (n + 63) / 64, 64, 0, s, g, c, (const float*)dpl, nf, heat);
   return cudaGetLastError();
 }
 
 cudaError_t c_mom(const Geom& g, const Consts& c, const void* ud, const void* vd, const double* pkap, const double* gz,
                   void* uc, void* vc, cudaStream_t s) {
   const StripPlan p = strips<MK_CMOM>(0, 0, g);
-  k_c_mom_m<T, S, C><<<p.grid, p.threads, p.threads / MW * FEED_BYTES<CMOM_NF, 0>, s>>>(
+  launch(k_c_mom_m<T, S, C>, p.grid, p.threads, p.threads / MW * FEED_BYTES<CMOM_NF, 0>, s, 
       g, c, (const S*)ud, (const S*)vd, pkap, gz, (C*)uc, (C*)vc, p.rows);
   return cudaGetLastError();
 }
@@ -77,13 +77,14 @@ cudaError_t c_mom(const Geom& g, const Consts& c, const void* ud, const void* vd
 cudaError_t d_mom(const Geom& g, const Consts& c, const void* ud, const void* vd, const void* uc, const void* vc,
                   const double* pkapb, const double* gzb, void* udo, void* vdo, int* nonfinite, cudaStream_t s) {
   const StripPlan p = strips<MK_DMOM>(0, 0, g);
-  k_d_mom_m<T, S, C><<<p.grid, p.threads, p.threads / MW * FEED_BYTES<DMOM_NF<std::is_same_v<S, T>>, 0>, s>>>(
+  launch(k_d_mom_m<T, S, C>, p.grid, p.threads, p.threads / MW * FEED_BYTES<DMOM_NF<std::is_same_v<S, T>>, 0>, s, 
       g, c, (const S*)ud, (const S*)vd, (const C*)uc, (const C*)vc, pkapb, gzb, (S*)udo, (S*)vdo, nonfinite, p.rows);
   return cudaGetLastError();
 }
 
 template <typename E>
-cudaError_t ring_t(const Geom& g, void* const* f, const void* const* src, int nf, int K, bool copy, cudaStream_t s) {
+cudaError_t ring_t(const Geom& g, void* const* f, const void* const* src, int nf, int K, bool copy, Status* reset,
+                   bool remap, cudaStream_t s) {
   int nring = 2 * H * (g.nx + 2 * H) + 2 * H * g.ny;
   dim3 grid((nring + 255) / 256, K, nf);
   E* d[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -93,18 +94,18 @@ cudaError_t ring_t(const Geom& g, void* const* f, const void* const* src, int nf
     if (src) q[i] = (const E*)src[i];
   }
   if (copy)
-    k_ring<E, true><<<grid, 256, 0, s>>>(g, d[0], d[1], d[2], d[3], q[0], q[1], q[2], q[3], K);
+    launch(k_ring<E, true>, grid, 256, 0, s, g, d[0], d[1], d[2], d[3], q[0], q[1], q[2], q[3], K, reset, remap);
   else
-    k_ring<E, false><<<grid, 256, 0, s>>>(g, d[0], d[1], d[2], d[3], q[0], q[1], q[2], q[3], K);
+    launch(k_ring<E, false>, grid, 256, 0, s, g, d[0], d[1], d[2], d[3], q[0], q[1], q[2], q[3], K, reset, remap);
   return cudaGetLastError();
 }
 
 // halo passes of the state fields and of the C-grid fields
 cudaError_t ring(const Geom& g, void* const* f, const void* const* src, int nf, int K, bool copy, cudaStream_t s) {
-  return ring_t<S>(g, f, src, nf, K, copy, s);
+  return ring_t<S>(g, f, src, nf, K, copy, nullptr, false, s);
 }
-cudaError_t ring_cg(const Geom& g, void* const* f, const void* const* src, int nf, int K, bool copy, cudaStream_t s) {
-  return ring_t<C>(g, f, src, nf, K, copy, s);
+cudaError_t ring_cg(const Geom& g, void* const* f, int nf, int K, Status* reset, bool remap, cudaStream_t s) {
+  return ring_t<C>(g, f, nullptr, nf, K, false, reset, remap, s);
 }
 
 cudaError_t remap_winds(const Geom& g, const RemapArgs& ra, const void* dp, const void* ud, const void* vd, void* urem,

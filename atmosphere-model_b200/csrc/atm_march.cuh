@@ -627,6 +627,7 @@ __global__ void __launch_bounds__(MW * MWARPS, MarchL<T, CGRID ? MK_CMASS : MK_D
                                                          typename MassM<T, CGRID, S, C>::O* __restrict__ dpo,
                                                          typename MassM<T, CGRID, S, C>::O* __restrict__ pto, int lo,
                                                          int hi, int* nonfinite, int tys) {
+  stream_order();
   extern __shared__ __align__(16) char feed_sm[];
   mass_strip<T, CGRID, S, C>(g, c, dp, pt, u, v, heat, dpo, pto, lo, hi, nonfinite, strip_x(), blockIdx.y, blockIdx.z,
                              tys, feed_sm + 8);
@@ -787,6 +788,7 @@ __global__ void __launch_bounds__(MW * MWARPS, MarchL<T, MK_CMOM>::min_blocks) k
                                                           const S* __restrict__ vd, const double* __restrict__ pkap,
                                                           const double* __restrict__ gz, C* __restrict__ uc,
                                                           C* __restrict__ vc, int tys) {
+  stream_order();
   extern __shared__ __align__(16) char feed_sm[];
   c_mom_strip<T, S, C>(g, c, ud, vd, pkap, gz, uc, vc, strip_x(), blockIdx.y, blockIdx.z, tys, feed_sm);
 }
@@ -962,6 +964,7 @@ __global__ void __launch_bounds__(MW * MWARPS, MarchL<T, MK_DMOM>::min_blocks) k
                                                           const C* __restrict__ vc, const double* __restrict__ pkapb,
                                                           const double* __restrict__ gzb, S* __restrict__ udo,
                                                           S* __restrict__ vdo, int* nonfinite, int tys) {
+  stream_order();
   extern __shared__ __align__(16) char feed_sm[];
   d_mom_strip<T, S, C>(g, c, ud, vd, uc, vc, pkapb, gzb, udo, vdo, nonfinite, strip_x(), blockIdx.y, blockIdx.z, tys,
                        feed_sm);

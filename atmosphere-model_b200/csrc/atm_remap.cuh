@@ -186,6 +186,7 @@ template <typename T, int LM, typename E = double>
 __global__ void __launch_bounds__(RM_LANES * RM_WARPS, 4) k_remap_winds_split(
     Geom g, RemapArgs ra, const T* __restrict__ dp, const T* __restrict__ ud, const T* __restrict__ vd,
     T* __restrict__ urem, T* __restrict__ vrem, int* trace, Status* st) {
+  stream_order();
   extern __shared__ double rm_sm[];
   __shared__ double ps[4][RM_LANES];
   __shared__ int bad[RM_LANES];
@@ -284,6 +285,7 @@ __global__ void __launch_bounds__(RM_LANES * RM_WARPS, 3) k_remap_energy_split(
     Geom g, RemapArgs ra, const T* __restrict__ dp, const T* __restrict__ pt, const T* __restrict__ ud,
     const T* __restrict__ vd, const T* __restrict__ urem, const T* __restrict__ vrem, const double* __restrict__ gzs,
     T* __restrict__ dpo, T* __restrict__ pto, T* __restrict__ udo, T* __restrict__ vdo, int* trace, Status* st) {
+  stream_order();
   extern __shared__ double rm_sm[];
   __shared__ int bad[RM_LANES];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -452,6 +454,7 @@ __global__ void __launch_bounds__(64, 16) k_remap_winds(Geom g, RemapArgs ra, co
                                                         const T* __restrict__ ud, const T* __restrict__ vd,
                                                         T* __restrict__ urem, T* __restrict__ vrem, int* trace,
                                                         Status* st) {
+  stream_order();
   remap_winds_at<T, LM, E>(g, ra, dp, ud, vd, urem, vrem, trace, st, blockIdx.x * blockDim.x + threadIdx.x,
                            blockIdx.y);
 }
@@ -462,6 +465,7 @@ __global__ void __launch_bounds__(64, 16) k_remap_energy(Geom g, RemapArgs ra, c
                                                          const T* __restrict__ vrem, const double* __restrict__ gzs,
                                                          T* __restrict__ dpo, T* __restrict__ pto, T* __restrict__ udo,
                                                          T* __restrict__ vdo, int* trace, Status* st) {
+  stream_order();
   remap_energy_at<T, LM, PW>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, dpo, pto, udo, vdo, trace, st,
                              blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -486,13 +490,13 @@ cudaError_t launch_remap_winds(const Geom& g, const RemapArgs& ra, const T* dp, 
                                T* vrem, int* trace, Status* st, cudaStream_t s) {
   const int n = (g.nx + 2) * (g.ny + 2);
   if (n > RM_WINDS_FEW) {
-    k_remap_winds<T, LM, E><<<dim3((n + 63) / 64, 2), 64, 0, s>>>(g, ra, dp, ud, vd, urem, vrem, trace, st);
+    launch(k_remap_winds<T, LM, E>, dim3((n + 63) / 64, 2), 64, 0, s, g, ra, dp, ud, vd, urem, vrem, trace, st);
     return cudaGetLastError();
   }
   const size_t sm = remap_smem(g.L, 3);
   const cudaError_t e = remap_smem_attr(k_remap_winds_split<T, LM, E>, remap_smem(LM, 3));
   if (e != cudaSuccess) return e;
-  k_remap_winds_split<T, LM, E><<<dim3((n + RM_LANES - 1) / RM_LANES, 2), RM_LANES * RM_WARPS, sm, s>>>(
+  launch(k_remap_winds_split<T, LM, E>, dim3((n + RM_LANES - 1) / RM_LANES, 2), RM_LANES * RM_WARPS, sm, s, 
       g, ra, dp, ud, vd, urem, vrem, trace, st);
   return cudaGetLastError();
 }
@@ -502,14 +506,14 @@ cudaError_t launch_remap_energy(const Geom& g, const RemapArgs& ra, const T* dp,
                                 int* trace, Status* st, cudaStream_t s) {
   const int n = g.nx * g.ny;
   if (n > RM_ENERGY_FEW) {
-    k_remap_energy<T, LM, PW><<<(n + 63) / 64, 64, 0, s>>>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, dpo, pto, udo, vdo,
+    launch(k_remap_energy<T, LM, PW>, (n + 63) / 64, 64, 0, s, g, ra, dp, pt, ud, vd, urem, vrem, gzs, dpo, pto, udo, vdo,
                                                            trace, st);
     return cudaGetLastError();
   }
   const size_t sm = remap_smem(g.L, 4);
   const cudaError_t e = remap_smem_attr(k_remap_energy_split<T, LM, PW>, remap_smem(LM, 4));
   if (e != cudaSuccess) return e;
-  k_remap_energy_split<T, LM, PW><<<(n + RM_LANES - 1) / RM_LANES, RM_LANES * RM_WARPS, sm, s>>>(
+  launch(k_remap_energy_split<T, LM, PW>, (n + RM_LANES - 1) / RM_LANES, RM_LANES * RM_WARPS, sm, s, 
       g, ra, dp, pt, ud, vd, urem, vrem, gzs, dpo, pto, udo, vdo, trace, st);
   return cudaGetLastError();
 }

@@ -353,6 +353,7 @@ __global__ void __launch_bounds__(RM_LANES * RMA_WARPS, 2) k_remap_winds_adj_spl
     Geom g, RemapArgs ra, const double* __restrict__ dp, const double* __restrict__ ud, const double* __restrict__ vd,
     const double* __restrict__ lam_ur, const double* __restrict__ lam_vr, double* lam_dp, double* lam_ud,
     double* lam_vd) {
+  stream_order();
   constexpr int N = (LM + RMA_WARPS - 1) / RMA_WARPS;
   extern __shared__ double rm_sm[];
   __shared__ double part[RMA_PART][RM_LANES];
@@ -472,6 +473,7 @@ __global__ void __launch_bounds__(RM_LANES * RMA_WARPS, 2) k_remap_energy_adj_sp
     const double* __restrict__ gzs, const double* __restrict__ lam_dpo, const double* __restrict__ lam_pto,
     const double* __restrict__ lam_udo, const double* __restrict__ lam_vdo, double* lam_dp, double* lam_pt,
     double* lam_ud, double* lam_vd, double* lam_ur, double* lam_vr) {
+  stream_order();
   constexpr int N = (LM + RMA_WARPS - 1) / RMA_WARPS;
   extern __shared__ double rm_sm[];
   __shared__ double part[RMA_PART][RM_LANES];
