@@ -520,7 +520,7 @@ int atm_init(atm_ctx* ctx) {
   k_fill<<<148, 256, 0, ctx->stream>>>(ctx->pkapb + g.S * ctx->L, g.S, ctx->cst.pk_top);
   CK(cudaGetLastError());
   // gzb(:,:,1) from the surface geopotential, src/mod_sw_dyn.f90:995-996
-  CK(atm::corners(g, ctx->pkap, ctx->gz, ctx->pkapb, ctx->gzb, 0, 0, 1, ctx->stream));
+  CK(atm::corners_gz0(g, ctx->gz, ctx->gzb, ctx->stream));
   ctx->initialized = true;
   ctx->flag_valid = false;
   return ATM_OK;
@@ -600,7 +600,7 @@ static int dgrid_step(atm_ctx* ctx, double dt, bool ring, bool reset) {
   }
   {
     Stage t(ctx, S_DCORN);
-    CK(atm::corners(g, ctx->pkap, ctx->gz, ctx->pkapb, ctx->gzb, 1, 0, ctx->L, ctx->stream));
+    CK(atm::corners(g, ctx->pkap, ctx->gz, ctx->pkapb, ctx->gzb, ctx->stream));
   }
   // ud, vd on the interior (src/mod_sw_dyn.f90:634-771)
   {
@@ -880,7 +880,7 @@ int fwd_d(atm_ctx* ctx, double dt, void* const* so, void* const* sn) {
   CK(ops.mass(g, k, so[F_DP], so[F_PT], ctx->cg[C_UC], ctx->cg[C_VC], nullptr, sn[F_DP], sn[F_PT], -3, 3,
               &ctx->status->nonfinite_step, false, ctx->stream));
   CK(ops.column(g, k, sn[F_DP], sn[F_PT], ops.elem, ctx->pkap, ctx->gz, -2, 2, nullptr, ctx->stream));
-  CK(atm::corners(g, ctx->pkap, ctx->gz, ctx->pkapb, ctx->gzb, 1, 0, ctx->L, ctx->stream));
+  CK(atm::corners(g, ctx->pkap, ctx->gz, ctx->pkapb, ctx->gzb, ctx->stream));
   CK(ops.d_mom(g, k, so[F_UD], so[F_VD], ctx->cg[C_UC], ctx->cg[C_VC], ctx->pkapb, ctx->gzb, sn[F_UD], sn[F_VD],
                &ctx->status->nonfinite_step, ctx->stream));
   ctx->launches += 5;

@@ -7,13 +7,18 @@
 
 namespace atm {
 
-cudaError_t corners(const Geom& g, const double* pkap, const double* gz, double* pkapb, double* gzb, int with_pkap,
-                    int lev0, int nlev, cudaStream_t s) {
-  int n = (g.nx + 1) * (g.ny + 1);
-  const int chunk = few_columns(n) ? 1 : 8;
-  launch(k_corners, dim3((n + 255) / 256, (nlev + chunk - 1) / chunk), 256, 0, s, g, pkap, gz, pkapb, gzb, with_pkap,
-                                                                             lev0, nlev, chunk);
-  return cudaGetLastError();
+template <bool PK>
+static cudaError_t corners_m(const Geom& g, const double* pkap, const double* gz, double* pkapb, double* gzb, int nlev,
+                             cudaStream_t s) {
+  const StripPlan p = plan_strips(g.nx + 1, g.ny + 1, nlev, COUT, 3, CORN_WARPS_SM);
+  return launch(k_corners_m<PK>, p.grid, p.threads, p.threads / MW * CORN_SMEM<PK>, s, g, pkap, gz, pkapb, gzb, p.rows);
+}
+
+cudaError_t corners(const Geom& g, const double* pkap, const double* gz, double* pkapb, double* gzb, cudaStream_t s) {
+  return corners_m<true>(g, pkap, gz, pkapb, gzb, g.L, s);
+}
+cudaError_t corners_gz0(const Geom& g, const double* gz, double* gzb, cudaStream_t s) {
+  return corners_m<false>(g, nullptr, gz, nullptr, gzb, 1, s);
 }
 
 static __global__ void k_pow_log(const double* x, double y, double* p, double* l, int n) {

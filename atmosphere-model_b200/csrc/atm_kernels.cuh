@@ -256,10 +256,10 @@ __device__ __forceinline__ double corner(const double* q, long long o, int P) {
   return out;
 }
 
-// B levels' loads are issued before their stores: 1 in the corner kernel
-// (measured fastest there), 4 in the persistent ensemble kernel, whose
-// pointers carry no no-alias promise and which runs at lower occupancy.
-template <int B = 1>
+// One corner's column of levels, of the persistent ensemble kernel (k_corners_m of
+// atm_march.cuh has the single domain's): B levels' loads are issued before their
+// stores, whose pointers carry no no-alias promise.
+template <int B>
 __device__ __forceinline__ void corner_at(const Geom& g, const double* pkap, const double* gz, double* pkapb,
                                           double* gzb, int with_pkap, int lev0, int nlev, int idx) {
   const int w = g.nx + 1, h = g.ny + 1;
@@ -282,19 +282,6 @@ __device__ __forceinline__ void corner_at(const Geom& g, const double* pkap, con
       gzb[g.at(x, y, l + (with_pkap ? 1 : 0))] = zb[u];
     }
   }
-}
-
-// blockIdx.y selects a chunk of `chunk` levels, so that more threads share the
-// levels' independent loads: 8 (0.67 ms at 1024x1024x64, against 0.72 / 0.67 /
-// 0.68 / 0.73 at 1 / 4 / 16 / 64), or 1 on domains of few columns (64x64x20:
-// 8.7 us against 12.0 and 16.9 at 4 and 8)
-static __global__ void k_corners(Geom g, const double* __restrict__ pkap, const double* __restrict__ gz,
-                          double* __restrict__ pkapb, double* __restrict__ gzb, int with_pkap, int lev0, int nlev,
-                          int chunk) {
-  stream_order();
-  const int l0 = lev0 + blockIdx.y * chunk;
-  const int n = min(chunk, lev0 + nlev - l0);
-  if (n > 0) corner_at(g, pkap, gz, pkapb, gzb, with_pkap, l0, n, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // =============================================================== halos ====

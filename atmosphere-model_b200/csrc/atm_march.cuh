@@ -970,4 +970,65 @@ __global__ void __launch_bounds__(MW * MWARPS, MarchL<T, MK_DMOM>::min_blocks) k
                        feed_sm);
 }
 
+// ================================================================ corners ==
+// interpolate_to_corners (src/mod_sw_dyn.f90:921-956; corner() of
+// atm_kernels.cuh, in its order) of pkap at level l into pkapb and of gz at level
+// l+1 into gzb on [0, nx] x [0, ny], l = blockIdx.z (PK = false: gz at level l
+// alone).  A strip as the sweeps': each point is loaded once, its interpolation
+// along x formed once and kept for four rows, that along y formed once and
+// passed between lanes; 29 of the 32 columns are outputs.  A thread a corner
+// loaded 32 values of L1 a corner: 0.67 ms at 1024x1024x64 -> 0.42 (251x187x27: 22 us -> 18), bound by the
+// four fields' traffic.
+constexpr int COUT = 29, CORN_WARPS_SM = 32;
+template <bool PK> constexpr int CORN_SMEM = FEED_BYTES<PK ? 2 : 1, 0>;
+struct CornerLine {
+  double q3 = 0, q2 = 0, q1 = 0, q0 = 0, t3 = 0, t2 = 0, t1 = 0, t0 = 0;  // values, x interpolations of rows j-3 .. j
+  __device__ __forceinline__ double push(double q) {  // the corner of row j-1
+    q3 = q2; q2 = q1; q1 = q0; q0 = q;
+    t3 = t2; t2 = t1; t1 = t0;
+    t0 = C7_12 * (q + shfl_up(q, 1)) - C1_12 * (shfl_dn(q, 1) + shfl_up(q, 2));
+    const double y = C7_12 * (q1 + q2) - C1_12 * (q0 + q3);
+    double out = C9_32 * (t1 + t2) - C1_32 * (t0 + t3);
+    out = out + C9_32 * (y + shfl_up(y, 1)) - C1_32 * (shfl_dn(y, 1) + shfl_up(y, 2));
+    return out;
+  }
+};
+template <bool PK>
+__global__ void __launch_bounds__(MW * MWARPS, CORN_WARPS_SM / MWARPS) k_corners_m(Geom g, const double* __restrict__ pkap,
+                                                                                 const double* __restrict__ gz,
+                                                                                 double* __restrict__ pkapb,
+                                                                                 double* __restrict__ gzb, int tys) {
+  stream_order();
+  extern __shared__ __align__(16) char feed_sm[];
+  const int lane = threadIdx.x & (MW - 1);
+  const int ox = strip_x() * COUT, oy = (int)blockIdx.y * tys;
+  if (ox > g.nx) return;
+  const int x = ox - 2 + lane, yend = min(oy + tys, g.ny + 1);
+  const bool out = lane >= 2 && lane < 2 + COUT && x <= g.nx;
+  const long long kS = (long long)blockIdx.z * g.S, zS = PK ? kS + g.S : kS;
+  const unsigned xi = col_of(g, x);
+  enum { F_GZ, F_PK };
+  FeedRing<PK ? 2 : 1, 0> feed(feed_sm);
+  auto copy = [&](int j) {
+    const unsigned r = row_of(g, j) + xi;
+    feed.early(j, F_GZ, gz + (zS + r));
+    if constexpr (PK) feed.early(j, F_PK, pkap + (kS + r));
+  };
+  auto none = [](int) {};
+  feed.start(copy, none, oy - 2);
+  CornerLine lz, lp;
+#pragma unroll 4
+  for (int j = oy - 2; j <= yend; ++j) {
+    feed.next(copy, none, j, yend + 1);
+    const double z = lz.push(feed.template get<double>(j, F_GZ));
+    double p = 0.;
+    if constexpr (PK) p = lp.push(feed.template get<double>(j, F_PK));
+    if (j > oy && out) {
+      const unsigned r = row_of(g, j - 1) + xi;
+      gzb[zS + r] = z;
+      if constexpr (PK) pkapb[kS + r] = p;
+    }
+  }
+}
+
 }  // namespace atm

@@ -48,8 +48,8 @@ extern const Ops ops_fp64;
 extern const Ops ops_mixed;
 
 // interpolate_to_corners of pkap/gz (double in both forms)
-cudaError_t corners(const Geom&, const double* pkap, const double* gz, double* pkapb, double* gzb, int with_pkap,
-                    int lev0, int nlev, cudaStream_t);
+cudaError_t corners(const Geom&, const double* pkap, const double* gz, double* pkapb, double* gzb, cudaStream_t);
+cudaError_t corners_gz0(const Geom&, const double* gz, double* gzb, cudaStream_t);  // level 0 of gzb
 
 // x**y and log(x) of the portable math on the device (tests)
 cudaError_t device_pow_log(const double* x, double y, double* p, double* l, int n, cudaStream_t);
