@@ -850,12 +850,12 @@ int require_adj(atm_ctx* c) {
 
 double** slot_fields(atm_ctx* c, int slot) { return c->lam[slot == ATM_ADJ_IN ? c->slot_in : 1 - c->slot_in]; }
 
-cudaError_t zero_fields(atm_ctx* c, double* const* f, int n, int K) {
-  for (int i = 0; i < n; ++i) {
-    cudaError_t e = cudaMemsetAsync(f[i], 0, (size_t)c->geo.S * K * 8, c->stream);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+// clears four fields, or four and four more
+cudaError_t zero_fields(atm_ctx* c, double* const* f, double* const* f2 = nullptr) {
+  atm::FieldList z;
+  for (int i = 0; i < 4; ++i) z.add(f[i], nullptr, c->geo.S * c->L);
+  for (int i = 0; f2 && i < 4; ++i) z.add(f2[i], nullptr, c->geo.S * c->L);
+  return atm::fields_zero(z, c->stream);
 }
 
 // forward C step from the state s into cg, pkap, gz (no halo)
@@ -959,8 +959,10 @@ int adj_r(atm_ctx* ctx, const void* const* s1, double* const* lout, double* cons
   Stage t(ctx, S_ARMP, 4);
   CK(ctx->ops->remap_winds(g, ra, s[F_DP], s[F_UD], s[F_VD], ctx->urem, ctx->vrem, nullptr, ctx->status,
                            ctx->stream));
-  CK(cudaMemsetAsync(ctx->lam_ur, 0, (size_t)g.S * ctx->L * 8, ctx->stream));
-  CK(cudaMemsetAsync(ctx->lam_vr, 0, (size_t)g.S * ctx->L * 8, ctx->stream));
+  atm::FieldList z;
+  z.add(ctx->lam_ur, nullptr, g.S * ctx->L);
+  z.add(ctx->lam_vr, nullptr, g.S * ctx->L);
+  CK(atm::fields_zero(z, ctx->stream));
   CK(atm::adj_remap_energy(g, ra, s[F_DP], s[F_PT], s[F_UD], s[F_VD], (const double*)ctx->urem,
                            (const double*)ctx->vrem, ctx->gz, lout[F_DP], lout[F_PT], lout[F_UD], lout[F_VD], lin[F_DP],
                            lin[F_PT], lin[F_UD], lin[F_VD], ctx->lam_ur, ctx->lam_vr, ctx->stream));
@@ -1013,9 +1015,8 @@ int atm_adj_enable(atm_ctx* ctx) {
 int atm_adj_zero(atm_ctx* ctx) {
   if (!ctx) return ATM_ERR_ARG;
   if (!ctx->adj) return fail(ctx, ATM_ERR_STATE, "atm_adj_enable has not been called");
-  CK(zero_fields(ctx, ctx->lam[0], 4, ctx->L));
-  CK(zero_fields(ctx, ctx->lam[1], 4, ctx->L));
-  CK(zero_fields(ctx, ctx->lam_cg, 4, ctx->L));
+  CK(zero_fields(ctx, ctx->lam[0], ctx->lam[1]));
+  CK(zero_fields(ctx, ctx->lam_cg));
   ctx->slot_in = 0;
   return ATM_OK;
 }
@@ -1118,13 +1119,12 @@ int adj_step_given(atm_ctx* ctx, double dt, int do_remap, const void* const* s0,
                    const void* const* s1) {
   const Geom& g = ctx->geo;
   if (do_remap) {
-    CK(zero_fields(ctx, slot_fields(ctx, ATM_ADJ_IN), 4, ctx->L));
+    CK(zero_fields(ctx, slot_fields(ctx, ATM_ADJ_IN)));
     int r = adj_r(ctx, s1, slot_fields(ctx, ATM_ADJ_OUT), slot_fields(ctx, ATM_ADJ_IN));
     if (r) return r;
     ctx->slot_in = 1 - ctx->slot_in;
   }
-  CK(zero_fields(ctx, slot_fields(ctx, ATM_ADJ_IN), 4, ctx->L));
-  CK(zero_fields(ctx, ctx->lam_cg, 4, ctx->L));
+  CK(zero_fields(ctx, slot_fields(ctx, ATM_ADJ_IN), ctx->lam_cg));
   int r = adj_d(ctx, dt, s0, s1, slot_fields(ctx, ATM_ADJ_OUT), slot_fields(ctx, ATM_ADJ_IN), cgf);
   if (r) return r;
   {
@@ -1180,18 +1180,22 @@ int atm_step_tape(atm_ctx* ctx, double dt, int do_remap, void* tape) {
   if (!tape) return ATM_ERR_ARG;
   const size_t fb = field_bytes(ctx), lb = level_bytes(ctx);
   char* t = (char*)tape;
-  for (int i = 0; i < 4; ++i)
-    CK(cudaMemcpyAsync(t + (TAPE_S0 + i) * fb, ctx->st[ctx->cur][i], fb, cudaMemcpyDeviceToDevice, ctx->stream));
+  const long long fe = (long long)(fb / 8), le = (long long)(lb / 8);
   if ((r = atm_cgrid_step(ctx, dt / 2.))) return r;
   if ((r = atm_cgrid_halo(ctx))) return r;
-  for (int i = 0; i < 4; ++i)
-    CK(cudaMemcpyAsync(t + (TAPE_CG + i) * fb, ctx->cg[i], fb, cudaMemcpyDeviceToDevice, ctx->stream));
+  atm::FieldList c1, c2;
+  for (int i = 0; i < 4; ++i) {  // the state before the step (the C-grid step leaves it) and the C-grid fields
+    c1.add((double*)(t + (TAPE_S0 + i) * fb), (const double*)ctx->st[ctx->cur][i], fe);
+    c1.add((double*)(t + (TAPE_CG + i) * fb), (const double*)ctx->cg[i], fe);
+  }
+  CK(atm::fields_copy(c1, ctx->stream));
   if ((r = atm_dgrid_step(ctx, dt))) return r;
   for (int i = 0; i < 4; ++i)
-    CK(cudaMemcpyAsync(t + (TAPE_S1 + i) * fb, ctx->st[ctx->cur][i], fb, cudaMemcpyDeviceToDevice, ctx->stream));
-  char* tb = t + TAPE_FIELDS * fb;
-  CK(cudaMemcpyAsync(tb, ctx->pkapb, lb, cudaMemcpyDeviceToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(tb + lb, ctx->gzb, lb, cudaMemcpyDeviceToDevice, ctx->stream));
+    c2.add((double*)(t + (TAPE_S1 + i) * fb), (const double*)ctx->st[ctx->cur][i], fe);
+  double* tb = (double*)(t + TAPE_FIELDS * fb);
+  c2.add(tb, ctx->pkapb, le);
+  c2.add(tb + le, ctx->gzb, le);
+  CK(atm::fields_copy(c2, ctx->stream));
   if (do_remap && (r = atm_remap(ctx))) return r;
   return atm_dgrid_halo(ctx);
 }

@@ -112,6 +112,21 @@ cudaError_t ensemble_launch(const EnsPlan& plan, int blocks, cudaStream_t);
 // 41; 350x350x64 111 -> 119, 512x512x64 191 -> 231)
 inline bool few_columns(long long n) { return n <= 148LL * 512; }
 
+// whole fields: destinations, sources (copies), elements
+struct FieldList {
+  double* d[10];
+  const double* s[10];
+  long long n[10];
+  int nf = 0;
+  void add(double* dst, const double* src, long long elems) {
+    d[nf] = dst;
+    s[nf] = src;
+    n[nf++] = elems;
+  }
+};
+cudaError_t fields_copy(const FieldList&, cudaStream_t);
+cudaError_t fields_zero(const FieldList&, cudaStream_t);
+
 // largest number of layers the vertical remap supports
 constexpr int MAX_LAYERS = 128;
 

@@ -285,3 +285,20 @@ def test_layer_counts_dot_product(nx, ny, nlay):
     lhs, scale = sum(np.sum(x) for x in terms), sum(np.sum(np.abs(x)) for x in terms)
     assert abs(lhs - rhs) <= TOL * scale, (lhs, rhs, scale)
     g.close()
+
+
+def test_tape_alignment():
+    """The tape is written alike on 16-byte and on 8-byte boundaries."""
+    import torch
+    st = generic_state(9, 8, 5, seed=3)
+    tapes = []
+    for shift in (0, 1):
+        g = Dycore(st)
+        n = g.tape_bytes() // 8
+        buf = torch.full((n + 2,), 7.0, dtype=torch.float64, device='cuda')
+        g.step_tape(st.dt, True, buf.data_ptr() + 8 * shift)
+        torch.cuda.synchronize()
+        tapes.append(buf[shift:shift + n].cpu().numpy())
+        assert buf[shift + n].item() == 7.0 and (shift == 0 or buf[0].item() == 7.0)
+        g.close()
+    np.testing.assert_array_equal(tapes[0], tapes[1])
