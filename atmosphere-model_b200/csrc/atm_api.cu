@@ -721,8 +721,13 @@ int atm_step(atm_ctx* ctx, double dt, int do_remap, int* stable) {
   // copying where the remap reads it (the winds' first ring points)
   if ((r = dgrid_step(ctx, dt, do_remap != 0, false))) return r;
   if (do_remap && (r = remap(ctx, false, false))) return r;
-  if ((r = atm_dgrid_halo(ctx))) return r;
-  if (stable) return atm_check_stability(ctx, stable);
+  if (!stable) return atm_dgrid_halo(ctx);
+  {
+    Stage t(ctx, S_DHALO);
+    CK(ctx->ops->ring_report(ctx->geo, ctx->st[ctx->cur], ctx->L, ctx->status, ctx->h_status, ctx->stream));
+  }
+  CK(cudaStreamSynchronize(ctx->stream));
+  *stable = (ctx->remapped ? ctx->h_status->nonfinite_remap : ctx->h_status->nonfinite_step) ? 0 : 1;
   return ATM_OK;
 }
 

@@ -218,25 +218,42 @@ __global__ void __launch_bounds__(32 * COL_WARPS) k_column_split(Geom g, Consts 
 // src/mod_sw_dyn.f90:89-106 (C) and 433-464 (D): pkap from dp (C step) or
 // dpc (D step) over the whole padded domain, playkap, then
 // heat = (nf(k+1) - nf(k)) / (cp dp / g) / playkap.
+// The levels of 32 columns are shared by a block's warps, as in k_column_split: one
+// warp sums the pressures, all share the powers and logarithms (shared memory:
+// plev and pkap of nlay x 32).  With a thread a column, its nlay powers and
+// logarithms in a row left the GPU waiting: 192x160x48 97 -> 46 us, 512x512x64 326 ->
+// 322.
+constexpr int HEAT_WARPS = 8;
 template <typename T>
-__global__ void __launch_bounds__(64) k_heating(Geom g, Consts c, const T* __restrict__ dpl,
-                                                const double* __restrict__ nf, double* __restrict__ heat) {
+__global__ void __launch_bounds__(32 * HEAT_WARPS) k_heating(Geom g, Consts c, const T* __restrict__ dpl,
+                                                                   const double* __restrict__ nf,
+                                                                   double* __restrict__ heat) {
   stream_order();
-  const int w = g.nx + 2 * H;
-  const int col = blockIdx.x * 64 + threadIdx.x;
-  if (col >= w * g.NYP) return;
-  const int x = -H + col % w, y = -H + col / w;
-  const long long o = g.at(x, y);
-  const int L = g.L;
-  double plev = c.ptop, pk_up = c.pk_top;
-  for (int k = L - 1; k >= 0; --k) {
-    long long ok = o + (long long)k * g.S;
-    double d = (double)dpl[ok];
-    plev = plev + d;
-    double pk = atm_pow(plev, KAPPA);
-    double playkap = (pk_up - pk) / atm_log(pk_up / pk);
-    heat[ok] = (nf[ok + g.S] - nf[ok]) / (CP_DRY * d / c.gravity) / playkap;
-    pk_up = pk;
+  extern __shared__ double heat_sm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int w = g.nx + 2 * H, L = g.L;
+  const int col = blockIdx.x * 32 + lane;
+  const bool in = col < w * g.NYP;
+  const int cc = in ? col : 0;
+  const long long o = g.at(-H + cc % w, -H + cc / w), S = g.S;
+  double *pl = heat_sm + lane, *pk = pl + 32 * L;
+  if (warp == 0) {
+    double plev = c.ptop;
+#pragma unroll 8
+    for (int k = L - 1; k >= 0; --k) {
+      plev = plev + (double)dpl[o + (long long)k * S];
+      pl[32 * k] = plev;
+    }
+  }
+  __syncthreads();
+  for (int k = warp; k < L; k += HEAT_WARPS) pk[32 * k] = atm_pow(pl[32 * k], KAPPA);
+  __syncthreads();
+  for (int k = warp; k < L; k += HEAT_WARPS) {
+    const long long ok = o + (long long)k * S;
+    const double p0 = pk[32 * k], p1 = k + 1 < L ? pk[32 * (k + 1)] : c.pk_top;
+    const double playkap = (p1 - p0) / atm_log(p1 / p0);
+    const double d = (double)dpl[ok];
+    if (in) heat[ok] = (nf[ok + S] - nf[ok]) / (CP_DRY * d / c.gravity) / playkap;
   }
 }
 
@@ -351,13 +368,26 @@ __device__ __forceinline__ void ring_batch(const Geom& g, T* f, const T* s, int 
     if (od[r] >= 0) f[od[r]] = v[r];
 }
 
+// What the first thread of a step's halo fill does with the status words beside:
+// clears those of the step (and of the remap), or hands all of them to the host
+// (host: mapped memory), which saves a small copy a step.
+struct RingStatus {
+  Status* clear = nullptr;
+  bool remap = false;
+  const Status* report = nullptr;
+  Status* host = nullptr;
+};
+
 template <typename T, bool COPY>
 __global__ void k_ring(Geom g, T* f0, T* f1, T* f2, T* f3, const T* s0, const T* s1, const T* s2, const T* s3, int K,
-                       Status* reset, bool remap) {
+                       RingStatus w) {
   stream_order();
-  if (reset && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) {
-    reset->nonfinite_step = 0;
-    if (remap) reset->nonfinite_remap = reset->fallback_pairs = 0;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) {
+    if (w.clear) {
+      w.clear->nonfinite_step = 0;
+      if (w.remap) w.clear->nonfinite_remap = w.clear->fallback_pairs = 0;
+    }
+    if (w.host) *w.host = *w.report;
   }
   const int k = blockIdx.y;
   if (k >= K) return;
@@ -1026,14 +1056,21 @@ __device__ __forceinline__ void remap_energy_at(const Geom& g, const RemapArgs& 
 
 // ============================================================ reductions ===
 // Finite check of the interior of four fields (src/mod_fields.f90:69-106).
+// A row of a level at a time, the grid filling the GPU (148 x 8 blocks): bound by
+// the four fields' traffic.  512x512x64: 0.45 ms with a division a point and a
+// quarter of the threads -> 0.14.
 template <typename T>
-__global__ void k_check_finite(Geom g, const T* f0, const T* f1, const T* f2, const T* f3, int* flag) {
-  const int n = g.nx * g.ny;
+__global__ void __launch_bounds__(256) k_check_finite(Geom g, const T* __restrict__ f0, const T* __restrict__ f1,
+                                                      const T* __restrict__ f2, const T* __restrict__ f3, int* flag) {
   bool bad = false;
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n * g.L; idx += gridDim.x * blockDim.x) {
-    int k = idx / n, r = idx - k * n;
-    long long o = g.at(r % g.nx, r / g.nx, k);
-    bad = bad || !(finite_(f0[o]) && finite_(f1[o]) && finite_(f2[o]) && finite_(f3[o]));
+  for (int r = blockIdx.x; r < g.ny * g.L; r += gridDim.x) {
+    const int k = r / g.ny;
+    const long long o = g.at(0, r - k * g.ny, k);
+#pragma unroll 2
+    for (int i = threadIdx.x; i < g.nx; i += 256) {
+      const T a = f0[o + i], b = f1[o + i], c = f2[o + i], d = f3[o + i];
+      bad = bad || !(finite_(a) && finite_(b) && finite_(c) && finite_(d));
+    }
   }
   flag_nonfinite(flag, bad);
 }

@@ -61,9 +61,12 @@ cudaError_t column(const Geom& g, const Consts& c, const void* dpl, const void* 
 cudaError_t heating(const Geom& g, const Consts& c, const void* dpl, int es, const double* nf, double* heat,
                     cudaStream_t s) {
   int n = (g.nx + 2 * H) * g.NYP;
-  if (es == 8) launch(k_heating<double>, (n + 63) / 64, 64, 0, s, g, c, (const double*)dpl, nf, heat);
-  else launch(k_heating<float>, (n + 63) / 64, 64, 0, s, g, c, (const float*)dpl, nf, heat);
-  return cudaGetLastError();
+  const int nb = (n + 31) / 32;
+  const size_t sm = (size_t)2 * g.L * 32 * sizeof(double), most = (size_t)2 * MAX_LAYERS * 32 * sizeof(double);
+  const cudaError_t e = es == 8 ? remap_smem_attr(k_heating<double>, most) : remap_smem_attr(k_heating<float>, most);
+  if (e != cudaSuccess) return e;
+  if (es == 8) return launch(k_heating<double>, nb, 32 * HEAT_WARPS, sm, s, g, c, (const double*)dpl, nf, heat);
+  return launch(k_heating<float>, nb, 32 * HEAT_WARPS, sm, s, g, c, (const float*)dpl, nf, heat);
 }
 
 cudaError_t c_mom(const Geom& g, const Consts& c, const void* ud, const void* vd, const double* pkap, const double* gz,
@@ -83,8 +86,8 @@ cudaError_t d_mom(const Geom& g, const Consts& c, const void* ud, const void* vd
 }
 
 template <typename E>
-cudaError_t ring_t(const Geom& g, void* const* f, const void* const* src, int nf, int K, bool copy, Status* reset,
-                   bool remap, cudaStream_t s) {
+cudaError_t ring_t(const Geom& g, void* const* f, const void* const* src, int nf, int K, bool copy,
+                   const RingStatus& w, cudaStream_t s) {
   int nring = 2 * H * (g.nx + 2 * H) + 2 * H * g.ny;
   dim3 grid((nring + 255) / 256, K, nf);
   E* d[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -94,18 +97,28 @@ cudaError_t ring_t(const Geom& g, void* const* f, const void* const* src, int nf
     if (src) q[i] = (const E*)src[i];
   }
   if (copy)
-    launch(k_ring<E, true>, grid, 256, 0, s, g, d[0], d[1], d[2], d[3], q[0], q[1], q[2], q[3], K, reset, remap);
+    launch(k_ring<E, true>, grid, 256, 0, s, g, d[0], d[1], d[2], d[3], q[0], q[1], q[2], q[3], K, w);
   else
-    launch(k_ring<E, false>, grid, 256, 0, s, g, d[0], d[1], d[2], d[3], q[0], q[1], q[2], q[3], K, reset, remap);
+    launch(k_ring<E, false>, grid, 256, 0, s, g, d[0], d[1], d[2], d[3], q[0], q[1], q[2], q[3], K, w);
   return cudaGetLastError();
 }
 
 // halo passes of the state fields and of the C-grid fields
 cudaError_t ring(const Geom& g, void* const* f, const void* const* src, int nf, int K, bool copy, cudaStream_t s) {
-  return ring_t<S>(g, f, src, nf, K, copy, nullptr, false, s);
+  return ring_t<S>(g, f, src, nf, K, copy, RingStatus{}, s);
 }
-cudaError_t ring_cg(const Geom& g, void* const* f, int nf, int K, Status* reset, bool remap, cudaStream_t s) {
-  return ring_t<C>(g, f, nullptr, nf, K, false, reset, remap, s);
+// the four state fields' halo, with the status words to mapped host memory
+cudaError_t ring_report(const Geom& g, void* const* f, int K, const Status* report, Status* host, cudaStream_t s) {
+  RingStatus w;
+  w.report = report;
+  w.host = host;
+  return ring_t<S>(g, f, nullptr, 4, K, false, w, s);
+}
+cudaError_t ring_cg(const Geom& g, void* const* f, int nf, int K, Status* clear, bool remap, cudaStream_t s) {
+  RingStatus w;
+  w.clear = clear;
+  w.remap = remap;
+  return ring_t<C>(g, f, nullptr, nf, K, false, w, s);
 }
 
 cudaError_t remap_winds(const Geom& g, const RemapArgs& ra, const void* dp, const void* ud, const void* vd, void* urem,
@@ -133,7 +146,7 @@ cudaError_t remap_energy(const Geom& g, const RemapArgs& ra, const void* dp, con
 }
 
 cudaError_t check_finite(const Geom& g, const void* const* f, int* flag, cudaStream_t s) {
-  k_check_finite<S><<<296, 256, 0, s>>>(g, (const S*)f[0], (const S*)f[1], (const S*)f[2], (const S*)f[3], flag);
+  k_check_finite<S><<<148 * 8, 256, 0, s>>>(g, (const S*)f[0], (const S*)f[1], (const S*)f[2], (const S*)f[3], flag);
   return cudaGetLastError();
 }
 
@@ -155,7 +168,7 @@ cudaError_t from_double(const double* src, void* dst, long long n, cudaStream_t 
 }  // namespace
 
 const Ops ATM_OPS_NAME = {(int)sizeof(S), (int)sizeof(C), mass,       column,
-                          heating,        c_mom,          d_mom,        ring,       ring_cg,
+                          heating,        c_mom,          d_mom,        ring,       ring_report,   ring_cg,
                           remap_winds,    remap_energy,   check_finite, mass_sum,   to_double,
                           from_double};
 

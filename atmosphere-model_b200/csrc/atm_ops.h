@@ -28,10 +28,12 @@ struct Ops {
                        const double* pkapb, const double* gzb, void* udo, void* vdo, int* nonfinite,
                        cudaStream_t);
   // periodic halo fill (copy = false) or ring copy src -> f (copy = true) of
-  // nf state fields (ring) or C-grid fields (ring_cg, which also clears the step's
-  // words of reset, and the remap's, where it is not null)
+  // nf state fields (ring), the four with the status words to the mapped memory
+  // host (ring_report), or C-grid fields (ring_cg, which clears the step's words of
+  // clear, and the remap's, where it is not null)
   cudaError_t (*ring)(const Geom&, void* const* f, const void* const* src, int nf, int K, bool copy, cudaStream_t);
-  cudaError_t (*ring_cg)(const Geom&, void* const* f, int nf, int K, Status* reset, bool remap, cudaStream_t);
+  cudaError_t (*ring_report)(const Geom&, void* const* f, int K, const Status* report, Status* host, cudaStream_t);
+  cudaError_t (*ring_cg)(const Geom&, void* const* f, int nf, int K, Status* clear, bool remap, cudaStream_t);
   cudaError_t (*remap_winds)(const Geom&, const RemapArgs&, const void* dp, const void* ud, const void* vd,
                              void* urem, void* vrem, int* trace, Status*, cudaStream_t);
   cudaError_t (*remap_energy)(const Geom&, const RemapArgs&, const void* dp, const void* pt, const void* ud,

@@ -102,3 +102,30 @@ def test_layer_counts_near_shared_limit(nlay):
     for name, f in FIELDS:
         np.testing.assert_array_equal(g.get(name, halo=True), o.get(f, halo=True), err_msg=name)
     g.close()
+
+
+@pytest.mark.parametrize('nx,ny,nlay', [(7, 8, 3), (19, 9, 33), (10, 9, 128), (300, 250, 4)])
+def test_heating_bit_exact(nx, ny, nlay):
+    """A step with the heating term of a radiative net flux, and the finite
+    check over the same shapes."""
+    import torch
+    st = ic.jet_case(nx, ny, nlay, 400e3, 400e3, width=900e3, seed=ny)
+    nf = np.random.default_rng(nx).normal(0, 150.0, (nlay + 1, ny + 14, nx + 14))
+    g, o = Dycore(st), pyoracle.OracleModel(st, threads=8)
+    for a in (g, o):
+        a.set_net_flux(nf)
+        a.cgrid_step(15.0)
+        a.cgrid_halo()
+        a.dgrid_step(30.0)
+        a.dgrid_halo()
+    for name, f in FIELDS:
+        np.testing.assert_array_equal(g.get(name, halo=True), o.get(f, halo=True), err_msg=name)
+    pt = g.get('pt')
+    assert g.check_stability()
+    for bad in (np.nan, np.inf):
+        for at in ((0, 0, 0), (nlay - 1, ny - 1, nx - 1)):
+            p = pt.copy()
+            p[at] = bad
+            g.upload_device('pt', torch.from_numpy(p).cuda())
+            assert not g.check_stability()
+    g.close()
