@@ -718,31 +718,20 @@ struct PPMLayers {
 
 // The pair loop as a monotone merge over the eliminated column: dst(m) for
 // m = 1..L in ascending order goes to put(m, value); dc(m) gives the
-// destination coordinate.  trace as in remap_column.
+// destination coordinate.  trace as in remap_column.  The loop runs over the
+// source layers, the lanes of a warp together, so that a layer's edges are
+// formed once a warp and its column arrays are read at one level: running over
+// the targets, lanes met a layer at different targets and formed its edges twice a
+// warp (1024x1024x64: winds 4.84 ms -> 4.09, energy 4.99 -> 4.34; 512x512x32 0.66 ->
+// 0.56 and 0.69 -> 0.60).
 template <typename FV, typename FD, typename FO, typename LA = ColArr>
 __device__ __forceinline__ void remap_merge(int L, ColArr sc, LA lv, LA gam, const FV& var, FD&& dc,
                                             FO&& put, int* trace, long long ts) {
   PPMLayers<FV, LA> ly(lv, gam, L, var);
-  int k0 = 1;
-  double d0 = dc(1);
-  for (int m = 1; m <= L; ++m) {
-    const double d1 = dc(m + 1);
-    while (k0 <= L && sc[k0 + 1] >= d0) ++k0;
-    double acc = 0.;
-    int first = -1, last = -1, w0 = -1, w1 = -1, cnt = 0;
-    for (int k = k0; k <= L; ++k) {
-      const double sk = sc[k];
-      if (!(sk > d1)) break;
-      while (ly.k < k) ly.next();
-      const int which = pair_add_case(acc, ly.btm, ly.top, ly.curv, ly.vk, sk, sc[k + 1], d0, d1);
-      if (first < 0) {
-        first = k;
-        w0 = which;
-      }
-      last = k;
-      w1 = which;
-      ++cnt;
-    }
+  int m = 1;
+  double d0 = dc(1), d1 = dc(2), acc = 0.;
+  int first = -1, last = -1, w0 = -1, w1 = -1, cnt = 0;
+  auto finish = [&]() {  // target m is complete
     put(m, acc);
     if (trace) {
       int* t = trace + (long long)(m - 1) * 5 * ts;
@@ -751,9 +740,36 @@ __device__ __forceinline__ void remap_merge(int L, ColArr sc, LA lv, LA gam, con
       t[2 * ts] = w0;
       t[3 * ts] = w1;
       t[4 * ts] = cnt;
+      first = last = w0 = w1 = -1;
+      cnt = 0;
     }
+    acc = 0.;
+    ++m;
     d0 = d1;
+    if (m <= L) d1 = dc(m + 1);
+  };
+  double sk1 = sc[1];
+  for (int k = 1; k <= L; ++k) {
+    const double sk = sk1;
+    sk1 = sc[k + 1];
+    ly.next();
+    while (m <= L && !(sk > d1)) finish();  // targets that end above the layer's base
+    while (m <= L && sk1 < d0) {
+      const int which = pair_add_case(acc, ly.btm, ly.top, ly.curv, ly.vk, sk, sk1, d0, d1);
+      if (trace) {
+        if (first < 0) {
+          first = k;
+          w0 = which;
+        }
+        last = k;
+        w1 = which;
+        ++cnt;
+      }
+      if (sk1 > d1) break;  // the target goes on in the next layer
+      finish();
+    }
   }
+  while (m <= L) finish();
 }
 
 // Winds on the cell faces over [isd-1, ied+1]^2, src/mod_remap.f90:80-105.
@@ -1023,13 +1039,19 @@ __device__ __forceinline__ void remap_energy_at(const Geom& g, const RemapArgs& 
   }
   int kc = L + 2, kv = L + 1;
   ppm_eliminate<false>(L, [&]() { return plev[--kc]; }, [&]() { return en[--kv]; }, plev, lv, gam);
-  // remapped energy -> potential temperature (:127-161), upward
+  // the remapped energy, kept where its potential temperature goes
+  static_assert(sizeof(T) == 8, "pto holds the remapped energy meanwhile");
+  remap_merge(L, plev, lv, gam, [&](int k) { return en[k]; }, tpl,
+              [&](int m, double erm) { pto[o + (long long)(m - 1) * S] = T(erm); }, tr, 1);
+  // remapped energy -> potential temperature (:127-161), upward; a pass of its
+  // own, as the lanes finish a target at different layers of the merge
   double gzr = gzs[o];
   double tpl0 = tpl(1);
   double tpk0 = PW::kappa(tpl0);
   bool bad = false;
-  auto put = [&](int m, double erm) {
+  for (int m = 1; m <= L; ++m) {
     const long long ok = o + (long long)(m - 1) * S;
+    const double erm = (double)pto[ok];
     const double tpl1 = tpl(m + 1);
     const double tpk1 = m < L ? PW::kappa(tpl1) : ra.pk_top;
     const double plog = PW::log(tpk1 / tpk0);
@@ -1049,8 +1071,7 @@ __device__ __forceinline__ void remap_energy_at(const Geom& g, const RemapArgs& 
     bad = bad || !(finite_(dpn) && finite_(tn) && finite_(un) && finite_(vn));
     tpl0 = tpl1;
     tpk0 = tpk1;
-  };
-  remap_merge(L, plev, lv, gam, [&](int k) { return en[k]; }, tpl, put, tr, 1);
+  }
   flag_nonfinite(&st->nonfinite_remap, bad);
 }
 

@@ -445,10 +445,8 @@ __global__ void __launch_bounds__(RM_LANES * RM_WARPS, 3) k_remap_energy_split(
 // One thread a column, for domains that fill the GPU with them: 16 blocks of 64
 // threads per SM (a 64-register budget, the column arrays in local memory
 // either way), as more columns in flight hide more of the local-memory latency
-// (1024x1024x64: winds 4.67 ms against 5.88 at the compiler's own budget, 5.34 at
-// 24 blocks, 7.05 at 32; energy 4.91 against 5.45), with every pair's quotients
-// formed; with those of its case only (pair_add_case) winds 5.29 -> 4.85 ms,
-// energy 5.25 -> 5.01.
+// (1024x1024x64, winds / energy: 4.09 / 4.34 ms, 4.51 / 5.00 at 12 blocks, 4.53 /
+// 4.39 at 20).
 template <typename T, int LM, typename E = double>
 __global__ void __launch_bounds__(64, 16) k_remap_winds(Geom g, RemapArgs ra, const T* __restrict__ dp,
                                                         const T* __restrict__ ud, const T* __restrict__ vd,
@@ -473,9 +471,9 @@ __global__ void __launch_bounds__(64, 16) k_remap_energy(Geom g, RemapArgs ra, c
 // Columns up to which the split kernels are the faster ones.  Their blocks wait
 // for one warp's chains, which other blocks hide only while few columns wait:
 // measured on B200 (us, split against one thread a column), winds 64x64x20 23 /
-// 60, 128x128x20 44 / 70, mixed 150x130x48 122 / 181, 251x187x27 142 / 138,
-// 301x203x40 257 / 224; energy 64x64x20 31 / 113, 128x128x20 66 / 121,
-// 256x256x32 232 / 293, 301x203x40 291 / 357, 350x350x64 893 / 709.
+// 52, 128x128x20 45 / 58, mixed 150x130x48 121 / 148, 192x160x48 166 / 177, 251x187x27
+// 144 / 121, 301x203x40 254 / 195; energy 64x64x20 31 / 97, 128x128x20 66 / 105,
+// 251x187x27 170 / 193, 256x256x32 232 / 242, 301x203x40 291 / 295, 350x350x64 965 / 610.
 constexpr long long RM_WINDS_FEW = 148LL * 256, RM_ENERGY_FEW = 148LL * 512;
 
 // Shared memory above the default limit, which the kernel's own variables count
