@@ -1108,6 +1108,61 @@ static __global__ void __launch_bounds__(128) k_pgf_adj_corners(Geom g, Consts c
   if (k1 == g.L) lam_gzb[pgf.o + (long long)g.L * g.S] = lo.z1;
 }
 
+// ==================================================== corners adjoint ====
+// Adjoint of interpolate_to_corners (src/mod_sw_dyn.f90:921-956): the 4x4-point
+// corner value has weights a(dx) b(dy) + b(dx) a(dy) with a = (-1/12, 7/12, 7/12,
+// -1/12) and b = (-1/32, 9/32, 9/32, -1/32) over dx, dy = -2..1.  Gathered over the
+// corners [0, nx] x [0, ny] that each point of [-2, nx+1]^2 feeds: pkapb(l) ->
+// pkap(l) and gzb(l+1) -> gz(l+1), l < nlay; the results are stored, not added.
+// Strips as the forward's (k_corners_m): the two sums along x of a row are formed
+// once and kept for four rows; 29 of the 32 columns are outputs.  A thread a point
+// gathered 32 values: 0.16 ms at 512x512x32 -> 0.07.
+struct CornerAdjLine {
+  double a3 = 0, a2 = 0, a1 = 0, a0 = 0, b3 = 0, b2 = 0, b1 = 0, b0 = 0;  // sums along x with a, b, rows j-3 .. j
+  __device__ __forceinline__ double push(double q) {  // the gather of row j-2
+    a3 = a2; a2 = a1; a1 = a0;
+    b3 = b2; b2 = b1; b1 = b0;
+    const double n = q + shfl_dn(q, 1), f = shfl_dn(q, 2) + shfl_up(q, 1);
+    a0 = C7_12 * n - C1_12 * f;
+    b0 = C9_32 * n - C1_32 * f;
+    return (C9_32 * (a2 + a1) - C1_32 * (a0 + a3)) + (C7_12 * (b2 + b1) - C1_12 * (b0 + b3));
+  }
+};
+static __global__ void __launch_bounds__(MW * MWARPS, CORN_WARPS_SM / MWARPS) k_corners_adj(
+    Geom g, const double* __restrict__ lam_pkb, const double* __restrict__ lam_gzb, double* __restrict__ lam_pk,
+    double* __restrict__ lam_gz, int tys) {
+  stream_order();
+  extern __shared__ __align__(16) char feed_sm[];
+  const int lane = threadIdx.x & (MW - 1);
+  const int ox = -2 + strip_x() * COUT, oy = -2 + (int)blockIdx.y * tys;
+  if (ox > g.nx + 1) return;
+  const int x = ox - 1 + lane, yend = min(oy + tys, g.ny + 2);
+  const bool out = lane >= 1 && lane < 1 + COUT && x <= g.nx + 1, inx = x >= 0 && x <= g.nx;
+  const long long kS = (long long)blockIdx.z * g.S, zS = kS + g.S;
+  const unsigned xi = col_of(g, x);
+  enum { F_GZ, F_PK };
+  FeedRing<2, 0> feed(feed_sm);
+  auto copy = [&](int j) {
+    const unsigned r = row_of(g, j) + xi;
+    feed.early(j, F_GZ, lam_gzb + (zS + r));
+    feed.early(j, F_PK, lam_pkb + (kS + r));
+  };
+  auto none = [](int) {};
+  feed.start(copy, none, oy - 1);
+  CornerAdjLine lz, lp;
+#pragma unroll 4
+  for (int j = oy - 1; j < yend + 2; ++j) {
+    feed.next(copy, none, j, yend + 2);
+    const bool ok = inx && j >= 0 && j <= g.ny;  // a corner
+    const double z = lz.push(ok ? feed.get<double>(j, F_GZ) : 0.), p = lp.push(ok ? feed.get<double>(j, F_PK) : 0.);
+    if (j >= oy + 2 && out) {
+      const unsigned r = row_of(g, j - 2) + xi;
+      lam_gz[zS + r] = z;
+      lam_pk[kS + r] = p;
+    }
+  }
+}
+
 // ================================================== D-momentum adjoint ====
 // Reverse of the D-grid momentum sweep, src/mod_sw_dyn.f90:634-771: ud, vd of
 // layer k from the old ud, vd, uc, vc of layers k and nlay (the pressure-

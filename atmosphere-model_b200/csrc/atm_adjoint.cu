@@ -150,9 +150,9 @@ cudaError_t adj_pgf_corners(const Geom& g, const Consts& c, const double* pkapb,
 
 cudaError_t adj_corners(const Geom& g, const double* lam_pkb, const double* lam_gzb, double* lam_pk, double* lam_gz,
                         cudaStream_t s) {
-  const int n = (g.nx + 4) * (g.ny + 4);
-  launch(k_corners_adj, dim3((n + 255) / 256, g.L), 256, 0, s, g, lam_pkb, lam_gzb, lam_pk, lam_gz);
-  return cudaGetLastError();
+  const StripPlan p = plan_strips(g.nx + 4, g.ny + 4, g.L, COUT, 3, CORN_WARPS_SM);
+  return launch(k_corners_adj, p.grid, p.threads, p.threads / MW * CORN_SMEM<true>, s, g, lam_pkb, lam_gzb, lam_pk, lam_gz,
+                p.rows);
 }
 
 cudaError_t adj_ring_fold(const Geom& g, double* const* f, int nf, int K, cudaStream_t s) {
