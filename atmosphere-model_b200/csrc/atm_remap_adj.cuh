@@ -15,8 +15,9 @@
 // Measured on B200 (the reverse of a remap with the forward winds it needs, ms;
 // before: one thread a column, about twenty column arrays in local memory, waits
 // of 16 to 18 cycles an issued instruction on them): 64x64x20 0.80 -> 0.15,
-// 301x203x40 3.83 -> 2.19, 512x512x32 7.46 -> 5.98.  Now the chains' barriers (5
-// cycles an issued instruction at two blocks an SM).  4 warps a block: 0.22 /
+// 301x203x40 3.83 -> 2.08, 512x512x32 7.46 -> 5.61.  Now the chains' barriers (5
+// cycles an issued instruction at two blocks an SM).  Before the layers' edges and the
+// target coordinate were kept: 0.15 / 2.19 / 5.98; with that, 4 warps a block: 0.22 /
 // 3.25 / 7.19; 16: 0.13 / 2.18 / 5.86; 8 warps at three blocks (80 registers,
 // spilling): 0.16 / 2.41 / 5.81.
 #pragma once
@@ -80,7 +81,8 @@ __device__ __forceinline__ double clamp_adj(double x0, double a, double b, doubl
 // i * RMA_WARPS of the lane's column: from the adjoint ldst(m) of the remapped
 // values, those of the source values (Lv) and of the source coordinate (Ls),
 // and Z += sum of bk(m) times that of the target coordinate dc(m), this
-// thread's part.  A, B from adj_solve; LL, Lg, T scratch; A, B, T are consumed.
+// thread's part.  A, B from adj_solve; LL, Lg, T scratch, consumed like A and B
+// (dc may read T: it is written after the pairs).
 template <int LM, typename FV, typename FD, typename FL, typename FB>
 __device__ __forceinline__ void remap_adj_core(int L, ShCol sc, ShCol A, ShCol B, ShCol LL, ShCol Lg, ShCol T,
                                                double (*ex)[RM_LANES], const FV& var, const FD& dc, const FL& ldst,
@@ -415,18 +417,20 @@ __global__ void __launch_bounds__(RM_LANES * RMA_WARPS, 2) k_remap_winds_adj_spl
     }
     return C7_12 * (ta + tb) - C1_12 * (tc + td);
   };
-  {
-    bool mono = true;
-    for (int k = 1 + warp; k <= L; k += RMA_WARPS) mono = mono && (dc(k + 1) <= dc(k));
-    if (!mono) bad[lane] = 1;
-  }
+  for (int k = 1 + warp; k <= L + 1; k += RMA_WARPS) T[k] = dc(k);  // until the core's scratch
   auto var = [&](int k) { return f[oa + (long long)(k - 1) * S]; };
   auto ldst = [&](int k) { return lr[oa + (long long)(k - 1) * S]; };
   auto bk = [&](int k) { return k <= L ? ra.bk[k - 1] : 0.; };
   adj_solve(L, sc, A, B, var, warp);
+  {
+    bool mono = true;
+    for (int k = 1 + warp; k <= L; k += RMA_WARPS) mono = mono && (T[k + 1] <= T[k]);
+    if (!mono) bad[lane] = 1;
+  }
+  auto td = [&](int k) { return T[k]; };
   double Lv[N], Ls[N], Z = 0.;
   // (ex: the partial sums' array, not read again before the core's barriers)
-  remap_adj_core<LM>(L, sc, A, B, LL, Lg, T, part, var, dc, ldst, bk, warp, Lv, Ls, Z);
+  remap_adj_core<LM>(L, sc, A, B, LL, Lg, T, part, var, td, ldst, bk, warp, Lv, Ls, Z);
   __syncthreads();
   Z = warps_sum(Z, part, warp, lane);
 #pragma unroll
@@ -564,7 +568,7 @@ __global__ void __launch_bounds__(RM_LANES * RMA_WARPS, 2) k_remap_energy_adj_sp
       atomicAdd(v + ok + 1 + P, .125 * lv);
     }
   };
-  double pk0[N], pk1[N], tk0[N], tk1[N], Dk[N];
+  double pk0[N], pk1[N], lyk[N], tk0[N], tk1[N], Dk[N], ke[N];
 #pragma unroll
   for (int q = 0; q < N; ++q) {
     const int k = 1 + warp + q * RMA_WARPS;
@@ -572,33 +576,45 @@ __global__ void __launch_bounds__(RM_LANES * RMA_WARPS, 2) k_remap_energy_adj_sp
     const long long ok = o + (long long)(k - 1) * S;
     pk0[q] = A[k];
     pk1[q] = A[k + 1];
-    const double lyk = (pk1[q] - pk0[q]) / atm_log(pk1[q] / pk0[q]);
+    lyk[q] = (pk1[q] - pk0[q]) / atm_log(pk1[q] / pk0[q]);
     double2 w = wind2(ud, vd, ok);
-    en[k] = CV_DRY * pt[ok] * lyk + .5 * (B[k + 1] + B[k] + w.x * w.x + w.y * w.y);
+    en[k] = CV_DRY * pt[ok] * lyk[q] + .5 * (B[k + 1] + B[k] + w.x * w.x + w.y * w.y);
     tk0[q] = T[k];
     tk1[q] = T[k + 1];
     const double tlyk = (tk1[q] - tk0[q]) / atm_log(tk1[q] / tk0[q]);
     w = wind2(urem, vrem, ok);
     Dk[q] = CV_DRY * tlyk + .5 * CP_DRY * (tk0[q] - tk1[q]);
-    LL[k] = .5 * (w.x * w.x + w.y * w.y);
-    Lg[k] = Dk[q];
+    ke[q] = .5 * (w.x * w.x + w.y * w.y);
   }
   __syncthreads();
   auto var = [&](int k) { return en[k]; };
   adj_solve(L, sc, A, B, var, warp);
-  for (int m = 1 + warp; m <= L; m += RMA_WARPS) {  // the remapped energy
+  for (int k = 1 + warp; k <= L; k += RMA_WARPS) {  // the layers' edges, for the remapped energy
+    double cb, ct, btm, top;
+    adj_edges(k, L, A, B, var, en[k], cb, ct, btm, top);
+    LL[k] = btm;
+    Lg[k] = top;
+  }
+  __syncthreads();
+  for (int m = 1 + warp; m <= L; m += RMA_WARPS) {
     const double d0 = tpl(m), d1 = tpl(m + 1);
     int k = m;
     while (k > 1 && !(sc[k] >= d0)) --k;
     while (k <= L && sc[k + 1] >= d0) ++k;
     double acc = 0.;
     for (; k <= L && sc[k] > d1; ++k) {
-      double cb, ct, btm, top;
-      const double vk = en[k];
-      adj_edges(k, L, A, B, var, vk, cb, ct, btm, top);
+      const double vk = en[k], btm = LL[k], top = Lg[k];
       pair_add_case(acc, btm, top, 6. * vk - 3. * (top + btm), vk, sc[k], sc[k + 1], d0, d1);
     }
     er[m] = acc;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    const int k = 1 + warp + q * RMA_WARPS;
+    if (k > L) continue;
+    LL[k] = ke[q];
+    Lg[k] = Dk[q];
   }
   __syncthreads();
   if (warp == 0) {
@@ -645,12 +661,14 @@ __global__ void __launch_bounds__(RM_LANES * RMA_WARPS, 2) k_remap_energy_adj_sp
       wind2_adj(lam_ur, lam_vr, ok, -w.x * ln, -w.y * ln);
     }
     er[m] = ln;  // (the level's own value, read above)
+    T[m] = tpl(m);
   }
   __syncthreads();
   auto ldst = [&](int k) { return er[k]; };
+  auto td = [&](int k) { return k <= L ? T[k] : ra.ptop; };
   auto bk = [&](int k) { return k <= L ? ra.bk[k - 1] : 0.; };
   double Lv[N], Ls[N];
-  remap_adj_core<LM>(L, sc, A, B, LL, Lg, T, part, var, tpl, ldst, bk, warp, Lv, Ls, Z);
+  remap_adj_core<LM>(L, sc, A, B, LL, Lg, T, part, var, td, ldst, bk, warp, Lv, Ls, Z);
   __syncthreads();
   Z = warps_sum(Z, part, warp, lane);
   // energy (:72-78), hydrostatic gz (:53-56), playkap (:46-52)
@@ -676,11 +694,10 @@ __global__ void __launch_bounds__(RM_LANES * RMA_WARPS, 2) k_remap_energy_adj_sp
     if (k > L) continue;
     const long long ok = o + (long long)(k - 1) * S;
     const double le = Lv[q], lz = LL[k], t = pt[ok], d = pk1[q] - pk0[q];
-    const double lg = atm_log(pk1[q] / pk0[q]), lyk = d / lg;
-    const double y = CV_DRY * t * le / lg;
-    Lpt[q] = CV_DRY * lyk * le - CP_DRY * d * lz;
-    Ls[q] += (y * (-1. + lyk / pk0[q]) + CP_DRY * t * lz) * KAPPA * pk0[q] / sc[k];  // pk = plev**kappa
-    T[k + 1] = k < L ? (y * (1. - lyk / pk1[q]) - CP_DRY * t * lz) * KAPPA * pk1[q] / sc[k + 1] : 0.;
+    const double ly = lyk[q], y = CV_DRY * t * le * ly / d;  // lyk = d / log(pk1 / pk0)
+    Lpt[q] = CV_DRY * ly * le - CP_DRY * d * lz;
+    Ls[q] += (y * (-1. + ly / pk0[q]) + CP_DRY * t * lz) * KAPPA * pk0[q] / sc[k];  // pk = plev**kappa
+    T[k + 1] = k < L ? (y * (1. - ly / pk1[q]) - CP_DRY * t * lz) * KAPPA * pk1[q] / sc[k + 1] : 0.;
     if (live) {
       const double2 w = wind2(ud, vd, ok);
       wind2_adj(lam_ud, lam_vd, ok, w.x * le, w.y * le);
