@@ -33,8 +33,8 @@ __global__ void __launch_bounds__(256) k_fields(FieldList f) {
 }
 
 // strips of a marching reverse over w x h points, `warm` rows beside the strip's own
-inline StripPlan adj_strips(int w, int h, int layers, int out, int warm) {
-  return plan_strips(w, h, layers, out, warm, 3 * MWARPS);
+inline StripPlan adj_strips(int w, int h, int layers, int out, int warm, int most = 128) {
+  return plan_strips(w, h, layers, out, warm, 3 * MWARPS, most);
 }
 
 }  // namespace
@@ -68,7 +68,10 @@ cudaError_t adj_mass(const Geom& g, const Consts& c, const double* dp, const dou
   const MassAdjArgs a{dp, pt, u, v, dpo, pto, lam_dpo, lam_pto, lam_dp, lam_pt, lam_u, lam_v};
   const int w = g.nx - lo + hi, h = g.ny - lo + hi;
   const bool xb = part == 1;
-  const StripPlan p = adj_strips(w, h, g.L, xb ? MOUT : YOUT_MASS, xb ? 4 : 11);
+  // the x kernels take few rows beside a strip's own, and short strips spread their
+  // adjoint sums: 512x512x32 C / D mass 0.362 / 0.473 ms at 18 rows, 0.379 / 0.514 at the
+  // 47 and 65 of an uncapped height, 301x203x40 0.130 / 0.169 at 14, 0.155 / 0.176 at 30
+  const StripPlan p = xb ? adj_strips(w, h, g.L, MOUT, 4, 20) : adj_strips(w, h, g.L, YOUT_MASS, 11);
   const int sm = p.threads / MW * mass_adj_smem(cgrid, xb);
   auto run = [&](auto kernel) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -18,12 +18,13 @@ struct StripPlan {
 // strip takes its rows and `warm` more to fill its windows; a row takes a time
 // that grows with the warps an SM holds, about as 16 + warps (B200, per row
 // of the FP64 C mass sweep: 0.91 us with 4, 1.28 us with 12 warps an SM); full
-// waves are followed by one that is only as crowded as what is left.
+// waves are followed by one that is only as crowded as what is left.  most: the
+// largest height.
 // Measured on B200, mixed form at 150x130x48 (us, C mass / C momentum / D mass
 // / D momentum): powers of two and a wave's cost independent of its size, 49 /
 // 54 / 47 / 58; over all heights from 4 to 128 the best is 33 / 33 / 34 / 37
 // and the heights chosen here are within 4% of it, as at 64x64x20 to 512x512x32.
-inline StripPlan plan_strips(int w, int h, int L, int out, int warm, int warps_sm) {
+inline StripPlan plan_strips(int w, int h, int L, int out, int warm, int warps_sm, int most = 128) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     sms = 148;
@@ -34,7 +35,7 @@ inline StripPlan plan_strips(int w, int h, int L, int out, int warm, int warps_s
   const long long slots = (long long)sms * (warps_sm / wpb * wpb);
   int best = 4;
   long long cost = -1;
-  for (int ns = (h + 127) / 128; ns <= (h + 3) / 4; ++ns) {
+  for (int ns = (h + most - 1) / most; ns <= (h + 3) / 4; ++ns) {
     const int rows = (h + ns - 1) / ns;
     const long long n = (long long)nsx * ((h + rows - 1) / rows) * L, full = n / slots, rem = n % slots;
     long long t = full * (16 + warps_sm);
