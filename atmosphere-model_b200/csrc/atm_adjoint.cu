@@ -181,10 +181,15 @@ static cudaError_t remap_energy_adj_lm(const Geom& g, const RemapArgs& ra, const
                                        const double* lam_udo, const double* lam_vdo, double* lam_dp, double* lam_pt,
                                        double* lam_ud, double* lam_vd, double* lam_ur, double* lam_vr, cudaStream_t s) {
   const int n = g.nx * g.ny;
-  if constexpr (LM > 64) {
+  // From 54 layers one block of the shared-level form fills an SM's shared memory,
+  // which loses on domains of many columns (both reverses of a remap, ms, shared
+  // levels / a thread a column: 64 layers 192x160 2.39 / 3.78, 301x203 4.22 / 4.23,
+  // 400x400 10.9 / 8.9, 512x512 17.6 / 12.5; 50 layers, two blocks, 512x512 10.6 / 11.9)
+  const bool one_block = 2 * (remap_smem(g.L, 8) + 3328) > 228 * 1024;
+  if (LM > 64 || (one_block && n > 148 * 400)) {
     launch(k_remap_energy_adj<LM>, (n + 63) / 64, 64, 0, s, g, ra, dp, pt, ud, vd, urem, vrem, gzs, lam_dpo, lam_pto,
                                                         lam_udo, lam_vdo, lam_dp, lam_pt, lam_ud, lam_vd, lam_ur, lam_vr);
-  } else {
+  } else if constexpr (LM <= 64) {
     const size_t sm = remap_smem(g.L, 8);
     const cudaError_t e = remap_smem_attr(k_remap_energy_adj_split<LM>, remap_smem(LM, 8));
     if (e != cudaSuccess) return e;

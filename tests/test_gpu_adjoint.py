@@ -240,7 +240,7 @@ def test_three_steps_dot_product(remap_every):
 
 
 @pytest.mark.parametrize('nx,ny,nlay', [(9, 8, 3), (13, 9, 20), (20, 17, 32), (9, 8, 33), (11, 8, 64), (8, 7, 65),
-                                        (7, 8, 128)])
+                                        (7, 8, 128), (250, 240, 54)])
 def test_layer_counts_dot_product(nx, ny, nlay):
     """The columns' and the remap's reverse over the ranges of their column
     arrays (up to 32, 64 and 128 layers), on columns that differ enough for
