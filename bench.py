@@ -11,7 +11,7 @@ Workload: the seeded zonal-jet case at 1024 x 1024 x 64 (dx = 25 km,
 dt = 30 s, remap every 8 steps), synthetic data from atmdyn.ic.jet_case.
 The headline ``value`` is forward + adjoint of the FP64 form through the
 torch.autograd binding: K steps forward with checkpoints every 8 steps,
-J = sum(theta^2) over the final state (every tile of the adjoint active),
+J = sum(theta^2) over the final state (every strip of the adjoint active),
 and the hand-written adjoint back to the initial state, per (K cells x
 steps) / (forward + backward time).  Beside it: the FP64 and mixed forward
 forms (``forms``), the masked loss of the differentiation case and its
@@ -82,8 +82,8 @@ def kernel_bytes(stage, form, cells):
 # DRAM bytes per interior cell and launch measured by ncu on the FP64 form
 # (dram__bytes_read.sum + dram__bytes_write.sum, jet 512x512x32, scaled by
 # cells)
-TRAFFIC_PER_CELL_FP64 = {'c_mass': 48.3, 'c_mom': 48.3, 'd_mass': 48.4, 'd_mom': 66.2, 'c_column': 31.4,
-                         'd_column': 31.4}
+TRAFFIC_PER_CELL_FP64 = {'c_mass': 50, 'c_mom': 52, 'd_mass': 49, 'd_mom': 70, 'c_column': 30, 'd_column': 30,
+                         'd_corners': 28}
 
 
 def load_peaks():
@@ -581,7 +581,8 @@ ADJ_WORDS = {
 # DRAM bytes per interior cell and launch of the adjoint kernels measured by
 # ncu (dram__bytes_read.sum + dram__bytes_write.sum, dense adjoint of the
 # jet at 512x512x32, scaled by cells)
-TRAFFIC_PER_CELL_ADJ = {}
+TRAFFIC_PER_CELL_ADJ = {'adj_d_mom_x': 95, 'adj_d_mom_y': 95, 'adj_d_mass_x': 130, 'adj_d_mass_y': 144,
+                        'adj_c_mass_x': 135, 'adj_c_mass_y': 144}
 
 
 def grad_leg(args, torch, barrier, max_over_ranks, world, peak, peak_kind):
@@ -755,7 +756,7 @@ def adjoint_leg(args, torch, max_over_ranks, world):
         return dyn, x, final_theta, mask, J, best
 
     # the headline workload with the masked loss of the differentiation case
-    # (a loss over a sub-domain: tiles outside its domain of dependence skip)
+    # (a loss over a sub-domain: strips outside its domain of dependence skip)
     st = ic.jet_case(args.nx, args.nx, args.nlay, 25e3, 25e3, seed=0)
     st.dt = DT
     nsteps = args.steps
