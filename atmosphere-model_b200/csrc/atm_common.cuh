@@ -101,14 +101,4 @@ template <int B> __device__ __forceinline__ double div_const(double x) {
 // multiplication by the rounded reciprocal.
 template <int B> __device__ __forceinline__ float div_const(float x) { return x * (1.0f / B); }
 
-// Monotone slope dqi_mono(i) and raw slope dqi(i) of src/mod_sw_dyn.f90:870-875
-// from q(i-1), q(i), q(i+1).
-template <typename T>
-__device__ __forceinline__ void slopes(T qm, T q0, T qp, T& dqi, T& mono) {
-  dqi = (qp - qm) * T(0.25);
-  T dmax = mx3(qp, q0, qm) - q0;
-  T dmin = q0 - mn3(qp, q0, qm);
-  mono = cpsign(mn3(fab(dqi), dmin, dmax), dqi);
-}
-
 }  // namespace atm

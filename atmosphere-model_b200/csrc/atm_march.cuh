@@ -108,9 +108,9 @@ __device__ __forceinline__ float mx_nan(float a, float b) {
 __device__ __forceinline__ double mn_nan(double a, double b) { return mn(a, b); }
 __device__ __forceinline__ double mx_nan(double a, double b) { return mx(a, b); }
 
-// Monotone slope of a cell (slopes() of atm_common.cuh) from the differences
+// Monotone slope of a cell (src/mod_sw_dyn.f90:870-875) from the differences
 // dm = q(0) - q(-1), dp = q(+1) - q(0) and dqi = (q(+1) - q(-1)) / 4.
-// slopes() bounds |dqi| by dmax = max(q(+1), q(0), q(-1)) - q(0) and dmin =
+// The reference bounds |dqi| by dmax = max(q(+1), q(0), q(-1)) - q(0) and dmin =
 // q(0) - min(...): where dm and dp agree in sign these two are |dm| and |dp|
 // (the same rounded differences), elsewhere one of them is zero.  So the
 // magnitude is the least of |dqi| and of dm, dp counted positive along dqi,
@@ -135,7 +135,7 @@ __device__ __forceinline__ double third(double x) {
 }
 __device__ __forceinline__ float third(float x) { return div_const<3>(x); }
 
-// The constrained limiter of a cell's raw edge anomalies (edges_pre) with
+// The constrained limiter (src/mod_sw_dyn.f90:878-911) of a cell's raw edge anomalies with
 // its raw slope dqi.
 __device__ __forceinline__ double lim_min(double lim, double e) { return mn(lim, fabs(e)); }
 __device__ __forceinline__ float lim_min(float lim, float e) { return fminf(lim, fabsf(e)); }
@@ -170,7 +170,7 @@ __device__ __forceinline__ void limit_nn(T q0, T dqi, T& eL, T& eR) {
 }
 
 // Upwind flux with Courant number c at the interface between cells m and 0
-// from their values and edges: the operations of flux_pre.
+// from their values and edges (src/mod_sw_dyn.f90:781-868).
 template <typename T>
 __device__ __forceinline__ T flux_e(T c, T qm, T eLm, T eRm, T q0, T eL0, T eR0) {
   const bool pos = c > T(0);
@@ -180,7 +180,7 @@ __device__ __forceinline__ T flux_e(T c, T qm, T eLm, T eRm, T q0, T eL0, T eR0)
   return fmadd(k2, pos ? eLm : eR0, fmadd(k1, pos ? eRm : eL0, pos ? qm : q0));
 }
 // PPM_CONSTRAINED: the upwind value itself where both cells' edges are
-// one-sided (flat_e of each), flux_con_pre
+// one-sided (flat_e of each)
 template <typename T>
 __device__ __forceinline__ bool flat_e(T eL, T eR) {
   return T(3) * fab(eL + eR) > fab(eL - eR);
