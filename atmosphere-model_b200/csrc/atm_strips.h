@@ -35,7 +35,11 @@ inline StripPlan plan_strips(int w, int h, int L, int out, int warm, int warps_s
   const long long slots = (long long)sms * (warps_sm / wpb * wpb);
   int best = 4;
   long long cost = -1;
-  for (int ns = (h + most - 1) / most; ns <= (h + 3) / 4; ++ns) {
+  // every number of strips, or on tall domains every height: at most 128 candidates
+  const bool tall = h > 512;
+  const int c0 = tall ? 4 : (h + most - 1) / most, c1 = tall ? most : (h + 3) / 4;
+  for (int c = c0; c <= c1; ++c) {
+    const int ns = tall ? (h + c - 1) / c : c;
     const int rows = (h + ns - 1) / ns;
     const long long n = (long long)nsx * ((h + rows - 1) / rows) * L, full = n / slots, rem = n % slots;
     long long t = full * (16 + warps_sm);
