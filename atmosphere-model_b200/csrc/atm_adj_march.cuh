@@ -885,34 +885,37 @@ static __global__ void __launch_bounds__(MW * MWARPS, 3) k_c_mom_adj_y(Geom g, C
 // lam_ud, lam_vd += the adjoints of the layer's C-grid winds (their direct
 // terms lam_uc, lam_vc, their part in the vorticity and as advected
 // quantities) through the averages that form them (:110-117), and, in layer
-// nlay, of the A-grid winds of the kinetic energy.  A thread a point of
-// [-4, n+3]^2 (blockIdx.y: row, blockIdx.z: layer).
+// nlay, of the A-grid winds of the kinetic energy.  A thread a column of
+// [-4, n+3]^2, blockIdx.y its first row and gridDim.y the step to the next (a
+// grid holds 65535 rows of blocks, a domain may have more), blockIdx.z the layer.
 static __global__ void __launch_bounds__(128) k_c_mom_adj_fin(Geom g, Consts c, CMomAdjArgs a) {
   stream_order();
-  const int x = -4 + (int)(blockIdx.x * blockDim.x + threadIdx.x), y = -4 + (int)blockIdx.y, k = blockIdx.z;
+  const int x = -4 + (int)(blockIdx.x * blockDim.x + threadIdx.x), k = blockIdx.z;
   if (x >= g.nx + 4) return;
-  const long long o = g.at(x, y, k);
   const int P = g.P;
-  const double* w = a.lam_w + o;
-  const double *s2 = a.lam_uc1 + o, *s3 = a.lam_vc1 + o, *lu = a.lam_uc + o, *lv = a.lam_vc + o;
   auto inx = [&](int q) { return q >= 0 && q < g.nx; };
   auto iny = [&](int q) { return q >= 0 && q < g.ny; };
-  const double wy = (w[-P] - w[P]) + (w[1 - P] - w[1 + P]);
-  const double wx = (w[-1] - w[1]) + (w[P - 1] - w[P + 1]);
-  double su = (s2[0] + s2[1]) + (s2[-P] + s2[1 - P]);
-  double sv = (s3[0] + s3[P]) + (s3[-1] + s3[P - 1]);
-  if (iny(y)) su += (inx(x) ? lu[0] : 0.) + (inx(x + 1) ? lu[1] : 0.);
-  if (iny(y - 1)) su += (inx(x) ? lu[-P] : 0.) + (inx(x + 1) ? lu[1 - P] : 0.);
-  if (iny(y)) sv += (inx(x) ? lv[0] : 0.) + (inx(x - 1) ? lv[-1] : 0.);
-  if (iny(y + 1)) sv += (inx(x) ? lv[P] : 0.) + (inx(x - 1) ? lv[P - 1] : 0.);
-  double du = .25 * (su - c.rdy * wy), dv = .25 * (sv + c.rdx * wx);
-  if (k == g.L - 1) {
-    const double *A = a.lam_ua + g.at(x, y), *B = a.lam_va + g.at(x, y);
-    du += .25 * (A[0] + A[-P]) + .125 * ((A[1] + A[-1]) + (A[1 - P] + A[-1 - P]));
-    dv += .25 * (B[0] + B[-1]) + .125 * ((B[P] + B[-P]) + (B[P - 1] + B[-P - 1]));
+  for (int y = -4 + (int)blockIdx.y; y < g.ny + 4; y += gridDim.y) {
+    const long long o = g.at(x, y, k);
+    const double* w = a.lam_w + o;
+    const double *s2 = a.lam_uc1 + o, *s3 = a.lam_vc1 + o, *lu = a.lam_uc + o, *lv = a.lam_vc + o;
+    const double wy = (w[-P] - w[P]) + (w[1 - P] - w[1 + P]);
+    const double wx = (w[-1] - w[1]) + (w[P - 1] - w[P + 1]);
+    double su = (s2[0] + s2[1]) + (s2[-P] + s2[1 - P]);
+    double sv = (s3[0] + s3[P]) + (s3[-1] + s3[P - 1]);
+    if (iny(y)) su += (inx(x) ? lu[0] : 0.) + (inx(x + 1) ? lu[1] : 0.);
+    if (iny(y - 1)) su += (inx(x) ? lu[-P] : 0.) + (inx(x + 1) ? lu[1 - P] : 0.);
+    if (iny(y)) sv += (inx(x) ? lv[0] : 0.) + (inx(x - 1) ? lv[-1] : 0.);
+    if (iny(y + 1)) sv += (inx(x) ? lv[P] : 0.) + (inx(x - 1) ? lv[P - 1] : 0.);
+    double du = .25 * (su - c.rdy * wy), dv = .25 * (sv + c.rdx * wx);
+    if (k == g.L - 1) {
+      const double *A = a.lam_ua + g.at(x, y), *B = a.lam_va + g.at(x, y);
+      du += .25 * (A[0] + A[-P]) + .125 * ((A[1] + A[-1]) + (A[1 - P] + A[-1 - P]));
+      dv += .25 * (B[0] + B[-1]) + .125 * ((B[P] + B[-P]) + (B[P - 1] + B[-P - 1]));
+    }
+    if (du != 0.) a.lam_ud[o] += du;
+    if (dv != 0.) a.lam_vd[o] += dv;
   }
-  if (du != 0.) a.lam_ud[o] += du;
-  if (dv != 0.) a.lam_vd[o] += dv;
 }
 
 // The four-point pressure-gradient term between two neighbours a (lower index)

@@ -101,7 +101,8 @@ cudaError_t adj_c_mom(const Geom& g, const Consts& c, const double* ud, const do
   launch(k_c_mom_adj_x, p.grid, p.threads, p.threads / MW * ADJ_RING7, s, g, c, a, p.rows);
   p = adj_strips(g.nx + 1, g.ny + 1, g.L, YOUT_CMOM, 10);
   launch(k_c_mom_adj_y, p.grid, p.threads, p.threads / MW * ADJ_RING7, s, g, c, a, p.rows);
-  launch(k_c_mom_adj_fin, dim3((g.nx + 8 + 127) / 128, g.ny + 8, g.L), 128, 0, s, g, c, a);
+  const int rows = g.ny + 8 < 65535 ? g.ny + 8 : 65535;
+  launch(k_c_mom_adj_fin, dim3((g.nx + 8 + 127) / 128, rows, g.L), 128, 0, s, g, c, a);
   return cudaGetLastError();
 }
 

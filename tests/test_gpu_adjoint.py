@@ -287,6 +287,33 @@ def test_layer_counts_dot_product(nx, ny, nlay):
     g.close()
 
 
+def test_tall_domain_dot_product():
+    """The reverse of a step of a domain of more rows than a grid holds rows of
+    blocks (65535).  The bound is on the sum of the products' magnitudes."""
+    nx, ny, nlay = 7, 65600, 3
+    st = generic_state(nx, ny, nlay, seed=9)
+    rng = np.random.default_rng(10)
+    dt = 30.0
+    g = Dycore(st)
+    g.adj_enable()
+    vs = {n: rand(rng, st, n) for n in NAMES}
+    t = tlm_from_gpu(g, st, vs)
+    t.cgrid_step(dt / 2)
+    t.cgrid_halo()
+    t.dgrid_step(dt)
+    w = {n: rand(rng, st, n) for n in NAMES}
+    terms = [w[n] * t.get(STATE[n], halo=True)[1] for n in NAMES]
+    for n in NAMES:
+        g.adj_set('out', n, w[n])
+    g.adj_dgrid_step(dt)
+    g.adj_cgrid_halo()
+    g.adj_cgrid_step(dt / 2)
+    rhs = sum(np.sum(vs[n] * g.adj_get('in', n)) for n in NAMES)
+    lhs, scale = sum(np.sum(x) for x in terms), sum(np.sum(np.abs(x)) for x in terms)
+    assert abs(lhs - rhs) <= TOL * scale, (lhs, rhs, scale)
+    g.close()
+
+
 def test_tape_alignment():
     """The tape is written alike on 16-byte and on 8-byte boundaries."""
     import torch
