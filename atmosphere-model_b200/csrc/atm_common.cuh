@@ -5,6 +5,9 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <type_traits>
+
 #include "atm_math.h"
 
 namespace atm {
@@ -53,6 +56,38 @@ struct Consts {
   double ptop, pk_top;    // Ak(1) and Ak(1)**kappa
   double dt, dtdx, dtdy;  // per call: dtdx = dt*rdx, dtdy = dt*rdy
 };
+
+// How the kernels that pass over whole rows share them: groups of 1 << lg threads,
+// each a row or one of its pieces of len points.  A group's threads fit the row
+// (their last round is not mostly empty), and rows too few to fill the GPU are cut up.  With 64 threads a row
+// whatever its width (256 in the finite check), four fields out of 16x2048x64 took
+// 96 us, in 111, and an upload with the finite check 261, of 7x4096x20 47, 52 and 107;
+// so 46, 86, 69 and 17, 46, 37.
+struct RowSplit {
+  int lg, pieces, len;
+};
+inline RowSplit row_split(int width, int rows, int lg_most) {
+  RowSplit r;
+  r.lg = lg_most;
+  while (r.lg > 3 && ((width - 1) >> r.lg << r.lg) + (1 << r.lg) > width + width / 2 + 2) --r.lg;
+  const int lanes = 1 << r.lg;
+  const int most = (width + 4 * lanes - 1) / (4 * lanes);  // four points a thread at least
+  const int want = (148 * 2048 / lanes + rows - 1) / rows;  // a piece to every group the GPU holds
+  r.pieces = want < most ? want : most;
+  r.len = ((width + r.pieces - 1) / r.pieces + lanes - 1) / lanes * lanes;
+  r.pieces = (width + r.len - 1) / r.len;
+  return r;
+}
+
+// f(the group's lg as a constant)
+template <typename F>
+inline cudaError_t with_lg(const RowSplit& r, F&& f) {
+  if (r.lg <= 3) return f(std::integral_constant<int, 3>{});
+  if (r.lg == 4) return f(std::integral_constant<int, 4>{});
+  if (r.lg == 5) return f(std::integral_constant<int, 5>{});
+  if (r.lg == 6) return f(std::integral_constant<int, 6>{});
+  return f(std::integral_constant<int, 8>{});
+}
 
 // Status words shared by every kernel of a context.
 struct Status {

@@ -1077,18 +1077,22 @@ __device__ __forceinline__ void remap_energy_at(const Geom& g, const RemapArgs& 
 
 // ============================================================ reductions ===
 // Finite check of the interior of four fields (src/mod_fields.f90:69-106).
-// A row of a level at a time, the grid filling the GPU (148 x 8 blocks): bound by
-// the four fields' traffic.  512x512x64: 0.45 ms with a division a point and a
-// quarter of the threads -> 0.14.
-template <typename T>
+// A row of a level, or a piece of one (RowSplit), at a time, the grid filling the
+// GPU (148 x 8 blocks): bound by the four fields' traffic.  512x512x64: 0.45 ms with
+// a division a point and a quarter of the threads -> 0.14.
+template <typename T, int LG>
 __global__ void __launch_bounds__(256) k_check_finite(Geom g, const T* __restrict__ f0, const T* __restrict__ f1,
-                                                      const T* __restrict__ f2, const T* __restrict__ f3, int* flag) {
+                                                      const T* __restrict__ f2, const T* __restrict__ f3, int* flag,
+                                                      RowSplit sp) {
   bool bad = false;
-  for (int r = blockIdx.x; r < g.ny * g.L; r += gridDim.x) {
+  const int n = g.ny * g.L * sp.pieces;
+  constexpr int per = 256 >> LG, lanes = 1 << LG;
+  for (int it = (int)blockIdx.x * per + (int)(threadIdx.x >> LG); it < n; it += (int)gridDim.x * per) {
+    const int r = sp.pieces > 1 ? it / sp.pieces : it, x0 = (it - r * sp.pieces) * sp.len, x1 = min(x0 + sp.len, g.nx);
     const int k = r / g.ny;
     const long long o = g.at(0, r - k * g.ny, k);
 #pragma unroll 2
-    for (int i = threadIdx.x; i < g.nx; i += 256) {
+    for (int i = x0 + ((int)threadIdx.x & (lanes - 1)); i < x1; i += lanes) {
       const T a = f0[o + i], b = f1[o + i], c = f2[o + i], d = f3[o + i];
       bad = bad || !(finite_(a) && finite_(b) && finite_(c) && finite_(d));
     }

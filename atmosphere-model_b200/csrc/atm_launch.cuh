@@ -146,8 +146,13 @@ cudaError_t remap_energy(const Geom& g, const RemapArgs& ra, const void* dp, con
 }
 
 cudaError_t check_finite(const Geom& g, const void* const* f, int* flag, cudaStream_t s) {
-  k_check_finite<S><<<148 * 8, 256, 0, s>>>(g, (const S*)f[0], (const S*)f[1], (const S*)f[2], (const S*)f[3], flag);
-  return cudaGetLastError();
+  RowSplit sp = row_split(g.nx, g.ny * g.L, 8);
+  if (sp.lg == 7) sp = row_split(g.nx, g.ny * g.L, 6);
+  return with_lg(sp, [&](auto lg) {
+    k_check_finite<S, decltype(lg)::value><<<148 * 8, 256, 0, s>>>(g, (const S*)f[0], (const S*)f[1], (const S*)f[2],
+                                                                   (const S*)f[3], flag, sp);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t mass_sum(const Geom& g, const void* dp, double* partial, int nblocks, double* out, cudaStream_t s) {
