@@ -469,12 +469,29 @@ __global__ void __launch_bounds__(64, 16) k_remap_energy(Geom g, RemapArgs ra, c
 }
 
 // Columns up to which the split kernels are the faster ones.  Their blocks wait
-// for one warp's chains, which other blocks hide only while few columns wait:
-// measured on B200 (us, split against one thread a column), winds 64x64x20 23 /
-// 52, 128x128x20 45 / 58, mixed 150x130x48 121 / 148, 192x160x48 166 / 177, 251x187x27
-// 144 / 121, 301x203x40 254 / 195; energy 64x64x20 31 / 97, 128x128x20 66 / 105,
-// 251x187x27 170 / 193, 256x256x32 232 / 242, 301x203x40 291 / 295, 350x350x64 965 / 610.
-constexpr long long RM_WINDS_FEW = 148LL * 256, RM_ENERGY_FEW = 148LL * 512;
+// for one warp's chains, which other blocks hide only while few columns wait: so
+// the limit is a number of columns a block that an SM holds (by the column
+// arrays' shared memory, at most `most` by registers), less where the layers leave
+// some of the block's warps without work.  Measured on B200, FP64 form (us, split
+// against one thread a column; columns in thousands), winds:
+//   3 layers 4.1 11/12, 9.2 14/12; 8 layers 9.2 19/23, 16 21/22, 26 27/23; 20 layers 16 38/47, 26 52/53;
+//   32 and 64 (four blocks) 26 74/89, 157/191, 37 103/100, 223/205;
+//   80 and 96 (three) 16 174/222, 220/267, 26 248/242, 312/292; 112 and 128 (two) 9.2 210/284, 250/329, 16 316/317, 375/365
+// and energy:
+//   3 layers 9.2 15/19, 16 23/19; 8 layers 26 31/37, 37 41/39; 20 layers 37 86/100, 50 118/114;
+//   32 and 64 (three blocks) 50 171/193, 372/402, 66 213/211, 467/436;
+//   80 and 96 (two) 26 368/450, 458/551, 37 500/476, 619/580; 112 and 128 (one) 16 553/608, 633/704, 26 817/650, 952/753
+// With a limit that did not know the layers, a remap of 256x256x128 took 2.70 ms, of
+// 272x272x96 1.61; a thread a column 1.82 and 1.41.
+inline int remap_blocks(int L, int n, int most) {
+  const int b = (int)(228 * 1024 / (remap_smem(L, n) + 2304));  // the kernels' own variables and the block's reserve
+  return b < most ? b : most;
+}
+inline long long remap_winds_few(int L) { return 148LL * 56 * remap_blocks(L, 3, 4) * (L < 32 ? L : 32) / 32; }
+// (more than two blocks of the 65- to 128-layer instance gain nothing: 65 layers 26 240/358, 50 472/408)
+inline long long remap_energy_few(int L) {
+  return 148LL * 120 * remap_blocks(L, 4, L > 64 ? 2 : 3) * (L < 28 ? L + 8 : 36) / 36;
+}
 
 // Shared memory above the default limit, which the kernel's own variables count
 // against too: always what the kernel's largest layer count takes, so that
@@ -487,7 +504,7 @@ template <typename T, int LM, typename E = double>
 cudaError_t launch_remap_winds(const Geom& g, const RemapArgs& ra, const T* dp, const T* ud, const T* vd, T* urem,
                                T* vrem, int* trace, Status* st, cudaStream_t s) {
   const int n = (g.nx + 2) * (g.ny + 2);
-  if (n > RM_WINDS_FEW) {
+  if (n > remap_winds_few(g.L)) {
     launch(k_remap_winds<T, LM, E>, dim3((n + 63) / 64, 2), 64, 0, s, g, ra, dp, ud, vd, urem, vrem, trace, st);
     return cudaGetLastError();
   }
@@ -503,7 +520,7 @@ cudaError_t launch_remap_energy(const Geom& g, const RemapArgs& ra, const T* dp,
                                 const T* urem, const T* vrem, const double* gzs, T* dpo, T* pto, T* udo, T* vdo,
                                 int* trace, Status* st, cudaStream_t s) {
   const int n = g.nx * g.ny;
-  if (n > RM_ENERGY_FEW) {
+  if (n > remap_energy_few(g.L)) {
     launch(k_remap_energy<T, LM, PW>, (n + 63) / 64, 64, 0, s, g, ra, dp, pt, ud, vd, urem, vrem, gzs, dpo, pto, udo, vdo,
                                                            trace, st);
     return cudaGetLastError();

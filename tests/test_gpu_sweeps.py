@@ -129,3 +129,29 @@ def test_heating_bit_exact(nx, ny, nlay):
             g.upload_device('pt', torch.from_numpy(p).cuda())
             assert not g.check_stability()
     g.close()
+
+
+# columns beyond which a thread has a column of its own, in each of the kernels'
+# layer ranges (the limits depend on the layers)
+@pytest.mark.parametrize('nx,ny,nlay', [(131, 130, 3), (171, 160, 8), (240, 230, 33), (203, 190, 65), (140, 137, 128)])
+@pytest.mark.parametrize('fields', ['smooth', 'crossed'])
+def test_remap_thread_a_column_bit_exact(nx, ny, nlay, fields):
+    """The remap of domains of many columns with its layer-pair trace."""
+    st = ic.jet_case(nx, ny, nlay, 400e3, 400e3, width=900e3, seed=ny)
+    rng = np.random.default_rng(nlay)
+    st.dp = st.dp * np.exp(rng.normal(0, 0.2, st.dp.shape))
+    st.u = st.u + rng.normal(0, 15.0, st.u.shape)
+    st.v = st.v + rng.normal(0, 15.0, st.v.shape)
+    if fields == 'crossed':
+        st.dp[1] = np.where(rng.random((ny, nx)) < 0.01, -0.2 * st.dp[1], st.dp[1])
+    g, o = Dycore(st), pyoracle.OracleModel(st, threads=8)
+    trace_o = o.enable_trace()
+    trace_g, fallback = g.remap_trace()
+    g.remap()
+    o.remap()
+    for name, f in FIELDS:
+        np.testing.assert_array_equal(g.get(name, halo=True), o.get(f, halo=True), err_msg=name)
+    np.testing.assert_array_equal(trace_g, trace_o)
+    if fields == 'crossed':
+        assert fallback.value > 0
+    g.close()
