@@ -175,6 +175,25 @@ cudaError_t adj_ring_copy(const Geom& g, double* const* dst, double* const* src,
   return cudaGetLastError();
 }
 
+// Whether the reverse of a remap of n columns takes a thread a column (beyond 64
+// layers always).  Of the energy: from 54 layers one block of the shared-level form
+// fills an SM's shared memory, and few layers leave most of a block's warps without
+// work, either of which loses on domains of many columns.  Measured on B200, both
+// reverses of a remap (us, shared levels / a thread a column; columns in thousands):
+// 3 layers 16 101/104, 37 180/165, 590 2630/1815; 8 layers 66 438/480, 147 964/844;
+// 16 layers 147 1674/1578; 28 layers 262 4947/4891; 32 layers 147 3119/3023, 262 5401/5503;
+// 40 layers 66 2108/2460, 147 4570/3914; 53 layers 66 2830/3283, 147 6184/5204;
+// 54 layers 37 2164/2831, 66 3654/3346; 64 layers 262 16752/11369.
+// Of the winds, whose blocks are smaller, only with few layers (energy by a thread a column):
+// 3 layers 16 104/101, 37 165/147, 590 1815/1055; 6 layers 66 387/344; 8 layers 147 844/806;
+// 11 layers 590 4628/4328; 12 layers 590 4749/4725; 16 layers 590 6021/6488.
+template <int LM>
+static bool remap_adj_columns(int n, int L) {
+  if (LM > 64) return true;
+  const bool one_block = 2 * (remap_smem(L, 8) + 3328) > 228 * 1024;
+  return n > 148 * (L < 10 ? 64 * L : one_block ? 400 : 640);
+}
+
 template <int LM>
 static cudaError_t remap_energy_adj_lm(const Geom& g, const RemapArgs& ra, const double* dp, const double* pt,
                                        const double* ud, const double* vd, const double* urem, const double* vrem,
@@ -182,12 +201,7 @@ static cudaError_t remap_energy_adj_lm(const Geom& g, const RemapArgs& ra, const
                                        const double* lam_udo, const double* lam_vdo, double* lam_dp, double* lam_pt,
                                        double* lam_ud, double* lam_vd, double* lam_ur, double* lam_vr, cudaStream_t s) {
   const int n = g.nx * g.ny;
-  // From 54 layers one block of the shared-level form fills an SM's shared memory,
-  // which loses on domains of many columns (both reverses of a remap, ms, shared
-  // levels / a thread a column: 64 layers 192x160 2.39 / 3.78, 301x203 4.22 / 4.23,
-  // 400x400 10.9 / 8.9, 512x512 17.6 / 12.5; 50 layers, two blocks, 512x512 10.6 / 11.9)
-  const bool one_block = 2 * (remap_smem(g.L, 8) + 3328) > 228 * 1024;
-  if (LM > 64 || (one_block && n > 148 * 400)) {
+  if (remap_adj_columns<LM>(n, g.L) && (LM != 32 || g.L <= 28)) {
     launch(k_remap_energy_adj<LM>, (n + 63) / 64, 64, 0, s, g, ra, dp, pt, ud, vd, urem, vrem, gzs, lam_dpo, lam_pto,
                                                         lam_udo, lam_vdo, lam_dp, lam_pt, lam_ud, lam_vd, lam_ur, lam_vr);
   } else if constexpr (LM <= 64) {
@@ -206,10 +220,10 @@ static cudaError_t remap_winds_adj_lm(const Geom& g, const RemapArgs& ra, const 
                                       const double* vd, const double* lam_ur, const double* lam_vr, double* lam_dp,
                                       double* lam_ud, double* lam_vd, cudaStream_t s) {
   const int n = (g.nx + 2) * (g.ny + 2);
-  if constexpr (LM > 64) {
+  if (remap_adj_columns<LM>(g.nx * g.ny, g.L) && (LM > 64 || g.L < 12)) {
     launch(k_remap_winds_adj<LM>, dim3((n + 63) / 64, 2), 64, 0, s, g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud,
                                                                 lam_vd);
-  } else {
+  } else if constexpr (LM <= 64) {
     const size_t sm = remap_smem(g.L, 6);
     const cudaError_t e = remap_smem_attr(k_remap_winds_adj_split<LM>, remap_smem(LM, 6));
     if (e != cudaSuccess) return e;

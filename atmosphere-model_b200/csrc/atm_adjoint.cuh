@@ -470,7 +470,7 @@ __device__ __noinline__ void remap_energy_pairs(int L, const double* en, double*
 // pre-remap dp, pt (this column), ud, vd (its A-grid neighbours) and of the
 // remapped face winds urem, vrem out.
 // One thread per column, its arrays in local memory: more than 64 layers, many
-// columns of more than 53, and columns whose coordinates are not monotone
+// columns (remap_adj_columns), and columns whose coordinates are not monotone
 // (atm_remap_adj.cuh has the others).
 template <int LM>
 __device__ __noinline__ void remap_energy_adj_at(const Geom& g, const RemapArgs& ra, const double* dp, const double* pt,

@@ -287,6 +287,13 @@ def test_layer_counts_dot_product(nx, ny, nlay):
     g.close()
 
 
+@pytest.mark.parametrize('nx,ny,nlay', [(190, 151, 3), (313, 287, 9), (310, 306, 12), (312, 305, 33)])
+def test_many_columns_dot_product(nx, ny, nlay):
+    """Domains of more columns than the limits beyond which a thread has a column
+    of its own, of few layers (both reverses of the remap) and of more."""
+    test_layer_counts_dot_product(nx, ny, nlay)
+
+
 def test_tall_domain_dot_product():
     """The reverse of a step of a domain of more rows than a grid holds rows of
     blocks (65535).  The bound is on the sum of the products' magnitudes."""
