@@ -159,6 +159,24 @@ struct RadSums {
   }
 };
 
+// The layer properties and flux sums of a column that one thread has to itself
+// (k_radiation_columns), and how its fluxes are added to them.
+template <int LM>
+struct OwnColumn {
+  double play[LM + 1], tlay[LM + 1], dm[LM + 1], tlev[LM + 2], sum[4][LM + 2];
+  unsigned code[LM + 1];
+  int kb[LM + 2];
+};
+template <int LM>
+struct OwnSums {
+  OwnColumn<LM>& c;
+  int which;
+  __device__ __forceinline__ void put(int, int k, double fu, double fd) {
+    c.sum[which][k] = c.sum[which][k] + fu;
+    c.sum[which + 1][k] = c.sum[which + 1][k] + fd;
+  }
+};
+
 // Per-lane working arrays of one g-point (1-based as in the reference).
 template <int LM>
 struct LayerArrays {
@@ -169,9 +187,9 @@ struct LayerArrays {
 // solve_shortwave_column (mod_radiation.f90:158-268) for g-point g: the layer
 // coefficients top-down (the direct beam is attenuated layer by layer), then
 // calculate_fluxes (:349-381); the beam is added to the downward flux.
-template <int LM>
-__device__ __forceinline__ void shortwave(const RadTables& tb, int g, int L, const RadColumn& col, double irradiance,
-                                          double mu0, double sfc_albedo, LayerArrays<LM>& c, RadSums& out) {
+template <int LM, typename Col, typename Out>
+__device__ __forceinline__ void shortwave(const RadTables& tb, int g, int L, const Col& col, double irradiance,
+                                          double mu0, double sfc_albedo, LayerArrays<LM>& c, Out& out) {
   const double* tab = tb.sw_abs + g;
   const double k_sca = tb.sw_sca[g];
   double beam = mu0 * irradiance;
@@ -279,9 +297,9 @@ __device__ __forceinline__ void shortwave(const RadTables& tb, int g, int L, con
 // solve_longwave_column (mod_radiation.f90:270-347) for g-point g: no
 // scattering, a Planck source linear in optical depth; the upward sweep of
 // calculate_fluxes inside its layer loop (both go upward)
-template <int LM>
-__device__ __forceinline__ void longwave(const RadTables& tb, int g, int L, const RadColumn& col, double ts, int kbs,
-                                         double emissivity, LayerArrays<LM>& c, RadSums& out) {
+template <int LM, typename Col, typename Out>
+__device__ __forceinline__ void longwave(const RadTables& tb, int g, int L, const Col& col, double ts, int kbs,
+                                         double emissivity, LayerArrays<LM>& c, Out& out) {
   const double* tab = tb.lw_abs + g;
   const double* plk = tb.plk + g;
   Lookup nx;
@@ -424,9 +442,89 @@ __global__ void __launch_bounds__(RG * RC, 4) k_radiation(Geom g, RadTables tb, 
   }
 }
 
+// The same with a thread a column, its g-points in turn and its arrays in local
+// memory: for tables of few g-points, whose other lanes k_radiation leaves idle,
+// and for few layers, whose work is little beside what a block sets up.  BLOCKS an
+// SM: 8 (64 registers) hide more of the local memory's latency where that many
+// columns come, 4 take fewer instructions (us at 4 / 6 / 8: 3 g-points 40 layers
+// 65536 columns 1081 / 1218 / 1265, 64 layers 262144 6633 / 6078 / 5057, 6 layers
+// 262144 422 / 470 / 474).
+template <int LM, int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS) k_radiation_columns(Geom g, RadTables tb, RadArgs a) {
+  const int col = blockIdx.x * blockDim.x + threadIdx.x;
+  if (col >= g.nx * g.ny) return;
+  const int L = g.L;
+  const long long S = g.S, o = g.at(col % g.nx, col / g.nx);
+  OwnColumn<LM> c;
+  bool bad = false;
+  {
+    double pu = a.ptop, pku = a.pk_top, lu = atm_log(a.ptop);  // level k + 1: pressure, pkap, log p
+    double lp2 = 0.;                                           // log play(k + 1)
+    auto level = [&bad, &tb](OwnColumn<LM>& c, int k, int m, double lm, double lm1, double lk) {
+      const double t = (c.tlay[m] * (lm1 - lk) + c.tlay[m + 1] * (lk - lm)) / (lm1 - lm);
+      c.tlev[k] = t;
+      c.kb[k] = bracket(t, tb.plk_t, tb.npl, bad);
+    };
+    const double ltop = lu;
+    for (int k = L; k >= 1; --k) {  // :54-84
+      const double dpk = a.dp[o + (long long)(k - 1) * S];
+      const double p = pu + dpk, pk = atm_pow(p, KAPPA), plog = atm_log(p / pu);
+      c.play[k] = dpk / plog;
+      c.tlay[k] = a.pt[o + (long long)(k - 1) * S] * ((pku - pk) / (-(plog * KAPPA)));
+      c.dm[k] = dpk / a.gravity;  // :118
+      c.code[k] = bracket_pt(tb, c.play[k], c.tlay[k], bad);
+      const double lp1 = atm_log(c.play[k]);
+      // the level above, between layers k and k + 1; the model top extrapolated (:86-93)
+      if (k < L) level(c, k + 1, k, lp1, lp2, lu);
+      if (k == L - 1) level(c, L + 1, L - 1, lp1, lp2, ltop);
+      pu = p;
+      pku = pk;
+      lu = atm_log(p);
+      if (k == 1) level(c, 1, 1, lp1, lp2, lu);  // the bottom extrapolated (:95-102)
+      lp2 = lp1;
+    }
+  }
+  const double ts = a.ts[o];
+  const int kbs = bracket(ts, tb.plk_t, tb.npl, bad);
+  for (int k = 1; k <= L + 1; ++k)
+    for (int i = 0; i < 4; ++i) c.sum[i][k] = 0.;  // :112-116
+  // solar_irradiance (mod_solar.f90:26-35)
+  const double r = a.radius[col] / SOLAR_SCALE;
+  const double irradiance = SOLAR_BASE * (1. + SOLAR_PEAK / (1. + r * r));
+  LayerArrays<LM> w;
+  OwnSums<LM> sw{c, 0}, lw{c, 2};
+  if (!bad)
+    for (int gp = 0; gp < tb.ng; ++gp) {
+      shortwave<LM>(tb, gp, L, c, tb.frac[gp] * irradiance, a.mu0, a.albedo, w, sw);
+      longwave<LM>(tb, gp, L, c, ts, kbs, a.emissivity, w, lw);
+    }
+  for (int k = 1; k <= L + 1; ++k)
+    a.nf[o + (long long)(k - 1) * S] = (c.sum[1][k] + c.sum[3][k]) - (c.sum[0][k] + c.sum[2][k]);
+  if (bad) atomicOr(a.range_error, 1);
+}
+
+// Whether n columns take a thread each.  Both forms' times grow with the columns, the
+// lanes' with the rounds of RG g-points, the threads' with the g-points and, for
+// latency, less than in proportion below 112000 columns; a column's round costs about 11
+// times a column's g-point in turn, more with many layers (fewer blocks an SM) and with
+// very few.  Measured on B200 (us, a lane a g-point / a thread a column):
+// 20 layers, 16384 columns 1 g-point 357/160, 3 358/323, 6 360/547; 262144 6 4911/2887, 10 4936/4582, 14 4965/6284;
+// 64 layers, 4096 1 361/430; 36000 3 2689/1515, 6 2698/2746; 262144 10 18175/14698, 14 18359/20239, 20 33584/28461, 40 49700/59697;
+// 128 layers, 160000 14 37249/33388, 16 37277/38637; 3 layers, 65536 16 308/219, 1048576 16 4840/2808.
+inline bool rad_columns(long long n, int L, int ng) {
+  const double round = L > 64 ? 15. : L > 32 ? 12. : 10.5 + 170. / (L * L);
+  const double cols = n > 112500 ? (double)n : 45000. + .6 * (double)n;
+  return (ng + 1.) * cols < round * ((ng + RG - 1) / RG) * (double)n;
+}
+
 template <int LM>
 cudaError_t launch(const Geom& g, const RadTables& t, const RadArgs& a, cudaStream_t s) {
   const int n = g.nx * g.ny;
+  if (rad_columns(n, g.L, t.ng)) {
+    if (n > 148 * 1024 && g.L > 8) k_radiation_columns<LM, 8><<<(n + 127) / 128, 128, 0, s>>>(g, t, a);
+    else k_radiation_columns<LM, 4><<<(n + 127) / 128, 128, 0, s>>>(g, t, a);
+    return cudaGetLastError();
+  }
   const size_t sm = (size_t)RC * rad_doubles(g.L) * sizeof(double);
   // what LM layers take whatever L is: launches on several threads set the same value
   const cudaError_t e = cudaFuncSetAttribute(k_radiation<LM>, cudaFuncAttributeMaxDynamicSharedMemorySize,

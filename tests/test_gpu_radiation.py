@@ -75,6 +75,26 @@ def test_g_point_counts_bit_exact(n_g, nx, ny, nlay):
     dy.close()
 
 
+# few g-points, or few layers, of enough columns that a thread has one of its own:
+# each layer range and number of blocks an SM, several rounds of g-points
+@pytest.mark.parametrize('n_g,nx,ny,nlay', [(1, 133, 127, 3), (16, 215, 206, 3), (3, 401, 379, 9), (17, 257, 250, 9),
+                                            (1, 130, 129, 33), (2, 393, 387, 34), (1, 131, 126, 65)])
+def test_thread_a_column_bit_exact(n_g, nx, ny, nlay):
+    go = gas_optics.synthetic(4, n_g=n_g)
+    st = radiative_state(nx, ny, nlay, seed=n_g)
+    xc, yc = ic.cell_axes(st)
+    dy = Dycore(st)
+    dy.set_radiation(go, xc, yc)
+    dy.radiative_heating(0.0)
+    np.testing.assert_array_equal(dy.get('net_flux'), oracle_flux(st, go, dy, xc, yc))
+    hot = st.ts.copy()
+    hot[ny // 2, nx - 1] = 1000.0
+    dy.upload('ts', np.pad(hot[None], ((0, 0), (H, H), (H, H))))
+    with pytest.raises(AtmError, match='outside the gas-optics tables'):
+        dy.radiative_heating()
+    dy.close()
+
+
 def test_mixed_form_and_parameters():
     """The radiation is FP64 in the mixed form too (its state is FP64);
     non-default zenith angle, albedo and emissivity."""
