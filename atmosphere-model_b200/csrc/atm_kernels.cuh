@@ -220,9 +220,8 @@ __global__ void __launch_bounds__(32 * COL_WARPS) k_column_split(Geom g, Consts 
 // heat = (nf(k+1) - nf(k)) / (cp dp / g) / playkap.
 // The levels of 32 columns are shared by a block's warps, as in k_column_split: one
 // warp sums the pressures, all share the powers and logarithms (shared memory:
-// plev and pkap of nlay x 32).  With a thread a column, its nlay powers and
-// logarithms in a row left the GPU waiting: 192x160x48 97 -> 46 us, 512x512x64 326 ->
-// 322.
+// plev and pkap of nlay x 32).  With a thread a column (k_heating_columns), its nlay
+// powers and logarithms in a row left the GPU waiting: 192x160x48 97 -> 46 us.
 constexpr int HEAT_WARPS = 8;
 template <typename T>
 __global__ void __launch_bounds__(32 * HEAT_WARPS) k_heating(Geom g, Consts c, const T* __restrict__ dpl,
@@ -254,6 +253,32 @@ __global__ void __launch_bounds__(32 * HEAT_WARPS) k_heating(Geom g, Consts c, c
     const double playkap = (p1 - p0) / atm_log(p1 / p0);
     const double d = (double)dpl[ok];
     if (in) heat[ok] = (nf[ok + S] - nf[ok]) / (CP_DRY * d / c.gravity) / playkap;
+  }
+}
+
+// The same with a thread a column, for domains that fill the GPU with them, where the
+// warps that wait for the pressures cost more than they save: the sooner the fewer
+// layers a warp of the shared form has, and beyond 88 layers, where an SM holds
+// few of its blocks.  Measured on B200 (us, shared levels / a thread a column; columns in
+// thousands): 3 layers 16 9/12, 31 12/12, 1049 137/60; 12 layers 66 28/31, 96 39/36; 20 layers
+// 96 55/56, 262 124/107; 64 layers 160 210/239, 262 324/327; 100 layers 66 190/214, 96 266/243;
+// 128 layers 31 152/254, 66 284/273, 160 622/469.
+inline bool heating_few(long long n, int L) { return n <= 148LL * (L > 88 ? 500 : 48 * (L < 32 ? L : 32)); }
+template <typename T>
+__global__ void __launch_bounds__(64) k_heating_columns(Geom g, Consts c, const T* __restrict__ dpl,
+                                                        const double* __restrict__ nf, double* __restrict__ heat) {
+  stream_order();
+  const int w = g.nx + 2 * H, col = blockIdx.x * 64 + threadIdx.x;
+  if (col >= w * g.NYP) return;
+  const long long o = g.at(-H + col % w, -H + col / w), S = g.S;
+  double plev = c.ptop, p1 = c.pk_top;
+  for (int k = g.L - 1; k >= 0; --k) {
+    const long long ok = o + (long long)k * S;
+    const double d = (double)dpl[ok];
+    plev = plev + d;
+    const double p0 = atm_pow(plev, KAPPA), playkap = (p1 - p0) / atm_log(p1 / p0);
+    heat[ok] = (nf[ok + S] - nf[ok]) / (CP_DRY * d / c.gravity) / playkap;
+    p1 = p0;
   }
 }
 

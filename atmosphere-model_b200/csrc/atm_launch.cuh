@@ -61,6 +61,10 @@ cudaError_t column(const Geom& g, const Consts& c, const void* dpl, const void* 
 cudaError_t heating(const Geom& g, const Consts& c, const void* dpl, int es, const double* nf, double* heat,
                     cudaStream_t s) {
   int n = (g.nx + 2 * H) * g.NYP;
+  if (!heating_few(n, g.L)) {
+    if (es == 8) return launch(k_heating_columns<double>, (n + 63) / 64, 64, 0, s, g, c, (const double*)dpl, nf, heat);
+    return launch(k_heating_columns<float>, (n + 63) / 64, 64, 0, s, g, c, (const float*)dpl, nf, heat);
+  }
   const int nb = (n + 31) / 32;
   const size_t sm = (size_t)2 * g.L * 32 * sizeof(double), most = (size_t)2 * MAX_LAYERS * 32 * sizeof(double);
   const cudaError_t e = es == 8 ? remap_smem_attr(k_heating<double>, most) : remap_smem_attr(k_heating<float>, most);

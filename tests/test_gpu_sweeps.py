@@ -131,6 +131,12 @@ def test_heating_bit_exact(nx, ny, nlay):
     g.close()
 
 
+@pytest.mark.parametrize('nx,ny,nlay', [(147, 143, 3), (300, 290, 10), (270, 263, 97)])
+def test_heating_thread_a_column_bit_exact(nx, ny, nlay):
+    """The heating term of domains of many columns."""
+    test_heating_bit_exact(nx, ny, nlay)
+
+
 # columns beyond which a thread has a column of its own, in each of the kernels'
 # layer ranges (the limits depend on the layers)
 @pytest.mark.parametrize('nx,ny,nlay', [(131, 130, 3), (171, 160, 8), (240, 230, 33), (203, 190, 65), (140, 137, 128)])
