@@ -38,7 +38,7 @@ cudaError_t mass(const Geom& g, const Consts& c, const void* dp, const void* pt,
 cudaError_t column(const Geom& g, const Consts& c, const void* dpl, const void* ptl, int es, double* pkap, double* gz,
                    int lo, int hi, double* plev, cudaStream_t s) {
   const int n = (g.nx - lo + hi) * (g.ny - lo + hi);
-  if (few_columns(n)) {
+  if (few_columns(n, g.L, es == 4)) {
     const int nb = (n + 31) / 32, nt = 32 * COL_WARPS;
     const size_t sm = (size_t)g.L * 32 * sizeof(double);  // at most 32 KB (128 layers)
     if (es == 8)

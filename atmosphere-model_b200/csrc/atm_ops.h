@@ -108,11 +108,15 @@ struct EnsPlan;
 int ensemble_max_blocks();
 cudaError_t ensemble_launch(const EnsPlan& plan, int blocks, cudaStream_t);
 
-// whether n columns leave a kernel of one thread a column with no more than four
-// blocks of 128 a multiprocessor, where levels are better shared (measured on B200,
-// FP64 column pass: 251x187x27 34 -> 29 us, 301x203x40 50 -> 44, 256x256x32 43 ->
-// 41; 350x350x64 111 -> 119, 512x512x64 191 -> 231)
-inline bool few_columns(long long n) { return n <= 148LL * 512; }
+// whether n columns of L layers leave a column pass of one thread a column with so
+// few blocks of 128 a multiprocessor that levels are better shared.  Measured on B200
+// (us, shared levels / a thread a column; columns in thousands): FP64 fields 3 layers 31
+// 8/10, 66 13/10, 32 layers 31 23/35, 66 40/39, 160 78/68; 64 layers 66 76/74; 128 layers
+// 31 96/112, 66 155/141; 301x203x40 44/50.  FP32 fields (single) 20 layers 66 20/21, 96 25/23; 64 layers
+// 66 43/47, 96 63/56; 128 layers 31 66/72, 66 112/93.
+inline bool few_columns(long long n, int L, bool single) {
+  return n <= 148LL * (L > 96 ? 400 : single && L > 8 ? 512 : 448);
+}
 
 // whole fields: destinations, sources (copies), elements
 struct FieldList {

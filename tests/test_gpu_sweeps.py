@@ -131,6 +131,13 @@ def test_heating_bit_exact(nx, ny, nlay):
     g.close()
 
 
+@pytest.mark.parametrize('nx,ny,nlay', [(257, 255, 3), (254, 241, 97), (249, 247, 64), (243, 240, 97)])
+def test_column_pass_both_sides_of_the_limit(nx, ny, nlay):
+    """Column passes of (nx + 4)(ny + 4) columns just above and just below the
+    limits up to which their levels are shared."""
+    test_step_bit_exact(nx, ny, nlay, 'smooth')
+
+
 @pytest.mark.parametrize('nx,ny,nlay', [(147, 143, 3), (300, 290, 10), (270, 263, 97)])
 def test_heating_thread_a_column_bit_exact(nx, ny, nlay):
     """The heating term of domains of many columns."""
