@@ -998,10 +998,14 @@ struct PgfColumn {
 // warp forms; the sums and the terms lie in shared memory (four arrays).
 // Measured on B200 (ms, C grid's / D grid's; before: a thread a column, its layers
 // one after the other): 64x64x20 0.059 / 0.055 -> 0.020 / 0.029, 301x203x40 0.160 /
-// 0.113 -> 0.116 / 0.084, 512x512x32 0.317 / 0.16 -> 0.316 / 0.17; 4 or 16 warps a
-// block: 10 to 20% slower there.
+// 0.113 -> 0.116 / 0.084; 4 or 16 warps a block: 10 to 20% slower there.
 constexpr int CADJ_WARPS = 8;
 inline size_t column_adj_smem(int L) { return (size_t)4 * L * 32 * sizeof(double); }
+// columns up to which this is the faster form
+inline long long column_adj_few(int L) {
+  const long long blocks = (long long)(228 * 1024 / (column_adj_smem(L) + 1024)), most = blocks > 2 ? 640 : 170 * blocks;
+  return 148 * (45 * L < most ? 45 * L : most);
+}
 template <bool CGRID>
 __global__ void __launch_bounds__(32 * CADJ_WARPS) k_column_adj(Geom g, Consts c, const double* __restrict__ dpl,
                                                                 const double* __restrict__ ptl,
@@ -1083,6 +1087,61 @@ __global__ void __launch_bounds__(32 * CADJ_WARPS) k_column_adj(Geom g, Consts c
   __syncthreads();
   if (!in) return;
   for (int k = warp; k < L; k += CADJ_WARPS) lam_dp[o + (long long)k * S] += Q[32 * k];
+}
+
+// The same with a thread a column, its layers in turn; the terms of a layer that its
+// neighbours complete wait a turn.  For domains of more columns than column_adj_few:
+// the warps of a block that wait for the sums are hidden by other blocks only while an
+// SM holds several, and few layers leave them idle.  Measured on B200 (us, C grid's
+// column stage, D grid's with the corners; shared levels / a thread a column; columns
+// in thousands): 3 layers 31 25/23 26/24, 1049 433/150 337/141; 12 layers 66 82/77 65/67,
+// 262 239/152 222/159; 20 layers 66 113/115 91/103, 96 148/122 132/118; 40 layers 96 228/230 223/234,
+// 262 523/521 534/489; 64 layers 66 289/326 272/311, 262 963/826 952/765; 100 layers (two blocks an SM)
+// 31 318/430 270/374, 66 627/511 520/413; 128 (one) 16 356/529 262/425, 31 619/570 456/472, 160 2729/1217 2160/904.
+template <int LM, bool CGRID>
+__global__ void __launch_bounds__(128) k_column_adj_columns(Geom g, Consts c, const double* __restrict__ dpl,
+                                                            const double* __restrict__ ptl,
+                                                            const double* __restrict__ pkap,
+                                                            const double* __restrict__ gz,
+                                                            const double* __restrict__ lam_u,
+                                                            const double* __restrict__ lam_v, double* lam_dp,
+                                                            double* lam_pt) {
+  stream_order();
+  const int w = g.nx + 4, L = g.L, col = blockIdx.x * blockDim.x + threadIdx.x;
+  if (col >= w * (g.ny + 4)) return;
+  const int x = -2 + col % w, y = -2 + col / w;
+  const long long o = g.at(x, y), S = g.S;
+  const PgfColumn<true> pgf(g, c, pkap, gz, lam_u, lam_v, x, y);
+  double q[LM];  // adjoint of plev(k)
+  double pl = c.ptop, lz = 0.;
+  double pl1 = 1., pk1 = c.pk_top, q1 = 0., cpz1 = 0., z1 = 0.;  // of layer k+1; z1: what it gives to gz(k+1)
+  for (int k = L - 1; k >= 0; --k) {
+    const long long ok = o + (long long)k * S;
+    PgfPoint l{0., 0., 0., 0.};
+    if constexpr (CGRID) {
+      l = pgf.layer(k);
+    } else {
+      l.p0 = lam_u[ok];
+      l.z1 = lam_v[ok + S];
+    }
+    pl = pl + dpl[ok];
+    const double pk = CGRID ? pkap[ok] : atm_pow(pl, KAPPA);
+    lz += k + 1 < L ? l.z1 + z1 : l.z1;
+    const double cpz = CP_DRY * ptl[ok] * lz;
+    lam_pt[ok] += CP_DRY * (pk - pk1) * lz;
+    if (k + 1 < L) q[k + 1] = ((CGRID ? q1 + l.p1 : q1) + cpz1 - cpz) * KAPPA * pk1 / pl1;
+    q1 = l.p0;
+    z1 = l.z0;
+    cpz1 = cpz;
+    pk1 = pk;
+    pl1 = pl;
+  }
+  q[0] = (q1 + cpz1) * KAPPA * pk1 / pl1;
+  double acc = 0.;
+  for (int k = 0; k < L; ++k) {
+    acc += q[k];
+    lam_dp[o + (long long)k * S] += acc;
+  }
 }
 
 // What the D grid's pressure-gradient force passes to pkapb (levels 1..nlay)

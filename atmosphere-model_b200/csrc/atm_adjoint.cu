@@ -125,6 +125,14 @@ static cudaError_t column_adj(const Geom& g, const Consts& c, const double* dp, 
                               const double* gz, const double* lam_u, const double* lam_v, double* lam_dp,
                               double* lam_pt, cudaStream_t s) {
   const int n = (g.nx + 4) * (g.ny + 4);
+  if (n > column_adj_few(g.L)) {
+    auto run = [&](auto kernel) {
+      return launch(kernel, (n + 127) / 128, 128, 0, s, g, c, dp, pt, pkap, gz, lam_u, lam_v, lam_dp, lam_pt);
+    };
+    if (g.L <= 32) return run(k_column_adj_columns<32, CGRID>);
+    if (g.L <= 64) return run(k_column_adj_columns<64, CGRID>);
+    return run(k_column_adj_columns<MAX_LAYERS, CGRID>);
+  }
   const size_t sm = column_adj_smem(g.L);
   const cudaError_t e = remap_smem_attr(k_column_adj<CGRID>, column_adj_smem(MAX_LAYERS));
   if (e != cudaSuccess) return e;

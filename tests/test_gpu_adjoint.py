@@ -287,10 +287,11 @@ def test_layer_counts_dot_product(nx, ny, nlay):
     g.close()
 
 
-@pytest.mark.parametrize('nx,ny,nlay', [(190, 151, 3), (313, 287, 9), (310, 306, 12), (312, 305, 33)])
+@pytest.mark.parametrize('nx,ny,nlay', [(190, 151, 3), (313, 287, 9), (310, 306, 12), (312, 305, 33),
+                                        (231, 224, 70), (162, 157, 113)])
 def test_many_columns_dot_product(nx, ny, nlay):
     """Domains of more columns than the limits beyond which a thread has a column
-    of its own, of few layers (both reverses of the remap) and of more."""
+    of its own, of few layers (both reverses of the remap, that of the columns) and of more."""
     test_layer_counts_dot_product(nx, ny, nlay)
 
 
