@@ -1007,12 +1007,12 @@ inline long long column_adj_few(int L) {
   return 148 * (45 * L < most ? 45 * L : most);
 }
 template <bool CGRID>
-__global__ void __launch_bounds__(32 * CADJ_WARPS) k_column_adj(Geom g, Consts c, const double* __restrict__ dpl,
-                                                                const double* __restrict__ ptl,
-                                                                const double* __restrict__ pkap,
-                                                                const double* __restrict__ gz,
-                                                                const double* __restrict__ lam_u,
-                                                                const double* __restrict__ lam_v, double* lam_dp,
+__global__ void __launch_bounds__(32 * CADJ_WARPS) k_column_adj(Geom g, Consts c, const double* dpl,
+                                                                const double* ptl,
+                                                                const double* pkap,
+                                                                const double* gz,
+                                                                const double* lam_u,
+                                                                const double* lam_v, double* lam_dp,
                                                                 double* lam_pt) {
   stream_order();
   extern __shared__ double adj_sm[];
@@ -1099,12 +1099,12 @@ __global__ void __launch_bounds__(32 * CADJ_WARPS) k_column_adj(Geom g, Consts c
 // 262 523/521 534/489; 64 layers 66 289/326 272/311, 262 963/826 952/765; 100 layers (two blocks an SM)
 // 31 318/430 270/374, 66 627/511 520/413; 128 (one) 16 356/529 262/425, 31 619/570 456/472, 160 2729/1217 2160/904.
 template <int LM, bool CGRID>
-__global__ void __launch_bounds__(128) k_column_adj_columns(Geom g, Consts c, const double* __restrict__ dpl,
-                                                            const double* __restrict__ ptl,
-                                                            const double* __restrict__ pkap,
-                                                            const double* __restrict__ gz,
-                                                            const double* __restrict__ lam_u,
-                                                            const double* __restrict__ lam_v, double* lam_dp,
+__global__ void __launch_bounds__(128) k_column_adj_columns(Geom g, Consts c, const double* dpl,
+                                                            const double* ptl,
+                                                            const double* pkap,
+                                                            const double* gz,
+                                                            const double* lam_u,
+                                                            const double* lam_v, double* lam_dp,
                                                             double* lam_pt) {
   stream_order();
   const int w = g.nx + 4, L = g.L, col = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1146,12 +1146,12 @@ __global__ void __launch_bounds__(128) k_column_adj_columns(Geom g, Consts c, co
 
 // What the D grid's pressure-gradient force passes to pkapb (levels 1..nlay)
 // and gzb (levels 2..nlay+1) of the corners [0, n]^2: a thread a corner.
-static __global__ void __launch_bounds__(128) k_pgf_adj_corners(Geom g, Consts c, const double* __restrict__ pkb,
-                                                                const double* __restrict__ gzb,
-                                                                const double* __restrict__ lam_u,
-                                                                const double* __restrict__ lam_v,
-                                                                double* __restrict__ lam_pkb,
-                                                                double* __restrict__ lam_gzb) {
+static __global__ void __launch_bounds__(128) k_pgf_adj_corners(Geom g, Consts c, const double* pkb,
+                                                                const double* gzb,
+                                                                const double* lam_u,
+                                                                const double* lam_v,
+                                                                double* lam_pkb,
+                                                                double* lam_gzb) {
   stream_order();
   const int w = g.nx + 1;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1191,8 +1191,8 @@ struct CornerAdjLine {
   }
 };
 static __global__ void __launch_bounds__(MW * MWARPS, CORN_WARPS_SM / MWARPS) k_corners_adj(
-    Geom g, const double* __restrict__ lam_pkb, const double* __restrict__ lam_gzb, double* __restrict__ lam_pk,
-    double* __restrict__ lam_gz, int tys) {
+    Geom g, const double* lam_pkb, const double* lam_gzb, double* lam_pk,
+    double* lam_gz, int tys) {
   stream_order();
   extern __shared__ __align__(16) char feed_sm[];
   const int lane = threadIdx.x & (MW - 1);

@@ -657,14 +657,14 @@ __device__ __noinline__ void remap_energy_adj_at(const Geom& g, const RemapArgs&
 // 16 blocks of 64 threads per SM (64 registers; more columns in flight to
 // hide the local-memory latency of the column arrays)
 template <int LM>
-__global__ void __launch_bounds__(64, 16) k_remap_energy_adj(Geom g, RemapArgs ra, const double* __restrict__ dp,
-                                                         const double* __restrict__ pt, const double* __restrict__ ud,
-                                                         const double* __restrict__ vd, const double* __restrict__ urem,
-                                                         const double* __restrict__ vrem, const double* __restrict__ gzs,
-                                                         const double* __restrict__ lam_dpo,
-                                                         const double* __restrict__ lam_pto,
-                                                         const double* __restrict__ lam_udo,
-                                                         const double* __restrict__ lam_vdo, double* lam_dp,
+__global__ void __launch_bounds__(64, 16) k_remap_energy_adj(Geom g, RemapArgs ra, const double* dp,
+                                                         const double* pt, const double* ud,
+                                                         const double* vd, const double* urem,
+                                                         const double* vrem, const double* gzs,
+                                                         const double* lam_dpo,
+                                                         const double* lam_pto,
+                                                         const double* lam_udo,
+                                                         const double* lam_vdo, double* lam_dp,
                                                          double* lam_pt, double* lam_ud, double* lam_vd, double* lam_ur,
                                                          double* lam_vr) {
   stream_order();
@@ -751,10 +751,10 @@ __device__ __noinline__ void remap_winds_adj_at(const Geom& g, const RemapArgs& 
 
 // (blockIdx.y: the direction)
 template <int LM>
-__global__ void __launch_bounds__(64, 16) k_remap_winds_adj(Geom g, RemapArgs ra, const double* __restrict__ dp,
-                                                        const double* __restrict__ ud, const double* __restrict__ vd,
-                                                        const double* __restrict__ lam_ur,
-                                                        const double* __restrict__ lam_vr, double* lam_dp,
+__global__ void __launch_bounds__(64, 16) k_remap_winds_adj(Geom g, RemapArgs ra, const double* dp,
+                                                        const double* ud, const double* vd,
+                                                        const double* lam_ur,
+                                                        const double* lam_vr, double* lam_dp,
                                                         double* lam_ud, double* lam_vd) {
   stream_order();
   const int w = g.nx + 2, h = g.ny + 2;

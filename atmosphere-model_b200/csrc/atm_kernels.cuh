@@ -121,9 +121,9 @@ __device__ __forceinline__ void column_at(const Geom& g, const Consts& c, const 
 }
 
 template <typename T, typename PW = PortablePow>
-__global__ void __launch_bounds__(128) k_column(Geom g, Consts c, const T* __restrict__ dpl, const T* __restrict__ ptl,
-                                                double* __restrict__ pkap, double* __restrict__ gz, int lo, int hi,
-                                                double* __restrict__ plev_out) {
+__global__ void __launch_bounds__(128) k_column(Geom g, Consts c, const T* dpl, const T* ptl,
+                                                double* pkap, double* gz, int lo, int hi,
+                                                double* plev_out) {
   stream_order();
   column_at<T, PW>(g, c, dpl, ptl, pkap, gz, lo, hi, plev_out, blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -139,10 +139,10 @@ __global__ void __launch_bounds__(128) k_column(Geom g, Consts c, const T* __res
 // 0.83 ms against 0.63).
 constexpr int COL_WARPS = 4;
 template <typename T, typename PW = PortablePow>
-__global__ void __launch_bounds__(32 * COL_WARPS) k_column_split(Geom g, Consts c, const T* __restrict__ dpl,
-                                                                 const T* __restrict__ ptl, double* __restrict__ pkap,
-                                                                 double* __restrict__ gz, int lo, int hi,
-                                                                 double* __restrict__ plev_out) {
+__global__ void __launch_bounds__(32 * COL_WARPS) k_column_split(Geom g, Consts c, const T* dpl,
+                                                                 const T* ptl, double* pkap,
+                                                                 double* gz, int lo, int hi,
+                                                                 double* plev_out) {
   stream_order();
   extern __shared__ double col_sm[];
   constexpr int B = 8;  // levels whose loads are in flight together
@@ -224,9 +224,9 @@ __global__ void __launch_bounds__(32 * COL_WARPS) k_column_split(Geom g, Consts 
 // powers and logarithms in a row left the GPU waiting: 192x160x48 97 -> 46 us.
 constexpr int HEAT_WARPS = 8;
 template <typename T>
-__global__ void __launch_bounds__(32 * HEAT_WARPS) k_heating(Geom g, Consts c, const T* __restrict__ dpl,
-                                                                   const double* __restrict__ nf,
-                                                                   double* __restrict__ heat) {
+__global__ void __launch_bounds__(32 * HEAT_WARPS) k_heating(Geom g, Consts c, const T* dpl,
+                                                                   const double* nf,
+                                                                   double* heat) {
   stream_order();
   extern __shared__ double heat_sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -265,8 +265,8 @@ __global__ void __launch_bounds__(32 * HEAT_WARPS) k_heating(Geom g, Consts c, c
 // 128 layers 31 152/254, 66 284/273, 160 622/469.
 inline bool heating_few(long long n, int L) { return n <= 148LL * (L > 88 ? 500 : 48 * (L < 32 ? L : 32)); }
 template <typename T>
-__global__ void __launch_bounds__(64) k_heating_columns(Geom g, Consts c, const T* __restrict__ dpl,
-                                                        const double* __restrict__ nf, double* __restrict__ heat) {
+__global__ void __launch_bounds__(64) k_heating_columns(Geom g, Consts c, const T* dpl,
+                                                        const double* nf, double* heat) {
   stream_order();
   const int w = g.nx + 2 * H, col = blockIdx.x * 64 + threadIdx.x;
   if (col >= w * g.NYP) return;

@@ -274,21 +274,13 @@ __device__ __forceinline__ T xline_flux_above(T q, T c) {
 // Column accessor of one level of a stored field: the value at (x, y) with x
 // the lane's column, both brought into the stored (halo-padded) array, so
 // that rows and lanes past it read some stored value (they only feed outputs
-// outside the kernel's range).  RO: no thread writes the field during the
-// launch, so it is read through the read-only data path; the persistent
-// ensemble kernel, whose later stages read what earlier stages of the same
-// launch wrote, uses plain (coherent) loads.  A level holds fewer than 2^32
+// outside the kernel's range).  A level holds fewer than 2^32
 // elements (three levels of 17 fields of that size exceed the device memory).
 __device__ __forceinline__ unsigned col_of(const Geom& g, int x) {
   return (unsigned)(min(max(x, -H), g.nx + H - 1) + H + XOFF);
 }
 __device__ __forceinline__ unsigned row_of(const Geom& g, int y) {
   return (unsigned)(min(max(y, -H), g.ny + H - 1) + H) * (unsigned)g.P;
-}
-template <bool RO, typename E>
-__device__ __forceinline__ E ld(const E* level, unsigned i) {
-  if constexpr (RO) return __ldg(level + i);
-  else return level[i];
 }
 
 // The inputs of a strip's rows, brought ahead of the row that works on them.
@@ -444,11 +436,11 @@ __device__ __forceinline__ void mass_strip(const Geom& g, const Consts& c, const
   T us = 0;                                       // D-grid u(x, j) + u(x-1, j) (C grid)
   T va_o = 0, vb_o = 0;                           // D-grid v at (x, j-3), (x+1, j-3) (C grid)
   if constexpr (CGRID) {
-    const T a = T(ld<RO>(u, row_of(g, oy - 3) + xi));
+    const T a = T(u[row_of(g, oy - 3) + xi]);
     us = a + shfl_up(a, 1);
     const unsigned rv = row_of(g, oy - 6);
-    va_o = T(ld<RO>(v, rv + xi));
-    vb_o = T(ld<RO>(v, rv + xr));
+    va_o = T(v[rv + xi]);
+    vb_o = T(v[rv + xr]);
   }
   bool bad = false;
   const int jend = min(oy + tys, yhi + 1) + 3;
@@ -619,13 +611,13 @@ constexpr int MASS_SMEM = FEED_BYTES<MASS_NF<true, CGRID, std::is_same_v<S, T>>,
 // across y, blockIdx.z the layer
 __device__ __forceinline__ int strip_x() { return (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); }
 template <typename T, bool CGRID, typename S, typename C>
-__global__ void __launch_bounds__(MW * MWARPS, MarchL<T, CGRID ? MK_CMASS : MK_DMASS>::min_blocks) k_mass_m(Geom g, Consts c, const S* __restrict__ dp,
-                                                         const S* __restrict__ pt,
-                                                         const typename MassM<T, CGRID, S, C>::UB* __restrict__ u,
-                                                         const typename MassM<T, CGRID, S, C>::UB* __restrict__ v,
-                                                         const double* __restrict__ heat,
-                                                         typename MassM<T, CGRID, S, C>::O* __restrict__ dpo,
-                                                         typename MassM<T, CGRID, S, C>::O* __restrict__ pto, int lo,
+__global__ void __launch_bounds__(MW * MWARPS, MarchL<T, CGRID ? MK_CMASS : MK_DMASS>::min_blocks) k_mass_m(Geom g, Consts c, const S* dp,
+                                                         const S* pt,
+                                                         const typename MassM<T, CGRID, S, C>::UB* u,
+                                                         const typename MassM<T, CGRID, S, C>::UB* v,
+                                                         const double* heat,
+                                                         typename MassM<T, CGRID, S, C>::O* dpo,
+                                                         typename MassM<T, CGRID, S, C>::O* pto, int lo,
                                                          int hi, int* nonfinite, int tys) {
   stream_order();
   extern __shared__ __align__(16) char feed_sm[];
@@ -663,9 +655,9 @@ __device__ __forceinline__ void c_mom_strip(const Geom& g, const Consts& c, cons
   // register windows of the column, named by their row offset from the
   // newest row j of the iteration
   unsigned r = row_of(g, oy - 3);
-  T u_x = T(ld<RO>(uk, r + xi)), u_xm = T(ld<RO>(uk, r + xl));  // ud(x, j), ud(x-1, j)
+  T u_x = T(uk[r + xi]), u_xm = T(uk[r + xl]);  // ud(x, j), ud(x-1, j)
   r = row_of(g, oy - 4);
-  T v_x = T(ld<RO>(vk, r + xi)), v_xp = T(ld<RO>(vk, r + xr));  // vd(x, j-1), vd(x+1, j-1)
+  T v_x = T(vk[r + xi]), v_xp = T(vk[r + xr]);  // vd(x, j-1), vd(x+1, j-1)
   T uw3 = 0, uw2 = 0, uw1 = 0, uw0 = 0;  // ud(x, j-3 .. j)
   T vw4 = 0, vw3 = 0, vw2 = 0, vw1 = 0, vw0 = 0;  // vd(x, j-4 .. j)
   T a3 = 0, a2 = 0, a1 = 0, a0 = 0;      // C-grid u of this layer, rows j-3 .. j
@@ -678,8 +670,8 @@ __device__ __forceinline__ void c_mom_strip(const Geom& g, const Consts& c, cons
   T ke1 = 0, ke0 = 0;                    // kinetic energy, rows j-4, j-3
   double pk0m = 0, pk1m = 0, gz0m = 0, gz1m = 0;  // pkap, gz at k and k+1, row j-4
   // layer-nlay ud at row y and vd at rows y-1, y of the first kinetic-energy row y = oy-1
-  T uL1 = T(ld<RO>(uL, row_of(g, oy - 1) + xi));
-  T vL2 = T(ld<RO>(vL, row_of(g, oy - 2) + xi)), vL1 = T(ld<RO>(vL, row_of(g, oy - 1) + xi));
+  T uL1 = T(uL[row_of(g, oy - 1) + xi]);
+  T vL2 = T(vL[row_of(g, oy - 2) + xi]), vL1 = T(vL[row_of(g, oy - 1) + xi]);
   const int jend = min(oy + tys, g.ny) + 3;
   enum { F_U, F_UM, F_V, F_VP, F_P0, F_P1, F_G0, F_G1, F_UN, F_VN };
   Feed<RO, CMOM_NF, 0> feed(sm);
@@ -784,10 +776,10 @@ __device__ __forceinline__ void c_mom_strip(const Geom& g, const Consts& c, cons
 }
 
 template <typename T, typename S, typename C>
-__global__ void __launch_bounds__(MW * MWARPS, MarchL<T, MK_CMOM>::min_blocks) k_c_mom_m(Geom g, Consts c, const S* __restrict__ ud,
-                                                          const S* __restrict__ vd, const double* __restrict__ pkap,
-                                                          const double* __restrict__ gz, C* __restrict__ uc,
-                                                          C* __restrict__ vc, int tys) {
+__global__ void __launch_bounds__(MW * MWARPS, MarchL<T, MK_CMOM>::min_blocks) k_c_mom_m(Geom g, Consts c, const S* ud,
+                                                          const S* vd, const double* pkap,
+                                                          const double* gz, C* uc,
+                                                          C* vc, int tys) {
   stream_order();
   extern __shared__ __align__(16) char feed_sm[];
   c_mom_strip<T, S, C>(g, c, ud, vd, pkap, gz, uc, vc, strip_x(), blockIdx.y, blockIdx.z, tys, feed_sm);
@@ -826,8 +818,8 @@ __device__ __forceinline__ void d_mom_strip(const Geom& g, const Consts& c, cons
   // register windows of the column, named by their row offset from the
   // newest row j of the iteration
   unsigned r = row_of(g, oy - 3) + xi;
-  T s3 = 0, s2 = 0, s1 = 0, s0 = T(ld<RO>(uk, r));  // ud(x, j-3 .. j)
-  T v0 = T(ld<RO>(vk, r)), v3 = 0;                  // vd(x, j), vd(x, j-3)
+  T s3 = 0, s2 = 0, s1 = 0, s0 = T(uk[r]);  // ud(x, j-3 .. j)
+  T v0 = T(vk[r]), v3 = 0;                  // vd(x, j), vd(x, j-3)
   YLine<T, CON> lv;                                 // vd along y
   lv.q0 = v0;
   T q2 = 0, q1 = 0, q0 = 0;                         // divergence, rows j-2 .. j
@@ -841,8 +833,8 @@ __device__ __forceinline__ void d_mom_strip(const Geom& g, const Consts& c, cons
   T fw1 = 0, fw0 = 0;                               // the vorticity's piecewise-constant y flux at interfaces j-3, j-2
   T ke3 = 0, ke2 = 0;                               // kinetic energy, rows j-3, j-2
   T lp4 = 0, lp3 = 0, lp2 = 0;                      // Laplacian of the vorticity, rows j-4 .. j-2
-  T cu3 = 0, cu2 = T(ld<RO>(uL, row_of(g, oy - 5) + xi)), cu1 = T(ld<RO>(uL, row_of(g, oy - 4) + xi));  // layer-nlay uc, rows j-3 .. j-1
-  T cv3 = 0, cv2 = T(ld<RO>(vL, row_of(g, oy - 5) + xi));  // layer-nlay vc, rows j-3, j-2
+  T cu3 = 0, cu2 = T(uL[row_of(g, oy - 5) + xi]), cu1 = T(uL[row_of(g, oy - 4) + xi]);  // layer-nlay uc, rows j-3 .. j-1
+  T cv3 = 0, cv2 = T(vL[row_of(g, oy - 5) + xi]);  // layer-nlay vc, rows j-3, j-2
   double pb0y = 0, pb1y = 0, gb0y = 0, gb1y = 0;    // pkapb, gzb at k, k+1, row j-3
   bool bad = false;
   const int jend = min(oy + tys, g.ny) + 3;
@@ -959,11 +951,11 @@ __device__ __forceinline__ void d_mom_strip(const Geom& g, const Consts& c, cons
 }
 
 template <typename T, typename S, typename C>
-__global__ void __launch_bounds__(MW * MWARPS, MarchL<T, MK_DMOM>::min_blocks) k_d_mom_m(Geom g, Consts c, const S* __restrict__ ud,
-                                                          const S* __restrict__ vd, const C* __restrict__ uc,
-                                                          const C* __restrict__ vc, const double* __restrict__ pkapb,
-                                                          const double* __restrict__ gzb, S* __restrict__ udo,
-                                                          S* __restrict__ vdo, int* nonfinite, int tys) {
+__global__ void __launch_bounds__(MW * MWARPS, MarchL<T, MK_DMOM>::min_blocks) k_d_mom_m(Geom g, Consts c, const S* ud,
+                                                          const S* vd, const C* uc,
+                                                          const C* vc, const double* pkapb,
+                                                          const double* gzb, S* udo,
+                                                          S* vdo, int* nonfinite, int tys) {
   stream_order();
   extern __shared__ __align__(16) char feed_sm[];
   d_mom_strip<T, S, C>(g, c, ud, vd, uc, vc, pkapb, gzb, udo, vdo, nonfinite, strip_x(), blockIdx.y, blockIdx.z, tys,
@@ -994,10 +986,10 @@ struct CornerLine {
   }
 };
 template <bool PK>
-__global__ void __launch_bounds__(MW * MWARPS, CORN_WARPS_SM / MWARPS) k_corners_m(Geom g, const double* __restrict__ pkap,
-                                                                                 const double* __restrict__ gz,
-                                                                                 double* __restrict__ pkapb,
-                                                                                 double* __restrict__ gzb, int tys) {
+__global__ void __launch_bounds__(MW * MWARPS, CORN_WARPS_SM / MWARPS) k_corners_m(Geom g, const double* pkap,
+                                                                                 const double* gz,
+                                                                                 double* pkapb,
+                                                                                 double* gzb, int tys) {
   stream_order();
   extern __shared__ __align__(16) char feed_sm[];
   const int lane = threadIdx.x & (MW - 1);

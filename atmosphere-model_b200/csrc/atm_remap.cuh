@@ -184,8 +184,8 @@ __device__ __forceinline__ double remap_layer(int m, int L, ShCol sc, ShCol A, S
 // and coefficients, later the edges.  E as in remap_winds_at.
 template <typename T, int LM, typename E = double>
 __global__ void __launch_bounds__(RM_LANES * RM_WARPS, 4) k_remap_winds_split(
-    Geom g, RemapArgs ra, const T* __restrict__ dp, const T* __restrict__ ud, const T* __restrict__ vd,
-    T* __restrict__ urem, T* __restrict__ vrem, int* trace, Status* st) {
+    Geom g, RemapArgs ra, const T* dp, const T* ud, const T* vd,
+    T* urem, T* vrem, int* trace, Status* st) {
   stream_order();
   extern __shared__ double rm_sm[];
   __shared__ double ps[4][RM_LANES];
@@ -282,9 +282,9 @@ __global__ void __launch_bounds__(RM_LANES * RM_WARPS, 4) k_remap_winds_split(
 // coefficients, top edges, pkap steps; energy, remapped energy.
 template <typename T, int LM, typename PW = PortablePow>
 __global__ void __launch_bounds__(RM_LANES * RM_WARPS, 3) k_remap_energy_split(
-    Geom g, RemapArgs ra, const T* __restrict__ dp, const T* __restrict__ pt, const T* __restrict__ ud,
-    const T* __restrict__ vd, const T* __restrict__ urem, const T* __restrict__ vrem, const double* __restrict__ gzs,
-    T* __restrict__ dpo, T* __restrict__ pto, T* __restrict__ udo, T* __restrict__ vdo, int* trace, Status* st) {
+    Geom g, RemapArgs ra, const T* dp, const T* pt, const T* ud,
+    const T* vd, const T* urem, const T* vrem, const double* gzs,
+    T* dpo, T* pto, T* udo, T* vdo, int* trace, Status* st) {
   stream_order();
   extern __shared__ double rm_sm[];
   __shared__ int bad[RM_LANES];
@@ -448,21 +448,21 @@ __global__ void __launch_bounds__(RM_LANES * RM_WARPS, 3) k_remap_energy_split(
 // (1024x1024x64, winds / energy: 4.09 / 4.34 ms, 4.51 / 5.00 at 12 blocks, 4.53 /
 // 4.39 at 20).
 template <typename T, int LM, typename E = double>
-__global__ void __launch_bounds__(64, 16) k_remap_winds(Geom g, RemapArgs ra, const T* __restrict__ dp,
-                                                        const T* __restrict__ ud, const T* __restrict__ vd,
-                                                        T* __restrict__ urem, T* __restrict__ vrem, int* trace,
+__global__ void __launch_bounds__(64, 16) k_remap_winds(Geom g, RemapArgs ra, const T* dp,
+                                                        const T* ud, const T* vd,
+                                                        T* urem, T* vrem, int* trace,
                                                         Status* st) {
   stream_order();
   remap_winds_at<T, LM, E>(g, ra, dp, ud, vd, urem, vrem, trace, st, blockIdx.x * blockDim.x + threadIdx.x,
                            blockIdx.y);
 }
 template <typename T, int LM, typename PW = PortablePow>
-__global__ void __launch_bounds__(64, 16) k_remap_energy(Geom g, RemapArgs ra, const T* __restrict__ dp,
-                                                         const T* __restrict__ pt, const T* __restrict__ ud,
-                                                         const T* __restrict__ vd, const T* __restrict__ urem,
-                                                         const T* __restrict__ vrem, const double* __restrict__ gzs,
-                                                         T* __restrict__ dpo, T* __restrict__ pto, T* __restrict__ udo,
-                                                         T* __restrict__ vdo, int* trace, Status* st) {
+__global__ void __launch_bounds__(64, 16) k_remap_energy(Geom g, RemapArgs ra, const T* dp,
+                                                         const T* pt, const T* ud,
+                                                         const T* vd, const T* urem,
+                                                         const T* vrem, const double* gzs,
+                                                         T* dpo, T* pto, T* udo,
+                                                         T* vdo, int* trace, Status* st) {
   stream_order();
   remap_energy_at<T, LM, PW>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, dpo, pto, udo, vdo, trace, st,
                              blockIdx.x * blockDim.x + threadIdx.x);

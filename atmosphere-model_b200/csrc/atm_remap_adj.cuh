@@ -351,11 +351,11 @@ __device__ __forceinline__ double warps_sum(double v, double (*part)[RM_LANES], 
 // Reverse of the wind remap (remap_winds_adj_at): blockIdx.y the direction.
 // Six column arrays.
 template <int LM>
-__global__ void __launch_bounds__(RM_LANES * RMA_WARPS, 2) k_remap_winds_adj_split(
-    Geom g, RemapArgs ra, const double* __restrict__ dp, const double* __restrict__ ud, const double* __restrict__ vd,
-    const double* __restrict__ lam_ur, const double* __restrict__ lam_vr, double* lam_dp, double* lam_ud,
-    double* lam_vd) {
-  stream_order();
+__device__ __forceinline__ void remap_winds_adj_block(const Geom& g, const RemapArgs& ra, const double* __restrict__ dp,
+                                                      const double* __restrict__ ud, const double* __restrict__ vd,
+                                                      const double* __restrict__ lam_ur,
+                                                      const double* __restrict__ lam_vr, double* lam_dp,
+                                                      double* lam_ud, double* lam_vd) {
   constexpr int N = (LM + RMA_WARPS - 1) / RMA_WARPS;
   extern __shared__ double rm_sm[];
   __shared__ double part[RMA_PART][RM_LANES];
@@ -467,17 +467,23 @@ __global__ void __launch_bounds__(RM_LANES * RMA_WARPS, 2) k_remap_winds_adj_spl
     atomicAdd(lam_dp + od + kk, -C1_12 * v);
   }
 }
+template <int LM>
+__global__ void __launch_bounds__(RM_LANES * RMA_WARPS, 2) k_remap_winds_adj_split(
+    Geom g, RemapArgs ra, const double* dp, const double* ud, const double* vd, const double* lam_ur,
+    const double* lam_vr, double* lam_dp, double* lam_ud, double* lam_vd) {
+  stream_order();
+  remap_winds_adj_block<LM>(g, ra, dp, ud, vd, lam_ur, lam_vr, lam_dp, lam_ud, lam_vd);
+}
 
 // Reverse of the energy remap (remap_energy_adj_at).  Eight column arrays; each
 // thread keeps the powers of its levels in registers.
 template <int LM>
-__global__ void __launch_bounds__(RM_LANES * RMA_WARPS, 2) k_remap_energy_adj_split(
-    Geom g, RemapArgs ra, const double* __restrict__ dp, const double* __restrict__ pt, const double* __restrict__ ud,
-    const double* __restrict__ vd, const double* __restrict__ urem, const double* __restrict__ vrem,
-    const double* __restrict__ gzs, const double* __restrict__ lam_dpo, const double* __restrict__ lam_pto,
-    const double* __restrict__ lam_udo, const double* __restrict__ lam_vdo, double* lam_dp, double* lam_pt,
-    double* lam_ud, double* lam_vd, double* lam_ur, double* lam_vr) {
-  stream_order();
+__device__ __forceinline__ void remap_energy_adj_block(
+    const Geom& g, const RemapArgs& ra, const double* __restrict__ dp, const double* __restrict__ pt,
+    const double* __restrict__ ud, const double* __restrict__ vd, const double* __restrict__ urem,
+    const double* __restrict__ vrem, const double* __restrict__ gzs, const double* __restrict__ lam_dpo,
+    const double* __restrict__ lam_pto, const double* __restrict__ lam_udo, const double* __restrict__ lam_vdo,
+    double* lam_dp, double* lam_pt, double* lam_ud, double* lam_vd, double* lam_ur, double* lam_vr) {
   constexpr int N = (LM + RMA_WARPS - 1) / RMA_WARPS;
   extern __shared__ double rm_sm[];
   __shared__ double part[RMA_PART][RM_LANES];
@@ -731,6 +737,16 @@ __global__ void __launch_bounds__(RM_LANES * RMA_WARPS, 2) k_remap_energy_adj_sp
     remap_energy_adj_at<LM>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, lam_dpo, lam_pto, lam_dp, lam_pt, lam_ud, lam_vd,
                               lam_ur, lam_vr, i, j);
   }
+}
+template <int LM>
+__global__ void __launch_bounds__(RM_LANES * RMA_WARPS, 2) k_remap_energy_adj_split(
+    Geom g, RemapArgs ra, const double* dp, const double* pt, const double* ud, const double* vd, const double* urem,
+    const double* vrem, const double* gzs, const double* lam_dpo, const double* lam_pto, const double* lam_udo,
+    const double* lam_vdo, double* lam_dp, double* lam_pt, double* lam_ud, double* lam_vd, double* lam_ur,
+    double* lam_vr) {
+  stream_order();
+  remap_energy_adj_block<LM>(g, ra, dp, pt, ud, vd, urem, vrem, gzs, lam_dpo, lam_pto, lam_udo, lam_vdo, lam_dp,
+                             lam_pt, lam_ud, lam_vd, lam_ur, lam_vr);
 }
 
 }  // namespace atm

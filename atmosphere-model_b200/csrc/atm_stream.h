@@ -8,7 +8,12 @@ namespace atm {
 
 // First statement of every kernel started by launch(): waits until the kernels
 // before it on the stream have completed and their writes are visible, then lets
-// the next one be set up.  Nothing is read or written before it.
+// the next one be set up.  Nothing is read or written before it: the kernel's
+// parameters carry no __restrict__, and nothing after it is read by __ldg or
+// ld.global.nc but constant tables, as a compiler may take such a load for one of
+// memory that never changes and move it above the wait.  What gains from the promise
+// that its pointers do not overlap is a function of its own, called after the wait
+// (interior_rows, remap_energy_adj_block).
 __device__ __forceinline__ void stream_order() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
