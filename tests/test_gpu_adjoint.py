@@ -322,6 +322,34 @@ def test_tall_domain_dot_product():
     g.close()
 
 
+def test_launch_count():
+    """Every kernel of the reverse is counted, the clears and the copies of a
+    tape among them."""
+    import torch
+    g = Dycore(generic_state(20, 17, 5, seed=3))
+    g.adj_enable()
+    tape = torch.empty(g.tape_bytes() // 8, dtype=torch.float64, device='cuda')
+
+    def count(f):
+        n = g.launch_count()
+        f()
+        return g.launch_count() - n
+    assert count(g.adj_zero) == 2
+    # C step recomputed 3, column 1, momentum 4 (clear, x, y, rest), column 1, mass 2
+    assert count(lambda: g.adj_cgrid_step(10.0)) == 11
+    # winds recomputed 1, clear 1, energy 1, winds 1, ring 1
+    assert count(g.adj_remap) == 5
+    # C step 3, halo 1, copy 1, D step 5, copy 1, halo 1
+    assert count(lambda: g.step_tape(20.0, False, tape.data_ptr())) == 12
+    # halo 1, clear 1, D step 2 + 3 + 2 + 1, halo 1, C step 8
+    assert count(lambda: g.adj_step_tape(20.0, False, tape.data_ptr())) == 19
+    # ... with the forward step recomputed (3 + 1 + 5)
+    assert count(lambda: g.adj_step(20.0, remap=False)) == 28
+    # ... and the remap's reverse with its clear
+    assert count(lambda: g.adj_step(20.0, remap=True)) == 34
+    g.close()
+
+
 def test_tape_alignment():
     """The tape is written alike on 16-byte and on 8-byte boundaries."""
     import torch
