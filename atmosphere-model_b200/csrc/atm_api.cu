@@ -249,14 +249,14 @@ cudaError_t d2h_pitched(atm_ctx* c, double* host, const double* dev, int K) {
 const char* const STAGE_NAMES[] = {"c_mass",  "c_column", "c_mom",        "c_halo",      "d_ring",
                                    "d_mass",  "d_column", "d_corners",    "d_mom",       "remap_ring",
                                    "remap_winds", "remap_energy", "d_halo", "heating", "check",
-                                   "adj_forward", "adj_remap", "adj_d_mom_x", "adj_d_column", "adj_d_mass_x",
-                                   "adj_c_column", "adj_c_mom", "adj_c_mass_x", "adj_halo",
-                                   "phys_tend", "phys_apply", "phys_halo", "adj_d_mom_y", "adj_d_mass_y",
-                                   "radiation", "radiation_halo", "adj_c_mass_y"};
-constexpr int NSTAGE = 32;
+                                   "adj_forward", "adj_remap", "adj_d_mom_ke", "adj_d_column", "adj_d_mass_x",
+                                   "adj_c_column", "adj_c_mom", "adj_c_mass", "adj_halo",
+                                   "phys_tend", "phys_apply", "phys_halo", "adj_d_mom_vf", "adj_d_mass_y",
+                                   "radiation", "radiation_halo"};
+constexpr int NSTAGE = 31;
 enum { S_CMASS, S_CCOL, S_CMOM, S_CHALO, S_DRING, S_DMASS, S_DCOL, S_DCORN, S_DMOM, S_RRING, S_RWIND, S_RENER,
        S_DHALO, S_HEAT, S_CHECK, S_AFWD, S_ARMP, S_ADMOM, S_ADCOL, S_ADMASS, S_ACCOL, S_ACMOM, S_ACMASS, S_AHALO,
-       S_PHYS_TEND, S_PHYS_APPLY, S_PHYS_HALO, S_ADMOM_Y, S_ADMASS_Y, S_RAD, S_RAD_HALO, S_ACMASS_Y };
+       S_PHYS_TEND, S_PHYS_APPLY, S_PHYS_HALO, S_ADMOM_Y, S_ADMASS_Y, S_RAD, S_RAD_HALO };
 
 // Brackets one stage (one kernel launch unless noted) with CUDA events on
 // the context's stream when profiling is on, and counts the launch.
@@ -935,11 +935,10 @@ int adj_c(atm_ctx* ctx, double dt_half, void* const* s, double* const* lin, cons
     CK(atm::adj_c_column(g, k, cg[C_DPC], cg[C_PTC], ctx->pkap, ctx->gz, ctx->lam_cg[C_UC], ctx->lam_cg[C_VC],
                          ctx->lam_cg[C_DPC], ctx->lam_cg[C_PTC], ctx->stream));
   }
-  for (int part = 1; part <= 2; ++part) {
-    Stage t(ctx, part == 1 ? S_ACMASS : S_ACMASS_Y);
+  Stage t(ctx, S_ACMASS, 2);
+  for (int part = 1; part <= 2; ++part)
     CK(atm::adj_mass(g, k, sd[F_DP], sd[F_PT], sd[F_UD], sd[F_VD], cg[C_DPC], cg[C_PTC], ctx->lam_cg[C_DPC],
                      ctx->lam_cg[C_PTC], lin[F_DP], lin[F_PT], lin[F_UD], lin[F_VD], -2, 2, true, ctx->stream, part));
-  }
   return ATM_OK;
 }
 
@@ -952,7 +951,8 @@ int adj_d(atm_ctx* ctx, double dt, const void* const* so, const void* const* sn,
   const double* const* o = (const double* const*)so;
   const double* const* n = (const double* const*)sn;
   const double* const* cg = (const double* const*)cgf;
-  // each sweep's x and y branch is its own kernel and profiled stage
+  // each sweep's x and y branch is its own kernel and profiled stage (the momentum's
+  // keep the names of the two kernels that they replaced)
   for (int part = 1; part <= 2; ++part) {
     Stage t(ctx, part == 1 ? S_ADMOM : S_ADMOM_Y);
     CK(atm::adj_d_mom(g, k, o[F_UD], o[F_VD], cg[C_UC], cg[C_VC], lout[F_UD], lout[F_VD], lin[F_UD], lin[F_VD],

@@ -160,7 +160,10 @@ int atm_remap_trace(atm_ctx* ctx, int32_t* buf, int* fallback_columns);
    launch with CUDA events on the context's stream (and clears earlier
    records); atm_profile_read synchronises and returns, per stage, the total
    milliseconds and the number of launches since then.  Stage i is named by
-   atm_profile_stage(i) (NULL past the last).  atm_launch_count returns how
+   atm_profile_stage(i) (NULL past the last): a kernel, or the kernels of one
+   part of a step (adj_c_mass: both branches of the C-grid mass reverse;
+   adj_d_mom_ke and adj_d_mom_vf: the x and the y branch of the D-grid momentum
+   reverse).  atm_launch_count returns how
    many kernels the context's step entry points have launched. */
 int atm_profile(atm_ctx* ctx, int enable);
 int atm_profile_read(atm_ctx* ctx, double* ms, int* count, int nstage);

@@ -40,6 +40,17 @@ def test_create_rejects_bad_arguments_without_touching_the_gpu():
         assert lib.atm_device_wait_check(polls, ctypes.byref(t)) == 1 and t.value == -1
 
 
+def test_profile_stages_keep_their_names():
+    """Callers find the stages of atm_profile_read by name and by index."""
+    lib = _lib.load()
+    names = ('c_mass c_column c_mom c_halo d_ring d_mass d_column d_corners d_mom remap_ring remap_winds remap_energy '
+             'd_halo heating check adj_forward adj_remap adj_d_mom_ke adj_d_column adj_d_mass_x adj_c_column adj_c_mom '
+             'adj_c_mass adj_halo phys_tend phys_apply phys_halo adj_d_mom_vf adj_d_mass_y radiation '
+             'radiation_halo').split()
+    assert [lib.atm_profile_stage(i).decode() for i in range(len(names))] == names
+    assert lib.atm_profile_stage(len(names)) is None
+
+
 def test_schedule_matches_calculate_dt():
     """calculate_dt (src/mod_model.f90:201-237): remap every 5 steps of 60 s,
     a last step shortened to reach t_final exactly."""
