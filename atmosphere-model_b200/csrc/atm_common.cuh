@@ -117,7 +117,7 @@ __device__ __forceinline__ double fab(double a) { return fabs(a); }
 __device__ __forceinline__ float fab(float a) { return fabsf(a); }
 
 // Division by the constants 3 and 12 of the PPM formulas
-// (src/mod_sw_dyn.f90:878-879,899), correctly rounded like an IEEE
+// (src/mod_sw_dyn.f90:878-879,899) and by 6 of the remap's overlaps, correctly rounded like an IEEE
 // division: q = x*RN(1/b) is within one ulp of x/b, the remainder
 // r = x - q*b is exact in one FMA, and RN(q + r*RN(1/b)) is the correctly
 // rounded quotient (P. Markstein, IBM J. Res. Dev. 34(1), 1990).  Zeros,

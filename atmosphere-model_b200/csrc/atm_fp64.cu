@@ -51,6 +51,8 @@ static __global__ void k_div_check(unsigned long long n, unsigned long long seed
     double q12 = div_const<12>(x), t12 = x / 12.0;
     ok = ok && (__double_as_longlong(q3) == __double_as_longlong(t3) || (q3 != q3 && t3 != t3));
     ok = ok && (__double_as_longlong(q12) == __double_as_longlong(t12) || (q12 != q12 && t12 != t12));
+    double q6 = div_const<6>(x), t6 = x / 6.0;
+    ok = ok && (__double_as_longlong(q6) == __double_as_longlong(t6) || (q6 != q6 && t6 != t6));
     const double q = third(x);
     ok = ok && (__double_as_longlong(q) == __double_as_longlong(t3) || (q != q && t3 != t3));
     if (!ok) ++local;

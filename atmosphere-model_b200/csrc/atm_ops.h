@@ -58,7 +58,7 @@ cudaError_t device_pow_log(const double* x, double y, double* p, double* l, int 
 // p**kappa as the mixed form evaluates it (atm_mixed.cu)
 cudaError_t device_kappa_pow(const double* x, double* out, int n, cudaStream_t);
 
-// count of arguments where div_const<3>/<12> differs from IEEE division (tests)
+// count of arguments where div_const<3>, <6>, <12> or third differs from IEEE division (tests)
 cudaError_t device_div_check(unsigned long long n, unsigned long long seed, unsigned long long* bad, cudaStream_t);
 // a bounded mbarrier wait on a barrier nothing completes: *flag = 1 when it gave up
 cudaError_t device_wait_timeout(int max_polls, int* flag, cudaStream_t);

@@ -272,7 +272,7 @@ int atm_ensemble_barrier_check(long long timeout_ns, int* timed_out);
 
 /* the number of the n pseudo-random FP64 arguments (all exponents, plus
    integers) for which the FP64 form's FMA-corrected division by the
-   constants 3 and 12 differs from IEEE division (expected: 0) */
+   constants 3, 6 and 12 differs from IEEE division (expected: 0) */
 int atm_device_div_check(long long n, long long seed, long long* mismatches);
 /* failure-detection check of a bounded device wait: a kernel arms an mbarrier
    for transactions that never arrive (no copy is issued) and waits on it for
