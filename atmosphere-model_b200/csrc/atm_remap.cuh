@@ -488,9 +488,14 @@ inline int remap_blocks(int L, int n, int most) {
   return b < most ? b : most;
 }
 inline long long remap_winds_few(int L) { return 148LL * 56 * remap_blocks(L, 3, 4) * (L < 32 ? L : 32) / 32; }
-// (more than two blocks of the 65- to 128-layer instance gain nothing: 65 layers 26 240/358, 50 472/408)
+// (more than two blocks of the 65- to 128-layer instance gain nothing: 65 layers 26
+// 240/358, 50 472/408; with three, columns that share the GPU with other kernels do
+// better in the split form also beyond the tie, so the line lies at its far end: eight
+// ensemble members 10.89 ms with it, 11.02 at 53000 columns, a gradient of 301x203x40
+// 30.13 and 30.34)
 inline long long remap_energy_few(int L) {
-  return 148LL * 120 * remap_blocks(L, 4, L > 64 ? 2 : 3) * (L < 28 ? L + 8 : 36) / 36;
+  const int b = remap_blocks(L, 4, L > 64 ? 2 : 3);
+  return 148LL * (b > 2 ? 512 : 120 * b) * (L < 28 ? L + 8 : 36) / 36;
 }
 
 // Shared memory above the default limit, which the kernel's own variables count

@@ -146,7 +146,7 @@ def test_heating_thread_a_column_bit_exact(nx, ny, nlay):
 
 # columns beyond which a thread has a column of its own, in each of the kernels'
 # layer ranges (the limits depend on the layers)
-@pytest.mark.parametrize('nx,ny,nlay', [(131, 130, 3), (171, 160, 8), (240, 230, 33), (203, 190, 65), (140, 137, 128)])
+@pytest.mark.parametrize('nx,ny,nlay', [(161, 152, 3), (211, 200, 8), (290, 270, 33), (203, 190, 65), (140, 137, 128)])
 @pytest.mark.parametrize('fields', ['smooth', 'crossed'])
 def test_remap_thread_a_column_bit_exact(nx, ny, nlay, fields):
     """The remap of domains of many columns with its layer-pair trace."""
