@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(MW * MWARPS, 3) k_mass_adj_y(Geom g, Consts c,
 // as advected quantities (lam_uc1, lam_vc1) and, summed over the layers, of
 // the layer-nlay A-grid winds (lam_ua, lam_va, one level each) in scratch
 // fields, which k_c_mom_adj_fin turns into those of ud, vd; the
-// pressure-gradient force is reversed with the columns (k_c_column_adj).
+// pressure-gradient force is reversed with the columns (k_column_adj<true>).
 struct CMomAdjArgs {
   const double *ud, *vd, *lam_uc, *lam_vc;
   double *lam_ud, *lam_vd, *lam_w, *lam_uc1, *lam_vc1, *lam_ua, *lam_va;

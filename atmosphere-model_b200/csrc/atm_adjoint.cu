@@ -69,8 +69,12 @@ cudaError_t adj_mass(const Geom& g, const Consts& c, const double* dp, const dou
   const int w = g.nx - lo + hi, h = g.ny - lo + hi;
   const bool xb = part == 1;
   // the x kernels take few rows beside a strip's own, and short strips spread their
-  // adjoint sums: 512x512x32 C / D mass 0.362 / 0.473 ms at 18 rows, 0.379 / 0.514 at the
-  // 47 and 65 of an uncapped height, 301x203x40 0.130 / 0.169 at 14, 0.155 / 0.176 at 30
+  // adjoint sums, whose contention plan_strips does not know: heights of at most 20 rows
+  // (C / D mass, us, against up to 128: 512x512x32 359 / 474, 375 / 513; 301x203x40 140 /
+  // 170, 154 / 176; 1024x1024x8 338 / 441, 408 / 539; 700x600x20 338 / 465, 422 / 578;
+  // 100x3000x10 158 / 252, 189 / 267; 512x512x64 686 / 910, 692 / 934; 192x160x48 105 / 113,
+  // 101 / 113; the one loss of sixteen grids 90x90x100 70 / 72, 62 / 70).  14 or 32 rows
+  // are within 5% of it on most.
   const StripPlan p = xb ? adj_strips(w, h, g.L, MOUT, 4, 20) : adj_strips(w, h, g.L, YOUT_MASS, 11);
   const int sm = p.threads / MW * mass_adj_smem(cgrid, xb);
   auto run = [&](auto kernel) {

@@ -433,14 +433,10 @@ int atm_upload_device(atm_ctx* ctx, int field, const void* dev, int dtype_bytes)
   if (!ctx || !dev || (dtype_bytes != 4 && dtype_bytes != 8)) return ATM_ERR_ARG;
   if (field < ATM_DP || field > ATM_GZ) return fail(ctx, ATM_ERR_ARG, "field cannot be uploaded");
   const int K = field == ATM_GZ ? 1 : ctx->L;
-  const bool dbl_field = field == ATM_GZ || ctx->ops->elem == 8;
-  void* dst = field == ATM_GZ ? (void*)ctx->gz : ctx->st[ctx->cur][field];
+  double* dst = field == ATM_GZ ? ctx->gz : (double*)ctx->st[ctx->cur][field];  // the state is FP64 in both forms
   // the halo of a device upload is the periodic image of the interior
-  auto up = [&](auto* to) {
-    return dtype_bytes == 8 ? interior<I_PERIODIC>(ctx->geo, (const double*)dev, to, K, ctx->stream)
-                            : interior<I_PERIODIC>(ctx->geo, (const float*)dev, to, K, ctx->stream);
-  };
-  CK(dbl_field ? up((double*)dst) : up((float*)dst));
+  CK(dtype_bytes == 8 ? interior<I_PERIODIC>(ctx->geo, (const double*)dev, dst, K, ctx->stream)
+                      : interior<I_PERIODIC>(ctx->geo, (const float*)dev, dst, K, ctx->stream));
   ctx->uploaded |= 1 << field;
   ctx->flag_valid = false;
   return ATM_OK;
@@ -449,13 +445,9 @@ int atm_upload_device(atm_ctx* ctx, int field, const void* dev, int dtype_bytes)
 int atm_download_device(atm_ctx* ctx, int field, void* dev, int dtype_bytes) {
   if (!ctx || !dev || (dtype_bytes != 4 && dtype_bytes != 8)) return ATM_ERR_ARG;
   if (field < ATM_DP || field > ATM_VD) return fail(ctx, ATM_ERR_ARG, "only prognostic fields");
-  const bool dbl_field = ctx->ops->elem == 8;
-  const void* src = ctx->st[ctx->cur][field];
-  auto down = [&](auto* from) {
-    return dtype_bytes == 8 ? interior<I_OUT>(ctx->geo, from, (double*)dev, ctx->L, ctx->stream)
-                            : interior<I_OUT>(ctx->geo, from, (float*)dev, ctx->L, ctx->stream);
-  };
-  CK(dbl_field ? down((const double*)src) : down((const float*)src));
+  const double* src = (const double*)ctx->st[ctx->cur][field];
+  CK(dtype_bytes == 8 ? interior<I_OUT>(ctx->geo, src, (double*)dev, ctx->L, ctx->stream)
+                      : interior<I_OUT>(ctx->geo, src, (float*)dev, ctx->L, ctx->stream));
   return ATM_OK;
 }
 

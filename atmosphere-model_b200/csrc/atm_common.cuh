@@ -1,6 +1,6 @@
 // Shared device definitions of the B200 dynamical core: field geometry in
-// HBM, physical constants, and the one-dimensional flux-form
-// semi-Lagrangian flux with its PPM reconstruction.
+// HBM, physical constants, how kernels share rows, status words, and division by
+// constants.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -59,10 +59,10 @@ struct Consts {
 
 // How the kernels that pass over whole rows share them: groups of 1 << lg threads,
 // each a row or one of its pieces of len points.  A group's threads fit the row
-// (their last round is not mostly empty), and rows too few to fill the GPU are cut up.  With 64 threads a row
-// whatever its width (256 in the finite check), four fields out of 16x2048x64 took
-// 96 us, in 111, and an upload with the finite check 261, of 7x4096x20 47, 52 and 107;
-// so 46, 86, 69 and 17, 46, 37.
+// (their last round is not mostly empty), and rows too few to fill the GPU are cut
+// up.  With 64 threads a row whatever its width (256 in the finite check), four
+// fields out of 16x2048x64 took 96 us, in 111, and an upload with the finite check
+// 261, of 7x4096x20 47, 52 and 107; so 46, 86, 69 and 17, 46, 37.
 struct RowSplit {
   int lg, pieces, len;
 };

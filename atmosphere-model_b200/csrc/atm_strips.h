@@ -19,7 +19,8 @@ struct StripPlan {
 // that grows with the warps an SM holds, about as 16 + warps (B200, per row
 // of the FP64 C mass sweep: 0.91 us with 4, 1.28 us with 12 warps an SM); full
 // waves are followed by one that is only as crowded as what is left.  most: the
-// largest height.
+// largest height; the least is 3 (strips of a height of about 4 share the rows
+// evenly), 4 on domains of more than 512 rows.
 // Measured on B200, mixed form at 150x130x48 (us, C mass / C momentum / D mass
 // / D momentum): powers of two and a wave's cost independent of its size, 49 /
 // 54 / 47 / 58; over all heights from 4 to 128 the best is 33 / 33 / 34 / 37
