@@ -28,23 +28,24 @@ enum { C_DPC = 0, C_PTC = 1, C_UC = 2, C_VC = 3 };
 
 // interior <-> contiguous (K, ny, nx) device buffer, with type conversion: out of a
 // field, or into it with its halo (the periodic image, or zeros).  A row, or a
-// piece of a wide one (RowSplit), to a group of 8 to 64 threads, a division or
-// two a piece: with two 64-bit divisions a point and the halo a launch of
+// piece of a wide one (RowSplit), to a group of 8 to 64 threads, a division a
+// piece: with two 64-bit divisions a point and the halo a launch of
 // its own, four fields in and out took 0.35 ms more at 1024x1024x64, 0.02 at 128x128x20.
+// CUT: rows in pieces, whose bounds take the instance from 32 registers to 40 and an
+// SM from eight blocks to six (90x800x20 whole rows in and out 30 and 31 us, 34 and 36 with it).
 enum { I_OUT, I_PERIODIC, I_ZERO };
-template <typename A, typename B, int MODE, int LG>
+template <typename A, typename B, int MODE, int LG, bool CUT>
 __device__ __forceinline__ void interior_rows(const Geom& g, const A* __restrict__ src, B* __restrict__ dst, int K,
-                                              const atm::RowSplit& sp) {
+                                              int len) {
   constexpr int h = MODE == I_OUT ? 0 : H;
-  const int nrow = g.ny + 2 * h, n = nrow * K * sp.pieces;
+  const int nrow = g.ny + 2 * h, rows = nrow * K;
   constexpr int per = 256 >> LG, lanes = 1 << LG;
-  for (int it = (int)blockIdx.x * per + (int)(threadIdx.x >> LG); it < n; it += (int)gridDim.x * per) {
-    const int r = sp.pieces > 1 ? it / sp.pieces : it, x0 = (it - r * sp.pieces) * sp.len - h;
+  const int x0 = CUT ? (int)blockIdx.y * len - h : -h, x1 = CUT ? min(x0 + len, g.nx + h) : g.nx + h;
+  for (int r = (int)blockIdx.x * per + (int)(threadIdx.x >> LG); r < rows; r += (int)gridDim.x * per) {
     const int k = r / nrow, y = r - k * nrow - h;
     const long long o = g.at(0, y, k);
     const int ys = y < 0 ? y + g.ny : (y >= g.ny ? y - g.ny : y);
     const long long q = ((long long)k * g.ny + ys) * g.nx;
-    const int x1 = min(x0 + sp.len, g.nx + h);
 #pragma unroll 4
     for (int x = x0 + ((int)threadIdx.x & (lanes - 1)); x < x1; x += lanes) {
       if constexpr (MODE == I_OUT) {
@@ -57,19 +58,20 @@ __device__ __forceinline__ void interior_rows(const Geom& g, const A* __restrict
     }
   }
 }
-template <typename A, typename B, int MODE, int LG>
-__global__ void __launch_bounds__(256) k_interior(Geom g, const A* src, B* dst, int K, atm::RowSplit sp) {
+template <typename A, typename B, int MODE, int LG, bool CUT>
+__global__ void __launch_bounds__(256) k_interior(Geom g, const A* src, B* dst, int K, int len) {
   atm::stream_order();
-  interior_rows<A, B, MODE, LG>(g, src, dst, K, sp);
+  interior_rows<A, B, MODE, LG, CUT>(g, src, dst, K, len);
 }
 template <int MODE, typename A, typename B>
 cudaError_t interior(const Geom& g, const A* src, B* dst, int K, cudaStream_t s) {
   const int h = MODE == I_OUT ? 0 : H, rows = (g.ny + 2 * h) * K;
   const atm::RowSplit sp = atm::row_split(g.nx + 2 * h, rows, 6);
-  const int per = 256 >> sp.lg, nb = (rows * sp.pieces + per - 1) / per;
+  const dim3 grid = atm::row_grid(sp, rows, 148 * 16);
   return atm::with_lg(sp, [&](auto lg) {
-    return atm::launch(k_interior<A, B, MODE, decltype(lg)::value < 6 ? decltype(lg)::value : 6>,
-                       nb < 148 * 16 ? nb : 148 * 16, 256, 0, s, g, src, dst, K, sp);
+    constexpr int LG = decltype(lg)::value < 6 ? decltype(lg)::value : 6;
+    return sp.pieces > 1 ? atm::launch(k_interior<A, B, MODE, LG, true>, grid, 256, 0, s, g, src, dst, K, sp.len)
+                         : atm::launch(k_interior<A, B, MODE, LG, false>, grid, 256, 0, s, g, src, dst, K, sp.len);
   });
 }
 

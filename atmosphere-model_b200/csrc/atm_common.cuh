@@ -61,8 +61,8 @@ struct Consts {
 // each a row or one of its pieces of len points.  A group's threads fit the row
 // (their last round is not mostly empty), and rows too few to fill the GPU are cut
 // up.  With 64 threads a row whatever its width (256 in the finite check), four
-// fields out of 16x2048x64 took 96 us, in 111, and an upload with the finite check
-// 261, of 7x4096x20 47, 52 and 107; so 46, 86, 69 and 17, 46, 37.
+// fields out of 16x2048x64 took 98 us, in 113 and the check 217, of 7x4096x20 46, 53
+// and 79; so 45, 84, 30 and 15, 42, 9.
 struct RowSplit {
   int lg, pieces, len;
 };
@@ -77,6 +77,13 @@ inline RowSplit row_split(int width, int rows, int lg_most) {
   r.len = ((width + r.pieces - 1) / r.pieces + lanes - 1) / lanes * lanes;
   r.pieces = (width + r.len - 1) / r.len;
   return r;
+}
+
+// Blocks of 256 threads that pass over the rows: blockIdx.y the piece, the row's
+// groups along x, at most `most` blocks.
+inline dim3 row_grid(const RowSplit& r, int rows, int most) {
+  const int per = 256 >> r.lg, nb = (rows + per - 1) / per, cap = most / r.pieces > 0 ? most / r.pieces : 1;
+  return dim3(nb < cap ? nb : cap, r.pieces);
 }
 
 // f(the group's lg as a constant)

@@ -1110,10 +1110,10 @@ __global__ void __launch_bounds__(256) k_check_finite(Geom g, const T* __restric
                                                       const T* __restrict__ f2, const T* __restrict__ f3, int* flag,
                                                       RowSplit sp) {
   bool bad = false;
-  const int n = g.ny * g.L * sp.pieces;
+  const int n = g.ny * g.L;
   constexpr int per = 256 >> LG, lanes = 1 << LG;
-  for (int it = (int)blockIdx.x * per + (int)(threadIdx.x >> LG); it < n; it += (int)gridDim.x * per) {
-    const int r = sp.pieces > 1 ? it / sp.pieces : it, x0 = (it - r * sp.pieces) * sp.len, x1 = min(x0 + sp.len, g.nx);
+  const int x0 = (int)blockIdx.y * sp.len, x1 = min(x0 + sp.len, g.nx);
+  for (int r = (int)blockIdx.x * per + (int)(threadIdx.x >> LG); r < n; r += (int)gridDim.x * per) {
     const int k = r / g.ny;
     const long long o = g.at(0, r - k * g.ny, k);
 #pragma unroll 2

@@ -153,7 +153,7 @@ cudaError_t check_finite(const Geom& g, const void* const* f, int* flag, cudaStr
   RowSplit sp = row_split(g.nx, g.ny * g.L, 8);
   if (sp.lg == 7) sp = row_split(g.nx, g.ny * g.L, 6);
   return with_lg(sp, [&](auto lg) {
-    k_check_finite<S, decltype(lg)::value><<<148 * 8, 256, 0, s>>>(g, (const S*)f[0], (const S*)f[1], (const S*)f[2],
+    k_check_finite<S, decltype(lg)::value><<<row_grid(sp, g.ny * g.L, 148 * 8), 256, 0, s>>>(g, (const S*)f[0], (const S*)f[1], (const S*)f[2],
                                                                    (const S*)f[3], flag, sp);
     return cudaGetLastError();
   });
