@@ -29,9 +29,10 @@
 // 512x512x32 (ms a launch; first: one or two kernels on 32 x 4-8 tiles that
 // kept every intermediate and its adjoint in shared memory, with shared-memory
 // atomics and block barriers between about ten stages, ~6000 instructions a
-// cell; then this march with its loads at their use, then with the rings):
-// C mass 3.37, 0.58 + 0.87, 0.37 + 0.56; C momentum 3.27, 1.05, 0.89; D mass
-// 3.53, 0.63 + 1.02, 0.47 + 0.79; D momentum 4.16, 0.59 + 0.57, 0.40 + 0.50.
+// cell; then this march with its loads at their use, then with the rings and
+// with the strips of atm_strips.h, every output with an adjoint):
+// C mass 3.37, 0.58 + 0.87, 0.36 + 0.45; C momentum 3.27, 1.05, 0.79; D mass
+// 3.53, 0.63 + 1.02, 0.47 + 0.63; D momentum 4.16, 0.59 + 0.57, 0.40 + 0.38.
 // With the rings, rows unrolled 2 or 3 times gain up to 4% in the momentum x
 // kernels and lose 10-25% in the y kernels; four blocks an SM lose 50% there.
 #pragma once

@@ -567,11 +567,10 @@ def probe_radiation(args):
 
 
 # Algorithmic HBM words per interior cell and launch of the adjoint
-# kernels: the forward inputs the kernel recomputes from, the output
-# adjoints it reads, and a read and a write of every adjoint it adds into
-# (layer-nlay slabs excluded, as for the forward).
+# kernels that are a profiled stage by themselves: the forward inputs the
+# kernel recomputes from, the output adjoints it reads, and a read and a write
+# of every adjoint it adds into (layer-nlay slabs excluded, as for the forward).
 ADJ_WORDS = {
-    'adj_c_mass': 32,    # both branches: dp, pt, ud, vd, dpc, ptc; lam dpc, ptc; += lam dp, pt, ud, vd
     'adj_d_mom_ke': 11,  # x branch: ud, vd, uc; lam ud, vd (out); += lam ud, vd, uc
     'adj_d_mom_vf': 11,  # y branch: ud, vd, vc; lam ud, vd (out); += lam ud, vd, vc
     'adj_d_mass_x': 16,  # dp, pt, uc, vc, new dp, pt; lam dp, pt (out); += lam dp, pt, uc, vc
@@ -580,8 +579,7 @@ ADJ_WORDS = {
 # DRAM bytes per interior cell and launch of the adjoint kernels measured by
 # ncu (dram__bytes_read.sum + dram__bytes_write.sum, dense adjoint of the
 # jet at 512x512x32, scaled by cells)
-TRAFFIC_PER_CELL_ADJ = {'adj_d_mom_ke': 95, 'adj_d_mom_vf': 95, 'adj_d_mass_x': 130, 'adj_d_mass_y': 144,
-                        'adj_c_mass': 279}
+TRAFFIC_PER_CELL_ADJ = {'adj_d_mom_ke': 95, 'adj_d_mom_vf': 95, 'adj_d_mass_x': 130, 'adj_d_mass_y': 144}
 
 
 def grad_leg(args, torch, barrier, max_over_ranks, world, peak, peak_kind):
