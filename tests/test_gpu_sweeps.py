@@ -168,3 +168,36 @@ def test_remap_thread_a_column_bit_exact(nx, ny, nlay, fields):
     if fields == 'crossed':
         assert fallback.value > 0
     g.close()
+
+
+@pytest.mark.parametrize('precision', ['fp64', 'mixed'])
+@pytest.mark.parametrize('nlay', [10, 70])
+def test_tiled_domain_same_bits(precision, nlay):
+    """A domain of copies of a smaller one: each copy is the smaller domain's
+    step, heating and remap bit for bit, although the larger one's columns are
+    too many for the forms that share a column's levels.  (The remap after the
+    halo fill: within a step it reads winds of the old halo, as the reference
+    does, which the larger domain's inner copies do not have.)"""
+    nx, ny, my, mx = 70, 65, 5, 4
+    st = ic.jet_case(nx, ny, nlay, 400e3, 400e3, width=900e3, seed=3)
+    rng = np.random.default_rng(nlay)
+    st.dp = st.dp * np.exp(rng.normal(0, 0.05, st.dp.shape))
+    st.u = st.u + rng.normal(0, 10.0, st.u.shape)
+    st.v = st.v + rng.normal(0, 10.0, st.v.shape)
+    nf = rng.normal(0, 150.0, (nlay + 1, ny, nx))
+    big = ic.jet_case(nx * mx, ny * my, nlay, 400e3, 400e3, width=900e3, seed=3)
+    for name in ('dp', 'pt', 'u', 'v', 'gzs'):
+        a = getattr(st, name)
+        setattr(big, name, np.tile(a, (1,) * (a.ndim - 2) + (my, mx)))
+    out = []
+    for s, flux in ((st, nf), (big, np.tile(nf, (1, my, mx)))):
+        g = Dycore(s, precision)
+        g.set_net_flux(np.pad(flux, ((0, 0), (7, 7), (7, 7)), mode='wrap'))
+        for _ in range(2):
+            assert g.step(20.0, remap=False, check_stable=True)
+            g.remap()
+            g.dgrid_halo()
+        out.append({name: g.get(name) for name, _ in FIELDS})
+        g.close()
+    for name, _ in FIELDS:
+        np.testing.assert_array_equal(out[1][name], np.tile(out[0][name], (1, my, mx)), err_msg=name)
